@@ -67,16 +67,17 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams 
 
 // m / rho into spos.w (0 for rho == 0: the field skips such particles), and the
 // isotropic kernel of every particle in the field's packed form: M = G^T G
-// with G = I / h (off-diagonals doubled), h_s^2 = h^2, and the weight
+// with G = I / h (off-diagonals doubled), the support's packed extents, and the weight
 // (m / rho) sigma det(G) = (m / rho) sigma / h^3; the anisotropy pass
 // overwrites the surface particles' entries.
 __global__ void __launch_bounds__(kThreads) k_inv_density(float4* __restrict__ spos, const float* __restrict__ rho,
                                                           float4* __restrict__ aniso, AnisoParams ap, uint32_t n) {
+    const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float r = rho[i];
         spos[i].w = r == 0.f ? 0.f : ap.mass / r;
         const float inv_h2 = ap.h_inv * ap.h_inv;
-        aniso[2 * (size_t)i + 0] = make_float4(inv_h2, 0.f, 0.f, ap.h_sq);
+        aniso[2 * (size_t)i + 0] = make_float4(inv_h2, 0.f, 0.f, __uint_as_float(ext));
         aniso[2 * (size_t)i + 1] = make_float4(inv_h2, 0.f, inv_h2, spos[i].w * ap.kdens);
     }
 }
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
         const float ox = m0.y / ws, oy = m0.z / ws, oz = m0.w / ws;   // mean - p
         const uint32_t nn = __float_as_uint(m2.z);
         float G[3][3], nv[3], maxv, flag;
+        float ext[3] = {ap.h, ap.h, ap.h};                   // half extents of the support's box
         if ((int)nn < ap.min_nn) {
             // isolated particle: isotropic kernel (Anisotropic_kernel.cuh:435-443)
 #pragma unroll
@@ -267,6 +269,13 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
                     G[a][b] = U[a][0] * k0 * U[b][0] + U[a][1] * k1 * U[b][1] + U[a][2] * k2 * U[b][2];
             nv[0] = U[0][2]; nv[1] = U[1][2]; nv[2] = U[2][2];
             maxv = sv0 / scale;
+            // the support is the ellipsoid with semi-axes 1 / k along U's columns
+            const float r0 = sv0 / cof, r1 = sv1 / cof, r2 = sv2 / cof;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float u0 = U[a][0] * r0, u1 = U[a][1] * r1, u2 = U[a][2] * r2;
+                ext[a] = sqrtf(u0 * u0 + u1 * u1 + u2 * u2);
+            }
         }
         // orient the normal away from the mean (Anisotropic_kernel.cuh:512-515)
         if (nv[0] * (-ox) + nv[1] * (-oy) + nv[2] * (-oz) < 0.f) { nv[0] = -nv[0]; nv[1] = -nv[1]; nv[2] = -nv[2]; }
@@ -274,7 +283,6 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
         const float det = G[0][0] * G[1][1] * G[2][2] + G[0][1] * G[1][2] * G[2][0] + G[0][2] * G[1][0] * G[2][1]
                         - G[0][0] * G[1][2] * G[2][1] - G[0][1] * G[1][0] * G[2][2] - G[0][2] * G[1][1] * G[2][0];
         const float hs = maxv * ap.h;
-        // symmetric G packed in two float4: {g00, g01, g02, hs^2}, {g11, g12, g22, sigma * det}
         // the field's packed form: M = G^T G = G G (G is symmetric), off-diagonals doubled,
         // so |G r|^2 = r^T M r costs 9 multiply-adds; w = (m / rho) sigma det(G)
         float M[3][3];
@@ -282,7 +290,8 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b) M[a][b] = G[a][0] * G[0][b] + G[a][1] * G[1][b] + G[a][2] * G[2][b];
-        aniso[2 * (size_t)i + 0] = make_float4(M[0][0], 2.f * M[0][1], 2.f * M[0][2], hs * hs);
+        aniso[2 * (size_t)i + 0] = make_float4(M[0][0], 2.f * M[0][1], 2.f * M[0][2],
+                                                __uint_as_float(pack_extents(ext[0], ext[1], ext[2], ap.h)));
         aniso[2 * (size_t)i + 1] = make_float4(M[1][1], 2.f * M[1][2], M[2][2], pi4.w * (kSigma * det));
         nrm4[i] = make_float4(nv[0], nv[1], nv[2], flag);
         mean4[s] = make_float4(pi4.x + ox, pi4.y + oy, pi4.z + oz, ws);
@@ -298,37 +307,6 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
         atomicMax(reinterpret_cast<unsigned int*>(&cell_rad[key]), __float_as_uint(hs));
         atomicMax(reinterpret_cast<unsigned int*>(&cell_rad[ap.sp_size + key / ap.spres_x]), __float_as_uint(hs));
         atomicMax(&cnt_w->rad_max_bits, __float_as_uint(hs));
-    }
-}
-
-// ---------------------------------------------------------------------------
-// per-cell culling record for the field: the bounding box of the cell's
-// particles and the square of the largest support among them (h, or the
-// cell's largest maxvalue * h), grown by kSupportGrow.  A vertex farther than
-// that from the box gets exactly 0 from every particle of the cell.  An empty
-// cell gets r^2 = -1, which no vertex reaches.
-// rec[2c] = {min x, min y, min z, r^2}, rec[2c + 1] = {max x, max y, max z, 0}.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) k_cell_records(const uint32_t* __restrict__ cell_start,
-                                                           const float4* __restrict__ spos,
-                                                           const float* __restrict__ cell_rad, float h, uint32_t S,
-                                                           float4* __restrict__ rec) {
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < S; c += gridDim.x * blockDim.x) {
-        const uint32_t j0 = cell_start[c], j1 = cell_start[c + 1];
-        if (j0 == j1) {
-            rec[2 * (size_t)c] = make_float4(0.f, 0.f, 0.f, -1.f);
-            continue;
-        }
-        const float4 q = spos[j0];
-        float lx = q.x, ly = q.y, lz = q.z, hx = q.x, hy = q.y, hz = q.z;
-        for (uint32_t j = j0 + 1; j < j1; ++j) {
-            const float4 p = spos[j];
-            lx = fminf(lx, p.x); ly = fminf(ly, p.y); lz = fminf(lz, p.z);
-            hx = fmaxf(hx, p.x); hy = fmaxf(hy, p.y); hz = fmaxf(hz, p.z);
-        }
-        const float r = fmaxf(cell_rad[c], h) * kSupportGrow;
-        rec[2 * (size_t)c] = make_float4(lx, ly, lz, r * r);
-        rec[2 * (size_t)c + 1] = make_float4(hx, hy, hz, 0.f);
     }
 }
 
@@ -387,10 +365,6 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
         ap, ctx->slist.as<uint32_t>(), cnt, ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->moments.as<float4>(),
         ctx->aniso.as<float4>(), ctx->nrm4.as<float4>(), ctx->mean4.as<float4>(), ctx->gdebug.as<float>(),
         ctx->nnb.as<uint32_t>(), ctx->cell_rad.as<float>(), cnt);
-    PMS_LAUNCHED(ctx);
-    k_cell_records<<<grid_for(g.sp_size, kThreads), kThreads, 0, ctx->stream>>>(
-        ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->cell_rad.as<float>(), P.h, g.sp_size,
-        ctx->cell_rec.as<float4>());
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }

@@ -108,6 +108,25 @@ constexpr float kRangeMargin = 0.01f;
 // float rounding of |G r|^2 moves that edge by ~1e-6 relative at most.
 constexpr float kSupportGrow = 1.0001f;
 
+// The half extents of the box around a particle's support {r : |G r| < 1}, per axis,
+// packed into the low 24 bits of a word as multiples of extent_unit(h), rounded up and
+// grown; bit 24 marks extents past the coded range (no culling).  The largest support is
+// 4^(2/3) h (the eigenvalue clamp), so steps of 2.6 h / 255 cover every particle.
+constexpr float kExtentRange = 2.6f;
+__host__ __device__ __forceinline__ float extent_unit(float h) { return h * (kExtentRange / 255.f); }
+__device__ __forceinline__ uint32_t pack_extents(float ex, float ey, float ez, float h) {
+    const float s = 1.002f * (255.f / kExtentRange) / h;
+    const float a = ceilf(ex * s), b = ceilf(ey * s), c = ceilf(ez * s);
+    if (!(a <= 255.f && b <= 255.f && c <= 255.f)) return 1u << 24;
+    return (uint32_t)a | (uint32_t)b << 8 | (uint32_t)c << 16;
+}
+__device__ __forceinline__ void unpack_extents(uint32_t p, float unit, float& ex, float& ey, float& ez) {
+    ex = (float)(p & 0xffu) * unit;
+    ey = (float)((p >> 8) & 0xffu) * unit;
+    ez = (float)((p >> 16) & 0xffu) * unit;
+    if (p >> 24) ex = ey = ez = __int_as_float(0x7f800000);
+}
+
 // First and one-past-last cell of [u - rc, u + rc] along one axis, clipped to [lo, hi).
 __device__ __forceinline__ void cell_range(float u, float rc, uint32_t lo, uint32_t hi, int& a, int& b) {
     a = max((int)floorf(u - rc), (int)lo);

@@ -11,21 +11,16 @@
 // sum > 2 * iso, which breaks only the innermost (x) loop: once the sum has
 // crossed the threshold, every later row adds exactly its first cell.
 //
-// GB300 design: thread per band vertex, consecutive threads on consecutive
-// band vertices (neighbours along x share almost all cells, so the particle
-// loads hit in L1).  Every particle carries its kernel in one packed form --
-// symmetric G, h_s^2 and sigma*det(G), with G = I/h, h_s = h for particles of
-// non-surface cells -- so one branch-free formula serves both kinds and the
-// loads of consecutive particles overlap.  The cells x in [xa, xb) of a row are
-// the contiguous particle range [cell_start[row + xa], cell_start[row + xb]);
-// slabs and rows are cut to those the largest support can reach, each row to
-// the cells its own largest support reaches, and a cell whose particles' bounding
-// box lies beyond the support of every particle in it (h, or the cell's largest
-// maxvalue * h recorded by the anisotropy pass) contributes exactly zero and is
-// skipped.
-// Adding a zero contribution leaves the sum unchanged, so no cut changes the
-// reference's sum or its early exit: the threshold test after a skipped cell
-// sees the same sum as the test before it.
+// GB300 design: a warp per tile of scalar vertices (k_field_tiles).  The vertices of a
+// tile share nearly all of the particles they sum, so the warp reads each particle
+// once, keeps it in shared memory if its support can reach the tile, and all lanes
+// evaluate it together.  Every particle carries its kernel in one packed form --
+// M = G^T G, the weight (m / rho) sigma det(G), and the extents of its support's box,
+// with G = I / h for particles of non-surface cells -- so one branch-free formula
+// serves both kinds.  Cells are sorted by key, so the cells x in [xa, xb) of a row are
+// the contiguous particle range [cell_start[row + xa], cell_start[row + xb]).
+// Adding a zero contribution leaves the sum unchanged, so leaving out particles that
+// cannot reach a vertex changes neither the reference's sum nor its early exit.
 //
 // Sign certification (the learned band's exact fallback; no reference
 // counterpart).  Every term of the sum is >= 0 and float addition of a
@@ -41,6 +36,7 @@
 // either way gets a placeholder above iso (its partial sum) and a bit in
 // `cert`; a vertex whose walk ran to the end has exactly the reference's value
 // (no early exit fired, the sum never exceeded iso).
+#include <algorithm>
 #include <type_traits>
 
 #include "pms_internal.h"
@@ -53,6 +49,7 @@ struct FieldParams {
     float thr;                // 2 * iso: the early-exit threshold (certification: iso)
     float grow;               // relative margin on culling radii
     float quick;              // certification: iso * (1 + 2^-9), the nearest-cells test
+    float ext_unit;           // step of the packed support extents
 };
 
 __device__ __forceinline__ float gap2_axis(float p, float lo, float cs, float pad) {
@@ -68,7 +65,8 @@ __device__ __forceinline__ float gap2_axis(float p, float lo, float cs, float pa
 // the two can differ only by rounding, where the contribution is ~0.  |G r|^2
 // is evaluated as r^T M r with the packed M = G^T G (off-diagonals doubled)
 // and the weight w = (m/rho) sigma det(G) stored per particle.
-// A work item is a run of up to K band vertices that are neighbours along x
+// The certification walks runs (k_field_cert), which visit only what their vertices
+// reach before they stop.  A work item is a run of up to K vertices that are neighbours along x
 // (ids id0, id0 + 1, ...; one row of the scalar grid): item = first band index
 // t0 | (count - 1) << 29.  The run shares the slabs and rows of its walk (same
 // y and z), each cell's bounds and record loads and each particle's loads;
@@ -83,16 +81,15 @@ static constexpr uint32_t kItemShift = 29;
 // (0 where none is anisotropic).  The z and y ranges are cut from the largest
 // support of the frame, each row's x range from the row's own radius, and each
 // non-empty cell by its record: the bounding box of its particles and its
-// largest support.  The value goes to field[t] (band order; skipped when field
-// is null) and to fdense[id] (the whole scalar grid).
-// CERT: sign certification (above); cert receives a bit per vertex stopped above
-// iso, n_cert their count.
-template <int BT, int K, bool CERT>
+// largest support.  The value, or the placeholder of a vertex stopped above iso, goes
+// to fdense[id] (the whole scalar grid); cert receives a bit per vertex stopped, n_cert
+// their count.
+template <int BT, int K>
 __global__ void __launch_bounds__(BT, (K == 1 ? 1280 : 1024) / BT)
-k_field(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_t* __restrict__ n_items_dev,
+k_field_cert(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_t* __restrict__ n_items_dev,
         const uint32_t* __restrict__ items, const uint32_t* __restrict__ vlist, const uint32_t* __restrict__ cell_start,
         const float* __restrict__ cell_rad, const float4* __restrict__ rec, const float4* __restrict__ spos,
-        const float4* __restrict__ aniso, float* __restrict__ field, float* __restrict__ fdense,
+        const float4* __restrict__ aniso, float* __restrict__ fdense,
         uint32_t* __restrict__ cert, uint32_t* __restrict__ n_cert, Counters* __restrict__ cnt_w) {
     const uint32_t n_items = *n_items_dev;
     uint32_t my_cert = 0;
@@ -129,7 +126,7 @@ k_field(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_
         bool done[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) done[k] = false;
-        if constexpr (CERT) {
+        {
             // the 2 x 2 x 2 cells nearest to each vertex (inside its window): the run
             // shares the two slabs and two rows, each vertex takes its own two x cells
             const int cz = (int)floorf(uz), cy = (int)floorf(uy);
@@ -215,29 +212,20 @@ k_field(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_
                 const float rr2 = rr * rr;
                 if (gyz >= rr2) continue;           // every cell of the row adds 0
                 const uint32_t row = rowi * srx;
-                // each vertex's cells of this row: past the threshold, only the window's
-                // first cell (the reference adds it, then breaks); else those the row's
-                // largest support reaches
+                // each vertex's cells of this row: those the row's largest support reaches
                 const float rxc = sqrtf(rr2 - gyz) * inv_cs + kRangeMargin;
                 int xs[K], xe[K];
                 bool live[K];
                 int X0 = 0x7fffffff, X1 = -1;
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
-                    if (!CERT && sum[k] > fp.thr) {
-                        xs[k] = wlo[k];
-                        xe[k] = min(wlo[k] + 1, whi[k]);
-                    } else {
-                        cell_range(ux[k], rxc, (uint32_t)wlo[k], (uint32_t)whi[k], xs[k], xe[k]);
-                    }
+                    cell_range(ux[k], rxc, (uint32_t)wlo[k], (uint32_t)whi[k], xs[k], xe[k]);
                     live[k] = xs[k] < xe[k];
                     if (live[k]) { X0 = min(X0, xs[k]); X1 = max(X1, xe[k]); }
                 }
                 for (int x0 = X0; x0 < X1; x0 += 32) {
                     const int nx = min(X1 - x0, 32);
-                    // cells of the chunk inside some live vertex's range (a vertex past the
-                    // threshold needs only its window's first cell, which can sit well left
-                    // of the others' ranges)
+                    // cells of the chunk inside some live vertex's range
                     uint32_t need = 0u;
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
@@ -266,8 +254,8 @@ k_field(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_
                     uint32_t any = 0u;
 #pragma unroll
                     for (int k = 0; k < K; ++k) any |= reach[k];
-                    // the reached cells in x order; a vertex stops for the row once its
-                    // sum passes the threshold after one of its cells
+                    // the reached cells in x order; a vertex stops once its sum passes the
+                    // threshold after one of its cells
                     while (any) {
                         const int i = __ffs(any) - 1;
                         const uint32_t bit = 1u << i;
@@ -307,7 +295,8 @@ k_field(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_
                             if (use[k] && sum[k] > fp.thr) {
                                 reach[k] = 0u;
                                 live[k] = false;
-                                if constexpr (CERT) { done[k] = true; whi[k] = wlo[k]; }   // certified: stop for good
+                                done[k] = true;
+                                whi[k] = wlo[k];         // certified: stop for good
                             }
                             still |= reach[k];
                         }
@@ -324,24 +313,475 @@ k_field(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_
 #pragma unroll
         for (int k = 0; k < K; ++k)
             if (k < m) {
-                if (field) field[t0 + k] = sum[k];
                 fdense[id + k] = sum[k];
                 if (done[k]) mask |= 1u << k;
             }
-        if (CERT && mask) {
+        if (mask) {
             const uint32_t w = id >> 5, sh = id & 31u;
             atomicOr(&cert[w], mask << sh);
             if (sh && (mask >> (32u - sh))) atomicOr(&cert[w + 1], mask >> (32u - sh));
             my_cert += (uint32_t)__popc(mask);
         }
     }
-    if constexpr (CERT) {
-        const uint32_t tot = __reduce_add_sync(0xffffffffu, my_cert);
-        if ((threadIdx.x & 31u) == 0 && tot) atomicAdd(n_cert, tot);
-    }
+    const uint32_t tot = __reduce_add_sync(0xffffffffu, my_cert);
+    if ((threadIdx.x & 31u) == 0 && tot) atomicAdd(n_cert, tot);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) my_pairs += __shfl_xor_sync(0xffffffffu, my_pairs, o);
     if ((threadIdx.x & 31u) == 0 && my_pairs) atomicAdd(&cnt_w->n_pairs, my_pairs);
+}
+
+// ---------------------------------------------------------------------------
+// Exact field, tile by tile.  One warp evaluates a tile of 32 K scalar vertices
+// (4 x 4 x 2 for K = 1, 4 x 4 x 4 for K = 2, 8 x 4 x 4 for K = 4; a lane owns K
+// x-neighbours).  The warp reads the particles that can reach the tile's band
+// vertices once, 32 at a time, in the reference's order -- ascending sorted index
+// -- keeps those whose support box meets the vertices' box, stages them in shared
+// memory, and every lane then runs over the staged particles, all lanes on the
+// same one.  A vertex adds every staged particle's contribution in that order, so
+// its sum is the one a walk of its own gives (particles left out add exactly 0).
+//
+// The early exit, restated per cell: a cell adds to a vertex when the vertex's sum
+// is not past 2 iso before it, or when it is the first cell of the vertex's window
+// in its row (the reference adds it, then breaks).  The sum never decreases, so
+// this is the reference's rule whatever was skipped in between.  Windows matter
+// only for cells that are not inside every vertex's window (or are some vertex's
+// first cell): a chunk with such a particle takes the general path, which tests
+// each vertex's own window.
+//
+// Bound by instruction issue.  A walk per run of vertices (18 of 32 lanes active, its
+// rows, records and cell bounds costing more than the pairs) took 2.89 / 2.56 / 7.24 ms
+// for the field stage of the crown 2M / dam 8M / spray 151k (ratio 3) frames; tiles take
+// 1.03 / 1.23 / 0.96 ms (30 of 32 lanes active).  Of that:
+// - support boxes and the separating plane leave 41, 66 and 28 staged particles per tile of
+//   about 52 band vertices; the boxes alone left 60, 99 and 42 (1.29 / 1.64 / 1.22 ms);
+// - a lane's x-neighbours go through the packed two-float operations, rounded as the
+//   scalar ones, and the early exit is a limit on |G r|^2 rather than a flag.
+// K = 2 is the default: K = 1 stages fewer particles per tile but shares less of each
+// (1.50 / 1.78 / 1.41 ms), K = 4 the reverse (1.31 / 1.53 / 1.03 ms).
+// ---------------------------------------------------------------------------
+template <int K> struct FieldTile {
+    static constexpr int X = K == 4 ? 8 : 4, Y = 4, Z = K == 1 ? 2 : 4;
+};
+static constexpr uint32_t kTileTicket = 4;      // consecutive listed tiles a warp takes at once
+// Resident warps per SM the registers are capped for.  Crown 2M / dam 8M field stage: 20 warps
+// (96 registers, no spills) 1.03 / 1.23 ms, 24 (80, spilling) 1.04 / 1.25, 16 1.15 / 1.36.
+static constexpr int kFieldWarps = 20;
+
+// The tiles holding a set bit of a bitmap over the scalar grid: list[t] its tile
+// index, mask[K t + k] the lanes whose vertex k is set.
+template <int K>
+__global__ void __launch_bounds__(256) k_field_tile_list(KGrid g, uint3 td, const uint32_t* __restrict__ bm,
+                                                         uint32_t* __restrict__ n_tiles, uint32_t* __restrict__ list,
+                                                         uint32_t* __restrict__ mask) {
+    using T = FieldTile<K>;
+    const uint32_t ntiles = td.x * td.y * td.z;
+    const uint32_t rx = g.scres[0], ry = g.scres[1], rz = g.scres[2];
+    // whole warps stay in the loop together (the append is a warp vote)
+    for (uint32_t t0 = blockIdx.x * blockDim.x; t0 < ntiles; t0 += gridDim.x * blockDim.x) {
+        const uint32_t t = t0 + threadIdx.x;
+        uint32_t m[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) m[k] = 0u;
+        if (t < ntiles) {
+            const uint32_t tx = t % td.x, tyz = t / td.x, ty = tyz % td.y, tz = tyz / td.y;
+            const uint32_t x0 = tx * T::X;
+            const uint32_t in = rx - x0 >= (uint32_t)T::X ? (1u << T::X) - 1u : (1u << (rx - x0)) - 1u;
+#pragma unroll
+            for (int z = 0; z < T::Z; ++z)
+#pragma unroll
+                for (int y = 0; y < T::Y; ++y) {
+                    const uint32_t vy = ty * T::Y + (uint32_t)y, vz = tz * T::Z + (uint32_t)z;
+                    if (vy >= ry || vz >= rz) continue;
+                    const uint64_t bit = ((uint64_t)vz * ry + vy) * rx + x0;
+                    const uint64_t w = bit >> 5;
+                    const uint32_t sh = (uint32_t)(bit & 31u);
+                    uint32_t b = __ldg(&bm[w]) >> sh;
+                    if (sh > 32u - (uint32_t)T::X) b |= __ldg(&bm[w + 1]) << (32u - sh);   // bitmaps hold a word more
+                    b &= in;
+#pragma unroll
+                    for (int i = 0; i < T::X; ++i)
+                        m[i % K] |= ((b >> i) & 1u) << (z * (32 / T::Z) + y * (T::X / K) + i / K);
+                }
+        }
+        uint32_t any = 0u;
+#pragma unroll
+        for (int k = 0; k < K; ++k) any |= m[k];
+        const uint32_t vote = __ballot_sync(0xffffffffu, any != 0u);
+        if (!vote) continue;
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t base = 0u;
+        if (lane == 0u) base = atomicAdd(n_tiles, (uint32_t)__popc(vote));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (any) {
+            const uint32_t e = base + (uint32_t)__popc(vote & ((1u << lane) - 1u));
+            list[e] = t;
+#pragma unroll
+            for (int k = 0; k < K; ++k) mask[(size_t)K * e + k] = m[k];
+        }
+    }
+}
+
+// A staged particle: position and packed kernel, its cell key, and whether its cell
+// differs from the one before.
+struct FieldStage {
+    float4 a;     // x, y, z, m00
+    float4 b;     // 2 m01, 2 m02, m11, 2 m12
+    float4 c;     // m22, w, key bits, new-cell flag
+};
+static constexpr int kFieldStage = 64;
+static constexpr float kNever = -1.0e30f;       // below any |G r|^2
+
+template <int BT, int K>
+__global__ void __launch_bounds__(BT, kFieldWarps * 32 / BT)
+k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cnt, const uint32_t* __restrict__ n_tiles_dev,
+              uint32_t* __restrict__ next, const uint32_t* __restrict__ list, const uint32_t* __restrict__ mask,
+              const uint32_t* __restrict__ cell_start, const float* __restrict__ cell_rad,
+              const uint32_t* __restrict__ skeys, const float4* __restrict__ spos, const float4* __restrict__ aniso,
+              const uint32_t* __restrict__ bm, const uint32_t* __restrict__ wprefix, float* __restrict__ field,
+              float* __restrict__ fdense, Counters* __restrict__ cnt_w) {
+    using T = FieldTile<K>;
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ FieldStage stage_all[BT / 32][kFieldStage];
+    const uint32_t lane = threadIdx.x & 31u;
+    FieldStage* stage = stage_all[threadIdx.x >> 5];
+    const uint32_t n_tiles = *n_tiles_dev;
+    const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
+    const int srx = (int)g.spres[0], sry = (int)g.spres[1], srz = (int)g.spres[2];
+    const int e2 = 2 * g.spexpand;
+    const float pad = 1e-4f * g.sp_cs, cs = g.sp_cs, inv_cs = 1.f / g.sp_cs;
+    const float* __restrict__ row_rad = cell_rad + g.sp_size;
+    const float rmax = fmaxf(__uint_as_float(cnt->rad_max_bits), fp.h) * fp.grow;
+    const float rmax2 = rmax * rmax;
+    // the lane's place in a tile
+    const uint32_t lx = K == 1 ? lane & 3u : (lane & 1u) * K, ly = K == 1 ? (lane >> 2) & 3u : (lane >> 1) & 3u,
+                   lz = K == 1 ? lane >> 4 : lane >> 3;
+    // few tiles are spread over all warps; many are taken in stretches, whose rows of cells
+    // stay in the SM's cache from tile to tile
+    const uint32_t ticket = min(max(n_tiles / (gridDim.x * (BT / 32u) * 4u), 1u), kTileTicket);
+    unsigned long long my_pairs = 0;
+    for (;;) {
+        uint32_t first = 0u;
+        if (lane == 0u) first = atomicAdd(next, ticket);
+        first = __shfl_sync(kAll, first, 0);
+        if (first >= n_tiles) break;
+        const uint32_t last = min(first + ticket, n_tiles);
+        for (uint32_t e = first; e < last; ++e) {
+            const uint32_t t = __ldg(&list[e]);
+            uint32_t m[K];
+#pragma unroll
+            for (int k = 0; k < K; ++k) m[k] = __ldg(&mask[(size_t)K * e + k]);
+            const uint32_t tx = t % td.x, tyz = t / td.x, ty = tyz % td.y, tz = tyz / td.y;
+            const uint32_t ix = tx * T::X + lx, iy = ty * T::Y + ly, iz = tz * T::Z + lz;
+            const float vy = sc_coord(g, iy, 1), vz = sc_coord(g, iz, 2);
+            float vx[K], sum[K];
+            float lim[K];                            // |G r|^2 below which a particle adds: 1, or never
+            bool have[K];
+            uint32_t nvert = 0u, x_lo = 0xffffffffu, x_hi = 0u;
+            bool some = false;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                vx[k] = sc_coord(g, ix + (uint32_t)k, 0);
+                have[k] = (m[k] >> lane) & 1u;
+                lim[k] = have[k] ? 1.f : kNever;
+                sum[k] = have[k] ? 0.f : INFINITY;   // no vertex: past the threshold from the start
+                nvert += (uint32_t)__popc(m[k]);
+                if (have[k]) { x_lo = min(x_lo, ix + (uint32_t)k); x_hi = max(x_hi, ix + (uint32_t)k); some = true; }
+            }
+            // the box of the tile's band vertices, and the spatial cells of its corners
+            x_lo = __reduce_min_sync(kAll, x_lo);
+            x_hi = __reduce_max_sync(kAll, x_hi);
+            const uint32_t y_lo = __reduce_min_sync(kAll, some ? iy : 0xffffffffu), y_hi = __reduce_max_sync(kAll, some ? iy : 0u);
+            const uint32_t z_lo = __reduce_min_sync(kAll, some ? iz : 0xffffffffu), z_hi = __reduce_max_sync(kAll, some ? iz : 0u);
+            const float bx0 = sc_coord(g, x_lo, 0), bx1 = sc_coord(g, x_hi, 0);
+            const float by0 = sc_coord(g, y_lo, 1), by1 = sc_coord(g, y_hi, 1);
+            const float bz0 = sc_coord(g, z_lo, 2), bz1 = sc_coord(g, z_hi, 2);
+            const uint3 c0 = sp_cell(g, bx0, by0, bz0), c1 = sp_cell(g, bx1, by1, bz1);
+            // cells some vertex's window holds [ulo, uhi), and cells that every window holds
+            // past its first column [ilo, ihi); near the grid's low side, where the reference's
+            // unsigned window wraps, every cell takes the general path
+            const bool regular = min(c0.x, min(c0.y, c0.z)) >= (uint32_t)e2;
+            const int ulx = regular ? (int)c0.x - e2 : 0, uhx = regular ? min((int)c1.x + e2, srx - 1) : srx;
+            const int uly = regular ? (int)c0.y - e2 : 0, uhy = regular ? min((int)c1.y + e2, sry - 1) : sry;
+            const int ulz = regular ? (int)c0.z - e2 : 0, uhz = regular ? min((int)c1.z + e2, srz - 1) : srz;
+            const int ilx = (int)c1.x - e2 + 1, ihx = regular ? min((int)c0.x + e2, srx - 1) : 0;
+            const int ily = (int)c1.y - e2, ihy = min((int)c0.y + e2, sry - 1);
+            const int ilz = (int)c1.z - e2, ihz = min((int)c0.z + e2, srz - 1);
+            const float ux0 = (bx0 - g.min_pos[0]) * inv_cs, ux1 = (bx1 - g.min_pos[0]) * inv_cs;
+            const float uy0 = (by0 - g.min_pos[1]) * inv_cs, uy1 = (by1 - g.min_pos[1]) * inv_cs;
+            const float uz0 = (bz0 - g.min_pos[2]) * inv_cs, uz1 = (bz1 - g.min_pos[2]) * inv_cs;
+            // rows (z, y) within the frame's largest support of the box
+            const float rc = rmax * inv_cs + kRangeMargin;
+            const int za = max((int)floorf(uz0 - rc), ulz), zb = min((int)floorf(uz1 + rc) + 1, uhz);
+            const int ya = max((int)floorf(uy0 - rc), uly), yb = min((int)floorf(uy1 + rc) + 1, uhy);
+            const int ny = yb - ya, nrow = ny > 0 && zb > za ? ny * (zb - za) : 0;
+
+            int staged = 0;
+            bool odd = false;                        // a staged particle needs the general path
+            uint32_t key_before = 0xffffffffu;       // cell of the last staged particle
+
+            // every lane over the staged particles
+            auto run = [&](auto general) {
+                constexpr bool G = decltype(general)::value;
+                int wx0[K], wx1[K], wy0 = 0, wy1 = 0, wz0 = 0, wz1 = 0;
+                if constexpr (G) {
+                    uint3 lo, hi;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        const uint3 c = sp_cell(g, vx[k], vy, vz);
+                        box_clamp(g, c, (uint32_t)e2, lo, hi);
+                        wx0[k] = (int)lo.x;
+                        wx1[k] = (int)hi.x;
+                    }
+                    wy0 = (int)lo.y; wy1 = (int)hi.y; wz0 = (int)lo.z; wz1 = (int)hi.z;
+                }
+#pragma unroll 2
+                for (int i = 0; i < staged; ++i) {
+                    const float4 a = stage[i].a, b = stage[i].b, c = stage[i].c;
+                    const bool fresh = c.w != 0.f;   // the first particle of a cell
+                    if constexpr (G) {
+                        if (fresh) {
+                            const uint32_t key = __float_as_uint(c.z);
+                            const int row = (int)(key / (uint32_t)srx), x = (int)(key - (uint32_t)row * (uint32_t)srx);
+                            const int z = row / sry, y = row - z * sry;
+                            const bool in = y >= wy0 && y < wy1 && z >= wz0 && z < wz1;
+#pragma unroll
+                            for (int k = 0; k < K; ++k)
+                                lim[k] = have[k] && in && x >= wx0[k] && x < wx1[k] && (x == wx0[k] || !(sum[k] > fp.thr)) ? 1.f : kNever;
+                        }
+                    } else {
+                        // (a cell inside every window: a vertex past the threshold takes no more of them)
+#pragma unroll
+                        for (int k = 0; k < K; ++k)
+                            if (fresh) lim[k] = sum[k] > fp.thr ? kNever : 1.f;
+                    }
+                    // r^T M r with every rounding spelled out (as in the run walk above); the
+                    // x-neighbours' parts two at a time
+                    const float ry = __fsub_rn(a.y, vy), rz = __fsub_rn(a.z, vz);
+                    const float pyz = __fmaf_rn(rz, __fmul_rn(c.x, rz), __fmul_rn(ry, __fmaf_rn(b.z, ry, __fmul_rn(b.w, rz))));
+                    const float cyz = __fmaf_rn(b.x, ry, __fmul_rn(b.y, rz));
+                    if constexpr (K == 1) {
+                        const float rxk = __fsub_rn(a.x, vx[0]);
+                        const float d2 = __fmaf_rn(rxk, __fmaf_rn(a.w, rxk, cyz), pyz);
+                        const float xx = __fsub_rn(1.f, d2);
+                        const float w = __fmul_rn(c.y, __fmul_rn(__fmul_rn(xx, xx), xx));
+                        if (d2 < lim[0]) sum[0] = __fadd_rn(sum[0], w);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < K; k += 2) {
+                            const float2 rr = __fadd2_rn(make_float2(a.x, a.x), make_float2(-vx[k], -vx[k + 1]));
+                            const float2 d2 = __ffma2_rn(rr, __ffma2_rn(make_float2(a.w, a.w), rr, make_float2(cyz, cyz)),
+                                                         make_float2(pyz, pyz));
+                            const float2 xx = __ffma2_rn(d2, make_float2(-1.f, -1.f), make_float2(1.f, 1.f));   // 1 - d2
+                            const float2 w = __fmul2_rn(make_float2(c.y, c.y), __fmul2_rn(__fmul2_rn(xx, xx), xx));
+                            if (d2.x < lim[k]) sum[k] = __fadd_rn(sum[k], w.x);
+                            if (d2.y < lim[k + 1]) sum[k + 1] = __fadd_rn(sum[k + 1], w.y);
+                        }
+                    }
+                }
+                my_pairs += (unsigned long long)(nvert * (uint32_t)staged);
+            };
+            auto flush = [&]() {
+                __syncwarp();
+                if (odd) run(std::true_type());
+                else run(std::false_type());
+                __syncwarp();
+                staged = 0;
+                odd = false;
+            };
+
+            for (int r0 = 0; r0 < nrow; r0 += 32) {
+                // a row per lane: its cells within the row's largest support of the box
+                const int r = r0 + (int)lane;
+                uint32_t ja = 0u, n = 0u, zy = 0u;
+                if (r < nrow) {
+                    const int z = za + r / ny, y = ya + r % ny;
+                    const uint32_t rowi = (uint32_t)z * (uint32_t)sry + (uint32_t)y;
+                    const float z0 = g.min_pos[2] + (float)z * cs, y0 = g.min_pos[1] + (float)y * cs;
+                    const float gz = fmaxf(fmaxf(z0 - pad - bz1, bz0 - (z0 + cs + pad)), 0.f);
+                    const float gy = fmaxf(fmaxf(y0 - pad - by1, by0 - (y0 + cs + pad)), 0.f);
+                    const float gyz = gz * gz + gy * gy;
+                    const float rr = fmaxf(__ldg(&row_rad[rowi]), fp.h) * fp.grow;
+                    const float rr2 = rr * rr;
+                    if (gyz < rr2) {
+                        const float rxc = sqrtf(rr2 - gyz) * inv_cs + kRangeMargin;
+                        const int xa = max((int)floorf(ux0 - rxc), ulx), xb = min((int)floorf(ux1 + rxc) + 1, uhx);
+                        if (xa < xb) {
+                            const uint32_t row = rowi * (uint32_t)srx;
+                            ja = __ldg(&cell_start[row + (uint32_t)xa]);
+                            n = __ldg(&cell_start[row + (uint32_t)xb]) - ja;
+                        }
+                    }
+                    zy = (z >= ilz && z < ihz && y >= ily && y < ihy) ? 1u : 0u;
+                }
+                uint32_t incl = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(kAll, incl, o);
+                    if (lane >= (uint32_t)o) incl += v;
+                }
+                const uint32_t total = __shfl_sync(kAll, incl, 31);
+                const uint32_t off = ja - (incl - n);          // particle index = off + position in the rows' list
+                for (uint32_t p0 = 0u; p0 < total; p0 += 32u) {
+                    const uint32_t p = p0 + lane;
+                    // the row holding position p: the first whose inclusive count exceeds p
+                    int row = 0;
+#pragma unroll
+                    for (int s = 16; s > 0; s >>= 1)
+                        if (__shfl_sync(kAll, incl, row + s - 1) <= p) row += s;
+                    const uint32_t j = __shfl_sync(kAll, off, row) + p;
+                    const uint32_t inner_row = __shfl_sync(kAll, zy, row);
+                    bool keep = false;
+                    float4 q, a0, a1;
+                    uint32_t key = 0u;
+                    if (p < total) {
+                        q = __ldg(&spos[j]);
+                        a0 = __ldg(&aniso[2 * (size_t)j]);
+                        key = __ldg(&skeys[j]);
+                        float ex, ey, ez;
+                        unpack_extents(__float_as_uint(a0.w), fp.ext_unit, ex, ey, ez);
+                        a1 = __ldg(&aniso[2 * (size_t)j + 1]);
+                        const float x0 = bx0 - q.x, x1 = bx1 - q.x, y0 = by0 - q.y, y1 = by1 - q.y, z0 = bz0 - q.z, z1 = bz1 - q.z;
+                        keep = !(x1 < -ex || x0 > ex || y1 < -ey || y0 > ey || z1 < -ez || z0 > ez);
+                        if (keep) {
+                            // a plane between the support and the box: its normal n = M r for the box's
+                            // nearest point r, the support's reach along it sqrt(n M^-1 n) = sqrt(r M r),
+                            // the box's lowest point along it (exact for a ball; never cuts a contribution)
+                            const float r0 = fminf(fmaxf(0.f, x0), x1), r1 = fminf(fmaxf(0.f, y0), y1), r2 = fminf(fmaxf(0.f, z0), z1);
+                            const float m01 = 0.5f * a0.y, m02 = 0.5f * a0.z, m12 = 0.5f * a1.y;
+                            const float n0 = a0.x * r0 + m01 * r1 + m02 * r2, n1 = m01 * r0 + a1.x * r1 + m12 * r2,
+                                        n2 = m02 * r0 + m12 * r1 + a1.z * r2;
+                            const float s = n0 * r0 + n1 * r1 + n2 * r2;
+                            const float low = fminf(n0 * x0, n0 * x1) + fminf(n1 * y0, n1 * y1) + fminf(n2 * z0, n2 * z1);
+                            keep = !(low > 0.f && low * low > 1.002f * s);
+                        }
+                    }
+                    const uint32_t kept = __ballot_sync(kAll, keep);
+                    if (!kept) continue;
+                    // a kept particle opens a cell when the kept one before it lies in another
+                    const uint32_t below = kept & ((1u << lane) - 1u);
+                    const uint32_t prev = __shfl_sync(kAll, key, below ? 31 - __clz(below) : 0);
+                    const uint32_t key_last = __shfl_sync(kAll, key, 31 - __clz(kept));
+                    if (keep) {
+                        const bool fresh = key != (below ? prev : key_before);
+                        FieldStage& s = stage[staged + __popc(below)];
+                        s.a = make_float4(q.x, q.y, q.z, a0.x);
+                        s.b = make_float4(a0.y, a0.z, a1.x, a1.y);
+                        s.c = make_float4(a1.z, a1.w, __uint_as_float(key), fresh ? 1.f : 0.f);
+                    }
+                    const int x = (int)(key % (uint32_t)srx);
+                    odd |= __any_sync(kAll, keep && !(inner_row && x >= ilx && x < ihx));
+                    key_before = key_last;
+                    staged += __popc(kept);
+                    if (staged > kFieldStage - 32) flush();
+                }
+            }
+            if (staged) flush();
+            // values, in band order and over the scalar grid
+            const uint32_t id = iz * rxy + iy * rx + ix;
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (have[k]) {
+                    const uint32_t v = id + (uint32_t)k;
+                    if (field) field[wprefix[v >> 5] + (uint32_t)__popc(__ldg(&bm[v >> 5]) & ((1u << (v & 31u)) - 1u))] = sum[k];
+                    fdense[v] = sum[k];
+                }
+        }
+    }
+    if (lane == 0u && my_pairs) atomicAdd(&cnt_w->n_pairs, my_pairs);
+}
+
+template <int K>
+static uint3 field_tile_dims(const pms_grid& g) {
+    using T = FieldTile<K>;
+    return make_uint3((g.scres[0] + T::X - 1) / T::X, (g.scres[1] + T::Y - 1) / T::Y, (g.scres[2] + T::Z - 1) / T::Z);
+}
+
+// the listed tiles of a bitmap of at most nv set bits: an index and K lane masks each
+template <int K>
+static uint64_t field_tile_most(const pms_grid& g, uint64_t nv) {
+    const uint3 td = field_tile_dims<K>(g);
+    return std::min<uint64_t>((uint64_t)td.x * td.y * td.z, nv);
+}
+template <int K>
+static size_t field_tile_bytes_of(const pms_grid& g, uint64_t nv) {
+    return 4 * (size_t)(1 + K) * (field_tile_most<K>(g, nv) + 1);
+}
+size_t field_tile_bytes(const pms_grid& g, int vpt, uint64_t nv) {
+    return vpt == 1 ? field_tile_bytes_of<1>(g, nv) : vpt == 4 ? field_tile_bytes_of<4>(g, nv) : field_tile_bytes_of<2>(g, nv);
+}
+
+template <int K>
+static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t n_host, float* out) {
+    const KGrid g = kgrid_of(ctx->grid);
+    const pms_params& P = ctx->prm;
+    FieldParams fp;
+    fp.h = P.h;
+    fp.thr = 2.f * P.iso_value;
+    fp.grow = kSupportGrow;
+    fp.quick = 0.f;
+    fp.ext_unit = extent_unit(P.h);
+    Counters* cnt = ctx->counters.as<Counters>();
+    const uint3 td = field_tile_dims<K>(ctx->grid);
+    const uint64_t ntiles = (uint64_t)td.x * td.y * td.z, most = field_tile_most<K>(ctx->grid, n_host);
+    PMS_CUDA(ctx, ctx->ftiles.ensure_grow(field_tile_bytes_of<K>(ctx->grid, n_host)));
+    uint32_t* list = ctx->ftiles.as<uint32_t>();
+    uint32_t* mask = list + most + 1;
+    // the list's length and the next ticket
+    PMS_CUDA(ctx, cudaMemsetAsync(&cnt->n_items, 0, 2 * sizeof(uint32_t), ctx->stream));
+    k_field_tile_list<K><<<grid_for(ntiles, 256), 256, 0, ctx->stream>>>(g, td, bm, &cnt->n_items, list, mask);
+    PMS_LAUNCHED(ctx);
+    const int bt = ctx->tune.field_threads;
+    const unsigned per_sm = kFieldWarps * 32u / (unsigned)bt;
+    const unsigned blocks = grid_for(most, (unsigned)bt / 32u, 152u * per_sm);
+    auto go = [&](auto kern) {
+        kern<<<blocks, bt, 0, ctx->stream>>>(g, fp, td, cnt, &cnt->n_items, &cnt->field_next, list, mask,
+                                             ctx->cell_start.as<uint32_t>(), ctx->cell_rad.as<float>(),
+                                             ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(), bm,
+                                             wprefix, out, ctx->fdense.as<float>(), cnt);
+    };
+    if (bt == 64) go(k_field_tiles<64, K>);
+    else if (bt == 256) go(k_field_tiles<256, K>);
+    else go(k_field_tiles<128, K>);
+    PMS_LAUNCHED(ctx);
+    return PMS_OK;
+}
+
+pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t n_host, float* out) {
+    if ((uint64_t)n_host >= (1ull << kItemShift)) return pms_fail(ctx, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices");
+    if (ctx->tune.field_vpt == 1) return field_tiles_of<1>(ctx, bm, wprefix, n_host, out);
+    if (ctx->tune.field_vpt == 4) return field_tiles_of<4>(ctx, bm, wprefix, n_host, out);
+    return field_tiles_of<2>(ctx, bm, wprefix, n_host, out);
+}
+
+// ---------------------------------------------------------------------------
+// per-cell culling record for the certification: the bounding box of the cell's
+// particles and the square of the largest support among them (h, or the
+// cell's largest maxvalue * h), grown by kSupportGrow.  A vertex farther than
+// that from the box gets exactly 0 from every particle of the cell.  An empty
+// cell gets r^2 = -1, which no vertex reaches.
+// rec[2c] = {min x, min y, min z, r^2}, rec[2c + 1] = {max x, max y, max z, 0}.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) k_cell_records(const uint32_t* __restrict__ cell_start,
+                                                           const float4* __restrict__ spos,
+                                                           const float* __restrict__ cell_rad, float h, uint32_t S,
+                                                           float4* __restrict__ rec) {
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < S; c += gridDim.x * blockDim.x) {
+        const uint32_t j0 = cell_start[c], j1 = cell_start[c + 1];
+        if (j0 == j1) {
+            rec[2 * (size_t)c] = make_float4(0.f, 0.f, 0.f, -1.f);
+            continue;
+        }
+        const float4 q = spos[j0];
+        float lx = q.x, ly = q.y, lz = q.z, hx = q.x, hy = q.y, hz = q.z;
+        for (uint32_t j = j0 + 1; j < j1; ++j) {
+            const float4 p = spos[j];
+            lx = fminf(lx, p.x); ly = fminf(ly, p.y); lz = fminf(lz, p.z);
+            hx = fmaxf(hx, p.x); hy = fmaxf(hy, p.y); hz = fmaxf(hz, p.z);
+        }
+        const float r = fmaxf(cell_rad[c], h) * kSupportGrow;
+        rec[2 * (size_t)c] = make_float4(lx, ly, lz, r * r);
+        rec[2 * (size_t)c + 1] = make_float4(hx, hy, hz, 0.f);
+    }
 }
 
 // Work items over vlist[0 .. *n_dev): group g = entries [g K, g K + K) splits
@@ -370,15 +810,16 @@ __global__ void __launch_bounds__(256) k_field_items(const uint32_t* __restrict_
     }
 }
 
-pms_status launch_field_on(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, float* out,
-                           uint32_t* cert, uint32_t* n_cert) {
+pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, uint32_t* cert,
+                             uint32_t* n_cert) {
     const KGrid g = kgrid_of(ctx->grid);
     const pms_params& P = ctx->prm;
     FieldParams fp;
     fp.h = P.h;
-    fp.thr = cert ? P.iso_value : 2.f * P.iso_value;
+    fp.thr = P.iso_value;
     fp.grow = kSupportGrow;
     fp.quick = P.iso_value * (1.f + 1.f / 512.f);
+    fp.ext_unit = 0.f;
     Counters* cnt = ctx->counters.as<Counters>();
     if ((uint64_t)n_host >= (1ull << kItemShift)) return pms_fail(ctx, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices");
     const uint32_t K = (uint32_t)ctx->tune.field_vpt;
@@ -386,6 +827,10 @@ pms_status launch_field_on(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* 
     PMS_CUDA(ctx, ctx->fitem_cnt.ensure(4 * ((size_t)ngroups + 1)));
     PMS_CUDA(ctx, ctx->fitem_off.ensure(4 * ((size_t)ngroups + 1)));
     PMS_CUDA(ctx, ctx->fitems.ensure(4 * ((size_t)n_host + 1)));
+    k_cell_records<<<grid_for(g.sp_size, 128), 128, 0, ctx->stream>>>(ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
+                                                                      ctx->cell_rad.as<float>(), P.h, g.sp_size,
+                                                                      ctx->cell_rec.as<float4>());
+    PMS_LAUNCHED(ctx);
     const unsigned gb = grid_for(ngroups, 256);
     k_field_items<<<gb, 256, 0, ctx->stream>>>(vlist, n_dev, ngroups, K, g.scres[0], nullptr, ctx->fitem_cnt.as<uint32_t>());
     PMS_LAUNCHED(ctx);
@@ -400,20 +845,14 @@ pms_status launch_field_on(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* 
     auto go = [&](auto kern) {
         kern<<<blocks, bt, 0, ctx->stream>>>(g, fp, cnt, &cnt->n_items, ctx->fitems.as<uint32_t>(), vlist,
                                              ctx->cell_start.as<uint32_t>(), ctx->cell_rad.as<float>(),
-                                             ctx->cell_rec.as<float4>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(), out,
+                                             ctx->cell_rec.as<float4>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(),
                                              ctx->fdense.as<float>(), cert, n_cert, cnt);
     };
     auto by_vpt = [&](auto bt_tag) {
         constexpr int B = decltype(bt_tag)::value;
-        if (cert) {
-            if (K == 1) go(k_field<B, 1, true>);
-            else if (K == 4) go(k_field<B, 4, true>);
-            else go(k_field<B, 2, true>);
-        } else {
-            if (K == 1) go(k_field<B, 1, false>);
-            else if (K == 4) go(k_field<B, 4, false>);
-            else go(k_field<B, 2, false>);
-        }
+        if (K == 1) go(k_field_cert<B, 1>);
+        else if (K == 4) go(k_field_cert<B, 4>);
+        else go(k_field_cert<B, 2>);
     };
     if (bt == 64) by_vpt(std::integral_constant<int, 64>());
     else if (bt == 256) by_vpt(std::integral_constant<int, 256>());
@@ -424,9 +863,8 @@ pms_status launch_field_on(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* 
 
 // the frame's first field evaluation: the dense field starts at 0 everywhere
 pms_status launch_field(pms_ctx* ctx) {
-    Counters* cnt = ctx->counters.as<Counters>();
     PMS_CUDA(ctx, cudaMemsetAsync(ctx->fdense.p, 0, 4 * (size_t)ctx->grid.sc_size, ctx->stream));
-    return launch_field_on(ctx, ctx->vlist.as<uint32_t>(), &cnt->nv, ctx->nv, ctx->field.as<float>());
+    return launch_field_bits(ctx, ctx->bm.as<uint32_t>(), ctx->wprefix.as<uint32_t>(), ctx->nv, ctx->field.as<float>());
 }
 
 // field[t] = fdense[vlist[t]]: the band-order field of a vertex list whose values are all computed

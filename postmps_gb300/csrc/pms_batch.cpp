@@ -323,9 +323,11 @@ static pms_status ensure_lane(pms_ctx* lc, pms_ctx* c, uint32_t nmax, const pms_
     PMS_CUDA(lc, lc->scan.partial.ensure(sizeof(unsigned long long) * 1024));
     lc->tune = c->tune;
     lc->tc_wait_polls = c->tc_wait_polls;     // the debug wait limit holds on every lane
+    for (const pms_grid& g : grid) PMS_CUDA(lc, lc->ftiles.ensure(field_tile_bytes(g, c->tune.field_vpt, g.sc_size)));
     if (!learned) return PMS_OK;
     const size_t S = (size_t)gmax.sc_size + 1;
     if ((st = ensure_learned_buffers(lc, gmax.sc_size, gmax.sc_size))) return st;
+    for (DBuf* d : {&lc->fitems, &lc->fitem_cnt, &lc->fitem_off}) PMS_CUDA(lc, d->ensure(4 * S));
     size_t ncoarse = 1;
     for (const pms_grid& g : grid)
         ncoarse = std::max(ncoarse, (size_t)(g.scres[0] / 2 + 2) * (g.scres[1] / 2 + 2) * (g.scres[2] / 2 + 2));

@@ -75,7 +75,8 @@ struct Counters {
     uint32_t l_nlist;       // band vertices certified (the rest of the band)
     uint32_t l_cert;        // ... of which stopped above iso without an exact value
     uint32_t l_recheck;     // certified corners of valid cubes, evaluated exactly afterwards
-    uint32_t n_items;       // work items of the last field launch
+    uint32_t n_items;       // work items (runs or tiles) of the last field launch
+    uint32_t field_next;    // the next listed tile a warp of the field takes (zeroed with n_items)
     uint32_t n_tiles;       // scalar-grid tiles the band marking visits
     uint32_t n_weld;        // vertices of the welded mesh (crossed grid edges)
     uint32_t n_df_total;    // generated + carried diffuse particles of a batched frame
@@ -210,8 +211,8 @@ struct pms_ctx {
     pms::DBuf w_bits, w_wc, w_wp, w_vert, w_vnorm, w_idx;
     uint64_t w_nvert = 0;
     bool have_weld = false, weld_normals = false;
-    // field work items (runs of x-neighbouring band vertices)
-    pms::DBuf fitems, fitem_cnt, fitem_off;
+    // field work: runs of x-neighbouring band vertices (certification), tiles (exact field)
+    pms::DBuf fitems, fitem_cnt, fitem_off, ftiles;
     bool have_values = false;
     // vertex normals of the current mesh: made by the emission only when a streamed
     // mesh asks for them, else on the first download that does
@@ -315,10 +316,15 @@ pms_status launch_density_aniso(pms_ctx* ctx);
 pms_status launch_band(pms_ctx* ctx);
 pms_status launch_band_list(pms_ctx* ctx);
 pms_status launch_field(pms_ctx* ctx);
-// field at the vertices vlist[0 .. *n_dev) into out (n_host: a bound for the grid); with
-// cert, sign certification: vertices stopped above iso get a bit there, n_cert counts them
-pms_status launch_field_on(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, float* out,
-                           uint32_t* cert = nullptr, uint32_t* n_cert = nullptr);
+// sign certification of the vertices vlist[0 .. *n_dev) (n_host: a bound for the grid):
+// values or placeholders into fdense, a bit of cert per vertex stopped above iso, their count
+pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, uint32_t* cert,
+                             uint32_t* n_cert);
+// exact field at the vertices of a bitmap over the scalar grid (n_host: a bound of their
+// number), into fdense and, unless null, in bitmap order into out (wprefix: the words' ranks)
+pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t n_host, float* out);
+// bytes of the tile list such a launch needs (field_vpt vertices per lane)
+size_t field_tile_bytes(const pms_grid& g, int vpt, uint64_t nv);
 pms_status launch_field_gather(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, float* out);
 // ascending list of the set bits of a bitmap over the scalar grid
 pms_status launch_bits_list(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t* vlist);

@@ -116,9 +116,8 @@ pms_status pms::learned_field(pms_ctx* c) {
     pms_status st;
     PMS_CUDA(c, cudaMemsetAsync(c->fdense.p, 0, 4 * (size_t)c->grid.sc_size, c->stream));
     PMS_CUDA(c, cudaMemsetAsync(c->l_cert.p, 0, 4 * W, c->stream));
-    if ((st = launch_field_on(c, c->l_e_list.as<uint32_t>(), &cnt->l_exact, nvb, nullptr))) return st;
-    if ((st = launch_field_on(c, c->l_n_list.as<uint32_t>(), &cnt->l_nlist, nvb, nullptr, c->l_cert.as<uint32_t>(),
-                              &cnt->l_cert)))
+    if ((st = launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nullptr, nvb, nullptr))) return st;
+    if ((st = launch_field_cert(c, c->l_n_list.as<uint32_t>(), &cnt->l_nlist, nvb, c->l_cert.as<uint32_t>(), &cnt->l_cert)))
         return st;
     if ((st = launch_mc_classify(c))) return st;
     // the certified corners of valid cubes: E's buffers hold them from here on
@@ -127,7 +126,7 @@ pms_status pms::learned_field(pms_ctx* c) {
     if ((st = launch_popc(c, c->l_e_bm.as<uint32_t>(), c->l_e_wc.as<uint32_t>()))) return st;
     if ((st = scan_u32(c, c->l_e_wc.as<uint32_t>(), c->l_e_wp.as<uint32_t>(), W, &cnt->l_recheck))) return st;
     if ((st = launch_bits_list(c, c->l_e_bm.as<uint32_t>(), c->l_e_wp.as<uint32_t>(), c->l_e_list.as<uint32_t>()))) return st;
-    if ((st = launch_field_on(c, c->l_e_list.as<uint32_t>(), &cnt->l_recheck, nvb, nullptr))) return st;
+    if ((st = launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nullptr, nvb, nullptr))) return st;
     return launch_field_gather(c, c->vlist.as<uint32_t>(), &cnt->nv, nvb, c->field.as<float>());
 }
 
