@@ -320,7 +320,7 @@ static pms_status ensure_lane(pms_ctx* lc, pms_ctx* c, uint32_t nmax, const pms_
     if ((st = ensure_particle_buffers(lc, nmax))) return st;
     if ((st = ensure_grid_buffers(lc, gmax))) return st;
     if ((st = ensure_band_buffers(lc, gmax.sc_size))) return st;
-    PMS_CUDA(lc, lc->scan.partial.ensure(sizeof(unsigned long long) * 1024));
+    PMS_CUDA(lc, lc->scan.partial.ensure(scan_scratch_bytes()));
     lc->tune = c->tune;
     lc->tc_wait_polls = c->tc_wait_polls;     // the debug wait limit holds on every lane
     for (const pms_grid& g : grid) PMS_CUDA(lc, lc->ftiles.ensure(field_tile_bytes(g, c->tune.field_vpt, g.sc_size)));
@@ -507,7 +507,7 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
         if (diffuse) {
             pms_ctx* dl = b->dlane;
             if ((st = ensure_diffuse_batch_buffers(dl, nmax, b->gen_cap, b->old_cap))) return st;
-            PMS_CUDA(c, dl->scan.partial.ensure(sizeof(unsigned long long) * 1024));
+            PMS_CUDA(c, dl->scan.partial.ensure(scan_scratch_bytes()));
             PMS_CUDA(c, b->dcnt.ensure(2 * sizeof(uint32_t)));
             PMS_CUDA(c, b->drun.ensure(sizeof(unsigned long long)));
             PMS_CUDA(c, b->dbase.ensure(sizeof(unsigned long long) * k));

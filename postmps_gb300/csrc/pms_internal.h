@@ -286,12 +286,14 @@ inline unsigned grid_for(uint64_t n, unsigned block, unsigned max_blocks = 152u 
 }
 
 // scans (scan.cu): exclusive prefix sums of n elements; *total_dev receives the
-// sum (may be null); with n_dev, elements at and past *n_dev count as zero
-// (n is then a bound).  All asynchronous on the stream.
+// sum (may be null); with n_dev, the scan covers the first *n_dev elements (n is
+// then a bound; out is not written past them).  All asynchronous on the stream.
 pms_status scan_u32(pms_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total_dev,
                     const uint32_t* n_dev = nullptr);
 pms_status scan_u64(pms_ctx* ctx, const unsigned long long* in, unsigned long long* out, uint64_t n,
                     unsigned long long* total_dev, const uint32_t* n_dev = nullptr);
+
+size_t scan_scratch_bytes();   // what a scan keeps in ScanTemp (captured launches: allocated before)
 
 // stage launchers (one .cu each)
 pms_status launch_bbox(pms_ctx* ctx);

@@ -2,112 +2,203 @@
 // thrust::exclusive_scan wrapper, Thrust.cuh:17-38, which also copied the
 // total back to the host; here the total stays on the device).
 //
-// Reduce-then-scan over a fixed number of blocks: each block owns one
-// contiguous chunk, (1) reduces it, (2) one block scans the chunk sums,
-// (3) each block rescans its chunk from its offset.  Tiles are staged through
-// shared memory so that global loads and stores stay coalesced.
+// Two forms, by size.
+// - Up to kClusterMax elements: one launch of one thread-block cluster.  Every warp keeps
+//   its stretch in registers, the blocks exchange their totals through distributed shared
+//   memory.  A frame of a few thousand particles runs six scans of this size, and their
+//   launches, not their bytes, are what they cost: three launches of about 3.3 us each
+//   (reduce, partials, down) before, one now.
+// - Above: reduce, then down.  Each block owns one contiguous chunk, each of its warps a
+//   contiguous part of it, read in rows of 32 lanes x 16 bytes with no shared memory on the
+//   way; the down pass adds up the blocks' sums before its own itself (at most kMaxBlocks
+//   values), so no third launch does.
+// With a device count the chunks divide that count, so a bound far above it idles no block.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
 #include "pms_internal.h"
 #include "k_common.cuh"
 
 namespace pms {
 
+namespace cg = cooperative_groups;
+
 static constexpr int kScanThreads = 256;
-static constexpr int kScanItems = 8;
-static constexpr int kScanTile = kScanThreads * kScanItems;   // 2048
-static constexpr int kScanMaxBlocks = 1024;
+static constexpr int kScanWarps = kScanThreads / 32;
+static constexpr int kMaxBlocks = 1024;
+// the one-launch form: kCluster blocks of kClusterThreads, kRows rows of 32 per warp
+static constexpr int kCluster = 8, kClusterThreads = 1024, kRows = 16;
+static constexpr uint64_t kClusterMax = (uint64_t)kCluster * kClusterThreads * kRows;   // 131072
+
+// scratch: a sum per block, then one per warp
+size_t scan_scratch_bytes() { return sizeof(unsigned long long) * kMaxBlocks * (1 + kScanWarps); }
 
 template <class T>
 __device__ __forceinline__ T warp_incl_scan(T v) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        T t = __shfl_up_sync(0xffffffffu, v, o);
+        const T t = __shfl_up_sync(0xffffffffu, v, o);
         if ((threadIdx.x & 31) >= o) v += t;
     }
     return v;
 }
-
-// exclusive scan of one value per thread across the block; returns block total
 template <class T>
-__device__ __forceinline__ T block_excl_scan(T v, T* smem_warp, T& total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    T inc = warp_incl_scan(v);
-    if (lane == 31) smem_warp[wid] = inc;
+__device__ __forceinline__ T warp_sum(T v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kClusterThreads) k_scan_cluster(const T* __restrict__ in, T* __restrict__ out, uint32_t n,
+                                                                  T* __restrict__ total_out, const uint32_t* __restrict__ n_dev) {
+    __shared__ T warp_tot[kClusterThreads / 32];
+    __shared__ T block_tot;
+    const cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t nn = n_dev ? min(*n_dev, n) : n;          // elements past nn count as 0
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    // rows of 32 per warp, the least that covers nn
+    const uint32_t warps = gridDim.x * (kClusterThreads / 32);
+    const uint32_t rows = min((nn + warps * 32u - 1u) / (warps * 32u), (uint32_t)kRows);
+    const uint32_t base = (blockIdx.x * (kClusterThreads / 32) + wid) * rows * 32u + lane;
+    T v[kRows], run = 0;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) v[r] = (uint32_t)r < rows && base + 32u * r < nn ? in[base + 32u * r] : T(0);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+        if ((uint32_t)r < rows) {
+            const T x = v[r], inc = warp_incl_scan(x);
+            v[r] = run + inc - x;
+            run += __shfl_sync(0xffffffffu, inc, 31);
+        }
+    if (lane == 0u) warp_tot[wid] = run;
     __syncthreads();
-    if (wid == 0) {
-        T s = (lane < kScanThreads / 32) ? smem_warp[lane] : T(0);
-        s = warp_incl_scan(s);
-        if (lane < kScanThreads / 32) smem_warp[lane] = s;
+    if (wid == 0u) {
+        const T x = warp_tot[lane], inc = warp_incl_scan(x);
+        warp_tot[lane] = inc - x;
+        if (lane == 31u) block_tot = inc;
     }
-    __syncthreads();
-    T base = wid ? smem_warp[wid - 1] : T(0);
-    total = smem_warp[kScanThreads / 32 - 1];
-    __syncthreads();
-    return base + inc - v;
+    T before = 0;
+    if (gridDim.x > 1u) {
+        cluster.sync();
+        for (uint32_t b = 0; b < cluster.block_rank(); ++b) before += *cluster.map_shared_rank(&block_tot, b);
+        cluster.sync();                                     // no block leaves while its total may be read
+    } else {
+        __syncthreads();
+    }
+    if (total_out && blockIdx.x == gridDim.x - 1u && threadIdx.x == 0u) *total_out = before + block_tot;
+    before += warp_tot[wid];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+        if ((uint32_t)r < rows && base + 32u * r < nn) out[base + 32u * r] = before + v[r];
 }
 
-template <class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restrict__ in, uint64_t n, uint64_t chunk,
-                                                              T* __restrict__ partial, const uint32_t* __restrict__ n_dev) {
-    __shared__ T warp_sums[kScanThreads / 32];
-    uint64_t b0 = (uint64_t)blockIdx.x * chunk;
-    uint64_t b1 = b0 + chunk < n ? b0 + chunk : n;
-    const uint64_t nn = n_dev && (uint64_t)*n_dev < n ? (uint64_t)*n_dev : n;   // elements past nn count as 0
-    T acc = 0;
-    for (uint64_t i = b0 + threadIdx.x; i < b1; i += kScanThreads) acc += i < nn ? in[i] : T(0);
-    T total;
-    block_excl_scan<T>(acc, warp_sums, total);
-    if (threadIdx.x == 0) partial[blockIdx.x] = total;
+// one block's and one warp's stretch of nn elements, in whole rows of 32 lanes x V elements
+struct Stretch { uint64_t begin, end; };
+template <int V>
+__device__ __forceinline__ Stretch scan_stretch(uint64_t nn) {
+    const uint64_t row = 32u * V, rows = (nn + row - 1) / row;
+    const uint64_t parts = (uint64_t)gridDim.x * kScanWarps, per = (rows + parts - 1) / parts;
+    const uint64_t w = (uint64_t)blockIdx.x * kScanWarps + (threadIdx.x >> 5);
+    const uint64_t b = w * per * row, e = b + per * row;
+    return {b < nn ? b : nn, e < nn ? e : nn};
 }
 
-template <class T>
-__global__ void __launch_bounds__(1024) k_scan_partials(T* __restrict__ partial, int nb, T* __restrict__ total_out) {
-    __shared__ T warp_sums[32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    T v = threadIdx.x < nb ? partial[threadIdx.x] : T(0);
-    T inc = warp_incl_scan(v);
-    if (lane == 31) warp_sums[wid] = inc;
-    __syncthreads();
-    if (wid == 0) warp_sums[lane] = warp_incl_scan(warp_sums[lane]);
-    __syncthreads();
-    T base = wid ? warp_sums[wid - 1] : T(0);
-    if (threadIdx.x < nb) partial[threadIdx.x] = base + inc - v;
-    if (threadIdx.x == 1023 && total_out) *total_out = base + inc;
+// V consecutive elements, 16 bytes in one access when V > 1 (the launcher checks the alignment)
+template <class T, int V>
+__device__ __forceinline__ void load_row(const T* __restrict__ p, uint64_t i, uint64_t end, T (&x)[V]) {
+    if (V > 1 && i + V <= end) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(p + i));
+        memcpy(x, &q, sizeof(x));
+    } else {
+#pragma unroll
+        for (int k = 0; k < V; ++k) x[k] = i + k < end ? p[i + k] : T(0);
+    }
 }
 
-template <class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_down(const T* __restrict__ in, T* __restrict__ out, uint64_t n,
-                                                             uint64_t chunk, const T* __restrict__ partial,
-                                                             const uint32_t* __restrict__ n_dev) {
-    __shared__ T tile[kScanTile];
-    __shared__ T warp_sums[kScanThreads / 32];
-    uint64_t b0 = (uint64_t)blockIdx.x * chunk;
-    uint64_t b1 = b0 + chunk < n ? b0 + chunk : n;
+template <class T, int V>
+__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restrict__ in, uint64_t n, T* __restrict__ block_sum,
+                                                              T* __restrict__ warp_sums, const uint32_t* __restrict__ n_dev) {
+    __shared__ T ws[kScanWarps];
     const uint64_t nn = n_dev && (uint64_t)*n_dev < n ? (uint64_t)*n_dev : n;
-    T carry = partial[blockIdx.x];
-    for (uint64_t t0 = b0; t0 < b1; t0 += kScanTile) {
+    const Stretch s = scan_stretch<V>(nn);
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    T acc = 0;
+#pragma unroll 4
+    for (uint64_t i = s.begin + lane * V; i < s.end; i += 32u * V) {
+        T x[V];
+        load_row<T, V>(in, i, s.end, x);
 #pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
-            uint64_t i = t0 + k * kScanThreads + threadIdx.x;
-            tile[k * kScanThreads + threadIdx.x] = i < nn && i < b1 ? in[i] : T(0);
-        }
-        __syncthreads();
-        T loc[kScanItems];
-        T sum = 0;
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) { loc[k] = tile[threadIdx.x * kScanItems + k]; sum += loc[k]; }
-        T total;
-        T run = block_excl_scan<T>(sum, warp_sums, total) + carry;
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) { T v = loc[k]; tile[threadIdx.x * kScanItems + k] = run; run += v; }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
-            uint64_t i = t0 + k * kScanThreads + threadIdx.x;
-            if (i < b1) out[i] = tile[k * kScanThreads + threadIdx.x];
-        }
-        carry += total;
-        __syncthreads();
+        for (int k = 0; k < V; ++k) acc += x[k];
     }
+    acc = warp_sum(acc);
+    if (lane == 0u) {
+        ws[wid] = acc;
+        warp_sums[(size_t)blockIdx.x * kScanWarps + wid] = acc;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        T t = 0;
+#pragma unroll
+        for (int w = 0; w < kScanWarps; ++w) t += ws[w];
+        block_sum[blockIdx.x] = t;
+    }
+}
+
+template <class T, int V>
+__global__ void __launch_bounds__(kScanThreads) k_scan_down(const T* __restrict__ in, T* __restrict__ out, uint64_t n,
+                                                            const T* __restrict__ block_sum, const T* __restrict__ warp_sums,
+                                                            T* __restrict__ total_out, const uint32_t* __restrict__ n_dev) {
+    __shared__ T ws[kScanWarps];
+    const uint64_t nn = n_dev && (uint64_t)*n_dev < n ? (uint64_t)*n_dev : n;
+    const Stretch s = scan_stretch<V>(nn);
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    // the blocks before this one, summed here
+    T acc = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kScanThreads) acc += block_sum[b];
+    acc = warp_sum(acc);
+    if (lane == 0u) ws[wid] = acc;
+    __syncthreads();
+    T run = 0;
+#pragma unroll
+    for (int w = 0; w < kScanWarps; ++w) run += ws[w];
+    if (total_out && blockIdx.x == gridDim.x - 1u && threadIdx.x == 0u) *total_out = run + block_sum[blockIdx.x];
+    for (uint32_t w = 0; w < wid; ++w) run += warp_sums[(size_t)blockIdx.x * kScanWarps + w];
+#pragma unroll 2
+    for (uint64_t r = s.begin; r < s.end; r += 32u * V) {
+        const uint64_t i = r + lane * V;
+        T x[V], sum = 0;
+        load_row<T, V>(in, i, s.end, x);
+#pragma unroll
+        for (int k = 0; k < V; ++k) { const T t = x[k]; x[k] = sum; sum += t; }
+        const T inc = warp_incl_scan(sum);
+        const T before = run + inc - sum;
+        run += __shfl_sync(0xffffffffu, inc, 31);
+#pragma unroll
+        for (int k = 0; k < V; ++k) x[k] += before;
+        if (V > 1 && i + V <= s.end) {
+            uint4 q;
+            memcpy(&q, x, sizeof(q));
+            *reinterpret_cast<uint4*>(out + i) = q;
+        } else {
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+                if (i + k < s.end) out[i + k] = x[k];
+        }
+    }
+}
+
+template <class T, int V>
+static pms_status scan_two(pms_ctx* ctx, const T* in, T* out, uint64_t n, T* total_dev, const uint32_t* n_dev) {
+    const uint64_t per = 4u * 32u * V * kScanWarps;          // at least four rows for each warp
+    const unsigned nb = (unsigned)std::min<uint64_t>((n + per - 1) / per, kMaxBlocks);
+    T *block_sum = ctx->scan.partial.as<T>(), *warp_sums = block_sum + kMaxBlocks;
+    k_scan_reduce<T, V><<<nb, kScanThreads, 0, ctx->stream>>>(in, n, block_sum, warp_sums, n_dev);
+    PMS_LAUNCHED(ctx);
+    k_scan_down<T, V><<<nb, kScanThreads, 0, ctx->stream>>>(in, out, n, block_sum, warp_sums, total_dev, n_dev);
+    PMS_LAUNCHED(ctx);
+    return PMS_OK;
 }
 
 template <class T>
@@ -116,19 +207,28 @@ static pms_status scan_impl(pms_ctx* ctx, const T* in, T* out, uint64_t n, T* to
         if (total_dev) PMS_CUDA(ctx, cudaMemsetAsync(total_dev, 0, sizeof(T), ctx->stream));
         return PMS_OK;
     }
-    uint64_t tiles = (n + kScanTile - 1) / kScanTile;
-    int nb = (int)(tiles < (uint64_t)kScanMaxBlocks ? tiles : (uint64_t)kScanMaxBlocks);
-    uint64_t chunk = ((tiles + nb - 1) / nb) * kScanTile;
-    nb = (int)((n + chunk - 1) / chunk);
-    PMS_CUDA(ctx, ctx->scan.partial.ensure(sizeof(unsigned long long) * kScanMaxBlocks));
-    T* partial = ctx->scan.partial.as<T>();
-    k_scan_reduce<T><<<nb, kScanThreads, 0, ctx->stream>>>(in, n, chunk, partial, n_dev);
-    PMS_LAUNCHED(ctx);
-    k_scan_partials<T><<<1, 1024, 0, ctx->stream>>>(partial, nb, total_dev);
-    PMS_LAUNCHED(ctx);
-    k_scan_down<T><<<nb, kScanThreads, 0, ctx->stream>>>(in, out, n, chunk, partial, n_dev);
-    PMS_LAUNCHED(ctx);
-    return PMS_OK;
+    if (n <= kClusterMax) {
+        // one block while it has few rows per warp, else the cluster
+        cudaLaunchConfig_t cfg = {};
+        const unsigned nb = n <= 4u * kClusterThreads ? 1u : (unsigned)kCluster;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = nb;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(nb);
+        cfg.blockDim = dim3(kClusterThreads);
+        cfg.stream = ctx->stream;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        PMS_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_scan_cluster<T>, in, out, (uint32_t)n, total_dev, n_dev));
+        PMS_LAUNCHED(ctx);
+        return PMS_OK;
+    }
+    PMS_CUDA(ctx, ctx->scan.partial.ensure(scan_scratch_bytes()));
+    constexpr int V = 16 / (int)sizeof(T);
+    // 16-byte accesses where both arrays start on a 16-byte boundary
+    if (((uintptr_t)in | (uintptr_t)out) & 15u) return scan_two<T, 1>(ctx, in, out, n, total_dev, n_dev);
+    return scan_two<T, V>(ctx, in, out, n, total_dev, n_dev);
 }
 
 pms_status scan_u32(pms_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total_dev,
