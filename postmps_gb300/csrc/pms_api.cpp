@@ -64,7 +64,7 @@ static void for_each_dbuf(pms_ctx* c, F f) {
                     &c->df_scan.partial, &c->df_tmp,
                     &c->l_dens, &c->l_clist, &c->l_counts, &c->l_model, &c->l_q, &c->l_cert, &c->l_e_bm, &c->l_e_wc,
                     &c->l_e_wp, &c->l_e_list, &c->l_n_bm, &c->l_n_wc, &c->l_n_wp, &c->l_n_list, &c->l_field_new,
-                    &c->l_cand, &c->l_logit, &c->l_label, &c->tile_bits, &c->tile_wc, &c->tile_wp, &c->tile_list,
+                    &c->l_cand, &c->l_logit, &c->l_label,
                     &c->w_bits, &c->w_wc, &c->w_wp, &c->w_vert, &c->w_vnorm, &c->w_idx};
     for (DBuf* b : bufs) f(*b);
 }
@@ -228,12 +228,6 @@ pms_status pms::ensure_grid_buffers(pms_ctx* c, const pms_grid& g) {
     PMS_CUDA(c, c->bm.ensure(4 * W));
     PMS_CUDA(c, c->wcount.ensure(4 * W));
     PMS_CUDA(c, c->wprefix.ensure(4 * W));
-    // the band marking's tiles of the scalar grid: at most one per vertex
-    const size_t T = (size_t)g.sc_size + 1, TW = T / 32 + 2;
-    PMS_CUDA(c, c->tile_bits.ensure(4 * TW));
-    PMS_CUDA(c, c->tile_wc.ensure(4 * TW));
-    PMS_CUDA(c, c->tile_wp.ensure(4 * TW));
-    PMS_CUDA(c, c->tile_list.ensure(4 * T));
     return PMS_OK;
 }
 

@@ -77,7 +77,7 @@ struct Counters {
     uint32_t l_recheck;     // certified corners of valid cubes, evaluated exactly afterwards
     uint32_t n_items;       // work items (runs or tiles) of the last field launch
     uint32_t field_next;    // the next listed tile a warp of the field takes (zeroed with n_items)
-    uint32_t n_tiles;       // scalar-grid tiles the band marking visits
+    uint32_t band_next;     // the next tile a warp of the band marking takes
     uint32_t n_weld;        // vertices of the welded mesh (crossed grid edges)
     uint32_t n_df_total;    // generated + carried diffuse particles of a batched frame
     uint32_t mc_piece[kMaxMcPieces + 1];  // first cube of each streamed emission range, then nvalid
@@ -199,8 +199,8 @@ struct pms_ctx {
     pms::DBuf cell_count, cell_start, cell_info, surf_count, surf_start, big_cells;
     // anisotropy
     pms::DBuf slist, moments, aniso, nrm4, mean4, gdebug, nnb, cell_rad, cell_rec;
-    // band (and the tiles of the scalar grid its marking visits)
-    pms::DBuf bm0, bm, wcount, wprefix, vlist, tile_bits, tile_wc, tile_wp, tile_list;
+    // band
+    pms::DBuf bm0, bm, wcount, wprefix, vlist;
     // field and marching cubes
     pms::DBuf field, mc_case, mc_key, mc_off, valid, vert, vnorm, sval;
     // the field over the whole scalar grid, 0 off the band (the marching cubes' lookups);
