@@ -277,15 +277,14 @@ __global__ void __launch_bounds__(256) k_df_count(DiffuseParams dp, float4* __re
     }
 }
 
-__global__ void k_df_totals(const unsigned long long* __restrict__ total, Counters* __restrict__ cnt) {
-    const unsigned long long t = *total;
-    cnt->n_spawning = (uint32_t)(t >> 32);
-    cnt->n_generated = (uint32_t)(t & 0xffffffffull);
-}
-
 __global__ void __launch_bounds__(256) k_df_spawnlist(const unsigned long long* __restrict__ key,
                                                       const unsigned long long* __restrict__ off, uint32_t n,
-                                                      uint32_t* __restrict__ list) {
+                                                      Counters* __restrict__ cnt, uint32_t* __restrict__ list) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const unsigned long long t = cnt->df_total;          // the scan's total
+        cnt->n_spawning = (uint32_t)(t >> 32);
+        cnt->n_generated = (uint32_t)(t & 0xffffffffull);
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         if (key[i]) list[(uint32_t)(off[i] >> 32)] = i;
 }
@@ -700,12 +699,11 @@ static pms_status diffuse_front(pms_ctx* ctx, const KGrid& g, const DiffuseParam
                                             ctx->d_isdiff.as<unsigned long long>());
     PMS_LAUNCHED(ctx);
     if ((st = scan_u64(ctx, ctx->d_isdiff.as<unsigned long long>(), ctx->d_isdiffscan.as<unsigned long long>(), n,
-                       ctx->tmp.as<unsigned long long>())))
+                       &cnt->df_total)))
         return st;
-    k_df_totals<<<1, 1, 0, ctx->stream>>>(ctx->tmp.as<unsigned long long>(), cnt);
-    PMS_LAUNCHED(ctx);
     k_df_spawnlist<<<gb, 256, 0, ctx->stream>>>(ctx->d_isdiff.as<unsigned long long>(),
-                                                ctx->d_isdiffscan.as<unsigned long long>(), n, ctx->d_difflist.as<uint32_t>());
+                                                ctx->d_isdiffscan.as<unsigned long long>(), n, cnt,
+                                                ctx->d_difflist.as<uint32_t>());
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }

@@ -437,7 +437,6 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
               uint32_t* __restrict__ next, const uint32_t* __restrict__ list, const uint32_t* __restrict__ mask,
               const uint32_t* __restrict__ cell_start, const float* __restrict__ cell_rad,
               const uint32_t* __restrict__ skeys, const float4* __restrict__ spos, const float4* __restrict__ aniso,
-              const uint32_t* __restrict__ bm, const uint32_t* __restrict__ wprefix, float* __restrict__ field,
               float* __restrict__ fdense, Counters* __restrict__ cnt_w) {
     using T = FieldTile<K>;
     constexpr unsigned kAll = 0xffffffffu;
@@ -676,15 +675,10 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
                 }
             }
             if (staged) flush();
-            // values, in band order and over the scalar grid
             const uint32_t id = iz * rxy + iy * rx + ix;
 #pragma unroll
             for (int k = 0; k < K; ++k)
-                if (have[k]) {
-                    const uint32_t v = id + (uint32_t)k;
-                    if (field) field[wprefix[v >> 5] + (uint32_t)__popc(__ldg(&bm[v >> 5]) & ((1u << (v & 31u)) - 1u))] = sum[k];
-                    fdense[v] = sum[k];
-                }
+                if (have[k]) fdense[id + (uint32_t)k] = sum[k];
         }
     }
     if (lane == 0u && my_pairs) atomicAdd(&cnt_w->n_pairs, my_pairs);
@@ -711,7 +705,7 @@ size_t field_tile_bytes(const pms_grid& g, int vpt, uint64_t nv) {
 }
 
 template <int K>
-static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t n_host, float* out) {
+static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, uint64_t n_host) {
     const KGrid g = kgrid_of(ctx->grid);
     const pms_params& P = ctx->prm;
     FieldParams fp;
@@ -736,8 +730,8 @@ static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, const uint32_
     auto go = [&](auto kern) {
         kern<<<blocks, bt, 0, ctx->stream>>>(g, fp, td, cnt, &cnt->n_items, &cnt->field_next, list, mask,
                                              ctx->cell_start.as<uint32_t>(), ctx->cell_rad.as<float>(),
-                                             ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(), bm,
-                                             wprefix, out, ctx->fdense.as<float>(), cnt);
+                                             ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(),
+                                             ctx->fdense.as<float>(), cnt);
     };
     if (bt == 64) go(k_field_tiles<64, K>);
     else if (bt == 256) go(k_field_tiles<256, K>);
@@ -746,11 +740,10 @@ static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, const uint32_
     return PMS_OK;
 }
 
-pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t n_host, float* out) {
-    if ((uint64_t)n_host >= (1ull << kItemShift)) return pms_fail(ctx, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices");
-    if (ctx->tune.field_vpt == 1) return field_tiles_of<1>(ctx, bm, wprefix, n_host, out);
-    if (ctx->tune.field_vpt == 4) return field_tiles_of<4>(ctx, bm, wprefix, n_host, out);
-    return field_tiles_of<2>(ctx, bm, wprefix, n_host, out);
+pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, uint64_t n_host) {
+    if (ctx->tune.field_vpt == 1) return field_tiles_of<1>(ctx, bm, n_host);
+    if (ctx->tune.field_vpt == 4) return field_tiles_of<4>(ctx, bm, n_host);
+    return field_tiles_of<2>(ctx, bm, n_host);
 }
 
 // ---------------------------------------------------------------------------
@@ -864,7 +857,7 @@ pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t
 // the frame's first field evaluation: the dense field starts at 0 everywhere
 pms_status launch_field(pms_ctx* ctx) {
     PMS_CUDA(ctx, cudaMemsetAsync(ctx->fdense.p, 0, 4 * (size_t)ctx->grid.sc_size, ctx->stream));
-    return launch_field_bits(ctx, ctx->bm.as<uint32_t>(), ctx->wprefix.as<uint32_t>(), ctx->nv, ctx->field.as<float>());
+    return launch_field_bits(ctx, ctx->bm.as<uint32_t>(), ctx->nv_pending ? ctx->grid.sc_size : ctx->nv);
 }
 
 // field[t] = fdense[vlist[t]]: the band-order field of a vertex list whose values are all computed

@@ -579,8 +579,9 @@ __device__ __forceinline__ uint32_t shifted(const uint32_t* __restrict__ b, uint
 // cubes null: no prediction, N = U
 __global__ void __launch_bounds__(256) k_band_split(const uint32_t* __restrict__ cubes, const uint32_t* __restrict__ band,
                                                     uint32_t* __restrict__ e_bm, uint32_t* __restrict__ n_bm,
-                                                    uint32_t* __restrict__ e_wc, uint32_t* __restrict__ n_wc, uint64_t nwords,
+                                                    uint32_t* __restrict__ n_wc, uint32_t* __restrict__ n_exact, uint64_t nwords,
                                                     uint64_t nbits, uint64_t sy, uint64_t sz) {
+    uint32_t my_exact = 0u;
     for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t v = 0u;
         if (cubes)
@@ -591,49 +592,35 @@ __global__ void __launch_bounds__(256) k_band_split(const uint32_t* __restrict__
         const uint32_t e = u & v, n = u & ~v;
         e_bm[w] = e;
         n_bm[w] = n;
-        e_wc[w] = __popc(e);
+        my_exact += (uint32_t)__popc(e);
         n_wc[w] = __popc(n);
     }
+    const uint32_t tot = __reduce_add_sync(0xffffffffu, my_exact);
+    if ((threadIdx.x & 31u) == 0u && tot) atomicAdd(n_exact, tot);
 }
 
-// The certified corners of the valid cubes (compaction records {vertex id,
-// case, ...}): their bits move from `cert` to `recheck`, whose vertices are
-// then evaluated exactly, so that `cert` ends holding the band vertices whose
-// field is a placeholder.  A cube's corners lie in 4 rows of 2 neighbouring
-// vertices.
-__global__ void __launch_bounds__(256) k_recheck_bits(KGrid g, const Counters* __restrict__ cnt, const uint4* __restrict__ cube,
-                                                      uint32_t* __restrict__ cert, uint32_t* __restrict__ recheck) {
-    const uint32_t n = cnt->nvalid;
-    const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const uint32_t id = __ldg(&cube[t]).x;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const uint32_t c = id + (uint32_t)(r & 1) * rx + (uint32_t)(r >> 1) * rxy;   // corners c, c + 1
-            const uint32_t w = c >> 5, sh = c & 31u;
-            const uint32_t pair = (cert[w] >> sh) & (sh == 31u ? 1u : 3u);
-            const uint32_t hi = sh == 31u ? (cert[w + 1] & 1u) : 0u;
-            if (pair) atomicOr(&recheck[w], pair << sh);
-            if (hi) atomicOr(&recheck[w + 1], 1u);
+// The certified corners of the valid cubes: their bits move from `cert` to `recheck`, whose
+// vertices are then evaluated exactly, so that `cert` ends holding the band vertices whose
+// field is a placeholder.  A vertex is a valid cube's corner when one of the eight cubes
+// around it is valid.
+__global__ void __launch_bounds__(256) k_recheck_bits(const uint32_t* __restrict__ valid, uint32_t* __restrict__ cert,
+                                                      uint32_t* __restrict__ recheck, uint32_t* __restrict__ n_recheck,
+                                                      uint64_t nwords, uint64_t sy, uint64_t sz) {
+    uint32_t mine = 0u;
+    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t c = cert[w];
+        uint32_t r = 0u;
+        if (c) {
+            r = c & (valid[w] | shifted(valid, w, 1) | shifted(valid, w, sy) | shifted(valid, w, sy + 1) | shifted(valid, w, sz) |
+                     shifted(valid, w, sz + 1) | shifted(valid, w, sz + sy) | shifted(valid, w, sz + sy + 1));
             // those vertices get exact values: they leave the certified set
-            if (pair) atomicAnd(&cert[w], ~(pair << sh));
-            if (hi) atomicAnd(&cert[w + 1], ~1u);
+            if (r) cert[w] = c & ~r;
         }
+        recheck[w] = r;
+        mine += (uint32_t)__popc(r);
     }
-}
-
-// popcount per word of a bitmap
-__global__ void __launch_bounds__(256) k_popc(const uint32_t* __restrict__ b, uint32_t* __restrict__ wcount, uint64_t nwords) {
-    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x)
-        wcount[w] = __popc(b[w]);
-}
-
-// cube bitmap of the plain method's valid cubes (training labels)
-__global__ void __launch_bounds__(256) k_label_bits(const uint32_t* __restrict__ n_dev, const uint32_t* __restrict__ vlist,
-                                                    const unsigned long long* __restrict__ mc_key, uint32_t* __restrict__ lbm) {
-    const uint32_t n = *n_dev;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-        if (mc_key[t]) atomicOr(&lbm[vlist[t] >> 5], 1u << (vlist[t] & 31u));
+    const uint32_t tot = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31u) == 0u && tot) atomicAdd(n_recheck, tot);
 }
 
 // features of explicit cubes (bf16 bits, 64 per cube), for checks against the oracle
@@ -998,39 +985,21 @@ pms_status launch_predict(pms_ctx* ctx, int use_model, uint32_t* q, uint32_t* ca
     return PMS_OK;
 }
 
-pms_status launch_band_split(pms_ctx* ctx, const uint32_t* cubes, uint32_t* e_bm, uint32_t* n_bm, uint32_t* e_wc,
-                             uint32_t* n_wc) {
+pms_status launch_band_split(pms_ctx* ctx, const uint32_t* cubes, uint32_t* e_bm, uint32_t* n_bm, uint32_t* n_wc) {
     const KGrid g = kgrid_of(ctx->grid);
     const uint64_t nbits = g.sc_size, nwords = (nbits + 31) / 32;
     const uint64_t sy = g.scres[0], sz = (uint64_t)g.scres[0] * g.scres[1];
-    k_band_split<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(cubes, ctx->bm.as<uint32_t>(), e_bm, n_bm, e_wc, n_wc,
-                                                                 nwords, nbits, sy, sz);
+    k_band_split<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(cubes, ctx->bm.as<uint32_t>(), e_bm, n_bm, n_wc,
+                                                                 &ctx->counters.as<Counters>()->l_exact, nwords, nbits, sy, sz);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }
-
-pms_status launch_bits_list(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t* vlist);
 
 pms_status launch_recheck_bits(pms_ctx* ctx, uint32_t* cert, uint32_t* recheck) {
     const KGrid g = kgrid_of(ctx->grid);
-    Counters* cnt = ctx->counters.as<Counters>();
-    // ctx->nv bounds the valid cubes; the kernel reads their count
-    k_recheck_bits<<<grid_for(ctx->nv, 256), 256, 0, ctx->stream>>>(g, cnt, ctx->cube.as<uint4>(), cert, recheck);
-    PMS_LAUNCHED(ctx);
-    return PMS_OK;
-}
-
-pms_status launch_popc(pms_ctx* ctx, const uint32_t* b, uint32_t* wcount) {
-    const uint64_t nwords = ((uint64_t)ctx->grid.sc_size + 31) / 32;
-    k_popc<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(b, wcount, nwords);
-    PMS_LAUNCHED(ctx);
-    return PMS_OK;
-}
-
-pms_status launch_label_bits(pms_ctx* ctx, uint32_t* lbm) {
-    Counters* cnt = ctx->counters.as<Counters>();
-    k_label_bits<<<grid_for(ctx->nv, 256), 256, 0, ctx->stream>>>(&cnt->nv, ctx->vlist.as<uint32_t>(),
-                                                                   ctx->mc_key.as<unsigned long long>(), lbm);
+    const uint64_t nwords = ((uint64_t)g.sc_size + 31) / 32, sy = g.scres[0], sz = sy * g.scres[1];
+    k_recheck_bits<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(ctx->mc_valid.as<uint32_t>(), cert, recheck,
+                                                                   &ctx->counters.as<Counters>()->l_recheck, nwords, sy, sz);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }

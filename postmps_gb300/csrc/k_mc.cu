@@ -11,16 +11,18 @@
 // differences of the field, zero outside the grid and outside the band,
 // myCuda.cuh:259-289) and writes the triangle soup in table order.
 //
-// GB300 design: the field is read from the dense scalar-grid copy the field
-// kernel writes (0 off the band, so a normal's out-of-band neighbour reads 0
-// as in the reference); band membership comes from the band bitmap.  One scan
-// over packed 64-bit keys (valid << 32 | nvert) yields both offsets; the
-// compaction writes one 16-byte record per valid cube {vertex id, case, first
-// mesh vertex}, so the emission reads its inputs coalesced.  Each warp emits
-// 32 consecutive valid cubes: their mesh vertices are contiguous, so the warp
-// stages them in shared memory and writes whole lines (scattered 4-byte stores
-// from each cube would leave partial sectors for the memory to merge).  Tables
-// sit in constant memory.
+// GB300 design: classification works on bits.  One pass reads the field over the band and
+// keeps a bit per band vertex, field <= iso; a word of 32 cubes then takes its corners' band
+// and sign bits from eight shifted words each, so which cubes are valid is a few logical
+// operations, and only valid cubes (a quarter of the band's) look at their case.  One scan
+// over a 64-bit key per word (valid << 32 | mesh vertices) yields both offsets; the
+// compaction writes one 16-byte record per valid cube {vertex id, case, first mesh vertex},
+// so the emission reads its inputs coalesced.  The field is read from the dense scalar-grid
+// copy the field kernel writes (0 off the band, so a normal's out-of-band neighbour reads 0
+// as in the reference).  Each warp emits 32 consecutive valid cubes: their mesh vertices
+// are contiguous, so the warp stages them in shared memory and writes whole lines
+// (scattered 4-byte stores from each cube would leave partial sectors for the memory to
+// merge).
 #include "pms_internal.h"
 #include "k_common.cuh"
 
@@ -73,55 +75,149 @@ pms_status upload_mc_tables(pms_ctx* ctx) {
     return PMS_OK;
 }
 
-// detectValidSurfaceCubes (6-argument version)
-__global__ void __launch_bounds__(kThreads) k_mc_classify(KGrid g, float iso, const Counters* __restrict__ cnt,
-                                                          const uint32_t* __restrict__ vlist, const uint32_t* __restrict__ bm,
-                                                          const float* __restrict__ fdense, uint32_t* __restrict__ mc_case,
-                                                          unsigned long long* __restrict__ mc_key) {
+// detectValidSurfaceCubes (6-argument version), in four steps over the scalar grid's words
+// of 32 vertices.  A pass per band vertex (eight corner lookups in the bitmap and the field, a
+// case and a 64-bit key each), a scan over those keys and a compaction pass took 0.27 ms on
+// the crown 2M frame and needed the band as a list (0.07 ms); the words take 0.11 ms.
+
+// (1) le[w]: the band vertices of word w with field <= iso.  A warp takes 32 words, all lanes
+// reading the field of one word with a band vertex at a time, four in flight.
+__global__ void __launch_bounds__(256) k_mc_signs(uint64_t nwords, float iso, const uint32_t* __restrict__ bm,
+                                                  const float* __restrict__ fdense, uint32_t* __restrict__ le) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t w0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; w0 < nwords; w0 += step) {
+        const uint64_t w = w0 + lane;
+        const uint32_t b = w < nwords ? bm[w] : 0u;
+        uint32_t mine = 0u;
+        for (uint32_t todo = __ballot_sync(0xffffffffu, b != 0u); todo;) {
+            int i[4];
+            uint32_t bi[4];
+            float v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                i[k] = todo ? __ffs((int)todo) - 1 : -1;
+                todo &= todo - 1u;
+                bi[k] = __shfl_sync(0xffffffffu, b, i[k] < 0 ? 0 : i[k]);
+                // only band vertices are read (and no word past the grid has any)
+                const bool in = i[k] >= 0 && ((bi[k] >> lane) & 1u);
+                v[k] = in ? __ldg(&fdense[32u * (w0 + (uint32_t)i[k]) + lane]) : INFINITY;
+                bi[k] = in;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t s = __ballot_sync(0xffffffffu, bi[k] && v[k] <= iso);
+                if ((int)lane == i[k]) mine = s;
+            }
+        }
+        if (w < nwords) le[w] = mine;
+    }
+}
+
+// The bits at `bit` and `bit` + 1 onwards of a bitmap (0 past its end): corner offsets in
+// linear order, as getCornerIndex1Ds' uint32 arithmetic has them, row wrap included.
+__device__ __forceinline__ void corner_pair(const uint32_t* __restrict__ b, uint64_t nwords, uint64_t bit, uint32_t out[2]) {
+    const uint64_t w = bit >> 5;
+    const uint32_t sh = (uint32_t)(bit & 31u);
+    const uint32_t lo = w < nwords ? __ldg(&b[w]) : 0u, hi = w + 1 < nwords ? __ldg(&b[w + 1]) : 0u;
+    out[0] = __funnelshift_rc(lo, hi, sh);
+    out[1] = __funnelshift_rc(lo, hi, sh + 1u);
+}
+// the words of the eight corners of 32 cubes, in corner order
+__device__ __forceinline__ void corner_words(const uint32_t* __restrict__ b, uint64_t nwords, uint64_t w, uint64_t rx, uint64_t rxy,
+                                             uint32_t out[8]) {
+    uint32_t p[2];
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+            corner_pair(b, nwords, 32u * w + (y ? rx : 0u) + (z ? rxy : 0u), p);
+            out[corner_at(0, y, z)] = p[0];
+            out[corner_at(1, y, z)] = p[1];
+        }
+}
+__device__ __forceinline__ uint32_t cube_case(const uint32_t le[8], uint32_t bit) {
+    uint32_t cs = 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) cs |= ((le[k] >> bit) & 1u) << k;
+    return cs;
+}
+
+// (2) the valid cubes of each word (all corners in the band, both signs among them), and
+// their number and mesh vertices as the scan's key
+__global__ void __launch_bounds__(256) k_mc_count(uint64_t nwords, uint64_t rx, uint64_t rxy, const uint32_t* __restrict__ bm,
+                                                  const uint32_t* __restrict__ le, uint32_t* __restrict__ valid,
+                                                  unsigned long long* __restrict__ key) {
+    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t v = 0u, nvert = 0u;
+        if (bm[w]) {
+            uint32_t c[8];
+            corner_words(bm, nwords, w, rx, rxy, c);
+            v = c[0] & c[1] & c[2] & c[3] & c[4] & c[5] & c[6] & c[7];
+            if (v) {
+                corner_words(le, nwords, w, rx, rxy, c);
+                v &= (c[0] | c[1] | c[2] | c[3] | c[4] | c[5] | c[6] | c[7]) & ~(c[0] & c[1] & c[2] & c[3] & c[4] & c[5] & c[6] & c[7]);
+                for (uint32_t m = v; m; m &= m - 1u) {
+                    const uint32_t bit = (uint32_t)(__ffs((int)m) - 1), n = __ldg(&g_case[cube_case(c, bit)]) >> 16;
+                    if (n) nvert += n;
+                    else v &= ~(1u << bit);                // a case without triangles
+                }
+            }
+        }
+        valid[w] = v;
+        key[w] = (unsigned long long)__popc(v) << 32 | nvert;
+    }
+}
+
+// (4) compactValidSurfaceCubes: the emission's per-cube records; unpacks the scanned total
+// {valid cubes << 32 | mesh vertices} into the counters the later kernels read
+__global__ void __launch_bounds__(256) k_mc_compact(uint64_t nwords, uint64_t rx, uint64_t rxy, const uint32_t* __restrict__ le,
+                                                    const uint32_t* __restrict__ valid,
+                                                    const unsigned long long* __restrict__ off, Counters* __restrict__ cnt,
+                                                    uint4* __restrict__ cube) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const unsigned long long t = cnt->mc_total;
+        cnt->nvalid = (uint32_t)(t >> 32);
+        cnt->nmesh = t & 0xffffffffull;
+    }
+    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t v = valid[w];
+        if (!v) continue;
+        uint32_t c[8];
+        corner_words(le, nwords, w, rx, rxy, c);
+        const unsigned long long o = off[w];
+        uint32_t k = (uint32_t)(o >> 32), base = (uint32_t)(o & 0xffffffffull);
+        for (uint32_t m = v; m; m &= m - 1u) {
+            const uint32_t bit = (uint32_t)(__ffs((int)m) - 1), cs = cube_case(c, bit);
+            cube[k++] = make_uint4((uint32_t)(32u * w) + bit, cs, base, 0u);
+            base += __ldg(&g_case[cs]) >> 16;
+        }
+    }
+}
+
+// the case and mesh vertices of every band vertex's cube, for parity tests (case 0 when not
+// all corners are band vertices)
+__global__ void __launch_bounds__(kThreads) k_mc_cases(KGrid g, float iso, const Counters* __restrict__ cnt,
+                                                       const uint32_t* __restrict__ vlist, const uint32_t* __restrict__ bm,
+                                                       const float* __restrict__ fdense, uint32_t* __restrict__ mc_case,
+                                                       uint32_t* __restrict__ mc_nvert) {
     const uint32_t nv = cnt->nv;
     const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
     const uint64_t nbits = g.sc_size;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nv; t += gridDim.x * blockDim.x) {
         const uint32_t id = vlist[t];
-        const uint32_t z = id / rxy, rem = id - z * rxy, y = rem / rx, x = rem - y * rx;
-        uint32_t cs = 0, nvert = 0;
+        uint32_t cs = 0;
         bool all = true;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            // uint32 corner index as getCornerIndex1Ds computes it
-            const uint32_t cid = (z + corner_off(k, 2)) * rxy + (y + corner_off(k, 1)) * rx + (x + corner_off(k, 0));
+            const uint32_t cid = id + corner_off(k, 2) * rxy + corner_off(k, 1) * rx + corner_off(k, 0);
             const bool in = bit_get(bm, nbits, cid);
             all = all && in;
             if (in) cs |= (__ldg(&fdense[cid]) <= iso ? 1u : 0u) << k;
         }
-        if (all) nvert = __ldg(&g_case[cs]) >> 16;
-        else cs = 0;
-        mc_case[t] = cs;
-        mc_key[t] = nvert ? ((1ull << 32) | nvert) : 0ull;
+        if (mc_case) mc_case[t] = all ? cs : 0u;
+        if (mc_nvert) mc_nvert[t] = all ? __ldg(&g_case[cs]) >> 16 : 0u;
     }
-}
-
-// unpack the scanned total {valid cubes << 32 | mesh vertices} into the counters
-__global__ void k_mc_totals(const unsigned long long* __restrict__ total, Counters* __restrict__ cnt) {
-    const unsigned long long t = *total;
-    cnt->nvalid = (uint32_t)(t >> 32);
-    cnt->nmesh = t & 0xffffffffull;
-}
-
-// compactValidSurfaceCubes, plus the emission's per-cube record
-__global__ void __launch_bounds__(256) k_mc_compact(const Counters* __restrict__ cnt,
-                                                    const unsigned long long* __restrict__ mc_key,
-                                                    const unsigned long long* __restrict__ mc_off,
-                                                    const uint32_t* __restrict__ vlist, const uint32_t* __restrict__ mc_case,
-                                                    uint32_t* __restrict__ valid, uint4* __restrict__ cube) {
-    const uint32_t nv = cnt->nv;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nv; t += gridDim.x * blockDim.x)
-        if (mc_key[t]) {
-            const unsigned long long off = mc_off[t];
-            const uint32_t k = (uint32_t)(off >> 32);
-            valid[k] = t;
-            cube[k] = make_uint4(vlist[t], mc_case[t], (uint32_t)(off & 0xffffffffull), 0u);
-        }
 }
 
 // field at scalar-grid vertex (x, y, z): 0 outside the grid and off the band
@@ -250,33 +346,40 @@ __global__ void __launch_bounds__(kThreads) k_mc_emit(KGrid g, float iso, Counte
     }
 }
 
-pms_status launch_mc_cases(pms_ctx* ctx) {
+pms_status launch_mc_count(pms_ctx* ctx) {
     const KGrid g = kgrid_of(ctx->grid);
     Counters* cnt = ctx->counters.as<Counters>();
-    k_mc_classify<<<grid_for(ctx->nv, kThreads), kThreads, 0, ctx->stream>>>(
-        g, ctx->prm.iso_value, cnt, ctx->vlist.as<uint32_t>(), ctx->bm.as<uint32_t>(), ctx->fdense.as<float>(),
-        ctx->mc_case.as<uint32_t>(), ctx->mc_key.as<unsigned long long>());
+    const uint64_t nwords = ((uint64_t)g.sc_size + 31) / 32, rx = g.scres[0], rxy = rx * g.scres[1];
+    k_mc_signs<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(nwords, ctx->prm.iso_value, ctx->bm.as<uint32_t>(),
+                                                               ctx->fdense.as<float>(), ctx->mc_le.as<uint32_t>());
+    PMS_LAUNCHED(ctx);
+    k_mc_count<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(nwords, rx, rxy, ctx->bm.as<uint32_t>(), ctx->mc_le.as<uint32_t>(),
+                                                               ctx->mc_valid.as<uint32_t>(), ctx->mc_key.as<unsigned long long>());
+    PMS_LAUNCHED(ctx);
+    return scan_u64(ctx, ctx->mc_key.as<unsigned long long>(), ctx->mc_off.as<unsigned long long>(), nwords, &cnt->mc_total);
+}
+
+pms_status launch_mc_compact(pms_ctx* ctx) {
+    const KGrid g = kgrid_of(ctx->grid);
+    const uint64_t nwords = ((uint64_t)g.sc_size + 31) / 32, rx = g.scres[0], rxy = rx * g.scres[1];
+    k_mc_compact<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(nwords, rx, rxy, ctx->mc_le.as<uint32_t>(),
+                                                                 ctx->mc_valid.as<uint32_t>(),
+                                                                 ctx->mc_off.as<unsigned long long>(),
+                                                                 ctx->counters.as<Counters>(), ctx->cube.as<uint4>());
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }
 
-pms_status launch_mc_compact(pms_ctx* ctx) {
-    Counters* cnt = ctx->counters.as<Counters>();
-    // ctx->nv may be a bound (batched frames): the scan stops at the device count
-    pms_status st = scan_u64(ctx, ctx->mc_key.as<unsigned long long>(), ctx->mc_off.as<unsigned long long>(), ctx->nv,
-                             ctx->tmp.as<unsigned long long>(), &cnt->nv);
-    if (st != PMS_OK) return st;
-    k_mc_totals<<<1, 1, 0, ctx->stream>>>(ctx->tmp.as<unsigned long long>(), cnt);
-    PMS_LAUNCHED(ctx);
-    k_mc_compact<<<grid_for(ctx->nv, 256), 256, 0, ctx->stream>>>(
-        cnt, ctx->mc_key.as<unsigned long long>(), ctx->mc_off.as<unsigned long long>(), ctx->vlist.as<uint32_t>(),
-        ctx->mc_case.as<uint32_t>(), ctx->valid.as<uint32_t>(), ctx->cube.as<uint4>());
+pms_status launch_mc_cases(pms_ctx* ctx, uint32_t nv, uint32_t* mc_case, uint32_t* mc_nvert) {
+    k_mc_cases<<<grid_for(nv, kThreads), kThreads, 0, ctx->stream>>>(
+        kgrid_of(ctx->grid), ctx->prm.iso_value, ctx->counters.as<Counters>(), ctx->vlist.as<uint32_t>(),
+        ctx->bm.as<uint32_t>(), ctx->fdense.as<float>(), mc_case, mc_nvert);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }
 
 pms_status launch_mc_classify(pms_ctx* ctx) {
-    pms_status st = launch_mc_cases(ctx);
+    pms_status st = launch_mc_count(ctx);
     return st ? st : launch_mc_compact(ctx);
 }
 

@@ -39,16 +39,15 @@ pms_status launch_coarse_counts(pms_ctx* ctx);
 pms_status launch_predict(pms_ctx* ctx, int use_model, uint32_t* q, uint32_t* cand, float* logit, uint32_t cand_cap);
 // the plain band (ctx->bm) split into the corners of the cubes of a cube bitmap (E,
 // evaluated exactly at once) and the rest (N, certified); cubes null: E empty
-pms_status launch_band_split(pms_ctx* ctx, const uint32_t* cubes, uint32_t* e_bm, uint32_t* n_bm, uint32_t* e_wc,
-                             uint32_t* n_wc);
+// (Counters::l_exact receives E's size, n_wc the words' counts of N)
+pms_status launch_band_split(pms_ctx* ctx, const uint32_t* cubes, uint32_t* e_bm, uint32_t* n_bm, uint32_t* n_wc);
 // the certified corners (bits of cert) of the classified valid cubes move to recheck
+// (Counters::l_recheck counts them)
 pms_status launch_recheck_bits(pms_ctx* ctx, uint32_t* cert, uint32_t* recheck);
-pms_status launch_popc(pms_ctx* ctx, const uint32_t* b, uint32_t* wcount);
-pms_status launch_label_bits(pms_ctx* ctx, uint32_t* lbm);
-// the learned band after the plain band (ctx->bm, ctx->vlist; ctx->nv its count, or a
+// the learned band after the plain band (ctx->bm; ctx->nv its count, or a
 // bound for batched frames): prediction and split, then the field stage (exact field
-// at E, certification of N, classification, exact field at the rechecked corners,
-// band-order field); no host synchronisation
+// at E, certification of N, classification, exact field at the rechecked corners); no
+// host synchronisation
 pms_status ensure_learned_buffers(pms_ctx* ctx, uint64_t sc_size, uint32_t nv);
 pms_status learned_split(pms_ctx* ctx, bool predict);
 pms_status learned_field(pms_ctx* ctx);

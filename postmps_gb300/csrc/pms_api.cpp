@@ -56,14 +56,14 @@ static void for_each_dbuf(pms_ctx* c, F f) {
     DBuf* bufs[] = {&c->in_pos, &c->in_vel, &c->in_rho, &c->keys, &c->slot, &c->order, &c->skeys, &c->spos,
                     &c->svel, &c->rho, &c->cell_count, &c->cell_start, &c->cell_info, &c->surf_count,
                     &c->surf_start, &c->big_cells, &c->slist, &c->moments, &c->cell_rad, &c->cell_rec, &c->aniso, &c->nrm4, &c->mean4, &c->gdebug,
-                    &c->nnb, &c->bm0, &c->bm, &c->wcount, &c->wprefix, &c->vlist, &c->field, &c->mc_case,
-                    &c->mc_key, &c->mc_off, &c->valid, &c->fdense, &c->cube, &c->fitems, &c->fitem_cnt, &c->fitem_off, &c->ftiles, &c->vert, &c->vnorm, &c->sval, &c->d_isfree, &c->d_freescan,
+                    &c->nnb, &c->bm0, &c->bm, &c->wcount, &c->wprefix, &c->vlist, &c->field, &c->mc_le,
+                    &c->mc_valid, &c->mc_key, &c->mc_off, &c->fdense, &c->cube, &c->fitems, &c->fitem_cnt, &c->fitem_off, &c->ftiles, &c->vert, &c->vnorm, &c->sval, &c->d_isfree, &c->d_freescan,
                     &c->d_freelist, &c->d_pot, &c->d_num, &c->d_numscan, &c->d_isdiff, &c->d_isdiffscan,
                     &c->d_difflist, &c->d_gen, &c->d_old, &c->d_all, &c->d_rand, &c->d_typescan,
                     &c->d_nrm_free, &c->d_tkey, &c->d_tscan, &c->d_perm, &c->counters, &c->scan.partial, &c->tmp,
                     &c->df_scan.partial, &c->df_tmp,
-                    &c->l_dens, &c->l_clist, &c->l_counts, &c->l_model, &c->l_q, &c->l_cert, &c->l_e_bm, &c->l_e_wc,
-                    &c->l_e_wp, &c->l_e_list, &c->l_n_bm, &c->l_n_wc, &c->l_n_wp, &c->l_n_list, &c->l_field_new,
+                    &c->l_dens, &c->l_clist, &c->l_counts, &c->l_model, &c->l_q, &c->l_cert, &c->l_e_bm,
+                    &c->l_e_list, &c->l_n_bm, &c->l_n_wc, &c->l_n_wp, &c->l_n_list, &c->l_field_new,
                     &c->l_cand, &c->l_logit, &c->l_label,
                     &c->w_bits, &c->w_wc, &c->w_wp, &c->w_vert, &c->w_vnorm, &c->w_idx};
     for (DBuf* b : bufs) f(*b);
@@ -228,6 +228,10 @@ pms_status pms::ensure_grid_buffers(pms_ctx* c, const pms_grid& g) {
     PMS_CUDA(c, c->bm.ensure(4 * W));
     PMS_CUDA(c, c->wcount.ensure(4 * W));
     PMS_CUDA(c, c->wprefix.ensure(4 * W));
+    PMS_CUDA(c, c->mc_le.ensure(4 * W));
+    PMS_CUDA(c, c->mc_valid.ensure(4 * W));
+    PMS_CUDA(c, c->mc_key.ensure(8 * W));
+    PMS_CUDA(c, c->mc_off.ensure(8 * W));
     return PMS_OK;
 }
 
@@ -237,16 +241,9 @@ void mark_stage(pms_ctx* c, int boundary);
 pms_status plain_band(pms_ctx* c);
 }  // namespace pms
 
-// the band's size changes from frame to frame: its buffers grow with headroom
+// a record per valid cube (at most nv): their number changes from frame to frame, so with headroom
 pms_status pms::ensure_band_buffers(pms_ctx* c, uint32_t nv) {
-    const size_t V = nv ? nv : 1;
-    PMS_CUDA(c, c->vlist.ensure_grow(4 * V));
-    PMS_CUDA(c, c->field.ensure_grow(4 * V));
-    PMS_CUDA(c, c->mc_case.ensure_grow(4 * V));
-    PMS_CUDA(c, c->mc_key.ensure_grow(8 * V));
-    PMS_CUDA(c, c->mc_off.ensure_grow(8 * V));
-    PMS_CUDA(c, c->valid.ensure_grow(4 * V));
-    PMS_CUDA(c, c->cube.ensure_grow(16 * V));
+    PMS_CUDA(c, c->cube.ensure_grow(16 * (size_t)(nv ? nv : 1)));
     return PMS_OK;
 }
 
@@ -367,6 +364,7 @@ static void begin_frame(pms_ctx* c, uint32_t n) {
     c->l_ncand = c->l_npred = c->l_nexact = c->l_ncert = c->l_nrecheck = 0;
     c->ns = c->nv = c->nvalid = 0;
     c->nmesh = 0;
+    c->nv_pending = false;
     for (int i = 0; i < kNumStages; ++i) c->ev_recorded[i] = false;
 }
 
@@ -544,37 +542,52 @@ extern "C" pms_status pms_anisotropy(pms_ctx* c) {
     return PMS_OK;
 }
 
-// The plain band's bitmap, count and ascending vertex list (one synchronisation).
+// The band's size on the host, from counters just synchronised.
+static pms_status take_band_size(pms_ctx* c) {
+    pms_status st = check_device_errors(c);
+    if (st) return st;
+    c->ns = c->h_counters->ns;
+    c->nv = c->h_counters->nv;
+    c->nv_pending = false;
+    if (c->nv >= (1u << 29)) return pms_fail(c, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices");
+    return PMS_OK;
+}
+
+// The plain band's bitmap and count (one synchronisation).
 pms_status pms::plain_band(pms_ctx* c) {
     pms_status st;
     if ((st = launch_band(c))) return st;
     if ((st = sync_counters(c))) return st;
-    if ((st = check_device_errors(c))) return st;
-    c->ns = c->h_counters->ns;
-    c->nv = c->h_counters->nv;
-    if ((st = ensure_band(c, c->nv))) return st;
-    return launch_band_list(c);
+    if ((st = take_band_size(c))) return st;
+    return ensure_band(c, c->nv);
+}
+
+// The band stage; inside a frame its size stays on the device (defer) until the marching
+// cubes synchronise for theirs: nothing before them is sized by it.
+static pms_status band_stage(pms_ctx* c, bool defer) {
+    c->band_learned = c->mc_classified = c->mc_compacted = false;
+    c->l_ncand = c->l_npred = c->l_nexact = c->l_ncert = c->l_nrecheck = 0;
+    if (c->n == 0) { c->nv = 0; c->have_band = true; return PMS_OK; }
+    pms_status st = defer ? launch_band(c) : plain_band(c);
+    if (st) return st;
+    c->nv_pending = defer;
+    c->have_band = true;
+    mark(c, kStageBand + 1);
+    return PMS_OK;
 }
 
 extern "C" pms_status pms_band(pms_ctx* c) {
     if (!c) return PMS_ERR_INVALID_ARGUMENT;
     if (!c->have_aniso) return pms_fail(c, PMS_ERR_STATE, "pms_band before pms_anisotropy");
     cudaSetDevice(c->device);
-    c->band_learned = c->mc_classified = c->mc_compacted = false;
-    c->l_ncand = c->l_npred = c->l_nexact = c->l_ncert = c->l_nrecheck = 0;
-    if (c->n == 0) { c->nv = 0; c->have_band = true; return PMS_OK; }
-    pms_status st;
-    if ((st = plain_band(c))) return st;
-    c->have_band = true;
-    mark(c, kStageBand + 1);
-    return PMS_OK;
+    return band_stage(c, false);
 }
 
 extern "C" pms_status pms_field(pms_ctx* c) {
     if (!c) return PMS_ERR_INVALID_ARGUMENT;
     if (!c->have_band) return pms_fail(c, PMS_ERR_STATE, "pms_field before pms_band");
     cudaSetDevice(c->device);
-    if (c->nv) { pms_status st = launch_field(c); if (st) return st; }
+    if (c->nv || c->nv_pending) { pms_status st = launch_field(c); if (st) return st; }
     c->have_field = true;
     mark(c, kStageField + 1);
     return PMS_OK;
@@ -588,16 +601,22 @@ extern "C" pms_status pms_marching_cubes(pms_ctx* c) {
     c->nmesh = 0;
     c->have_weld = false;
     int slot = -1;                     // the frame's record in the streamed-mesh queue
-    if (c->nv) {
+    if (c->nv || c->nv_pending) {
         pms_status st;
-        // the learned band's last border check already computed the final vertex set's cases
-        if (!c->mc_classified && (st = launch_mc_cases(c))) return st;
+        // the learned band has classified already
+        if (!c->mc_classified && (st = launch_mc_count(c))) return st;
         if (!(c->mc_classified && c->mc_compacted)) {
-            if ((st = launch_mc_compact(c))) return st;
             if ((st = sync_counters(c))) return st;
+            if (c->nv_pending && (st = take_band_size(c))) return st;
+            const uint64_t total = c->h_counters->mc_total;
+            if ((st = ensure_band(c, (uint32_t)(total >> 32)))) return st;
+            if ((st = launch_mc_compact(c))) return st;
+            c->nvalid = (uint32_t)(total >> 32);
+            c->nmesh = total & 0xffffffffull;
+        } else {
+            c->nvalid = c->h_counters->nvalid;
+            c->nmesh = c->h_counters->nmesh;
         }
-        c->nvalid = c->h_counters->nvalid;
-        c->nmesh = c->h_counters->nmesh;
         const size_t M = c->nmesh ? c->nmesh : 1;
         // earlier frames' meshes may still be on their way to the host: a buffer that
         // grows waits for them on the host (its old allocation is freed), the emission
@@ -673,7 +692,7 @@ extern "C" pms_status pms_download_scalar_values(pms_ctx* c, float* vel_xyz, flo
 extern "C" pms_status pms_surface(pms_ctx* c) {
     pms_status st;
     if ((st = pms_anisotropy(c))) return st;
-    if ((st = pms_band(c))) return st;
+    if ((st = band_stage(c, true))) return st;
     if ((st = pms_field(c))) return st;
     return pms_marching_cubes(c);
 }
@@ -718,8 +737,8 @@ struct DiffuseJoin {
 // depends only on the grid and the anisotropy pass, and the surface stages only on
 // those too, so after the anisotropy the diffuse parts run on a stream of their own
 // beside the band, field and marching cubes.  Each part is issued where the surface
-// chain has a long stretch of work queued: the front before the band's
-// synchronisation, the tail after the field is queued, the finish after the emission.
+// chain has a long stretch of work queued: the front before the band, the tail after the
+// field is queued, the finish after the emission.
 // Results are those of the stages one after the other (no stage reads what the other
 // chain writes; counters are separate fields, errors are OR-ed).
 static pms_status run_frame_overlapped(pms_ctx* c) {
@@ -743,7 +762,7 @@ static pms_status run_frame_overlapped(pms_ctx* c) {
     if (c->band_mode != PMS_BAND_PLAIN) {
         if ((st = pms_band_learned(c))) return st;
     } else {
-        if ((st = pms_band(c))) return st;
+        if ((st = band_stage(c, true))) return st;
         if ((st = pms_field(c))) return st;
     }
     {
@@ -1040,22 +1059,24 @@ extern "C" pms_status pms_debug_download(pms_ctx* c, int id, void* dst, uint64_t
             put(v.data(), 4 * v.size());
             break;
         }
-        case PMS_ARRAY_BAND_LIST: case PMS_ARRAY_FIELD: case PMS_ARRAY_CUBE_CASE: {
+        case PMS_ARRAY_BAND_LIST: case PMS_ARRAY_FIELD: case PMS_ARRAY_CUBE_CASE: case PMS_ARRAY_CUBE_NVERT: {
             const bool ok = id == PMS_ARRAY_BAND_LIST ? c->have_band : id == PMS_ARRAY_FIELD ? c->have_field : c->have_mc;
             if (!ok) return PMS_ERR_STATE;
-            const DBuf& b = id == PMS_ARRAY_BAND_LIST ? c->vlist : id == PMS_ARRAY_FIELD ? c->field : c->mc_case;
+            // the stages keep the band as bits and the field over the grid: the band-order arrays are made here
+            if (nv) {
+                PMS_CUDA(c, c->vlist.ensure(4 * (size_t)nv));
+                PMS_CUDA(c, c->field.ensure(4 * (size_t)nv));
+                if ((st = launch_band_list(c))) return st;
+                uint32_t* out = c->field.as<uint32_t>();
+                if (id == PMS_ARRAY_FIELD)
+                    st = launch_field_gather(c, c->vlist.as<uint32_t>(), &c->counters.as<Counters>()->nv, nv, c->field.as<float>());
+                else if (id != PMS_ARRAY_BAND_LIST)
+                    st = launch_mc_cases(c, nv, id == PMS_ARRAY_CUBE_CASE ? out : nullptr, id == PMS_ARRAY_CUBE_NVERT ? out : nullptr);
+                if (st) return st;
+            }
             std::vector<uint32_t> v;
-            if ((st = d2h(c, v, b.p, nv))) return st;
-            put(v.data(), 4 * v.size());
-            break;
-        }
-        case PMS_ARRAY_CUBE_NVERT: {
-            if (!c->have_mc) return PMS_ERR_STATE;
-            std::vector<unsigned long long> v;
-            if ((st = d2h(c, v, c->mc_key.p, nv))) return st;
-            std::vector<uint32_t> o(nv);
-            for (size_t i = 0; i < nv; ++i) o[i] = (uint32_t)(v[i] & 0xffffffffull);
-            put(o.data(), 4 * o.size());
+            if ((st = d2h(c, v, id == PMS_ARRAY_BAND_LIST ? c->vlist.p : c->field.p, nv))) return st;
+            put(v.data(), 4 * (size_t)nv);
             break;
         }
         default: {

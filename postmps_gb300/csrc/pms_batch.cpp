@@ -187,12 +187,10 @@ static pms_status capture_frame(pms_ctx* c, BatchState* b, uint32_t f, int band,
     if (fork) PMS_CUDA(c, cudaEventRecord(fork, c->stream));
     if (band) {
         if ((st = launch_band(c))) return st;
-        if ((st = launch_band_list(c))) return st;
         if ((st = learned_split(c, band == 1))) return st;
         if ((st = learned_field(c))) return st;
     } else {
         if ((st = launch_band(c))) return st;
-        if ((st = launch_band_list(c))) return st;
         if ((st = launch_field(c))) return st;
         if ((st = launch_mc_classify(c))) return st;
     }

@@ -54,6 +54,8 @@ struct Counters {
     uint32_t nv;            // band vertices
     uint32_t nvalid;        // valid cubes
     unsigned long long nmesh;  // mesh vertices
+    unsigned long long mc_total;  // the marching cubes' scan total, valid cubes << 32 | mesh vertices
+    unsigned long long df_total;  // the spawn counts' scan total, spawning << 32 | generated
     unsigned long long n_pairs;  // (vertex, particle) pairs the field launches evaluated
     uint32_t n_fp64;        // covariances solved in FP64
     uint32_t n_big_cells;   // cells with more particles than the per-thread sort handles
@@ -191,6 +193,7 @@ struct pms_ctx {
     // host mirrors of device counters, valid after the stage that syncs
     uint32_t ns = 0, nv = 0, nvalid = 0;
     uint64_t nmesh = 0;
+    bool nv_pending = false;     // nv is on the device: the marching cubes' synchronisation reads it
 
     // particle inputs
     pms::DBuf in_pos, in_vel, in_rho;
@@ -202,7 +205,9 @@ struct pms_ctx {
     // band
     pms::DBuf bm0, bm, wcount, wprefix, vlist;
     // field and marching cubes
-    pms::DBuf field, mc_case, mc_key, mc_off, valid, vert, vnorm, sval;
+    // (field: the band-order copy, made for debug downloads and tests; mc_*: per word of the
+    // scalar grid the band vertices at or below iso, the valid cubes, their key and its scan)
+    pms::DBuf field, mc_le, mc_valid, mc_key, mc_off, vert, vnorm, sval;
     // the field over the whole scalar grid, 0 off the band (the marching cubes' lookups);
     // per valid cube {vertex id, case, first mesh vertex, 0}
     pms::DBuf fdense, cube;
@@ -223,8 +228,9 @@ struct pms_ctx {
     // learned band: coarse counts, model, cube bitmaps, merge buffers, training data
     pms::DBuf l_dens, l_clist;   // bf16 coarse density pairs (padded grid), candidate cube records
     // l_q: predicted cubes; l_cert: certified vertices; E / N: vertices evaluated exactly first /
-    // certified (bitmaps, popcounts, prefixes, lists); the rechecked corners reuse E's buffers
-    pms::DBuf l_counts, l_model, l_q, l_cert, l_e_bm, l_e_wc, l_e_wp, l_e_list, l_n_bm, l_n_wc, l_n_wp, l_n_list,
+    // certified (bitmaps; N's popcounts, prefixes and list); the rechecked corners reuse E's bitmap
+    // (l_e_list: scratch of the candidate downloads)
+    pms::DBuf l_counts, l_model, l_q, l_cert, l_e_bm, l_e_list, l_n_bm, l_n_wc, l_n_wp, l_n_list,
               l_field_new, l_cand, l_logit, l_label;
     bool have_model = false, band_learned = false, mc_classified = false, mc_compacted = false;
     // polls + 1 of the first bounded wait on the tensor cores (0: the default bound)
@@ -323,17 +329,19 @@ pms_status launch_field(pms_ctx* ctx);
 pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, uint32_t* cert,
                              uint32_t* n_cert);
 // exact field at the vertices of a bitmap over the scalar grid (n_host: a bound of their
-// number), into fdense and, unless null, in bitmap order into out (wprefix: the words' ranks)
-pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t n_host, float* out);
+// number), into fdense
+pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, uint64_t n_host);
 // bytes of the tile list such a launch needs (field_vpt vertices per lane)
 size_t field_tile_bytes(const pms_grid& g, int vpt, uint64_t nv);
 pms_status launch_field_gather(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, float* out);
 // ascending list of the set bits of a bitmap over the scalar grid
 pms_status launch_bits_list(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t* vlist);
-// marching-cube cases of the band vertices, then the scan and compaction; classify = both
-pms_status launch_mc_cases(pms_ctx* ctx);
+// the valid cubes per word and their scan (Counters::mc_total); then the compaction; classify = both
+pms_status launch_mc_count(pms_ctx* ctx);
 pms_status launch_mc_compact(pms_ctx* ctx);
 pms_status launch_mc_classify(pms_ctx* ctx);
+// case and / or vertex count of every band vertex's cube (vlist made before)
+pms_status launch_mc_cases(pms_ctx* ctx, uint32_t nv, uint32_t* mc_case, uint32_t* mc_nvert);
 // the mesh in `pieces` vertex ranges [nmesh * q / pieces, nmesh * (q + 1) / pieces): the first
 // cube of each range into Counters::mc_piece (pieces <= kMaxMcPieces)
 pms_status launch_mc_piece_bounds(pms_ctx* ctx, uint32_t pieces);

@@ -78,14 +78,13 @@ extern "C" pms_status pms_load_band_model(const char* path, pms_band_model* out)
 // of at most nv of them.
 pms_status pms::ensure_learned_buffers(pms_ctx* c, uint64_t sc_size, uint32_t nv) {
     const uint64_t W = (sc_size + 31) / 32 + 1;
-    for (DBuf* d : {&c->l_q, &c->l_cert, &c->l_e_bm, &c->l_e_wc, &c->l_e_wp, &c->l_n_bm, &c->l_n_wc, &c->l_n_wp})
-        PMS_CUDA(c, d->ensure(4 * W));
-    for (DBuf* d : {&c->l_e_list, &c->l_n_list}) PMS_CUDA(c, d->ensure(4 * ((size_t)nv + 1)));
+    for (DBuf* d : {&c->l_q, &c->l_cert, &c->l_e_bm, &c->l_n_bm, &c->l_n_wc, &c->l_n_wp}) PMS_CUDA(c, d->ensure(4 * W));
+    PMS_CUDA(c, c->l_n_list.ensure(4 * ((size_t)nv + 1)));
     return PMS_OK;
 }
 
 // The network's prediction (when asked) and the split of the plain band into the
-// corners of predicted cubes E and the rest N, both as ascending lists.
+// corners of predicted cubes E and the rest N, which also as an ascending list.
 pms_status pms::learned_split(pms_ctx* c, bool predict) {
     Counters* cnt = c->counters.as<Counters>();
     const uint64_t W = words_of(c);
@@ -97,18 +96,16 @@ pms_status pms::learned_split(pms_ctx* c, bool predict) {
         if ((st = launch_predict(c, 1, c->l_q.as<uint32_t>(), nullptr, nullptr, 0))) return st;
     }
     if ((st = launch_band_split(c, predict ? c->l_q.as<uint32_t>() : nullptr, c->l_e_bm.as<uint32_t>(),
-                                c->l_n_bm.as<uint32_t>(), c->l_e_wc.as<uint32_t>(), c->l_n_wc.as<uint32_t>())))
+                                c->l_n_bm.as<uint32_t>(), c->l_n_wc.as<uint32_t>())))
         return st;
-    if ((st = scan_u32(c, c->l_e_wc.as<uint32_t>(), c->l_e_wp.as<uint32_t>(), W, &cnt->l_exact))) return st;
     if ((st = scan_u32(c, c->l_n_wc.as<uint32_t>(), c->l_n_wp.as<uint32_t>(), W, &cnt->l_nlist))) return st;
-    if ((st = launch_bits_list(c, c->l_e_bm.as<uint32_t>(), c->l_e_wp.as<uint32_t>(), c->l_e_list.as<uint32_t>()))) return st;
     return launch_bits_list(c, c->l_n_bm.as<uint32_t>(), c->l_n_wp.as<uint32_t>(), c->l_n_list.as<uint32_t>());
 }
 
 // The field stage of the learned band: the exact field at E, signs at N, the
 // classification of every band cube (the signs are those of the exact field
-// everywhere), the exact field at the certified corners of the valid cubes, and
-// the band-order field.  c->nv bounds every list.
+// everywhere), and the exact field at the certified corners of the valid cubes.
+// c->nv bounds every list.
 pms_status pms::learned_field(pms_ctx* c) {
     Counters* cnt = c->counters.as<Counters>();
     const uint64_t W = words_of(c);
@@ -116,18 +113,13 @@ pms_status pms::learned_field(pms_ctx* c) {
     pms_status st;
     PMS_CUDA(c, cudaMemsetAsync(c->fdense.p, 0, 4 * (size_t)c->grid.sc_size, c->stream));
     PMS_CUDA(c, cudaMemsetAsync(c->l_cert.p, 0, 4 * W, c->stream));
-    if ((st = launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nullptr, nvb, nullptr))) return st;
+    if ((st = launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nvb))) return st;
     if ((st = launch_field_cert(c, c->l_n_list.as<uint32_t>(), &cnt->l_nlist, nvb, c->l_cert.as<uint32_t>(), &cnt->l_cert)))
         return st;
     if ((st = launch_mc_classify(c))) return st;
-    // the certified corners of valid cubes: E's buffers hold them from here on
-    PMS_CUDA(c, cudaMemsetAsync(c->l_e_bm.p, 0, 4 * W, c->stream));
+    // the certified corners of valid cubes: E's bitmap holds them from here on
     if ((st = launch_recheck_bits(c, c->l_cert.as<uint32_t>(), c->l_e_bm.as<uint32_t>()))) return st;
-    if ((st = launch_popc(c, c->l_e_bm.as<uint32_t>(), c->l_e_wc.as<uint32_t>()))) return st;
-    if ((st = scan_u32(c, c->l_e_wc.as<uint32_t>(), c->l_e_wp.as<uint32_t>(), W, &cnt->l_recheck))) return st;
-    if ((st = launch_bits_list(c, c->l_e_bm.as<uint32_t>(), c->l_e_wp.as<uint32_t>(), c->l_e_list.as<uint32_t>()))) return st;
-    if ((st = launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nullptr, nvb, nullptr))) return st;
-    return launch_field_gather(c, c->vlist.as<uint32_t>(), &cnt->nv, nvb, c->field.as<float>());
+    return launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nvb);
 }
 
 extern "C" pms_status pms_band_learned(pms_ctx* c) {
@@ -183,8 +175,9 @@ extern "C" pms_status pms_learn_prepare(pms_ctx* c, uint32_t* n_candidates, uint
     const uint64_t W = words_of(c);
     pms_status st;
     PMS_CUDA(c, c->l_label.ensure(4 * (W + 1)));
-    PMS_CUDA(c, cudaMemsetAsync(c->l_label.p, 0, 4 * W, c->stream));
-    if (c->nv && (st = launch_label_bits(c, c->l_label.as<uint32_t>()))) return st;
+    // the plain method's valid cubes are the labels
+    if (c->nv) PMS_CUDA(c, cudaMemcpyAsync(c->l_label.p, c->mc_valid.p, 4 * W, cudaMemcpyDeviceToDevice, c->stream));
+    else PMS_CUDA(c, cudaMemsetAsync(c->l_label.p, 0, 4 * W, c->stream));
     if ((st = launch_coarse_counts(c))) return st;
     if ((st = zero_learn_counters(c))) return st;
     if ((st = launch_predict(c, 0, nullptr, nullptr, nullptr, 0))) return st;
