@@ -34,16 +34,25 @@ struct AnisoParams {
     double cond_limit;
 };
 
+// m / rho, 0 for rho == 0
+__device__ __forceinline__ float mass_over(float mass, float r) { return r == 0.f ? 0.f : mass / r; }
+
 // ---------------------------------------------------------------------------
 // density (calculationOfDensity): rho_i = sum_j sigma/h^3 (1 - (d/h)^2)^3, d < h,
-// over cells [c - e, c + e]; also stores m / rho into spos.w for the field.
+// over cells [c - e, c + e].  Also the isotropic kernel of every particle in the field's
+// packed form: M = G^T G with G = I / h (off-diagonals doubled), the support's packed
+// extents, and the weight (m / rho) sigma det(G) = (m / rho) sigma / h^3, 0 for rho == 0
+// (the field skips such particles); the anisotropy pass overwrites the surface
+// particles' entries.
 // ---------------------------------------------------------------------------
 template <int BT>
 __global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams ap, const uint32_t* __restrict__ skeys,
-                                                      const uint32_t* __restrict__ cell_start, float4* __restrict__ spos,
-                                                      float* __restrict__ rho, uint32_t n) {
+                                                      const uint32_t* __restrict__ cell_start, const float4* __restrict__ spos,
+                                                      float* __restrict__ rho, float4* __restrict__ aniso, uint32_t n) {
     const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1];
     const float pad = 1e-4f * g.sp_cs;
+    const float inv_h2 = ap.h_inv * ap.h_inv;
+    const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 pi4 = spos[i];
         const float3 p = make_float3(pi4.x, pi4.y, pi4.z);
@@ -61,24 +70,10 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams 
             const float s = fmaxf(fmaf(-d2, ap.inv_h2, 1.f), 0.f);   // 0 beyond h: adds nothing
             w = fmaf(s * s, s, w);
         });
-        rho[i] = ap.kdens * w;
-    }
-}
-
-// m / rho into spos.w (0 for rho == 0: the field skips such particles), and the
-// isotropic kernel of every particle in the field's packed form: M = G^T G
-// with G = I / h (off-diagonals doubled), the support's packed extents, and the weight
-// (m / rho) sigma det(G) = (m / rho) sigma / h^3; the anisotropy pass
-// overwrites the surface particles' entries.
-__global__ void __launch_bounds__(kThreads) k_inv_density(float4* __restrict__ spos, const float* __restrict__ rho,
-                                                          float4* __restrict__ aniso, AnisoParams ap, uint32_t n) {
-    const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float r = rho[i];
-        spos[i].w = r == 0.f ? 0.f : ap.mass / r;
-        const float inv_h2 = ap.h_inv * ap.h_inv;
+        const float r = ap.kdens * w;
+        rho[i] = r;
         aniso[2 * (size_t)i + 0] = make_float4(inv_h2, 0.f, 0.f, __uint_as_float(ext));
-        aniso[2 * (size_t)i + 1] = make_float4(inv_h2, 0.f, inv_h2, spos[i].w * ap.kdens);
+        aniso[2 * (size_t)i + 1] = make_float4(inv_h2, 0.f, inv_h2, mass_over(ap.mass, r) * ap.kdens);
     }
 }
 
@@ -208,8 +203,8 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_moments(KGrid g, AnisoParams 
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32_t* __restrict__ slist,
                                                     const Counters* __restrict__ cnt, const uint32_t* __restrict__ skeys,
-                                                    const float4* __restrict__ spos, const float4* __restrict__ mom,
-                                                    float4* __restrict__ aniso, float4* __restrict__ nrm4,
+                                                    const float4* __restrict__ spos, const float* __restrict__ rho,
+                                                    const float4* __restrict__ mom, float4* __restrict__ aniso, float4* __restrict__ nrm4,
                                                     float4* __restrict__ mean4, float* __restrict__ gdebug,
                                                     uint32_t* __restrict__ nnb, float* __restrict__ cell_rad,
                                                     Counters* __restrict__ cnt_w) {
@@ -292,7 +287,8 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
             for (int b = 0; b < 3; ++b) M[a][b] = G[a][0] * G[0][b] + G[a][1] * G[1][b] + G[a][2] * G[2][b];
         aniso[2 * (size_t)i + 0] = make_float4(M[0][0], 2.f * M[0][1], 2.f * M[0][2],
                                                 __uint_as_float(pack_extents(ext[0], ext[1], ext[2], ap.h)));
-        aniso[2 * (size_t)i + 1] = make_float4(M[1][1], 2.f * M[1][2], M[2][2], pi4.w * (kSigma * det));
+        aniso[2 * (size_t)i + 1] = make_float4(M[1][1], 2.f * M[1][2], M[2][2],
+                                                mass_over(ap.mass, rho[i]) * (kSigma * det));
         nrm4[i] = make_float4(nv[0], nv[1], nv[2], flag);
         mean4[s] = make_float4(pi4.x + ox, pi4.y + oy, pi4.z + oz, ws);
         float* gd = gdebug + 10 * (size_t)s;
@@ -340,14 +336,11 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
     auto dens = [&](auto kern) {
         kern<<<grid_for(ctx->n, (unsigned)bd), bd, 0, ctx->stream>>>(g, ap, ctx->skeys.as<uint32_t>(),
                                                                     ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
-                                                                    ctx->rho.as<float>(), ctx->n);
+                                                                    ctx->rho.as<float>(), ctx->aniso.as<float4>(), ctx->n);
     };
     if (bd == 64) dens(k_density<64>);
     else if (bd == 256) dens(k_density<256>);
     else dens(k_density<128>);
-    PMS_LAUNCHED(ctx);
-    k_inv_density<<<grid_for(ctx->n, kThreads), kThreads, 0, ctx->stream>>>(ctx->spos.as<float4>(), ctx->rho.as<float>(),
-                                                                           ctx->aniso.as<float4>(), ap, ctx->n);
     PMS_LAUNCHED(ctx);
     // ns is on the device; grids are sized by the particle count (an upper bound)
     auto mom = [&](auto kern) {
@@ -359,11 +352,9 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
     else if (bm == 256) mom(k_moments<256>);
     else mom(k_moments<128>);
     PMS_LAUNCHED(ctx);
-    PMS_CUDA(ctx, cudaMemsetAsync(ctx->cell_rad.p, 0,
-                                  sizeof(float) * ((size_t)g.sp_size + (size_t)g.spres[1] * g.spres[2]), ctx->stream));
     k_eigen<<<grid_for(ctx->n, kThreads), kThreads, 0, ctx->stream>>>(
-        ap, ctx->slist.as<uint32_t>(), cnt, ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->moments.as<float4>(),
-        ctx->aniso.as<float4>(), ctx->nrm4.as<float4>(), ctx->mean4.as<float4>(), ctx->gdebug.as<float>(),
+        ap, ctx->slist.as<uint32_t>(), cnt, ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->rho.as<float>(),
+        ctx->moments.as<float4>(), ctx->aniso.as<float4>(), ctx->nrm4.as<float4>(), ctx->mean4.as<float4>(), ctx->gdebug.as<float>(),
         ctx->nnb.as<uint32_t>(), ctx->cell_rad.as<float>(), cnt);
     PMS_LAUNCHED(ctx);
     return PMS_OK;

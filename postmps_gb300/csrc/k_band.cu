@@ -261,7 +261,9 @@ __device__ __forceinline__ uint32_t shifted_word(const uint32_t* __restrict__ b,
 // LOWRES dilation (Anisotropic_kernel.cuh:610-629) and popcount per word
 __global__ void __launch_bounds__(256) k_band_dilate(const uint32_t* __restrict__ bm0, uint32_t* __restrict__ bm,
                                                      uint32_t* __restrict__ wcount, uint64_t nwords, uint64_t nbits,
-                                                     uint64_t sy, uint64_t sz) {
+                                                     uint64_t sy, uint64_t sz, Counters* __restrict__ cnt) {
+    // the tickets of the next launches that take any start at 0
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt->band_next = cnt->n_items = cnt->field_next = 0u;
     for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t v = bm0[w] | shifted_word(bm0, w, 1) | shifted_word(bm0, w, sy) | shifted_word(bm0, w, sz);
         if (w == nwords - 1 && (nbits & 31u)) v &= (1u << (nbits & 31u)) - 1u;
@@ -298,8 +300,8 @@ pms_status launch_band(pms_ctx* ctx) {
     const uint64_t nbits = g.sc_size, nwords = (nbits + 31) / 32;
     const TileDims td = tile_dims(g);
     const uint64_t ntiles = (uint64_t)td.n[0] * td.n[1] * td.n[2];
-    PMS_CUDA(ctx, cudaMemsetAsync(&cnt->band_next, 0, sizeof(uint32_t), ctx->stream));
-    PMS_CUDA(ctx, cudaMemsetAsync(ctx->bm0.p, 0, sizeof(uint32_t) * nwords, ctx->stream));
+    // (the marks and the ticket are 0: the frame's start and the dilation leave them so, and a
+    // second band of the same frame sets the same bits)
     // extent = ceil(maxdistance / scGridSize) (Anisotropic_kernel.cuh:551), a correctly rounded float quotient
     const int ext_dev = (int)(uint32_t)ceilf(ctx->prm.h / g.sc_cs);
     const uint64_t warps = 152u * 8u * (kBandThreads / 32);
@@ -311,8 +313,9 @@ pms_status launch_band(pms_ctx* ctx) {
     PMS_LAUNCHED(ctx);
     const uint64_t sy = g.scres[0], sz = (uint64_t)g.scres[0] * g.scres[1];
     k_band_dilate<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(ctx->bm0.as<uint32_t>(), ctx->bm.as<uint32_t>(),
-                                                                  ctx->wcount.as<uint32_t>(), nwords, nbits, sy, sz);
+                                                                  ctx->wcount.as<uint32_t>(), nwords, nbits, sy, sz, cnt);
     PMS_LAUNCHED(ctx);
+    ctx->field_tickets_zero = true;
     return scan_u32(ctx, ctx->wcount.as<uint32_t>(), ctx->wprefix.as<uint32_t>(), nwords, &cnt->nv);
 }
 

@@ -720,8 +720,9 @@ static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, uint64_t n_ho
     PMS_CUDA(ctx, ctx->ftiles.ensure_grow(field_tile_bytes_of<K>(ctx->grid, n_host)));
     uint32_t* list = ctx->ftiles.as<uint32_t>();
     uint32_t* mask = list + most + 1;
-    // the list's length and the next ticket
-    PMS_CUDA(ctx, cudaMemsetAsync(&cnt->n_items, 0, 2 * sizeof(uint32_t), ctx->stream));
+    // the list's length and the next ticket start at 0: the band left them so, for one launch
+    if (!ctx->field_tickets_zero) PMS_CUDA(ctx, cudaMemsetAsync(&cnt->n_items, 0, 2 * sizeof(uint32_t), ctx->stream));
+    ctx->field_tickets_zero = false;
     k_field_tile_list<K><<<grid_for(ntiles, 256), 256, 0, ctx->stream>>>(g, td, bm, &cnt->n_items, list, mask);
     PMS_LAUNCHED(ctx);
     const int bt = ctx->tune.field_threads;
@@ -854,9 +855,7 @@ pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t
     return PMS_OK;
 }
 
-// the frame's first field evaluation: the dense field starts at 0 everywhere
 pms_status launch_field(pms_ctx* ctx) {
-    PMS_CUDA(ctx, cudaMemsetAsync(ctx->fdense.p, 0, 4 * (size_t)ctx->grid.sc_size, ctx->stream));
     return launch_field_bits(ctx, ctx->bm.as<uint32_t>(), ctx->nv_pending ? ctx->grid.sc_size : ctx->nv);
 }
 

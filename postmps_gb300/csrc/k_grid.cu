@@ -9,9 +9,8 @@
 // GB300 design: keys are cell indices < sp_size, so the stable sort is a
 // counting sort -- one atomic histogram (which doubles as the cell-count
 // array), one scan (which doubles as the cell-start array), one scatter, and a
-// per-cell ordering fix that restores the input order inside each cell (the
-// order a stable sort produces).  Only a uint32 permutation moves; the
-// payload is gathered once into SoA float4 arrays (x, y, z, m/rho) that the
+// placement that restores the input order inside each cell (the order a stable
+// sort produces) and writes the payload once into SoA float4 arrays that the
 // neighbour loops read with one 16-byte load per particle.
 #include "pms_internal.h"
 #include "k_common.cuh"
@@ -38,22 +37,25 @@ __global__ void __launch_bounds__(kThreads) k_bbox(const float* __restrict__ pos
             mx[k] = max(mx[k], o);
         }
     }
+    // one set of atomics per block: a warp's own would queue up on the six words (2M
+    // particles: 42 us with 58k atomics, the reads take 6)
+    __shared__ uint32_t s_mn[kThreads / 32][3], s_mx[kThreads / 32][3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[k] = min(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-            mx[k] = max(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-        }
+        mn[k] = __reduce_min_sync(0xffffffffu, mn[k]);
+        mx[k] = __reduce_max_sync(0xffffffffu, mx[k]);
+        if ((threadIdx.x & 31) == 0) { s_mn[threadIdx.x >> 5][k] = mn[k]; s_mx[threadIdx.x >> 5][k] = mx[k]; }
     }
-    if ((threadIdx.x & 31) == 0) {
+    const bool any_bad = __syncthreads_or(bad);
+    if (threadIdx.x < 3) {
+        const int k = threadIdx.x;
+        uint32_t lo = s_mn[0][k], hi = s_mx[0][k];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            atomicMin(&cnt->bbox_min[k], mn[k]);
-            atomicMax(&cnt->bbox_max[k], mx[k]);
-        }
+        for (int w = 1; w < kThreads / 32; ++w) { lo = min(lo, s_mn[w][k]); hi = max(hi, s_mx[w][k]); }
+        atomicMin(&cnt->bbox_min[k], lo);
+        atomicMax(&cnt->bbox_max[k], hi);
     }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&cnt->err, kErrNonFinite);
+    if (any_bad && threadIdx.x == 0) atomicOr(&cnt->err, kErrNonFinite);
 }
 
 __global__ void k_counters_init(Counters* cnt, uint32_t n) {
@@ -82,7 +84,7 @@ pms_status launch_bbox(pms_ctx* ctx) {
     Counters* cnt = ctx->counters.as<Counters>();
     k_counters_init<<<1, 1, 0, ctx->stream>>>(cnt, ctx->n);
     PMS_LAUNCHED(ctx);
-    k_bbox<<<grid_for(ctx->n, kThreads, 152 * 8), kThreads, 0, ctx->stream>>>(ctx->in_pos.as<float>(), ctx->n, cnt);
+    k_bbox<<<grid_for(ctx->n, kThreads, 152 * 4), kThreads, 0, ctx->stream>>>(ctx->in_pos.as<float>(), ctx->n, cnt);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }
@@ -109,37 +111,68 @@ __global__ void __launch_bounds__(kThreads) k_scatter(const uint32_t* __restrict
         order[cell_start[keys[i]] + slot[i]] = i;
 }
 
-// Restores ascending input order inside every cell: what a stable sort by key
-// yields.  Cells up to kSmallCell are sorted by one thread; larger ones are
-// queued for k_cell_sort_big.
-__global__ void __launch_bounds__(kThreads) k_cell_sort(const uint32_t* __restrict__ cell_count,
-                                                        const uint32_t* __restrict__ cell_start, uint32_t ncells,
-                                                        uint32_t* __restrict__ order, uint32_t* __restrict__ big,
-                                                        Counters* __restrict__ cnt) {
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x) {
-        uint32_t m = cell_count[c];
-        if (m < 2) continue;
-        if (m > kSmallCell) {
-            uint32_t k = atomicAdd(&cnt->n_big_cells, 1u);
-            big[k] = c;
-            if (m > kBigCell) atomicOr(&cnt->err, kErrBigCell);
-            continue;
-        }
-        uint32_t* a = order + cell_start[c];
-        for (uint32_t i = 1; i < m; ++i) {
-            uint32_t v = a[i];
-            uint32_t j = i;
-            while (j > 0 && a[j - 1] > v) { a[j] = a[j - 1]; --j; }
-            a[j] = v;
-        }
+// Up to three arrays zeroed in one launch (a frame of a few thousand particles pays the
+// launches, not the bytes).
+struct ZeroList {
+    uint32_t* p[3];
+    uint64_t n[3];
+};
+__global__ void __launch_bounds__(kThreads) k_zero(ZeroList z) {
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        // whole 16-byte words, then the rest (the arrays are allocations of their own)
+        uint4* q = reinterpret_cast<uint4*>(z.p[k]);
+        for (uint64_t i = t; i < z.n[k] / 4; i += step) q[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (uint64_t i = z.n[k] / 4 * 4 + t; i < z.n[k]; i += step) z.p[k][i] = 0u;
     }
 }
 
-// One block per queued cell: bitonic sort in shared memory (<= kBigCell entries).
+// One sorted particle.
+__device__ __forceinline__ void place(uint32_t dest, uint32_t i, uint32_t key, const float* __restrict__ pos,
+                                      const float* __restrict__ vel, uint32_t* __restrict__ skeys, float4* __restrict__ spos,
+                                      float4* __restrict__ svel) {
+    skeys[dest] = key;
+    spos[dest] = make_float4(pos[3 * (size_t)i], pos[3 * (size_t)i + 1], pos[3 * (size_t)i + 2], 0.f);
+    svel[dest] = make_float4(vel[3 * (size_t)i], vel[3 * (size_t)i + 1], vel[3 * (size_t)i + 2], 0.f);
+}
+
+// Ascending input order inside every cell, what a stable sort by key yields, and the payload
+// in that order.  In a cell of up to kSmallCell particles each finds its place by counting
+// the smaller indices among the cell's entries (neighbouring threads read the same few);
+// larger cells are queued for k_cell_sort_big.  (A thread per cell sorting its entries in
+// place, then a gather, took 35 + 35 us on 2M particles and 13 + 4 us on 4k, where the
+// serial sort of a cell is the latency; this takes 39 and 5.)
+__global__ void __launch_bounds__(kThreads) k_place(const uint32_t* __restrict__ scattered, const uint32_t* __restrict__ keys,
+                                                    const uint32_t* __restrict__ cell_start, const float* __restrict__ pos,
+                                                    const float* __restrict__ vel, uint32_t n, uint32_t* __restrict__ order,
+                                                    uint32_t* __restrict__ skeys, float4* __restrict__ spos,
+                                                    float4* __restrict__ svel, uint32_t* __restrict__ big,
+                                                    Counters* __restrict__ cnt) {
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        const uint32_t i = __ldg(&scattered[s]), key = __ldg(&keys[i]);
+        const uint32_t st = __ldg(&cell_start[key]), m = __ldg(&cell_start[key + 1u]) - st;
+        uint32_t dest = s;
+        if (m <= kSmallCell) {
+            dest = st;
+            for (uint32_t t = 0; t < m; ++t) dest += __ldg(&scattered[st + t]) < i ? 1u : 0u;
+        } else if (s == st) {
+            big[atomicAdd(&cnt->n_big_cells, 1u)] = key;
+            if (m > kBigCell) atomicOr(&cnt->err, kErrBigCell);
+        }
+        order[dest] = i;
+        place(dest, i, key, pos, vel, skeys, spos, svel);
+    }
+}
+
+// One block per queued cell: bitonic sort in shared memory (<= kBigCell entries), and the
+// payload in the sorted order.
 __global__ void __launch_bounds__(1024) k_cell_sort_big(const uint32_t* __restrict__ cell_count,
                                                         const uint32_t* __restrict__ cell_start,
                                                         const uint32_t* __restrict__ big, const Counters* __restrict__ cnt,
-                                                        uint32_t* __restrict__ order) {
+                                                        const float* __restrict__ pos, const float* __restrict__ vel,
+                                                        uint32_t* __restrict__ order, uint32_t* __restrict__ skeys,
+                                                        float4* __restrict__ spos, float4* __restrict__ svel) {
     __shared__ uint32_t s[kBigCell];
     uint32_t nb = cnt->n_big_cells;
     for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
@@ -164,21 +197,11 @@ __global__ void __launch_bounds__(1024) k_cell_sort_big(const uint32_t* __restri
                 __syncthreads();
             }
         }
-        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) a[i] = s[i];
+        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+            a[i] = s[i];
+            place(cell_start[c] + i, s[i], c, pos, vel, skeys, spos, svel);
+        }
         __syncthreads();
-    }
-}
-
-// Gathers the payload into sorted SoA arrays.
-__global__ void __launch_bounds__(kThreads) k_gather(const uint32_t* __restrict__ order, const uint32_t* __restrict__ keys,
-                                                     const float* __restrict__ pos, const float* __restrict__ vel,
-                                                     uint32_t n, uint32_t* __restrict__ skeys, float4* __restrict__ spos,
-                                                     float4* __restrict__ svel) {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        uint32_t i = order[j];
-        skeys[j] = keys[i];
-        spos[j] = make_float4(pos[3 * (size_t)i], pos[3 * (size_t)i + 1], pos[3 * (size_t)i + 2], 0.f);
-        svel[j] = make_float4(vel[3 * (size_t)i], vel[3 * (size_t)i + 1], vel[3 * (size_t)i + 2], 0.f);
     }
 }
 
@@ -186,7 +209,12 @@ pms_status launch_hash_sort(pms_ctx* ctx) {
     const uint32_t n = ctx->n;
     const KGrid g = kgrid_of(ctx->grid);
     Counters* cnt = ctx->counters.as<Counters>();
-    PMS_CUDA(ctx, cudaMemsetAsync(ctx->cell_count.p, 0, sizeof(uint32_t) * (size_t)g.sp_size, ctx->stream));
+    // the cell counts, the support radii the anisotropy pass raises, the band's marks: all start
+    // at 0, and a stage run again on the same frame sets the same values
+    const ZeroList z = {{ctx->cell_count.as<uint32_t>(), ctx->cell_rad.as<uint32_t>(), ctx->bm0.as<uint32_t>()},
+                        {g.sp_size, (uint64_t)g.sp_size + (uint64_t)g.spres[1] * g.spres[2], ((uint64_t)g.sc_size + 31) / 32}};
+    k_zero<<<grid_for((z.n[0] + z.n[1] + z.n[2]) / 16 + 1, kThreads, 152 * 8), kThreads, 0, ctx->stream>>>(z);
+    PMS_LAUNCHED(ctx);
     const unsigned gb = grid_for(n, kThreads);
     k_hash_count<<<gb, kThreads, 0, ctx->stream>>>(g, ctx->in_pos.as<float>(), n, ctx->keys.as<uint32_t>(),
                                                    ctx->slot.as<uint32_t>(), ctx->cell_count.as<uint32_t>(), cnt);
@@ -196,23 +224,23 @@ pms_status launch_hash_sort(pms_ctx* ctx) {
     pms_status st = scan_u32(ctx, ctx->cell_count.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), g.sp_size,
                              ctx->cell_start.as<uint32_t>() + g.sp_size);
     if (st != PMS_OK) return st;
+    // (the surface list's buffer holds the scattered indices until the surface pass)
     k_scatter<<<gb, kThreads, 0, ctx->stream>>>(ctx->keys.as<uint32_t>(), ctx->slot.as<uint32_t>(),
-                                                ctx->cell_start.as<uint32_t>(), n, ctx->order.as<uint32_t>());
-    PMS_LAUNCHED(ctx);
-    k_cell_sort<<<grid_for(g.sp_size, kThreads), kThreads, 0, ctx->stream>>>(
-        ctx->cell_count.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), g.sp_size, ctx->order.as<uint32_t>(),
-        ctx->big_cells.as<uint32_t>(), cnt);
-    PMS_LAUNCHED(ctx);
-    k_cell_sort_big<<<32, 1024, 0, ctx->stream>>>(ctx->cell_count.as<uint32_t>(), ctx->cell_start.as<uint32_t>(),
-                                                   ctx->big_cells.as<uint32_t>(), cnt, ctx->order.as<uint32_t>());
+                                                ctx->cell_start.as<uint32_t>(), n, ctx->slist.as<uint32_t>());
     PMS_LAUNCHED(ctx);
     if (ctx->vel_pending) {
         PMS_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->vel_ready, 0));   // the uploaded velocities
         ctx->vel_pending = false;
     }
-    k_gather<<<gb, kThreads, 0, ctx->stream>>>(ctx->order.as<uint32_t>(), ctx->keys.as<uint32_t>(),
-                                               ctx->in_pos.as<float>(), ctx->in_vel.as<float>(), n,
-                                               ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->svel.as<float4>());
+    k_place<<<gb, kThreads, 0, ctx->stream>>>(ctx->slist.as<uint32_t>(), ctx->keys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(),
+                                              ctx->in_pos.as<float>(), ctx->in_vel.as<float>(), n, ctx->order.as<uint32_t>(),
+                                              ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->svel.as<float4>(),
+                                              ctx->big_cells.as<uint32_t>(), cnt);
+    PMS_LAUNCHED(ctx);
+    k_cell_sort_big<<<32, 1024, 0, ctx->stream>>>(ctx->cell_count.as<uint32_t>(), ctx->cell_start.as<uint32_t>(),
+                                                   ctx->big_cells.as<uint32_t>(), cnt, ctx->in_pos.as<float>(),
+                                                   ctx->in_vel.as<float>(), ctx->order.as<uint32_t>(), ctx->skeys.as<uint32_t>(),
+                                                   ctx->spos.as<float4>(), ctx->svel.as<float4>());
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }

@@ -18,8 +18,8 @@
 // over a 64-bit key per word (valid << 32 | mesh vertices) yields both offsets; the
 // compaction writes one 16-byte record per valid cube {vertex id, case, first mesh vertex},
 // so the emission reads its inputs coalesced.  The field is read from the dense scalar-grid
-// copy the field kernel writes (0 off the band, so a normal's out-of-band neighbour reads 0
-// as in the reference).  Each warp emits 32 consecutive valid cubes: their mesh vertices
+// copy the field kernel writes (a normal's out-of-band neighbour reads 0, as in the
+// reference: the bitmap decides).  Each warp emits 32 consecutive valid cubes: their mesh vertices
 // are contiguous, so the warp stages them in shared memory and writes whole lines
 // (scattered 4-byte stores from each cube would leave partial sectors for the memory to
 // merge).
@@ -220,11 +220,14 @@ __global__ void __launch_bounds__(kThreads) k_mc_cases(KGrid g, float iso, const
     }
 }
 
-// field at scalar-grid vertex (x, y, z): 0 outside the grid and off the band
-__device__ __forceinline__ float grid_value(const KGrid& g, const float* __restrict__ fdense, int x, int y, int z) {
+// field at scalar-grid vertex (x, y, z): 0 outside the grid and off the band (the dense array
+// holds values at band vertices only; elsewhere it is whatever an earlier frame left)
+__device__ __forceinline__ float grid_value(const KGrid& g, const uint32_t* __restrict__ bm, const float* __restrict__ fdense,
+                                            int x, int y, int z) {
     if (x < 0 || y < 0 || z < 0 || (uint32_t)x >= g.scres[0] || (uint32_t)y >= g.scres[1] || (uint32_t)z >= g.scres[2])
         return 0.f;
-    return __ldg(&fdense[((size_t)z * g.scres[1] + (size_t)y) * g.scres[0] + (size_t)x]);
+    const size_t i = ((size_t)z * g.scres[1] + (size_t)y) * g.scres[0] + (size_t)x;
+    return (__ldg(&bm[i >> 5]) >> (i & 31u)) & 1u ? __ldg(&fdense[i]) : 0.f;
 }
 
 __device__ __forceinline__ float3 normalized(float3 v) {
@@ -242,7 +245,8 @@ static constexpr int kEmitStage = 32 * 15 * 6;     // floats: 32 cubes x 15 mesh
 // are made, from the same arithmetic, so the positions are the same either way.
 template <bool kNormals>
 __global__ void __launch_bounds__(kThreads) k_mc_emit(KGrid g, float iso, Counters* __restrict__ cnt,
-                                                      const uint4* __restrict__ cube, const float* __restrict__ fdense,
+                                                      const uint4* __restrict__ cube, const uint32_t* __restrict__ bm,
+                                                      const float* __restrict__ fdense,
                                                       float* __restrict__ vert, float* __restrict__ vnorm,
                                                       const unsigned long long* __restrict__ frame_base,
                                                       unsigned long long cap, int piece) {
@@ -289,9 +293,9 @@ __global__ void __launch_bounds__(kThreads) k_mc_emit(KGrid g, float iso, Counte
             for (int c = 0; c < 8 && kNormals; ++c) {
                 const int ox = corner_off(c, 0), oy = corner_off(c, 1), oz = corner_off(c, 2);
                 const int X = x + ox, Y = y + oy, Z = z + oz;
-                const float fx = grid_value(g, fdense, ox ? X + 1 : X - 1, Y, Z);
-                const float fy = grid_value(g, fdense, X, oy ? Y + 1 : Y - 1, Z);
-                const float fz = grid_value(g, fdense, X, Y, oz ? Z + 1 : Z - 1);
+                const float fx = grid_value(g, bm, fdense, ox ? X + 1 : X - 1, Y, Z);
+                const float fy = grid_value(g, bm, fdense, X, oy ? Y + 1 : Y - 1, Z);
+                const float fz = grid_value(g, bm, fdense, X, Y, oz ? Z + 1 : Z - 1);
                 const float qx = cf[corner_partner(c, 0)], qy = cf[corner_partner(c, 1)], qz = cf[corner_partner(c, 2)];
                 cn[c] = normalized(make_float3(ox ? qx - fx : fx - qx, oy ? qy - fy : fy - qy, oz ? qz - fz : fz - qz));
             }
@@ -519,11 +523,13 @@ pms_status launch_mc_emit_to(pms_ctx* ctx, float* vert, float* vnorm, const unsi
     const unsigned blocks = grid_for(work, kThreads);
     if (vnorm)
         k_mc_emit<true><<<blocks, kThreads, 0, ctx->stream>>>(g, ctx->prm.iso_value, cnt, ctx->cube.as<uint4>(),
-                                                              ctx->fdense.as<float>(), vert, vnorm, frame_base, cap,
+                                                              ctx->bm.as<uint32_t>(), ctx->fdense.as<float>(), vert, vnorm,
+                                                              frame_base, cap,
                                                               piece);
     else
         k_mc_emit<false><<<blocks, kThreads, 0, ctx->stream>>>(g, ctx->prm.iso_value, cnt, ctx->cube.as<uint4>(),
-                                                               ctx->fdense.as<float>(), vert, nullptr, frame_base,
+                                                               ctx->bm.as<uint32_t>(), ctx->fdense.as<float>(), vert,
+                                                               nullptr, frame_base,
                                                                cap, piece);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
@@ -569,16 +575,16 @@ __global__ void __launch_bounds__(256) k_weld_popc(const uint32_t* __restrict__ 
 
 // the negative field gradient at a scalar vertex (central differences, 0 outside the grid
 // and the band), the vertex normal of getVertexNorm (myCuda.cuh:259-289)
-__device__ __forceinline__ float3 vertex_normal(const KGrid& g, const float* __restrict__ fdense, int x, int y, int z) {
-    return normalized(make_float3(grid_value(g, fdense, x - 1, y, z) - grid_value(g, fdense, x + 1, y, z),
-                                  grid_value(g, fdense, x, y - 1, z) - grid_value(g, fdense, x, y + 1, z),
-                                  grid_value(g, fdense, x, y, z - 1) - grid_value(g, fdense, x, y, z + 1)));
+__device__ __forceinline__ float3 vertex_normal(const KGrid& g, const uint32_t* __restrict__ bm, const float* __restrict__ fdense, int x, int y, int z) {
+    return normalized(make_float3(grid_value(g, bm, fdense, x - 1, y, z) - grid_value(g, bm, fdense, x + 1, y, z),
+                                  grid_value(g, bm, fdense, x, y - 1, z) - grid_value(g, bm, fdense, x, y + 1, z),
+                                  grid_value(g, bm, fdense, x, y, z - 1) - grid_value(g, bm, fdense, x, y, z + 1)));
 }
 
 // one welded vertex per set edge bit, at the edge's rank
 __global__ void __launch_bounds__(256) k_weld_vertices(KGrid g, float iso, const uint32_t* __restrict__ ebits,
                                                        const uint32_t* __restrict__ wprefix, uint64_t nw,
-                                                       const float* __restrict__ fdense, uint64_t cap,
+                                                       const uint32_t* __restrict__ bm, const float* __restrict__ fdense, uint64_t cap,
                                                        float* __restrict__ vert, float* __restrict__ vnorm) {
     const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
     const float sgn = (iso < 0.f) ? -1.f : 1.f;
@@ -592,7 +598,7 @@ __global__ void __launch_bounds__(256) k_weld_vertices(KGrid g, float iso, const
             const uint32_t v = (uint32_t)(key / 3ull), axis = (uint32_t)(key - 3ull * v);
             const int z = (int)(v / rxy), rem = (int)(v - (uint32_t)z * rxy), y = rem / (int)rx, x = rem - y * (int)rx;
             const int X = x + (axis == 0), Y = y + (axis == 1), Z = z + (axis == 2);
-            const float fa = grid_value(g, fdense, x, y, z), fb = grid_value(g, fdense, X, Y, Z);
+            const float fa = grid_value(g, bm, fdense, x, y, z), fb = grid_value(g, bm, fdense, X, Y, Z);
             const float d = fb - fa;
             const float tt = fabsf(d) < 1.0e-7f ? 0.5f : (iso - fa) / d;   // getLerpFac's test, as above
             const float ax = sc_coord_i(g, x, 0), ay = sc_coord_i(g, y, 1), az = sc_coord_i(g, z, 2);
@@ -601,7 +607,7 @@ __global__ void __launch_bounds__(256) k_weld_vertices(KGrid g, float iso, const
             vert[3 * (size_t)r + 1] = ay + tt * (by - ay);
             vert[3 * (size_t)r + 2] = az + tt * (bz - az);
             if (vnorm) {
-                const float3 na = vertex_normal(g, fdense, x, y, z), nb = vertex_normal(g, fdense, X, Y, Z);
+                const float3 na = vertex_normal(g, bm, fdense, x, y, z), nb = vertex_normal(g, bm, fdense, X, Y, Z);
                 const float3 nn = normalized(make_float3(na.x + tt * (nb.x - na.x), na.y + tt * (nb.y - na.y),
                                                          na.z + tt * (nb.z - na.z)));
                 vnorm[3 * (size_t)r + 0] = sgn * nn.x;
@@ -647,7 +653,8 @@ pms_status launch_weld(pms_ctx* ctx, uint32_t* ebits, uint32_t* wc, uint32_t* wp
     if (st) return st;
     if (vert) {
         k_weld_vertices<<<grid_for(nw, 256), 256, 0, ctx->stream>>>(g, ctx->prm.iso_value, ebits, wprefix, nw,
-                                                                    ctx->fdense.as<float>(), cap, vert, vnorm);
+                                                                    ctx->bm.as<uint32_t>(), ctx->fdense.as<float>(), cap, vert,
+                                                                    vnorm);
         PMS_LAUNCHED(ctx);
     }
     if (idx) {

@@ -78,8 +78,8 @@ struct Counters {
     uint32_t l_cert;        // ... of which stopped above iso without an exact value
     uint32_t l_recheck;     // certified corners of valid cubes, evaluated exactly afterwards
     uint32_t n_items;       // work items (runs or tiles) of the last field launch
-    uint32_t field_next;    // the next listed tile a warp of the field takes (zeroed with n_items)
-    uint32_t band_next;     // the next tile a warp of the band marking takes
+    uint32_t field_next;    // the next listed tile a warp of the field takes (both 0 before a launch)
+    uint32_t band_next;     // the next tile a warp of the band marking takes (0 between launches)
     uint32_t n_weld;        // vertices of the welded mesh (crossed grid edges)
     uint32_t n_df_total;    // generated + carried diffuse particles of a batched frame
     uint32_t mc_piece[kMaxMcPieces + 1];  // first cube of each streamed emission range, then nvalid
@@ -208,7 +208,7 @@ struct pms_ctx {
     // (field: the band-order copy, made for debug downloads and tests; mc_*: per word of the
     // scalar grid the band vertices at or below iso, the valid cubes, their key and its scan)
     pms::DBuf field, mc_le, mc_valid, mc_key, mc_off, vert, vnorm, sval;
-    // the field over the whole scalar grid, 0 off the band (the marching cubes' lookups);
+    // the field over the whole scalar grid, written at band vertices (the marching cubes' lookups);
     // per valid cube {vertex id, case, first mesh vertex, 0}
     pms::DBuf fdense, cube;
     // welded mesh: crossed-edge bitmap (3 bits per scalar vertex), its word popcounts and
@@ -218,6 +218,7 @@ struct pms_ctx {
     bool have_weld = false, weld_normals = false;
     // field work: runs of x-neighbouring band vertices (certification), tiles (exact field)
     pms::DBuf fitems, fitem_cnt, fitem_off, ftiles;
+    bool field_tickets_zero = false;   // Counters::n_items and field_next are 0 (the band's last launch)
     bool have_values = false;
     // vertex normals of the current mesh: made by the emission only when a streamed
     // mesh asks for them, else on the first download that does

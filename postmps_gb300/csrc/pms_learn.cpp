@@ -111,7 +111,6 @@ pms_status pms::learned_field(pms_ctx* c) {
     const uint64_t W = words_of(c);
     const uint32_t nvb = c->nv;
     pms_status st;
-    PMS_CUDA(c, cudaMemsetAsync(c->fdense.p, 0, 4 * (size_t)c->grid.sc_size, c->stream));
     PMS_CUDA(c, cudaMemsetAsync(c->l_cert.p, 0, 4 * W, c->stream));
     if ((st = launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nvb))) return st;
     if ((st = launch_field_cert(c, c->l_n_list.as<uint32_t>(), &cnt->l_nlist, nvb, c->l_cert.as<uint32_t>(), &cnt->l_cert)))
