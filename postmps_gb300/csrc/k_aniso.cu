@@ -15,6 +15,7 @@
 // with exact rotations runs in float32, and covariances whose condition
 // number exceeds cfg.fp64_svd_cond are re-solved in float64.  Sums are
 // accumulated relative to the particle's own position for accuracy.
+#include <algorithm>
 #include <cmath>
 
 #include "pms_internal.h"
@@ -23,6 +24,8 @@
 namespace pms {
 
 static constexpr int kThreads = 128;
+// frames of up to this many particles take a warp per particle for the density
+static constexpr uint32_t kDensityWarp = 16384;
 static constexpr float kSigma = 1.56668147f;      // Define.h:11, 315/(64 pi)
 
 struct AnisoParams {
@@ -34,6 +37,12 @@ struct AnisoParams {
     double cond_limit;
 };
 
+// max(1 - |r|^2 / h^2, 0), every rounding spelled out: 0 beyond h
+__device__ __forceinline__ float density_term(float dx, float dy, float dz, float inv_h2) {
+    const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+    return __saturatef(__fmaf_rn(-d2, inv_h2, 1.f));         // (never above 1)
+}
+
 // m / rho, 0 for rho == 0
 __device__ __forceinline__ float mass_over(float mass, float r) { return r == 0.f ? 0.f : mass / r; }
 
@@ -44,14 +53,34 @@ __device__ __forceinline__ float mass_over(float mass, float r) { return r == 0.
 // extents, and the weight (m / rho) sigma det(G) = (m / rho) sigma / h^3, 0 for rho == 0
 // (the field skips such particles); the anisotropy pass overwrites the surface
 // particles' entries.
+//
+// Three forms, chosen by the launcher:
+// - k_density_tiles: a warp per block of 4 x 2 x 2 cells.  Its particles (54 at rest, two per
+//   lane) share their neighbours: the warp reads each once, keeps those within h of the
+//   particles' box in shared memory, and all lanes add them.  Used where every particle's
+//   window [c - e, c + e] surely holds its support (e cells exceed h by kRangeMargin: the
+//   sum then does not depend on the window).
+// - k_density: a thread per particle over its own window, else.
+// - k_density_warp: a warp per particle for frames too small to fill the GPU with
+//   either, where one particle's serial walk is the pass's time.
+// All add the same contributions in the same order (ascending sorted index; what lies
+// beyond h adds exactly 0).  Bound by L1 (93 %: each lane loading its own neighbours)
+// before, by instruction issue now: dam 8M 1.47 -> 1.17 ms, crown 2M 0.36 -> 0.28, block 4k 23 -> 7 us.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void put_density(const AnisoParams& ap, uint32_t i, float w, uint32_t ext, float* __restrict__ rho,
+                                            float4* __restrict__ aniso) {
+    const float r = ap.kdens * w, inv_h2 = ap.h_inv * ap.h_inv;
+    rho[i] = r;
+    aniso[2 * (size_t)i + 0] = make_float4(inv_h2, 0.f, 0.f, __uint_as_float(ext));
+    aniso[2 * (size_t)i + 1] = make_float4(inv_h2, 0.f, inv_h2, mass_over(ap.mass, r) * ap.kdens);
+}
+
 template <int BT>
 __global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams ap, const uint32_t* __restrict__ skeys,
                                                       const uint32_t* __restrict__ cell_start, const float4* __restrict__ spos,
                                                       float* __restrict__ rho, float4* __restrict__ aniso, uint32_t n) {
     const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1];
     const float pad = 1e-4f * g.sp_cs;
-    const float inv_h2 = ap.h_inv * ap.h_inv;
     const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 pi4 = spos[i];
@@ -65,15 +94,165 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams 
         float w = 0.f;
         row_walk(g, p, lo, hi, ap.h_sq, pad, cell_start, [&](uint32_t j) {
             const float4 q = __ldg(&spos[j]);
-            const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-            const float d2 = dx * dx + dy * dy + dz * dz;
-            const float s = fmaxf(fmaf(-d2, ap.inv_h2, 1.f), 0.f);   // 0 beyond h: adds nothing
+            const float s = density_term(p.x - q.x, p.y - q.y, p.z - q.z, ap.inv_h2);
             w = fmaf(s * s, s, w);
         });
-        const float r = ap.kdens * w;
-        rho[i] = r;
-        aniso[2 * (size_t)i + 0] = make_float4(inv_h2, 0.f, 0.f, __uint_as_float(ext));
-        aniso[2 * (size_t)i + 1] = make_float4(inv_h2, 0.f, inv_h2, mass_over(ap.mass, r) * ap.kdens);
+        put_density(ap, i, w, ext, rho, aniso);
+    }
+}
+
+// a warp per particle: the lanes work out 32 neighbours' terms, then add the non-zero ones in
+// their order
+__global__ void __launch_bounds__(kThreads) k_density_warp(KGrid g, AnisoParams ap, const uint32_t* __restrict__ skeys,
+                                                           const uint32_t* __restrict__ cell_start,
+                                                           const float4* __restrict__ spos, float* __restrict__ rho,
+                                                           float4* __restrict__ aniso, uint32_t n) {
+    const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1], lane = threadIdx.x & 31u;
+    const float pad = 1e-4f * g.sp_cs;
+    const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+        const float4 pi4 = spos[i];
+        const float3 p = make_float3(pi4.x, pi4.y, pi4.z);
+        const uint32_t key = skeys[i];
+        const uint3 c = make_uint3(key % rx, (key / rx) % g.spres[1], key / rxy);
+        uint3 lo, hi;
+        box_clamp(g, c, (uint32_t)g.spexpand, lo, hi);
+        hi = make_uint3(hi.x + 1, hi.y + 1, hi.z + 1);
+        float w = 0.f;
+        warp_walk(g, p, lo, hi, ap.h_sq, pad, cell_start, [&](bool valid, uint32_t j) {
+            float s = 0.f;
+            if (valid) {
+                const float4 q = __ldg(&spos[j]);
+                s = density_term(p.x - q.x, p.y - q.y, p.z - q.z, ap.inv_h2);
+            }
+            const float ss = s * s;
+            for (uint32_t m = __ballot_sync(0xffffffffu, s > 0.f); m; m &= m - 1u) {
+                const int l = __ffs((int)m) - 1;
+                w = fmaf(__shfl_sync(0xffffffffu, ss, l), __shfl_sync(0xffffffffu, s, l), w);
+            }
+        });
+        if (lane == 0u) put_density(ap, i, w, ext, rho, aniso);
+    }
+}
+
+static constexpr int kDensX = 2, kDensY = 2, kDensZ = 2;      // cells of a block
+static constexpr int kDensStage = 64;
+
+// the blocks that hold particles
+__global__ void __launch_bounds__(256) k_density_list(KGrid g, uint3 bd, const uint32_t* __restrict__ cell_start,
+                                                      uint32_t* __restrict__ n_blocks, uint32_t* __restrict__ list) {
+    const uint32_t nb = bd.x * bd.y * bd.z;
+    for (uint32_t t0 = blockIdx.x * blockDim.x; t0 < nb; t0 += gridDim.x * blockDim.x) {    // whole warps together
+        const uint32_t t = t0 + threadIdx.x;
+        bool any = false;
+        if (t < nb) {
+            const uint32_t x0 = t % bd.x * kDensX, y0 = t / bd.x % bd.y * kDensY, z0 = t / bd.x / bd.y * kDensZ;
+            const uint32_t x1 = min(x0 + kDensX, g.spres[0]);
+#pragma unroll
+            for (int k = 0; k < kDensY * kDensZ; ++k) {
+                const uint32_t y = y0 + k % kDensY, z = z0 + k / kDensY;
+                if (y >= g.spres[1] || z >= g.spres[2]) continue;
+                const uint32_t row = (z * g.spres[1] + y) * g.spres[0];
+                any |= __ldg(&cell_start[row + x0]) != __ldg(&cell_start[row + x1]);
+            }
+        }
+        const uint32_t vote = __ballot_sync(0xffffffffu, any);
+        if (!vote) continue;
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t base = 0u;
+        if (lane == 0u) base = atomicAdd(n_blocks, (uint32_t)__popc(vote));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (any) list[base + (uint32_t)__popc(vote & ((1u << lane) - 1u))] = t;
+    }
+}
+
+__device__ __forceinline__ float warp_min(float v) { return from_ordered_bits(__reduce_min_sync(0xffffffffu, ordered_bits(v))); }
+__device__ __forceinline__ float warp_max(float v) { return from_ordered_bits(__reduce_max_sync(0xffffffffu, ordered_bits(v))); }
+
+template <int BT>
+__global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoParams ap, uint3 bd,
+                                                                 const uint32_t* __restrict__ n_blocks_dev,
+                                                                 uint32_t* __restrict__ next, const uint32_t* __restrict__ list,
+                                                                 const uint32_t* __restrict__ cell_start,
+                                                                 const float4* __restrict__ spos, float* __restrict__ rho,
+                                                                 float4* __restrict__ aniso) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ float4 stage_all[BT / 32][kDensStage];
+    float4* stage = stage_all[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, n_blocks = *n_blocks_dev;
+    const float pad = 1e-4f * g.sp_cs, inv_cs = 1.f / g.sp_cs;
+    const float rc = ap.h * inv_cs + kRangeMargin, reach2 = ap.h_sq * 1.001f;
+    const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
+    for (;;) {
+        uint32_t bi = 0u;
+        if (lane == 0u) bi = atomicAdd(next, 1u);
+        bi = __shfl_sync(kAll, bi, 0);
+        if (bi >= n_blocks) break;
+        const uint32_t t = __ldg(&list[bi]);
+        // the block's particles: a contiguous range per row of cells
+        const uint32_t x0 = t % bd.x * kDensX, y0 = t / bd.x % bd.y * kDensY, z0 = t / bd.x / bd.y * kDensZ;
+        uint32_t first = 0u, n = 0u;
+        if (lane < kDensY * kDensZ) {
+            const uint32_t y = y0 + lane % kDensY, z = z0 + lane / kDensY;
+            if (y < g.spres[1] && z < g.spres[2]) {
+                const uint32_t row = (z * g.spres[1] + y) * g.spres[0];
+                first = __ldg(&cell_start[row + x0]);
+                n = __ldg(&cell_start[row + min(x0 + kDensX, g.spres[0])]) - first;
+            }
+        }
+        const WarpRows mine = warp_rows(first, n);
+        for (uint32_t t0 = 0u; t0 < mine.total; t0 += 32u) {
+            // lanes past the block's particles repeat its last one
+            const uint32_t own = min(t0 + lane, mine.total - 1u);
+            const int own_row = warp_row_of(mine, own);
+            const uint32_t id = __shfl_sync(kAll, mine.off, own_row) + own;
+            const float4 pi4 = __ldg(&spos[id]);
+            const float3 b0 = make_float3(warp_min(pi4.x), warp_min(pi4.y), warp_min(pi4.z));
+            const float3 b1 = make_float3(warp_max(pi4.x), warp_max(pi4.y), warp_max(pi4.z));
+            float w = 0.f;
+            int staged = 0;
+            auto flush = [&]() {
+                __syncwarp();
+#pragma unroll 4
+                for (int i = 0; i < staged; ++i) {
+                    const float4 q = stage[i];
+                    const float s = density_term(pi4.x - q.x, pi4.y - q.y, pi4.z - q.z, ap.inv_h2);
+                    w = __fmaf_rn(__fmul_rn(s, s), s, w);
+                }
+                __syncwarp();
+                staged = 0;
+            };
+            const int za = max((int)floorf((b0.z - g.min_pos[2]) * inv_cs - rc), 0);
+            const int zb = min((int)floorf((b1.z - g.min_pos[2]) * inv_cs + rc) + 1, (int)g.spres[2]);
+            const int ya = max((int)floorf((b0.y - g.min_pos[1]) * inv_cs - rc), 0);
+            const int yb = min((int)floorf((b1.y - g.min_pos[1]) * inv_cs + rc) + 1, (int)g.spres[1]);
+            const int ny = yb - ya, nrow = ny > 0 && zb > za ? ny * (zb - za) : 0;
+            for (int r0 = 0; r0 < nrow; r0 += 32) {
+                const int r = r0 + (int)lane;
+                uint32_t ja = 0u, m = 0u;
+                if (r < nrow) m = box_row(g, b0, b1, ap.h_sq, pad, za + r / ny, ya + r % ny, 0, (int)g.spres[0], cell_start, ja);
+                const WarpRows rows = warp_rows(ja, m);
+                for (uint32_t p0 = 0u; p0 < rows.total; p0 += 32u) {
+                    const uint32_t p = p0 + lane;
+                    const int row = warp_row_of(rows, p);
+                    const uint32_t j = __shfl_sync(kAll, rows.off, row) + p;
+                    float4 q;
+                    bool keep = false;
+                    if (p < rows.total) {
+                        q = __ldg(&spos[j]);
+                        const float ex = fmaxf(fmaxf(b0.x - q.x, q.x - b1.x), 0.f), ey = fmaxf(fmaxf(b0.y - q.y, q.y - b1.y), 0.f),
+                                    ez = fmaxf(fmaxf(b0.z - q.z, q.z - b1.z), 0.f);
+                        keep = ex * ex + ey * ey + ez * ez < reach2;
+                    }
+                    const uint32_t kept = __ballot_sync(kAll, keep);
+                    if (keep) stage[staged + __popc(kept & ((1u << lane) - 1u))] = q;
+                    staged += __popc(kept);
+                    if (staged > kDensStage - 32) flush();
+                }
+            }
+            if (staged) flush();
+            if (t0 + lane < mine.total) put_density(ap, id, w, ext, rho, aniso);
+        }
     }
 }
 
@@ -154,6 +333,100 @@ __device__ __forceinline__ void eig_sym3(T a[3][3], T e[3], T v[3][3], T tol) {
 // rounded square root (the same decisions as comparing |u|); the weight uses
 // the hardware reciprocal square root (a few ulp, inside the weight's rounding).
 // ---------------------------------------------------------------------------
+// w = 1 - (|u| / 2h)^3 within the support, 0 beyond, 1 at the particle itself
+__device__ __forceinline__ float moment_weight(float d2, float w_d2, float inv_r2h) {
+    const float t = d2 * rsqrtf(d2) * inv_r2h;                       // d2 = 0 gives NaN, selected away
+    return (d2 <= w_d2 && d2 > 0.f) ? __fmaf_rn(-(t * t), t, 1.f) : (d2 > 0.f ? 0.f : 1.f);
+}
+
+// Few surface particles leave the GPU idle, and the pass then takes as long as one particle's
+// serial walk (about 80 us whatever the count).  So up to kMomentsWarp of them get a warp
+// each: the lanes work out 32 neighbours' weights, those within the support are staged in
+// shared memory in their order, and ten lanes run the ten sums over them.  Every product and
+// sum is the thread-per-particle form's.  Block 4k (1353 surface particles) 79 -> 12 us; the
+// two forms meet near 45,000.
+static constexpr uint32_t kMomentsWarp = 32768;
+
+template <int BT>
+__device__ __forceinline__ void moments_warp(const KGrid& g, const AnisoParams& ap, const uint32_t* __restrict__ slist, uint32_t ns,
+                                             const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ cell_start,
+                                             const float4* __restrict__ spos, float4* __restrict__ mom) {
+    constexpr unsigned kAll = 0xffffffffu;
+    // five columns of staged neighbours {w, ux, uy, uz, 1}, padded so that the ten lanes' 16-byte
+    // reads fall on different banks
+    constexpr int kCol = 68;
+    __shared__ __align__(16) float hits_all[BT / 32][5 * kCol];
+    float* hits = hits_all[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t k = lane; k < 64u; k += 32u) hits[4 * kCol + k] = 1.f;
+    __syncwarp();
+    const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1];
+    const float pad = 1e-4f * g.sp_cs, r2h_sq = ap.r2h * ap.r2h, inv_r2h = 1.f / ap.r2h;
+    // lane q's sum adds (w f1) f2: s0 | sx sy sz | sxx sxy sxz syy syz szz
+    const int f1 = lane == 0u ? 4 : (lane < 4u ? (int)lane : (lane < 7u ? 1 : (lane < 9u ? 2 : 3)));
+    const int f2 = lane < 4u ? 4 : (lane < 7u ? (int)lane - 3 : (lane < 9u ? (int)lane - 5 : 3));
+    for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < ns; s += (gridDim.x * blockDim.x) >> 5) {
+        const uint32_t i = slist[s];
+        const float4 pi4 = spos[i];
+        const float3 p = make_float3(pi4.x, pi4.y, pi4.z);
+        const uint32_t key = skeys[i];
+        const uint3 c = make_uint3(key % rx, (key / rx) % g.spres[1], key / rxy);
+        uint3 lo, hi;
+        box_clamp(g, c, 2u * (uint32_t)g.spexpand, lo, hi);
+        hi = make_uint3(hi.x + 1, hi.y + 1, hi.z + 1);
+        uint32_t nn = 0u;
+        int staged = 0;
+        float acc = 0.f;
+        auto flush = [&]() {
+            __syncwarp();
+            if (lane < 10u) {
+                const float *W = hits, *A = hits + kCol * f1, *B = hits + kCol * f2;
+                int k = 0;
+                for (; k + 4 <= staged; k += 4) {
+                    const float4 w = *reinterpret_cast<const float4*>(W + k), a = *reinterpret_cast<const float4*>(A + k),
+                                 b = *reinterpret_cast<const float4*>(B + k);
+                    acc = __fmaf_rn(__fmul_rn(w.x, a.x), b.x, acc);
+                    acc = __fmaf_rn(__fmul_rn(w.y, a.y), b.y, acc);
+                    acc = __fmaf_rn(__fmul_rn(w.z, a.z), b.z, acc);
+                    acc = __fmaf_rn(__fmul_rn(w.w, a.w), b.w, acc);
+                }
+                for (; k < staged; ++k) acc = __fmaf_rn(__fmul_rn(W[k], A[k]), B[k], acc);
+            }
+            __syncwarp();
+            staged = 0;
+        };
+        warp_walk(g, p, lo, hi, r2h_sq, pad, cell_start, [&](bool valid, uint32_t j) {
+            float ux = 0.f, uy = 0.f, uz = 0.f, w = 0.f;
+            bool keep = false;
+            if (valid) {
+                const float4 q = __ldg(&spos[j]);
+                ux = __fsub_rn(q.x, p.x); uy = __fsub_rn(q.y, p.y); uz = __fsub_rn(q.z, p.z);
+                const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(ux, ux), __fmul_rn(uy, uy)), __fmul_rn(uz, uz));
+                keep = d2 <= ap.w_d2;                        // beyond the support everything adds exactly 0
+                nn += d2 <= ap.nn_d2 ? 1u : 0u;
+                w = moment_weight(d2, ap.w_d2, inv_r2h);
+            }
+            const uint32_t kept = __ballot_sync(kAll, keep);
+            if (keep) {
+                float* h = hits + staged + __popc(kept & ((1u << lane) - 1u));
+                h[0] = w; h[kCol] = ux; h[2 * kCol] = uy; h[3 * kCol] = uz;
+            }
+            staged += __popc(kept);
+            if (staged > 32) flush();
+        });
+        if (staged) flush();
+        nn = __reduce_add_sync(kAll, nn);
+        float v[10];
+#pragma unroll
+        for (int k = 0; k < 10; ++k) v[k] = __shfl_sync(kAll, acc, k);
+        if (lane == 0u) {
+            mom[3 * (size_t)s + 0] = make_float4(v[0], v[1], v[2], v[3]);
+            mom[3 * (size_t)s + 1] = make_float4(v[4], v[5], v[6], v[7]);
+            mom[3 * (size_t)s + 2] = make_float4(v[8], v[9], __uint_as_float(nn), 0.f);
+        }
+    }
+}
+
 template <int BT>
 __global__ void __launch_bounds__(BT, 1024 / BT) k_moments(KGrid g, AnisoParams ap, const uint32_t* __restrict__ slist,
                                                       const Counters* __restrict__ cnt, const uint32_t* __restrict__ skeys,
@@ -164,6 +437,10 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_moments(KGrid g, AnisoParams 
     const float pad = 1e-4f * g.sp_cs;
     const float r2h_sq = ap.r2h * ap.r2h;
     const float inv_r2h = 1.f / ap.r2h;
+    if (ns <= kMomentsWarp) {
+        moments_warp<BT>(g, ap, slist, ns, skeys, cell_start, spos, mom);
+        return;
+    }
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
         const uint32_t i = slist[s];
         const float4 pi4 = spos[i];
@@ -182,12 +459,11 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_moments(KGrid g, AnisoParams 
             const float ux = __fsub_rn(q.x, p.x), uy = __fsub_rn(q.y, p.y), uz = __fsub_rn(q.z, p.z);
             const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(ux, ux), __fmul_rn(uy, uy)), __fmul_rn(uz, uz));
             nn += (d2 <= ap.nn_d2) ? 1u : 0u;
-            const float t = d2 * rsqrtf(d2) * inv_r2h;               // d2 = 0 gives NaN, selected away
-            const float w = (d2 <= ap.w_d2 && d2 > 0.f) ? 1.f - t * t * t : (d2 > 0.f ? 0.f : 1.f);
-            const float wx = w * ux, wy = w * uy, wz = w * uz;
+            const float w = moment_weight(d2, ap.w_d2, inv_r2h);
+            const float wx = __fmul_rn(w, ux), wy = __fmul_rn(w, uy), wz = __fmul_rn(w, uz);
             s0 += w; sx += wx; sy += wy; sz += wz;
-            sxx += wx * ux; sxy += wx * uy; sxz += wx * uz;
-            syy += wy * uy; syz += wy * uz; szz += wz * uz;
+            sxx = __fmaf_rn(wx, ux, sxx); sxy = __fmaf_rn(wx, uy, sxy); sxz = __fmaf_rn(wx, uz, sxz);
+            syy = __fmaf_rn(wy, uy, syy); syz = __fmaf_rn(wy, uz, syz); szz = __fmaf_rn(wz, uz, szz);
         });
         mom[3 * (size_t)s + 0] = make_float4(s0, sx, sy, sz);
         mom[3 * (size_t)s + 1] = make_float4(sxx, sxy, sxz, syy);
@@ -209,6 +485,7 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
                                                     uint32_t* __restrict__ nnb, float* __restrict__ cell_rad,
                                                     Counters* __restrict__ cnt_w) {
     const uint32_t ns = cnt->ns;
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt_w->dens_blocks = cnt_w->dens_next = 0u;   // the next density pass's tickets
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
         const uint32_t i = slist[s];
         const float4 pi4 = spos[i];
@@ -332,19 +609,44 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
     ap.spres_x = g.spres[0];
     Counters* cnt = ctx->counters.as<Counters>();
     // block sizes of the neighbour walks are autotuned (64, 128 or 256 threads)
-    const int bd = ctx->tune.density_threads, bm = ctx->tune.moments_threads;
-    auto dens = [&](auto kern) {
-        kern<<<grid_for(ctx->n, (unsigned)bd), bd, 0, ctx->stream>>>(g, ap, ctx->skeys.as<uint32_t>(),
-                                                                    ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
-                                                                    ctx->rho.as<float>(), ctx->aniso.as<float4>(), ctx->n);
-    };
-    if (bd == 64) dens(k_density<64>);
-    else if (bd == 256) dens(k_density<256>);
-    else dens(k_density<128>);
+    const int bd_threads = ctx->tune.density_threads, bm = ctx->tune.moments_threads;
+    const uint32_t n = ctx->n;
+    if (n <= kDensityWarp) {
+        k_density_warp<<<grid_for((uint64_t)n * 32, kThreads, 152u * 16u), kThreads, 0, ctx->stream>>>(
+            g, ap, ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->rho.as<float>(),
+            ctx->aniso.as<float4>(), n);
+    } else if ((float)g.spexpand * g.sp_cs - P.h >= kRangeMargin * g.sp_cs) {
+        const uint3 bd = make_uint3((g.spres[0] + kDensX - 1) / kDensX, (g.spres[1] + kDensY - 1) / kDensY,
+                                    (g.spres[2] + kDensZ - 1) / kDensZ);
+        // (the moments' buffer holds the list until the moments are made: at most a block per particle)
+        uint32_t* list = ctx->moments.as<uint32_t>();
+        k_density_list<<<grid_for((uint64_t)bd.x * bd.y * bd.z, 256), 256, 0, ctx->stream>>>(
+            g, bd, ctx->cell_start.as<uint32_t>(), &cnt->dens_blocks, list);
+        PMS_LAUNCHED(ctx);
+        auto tiles = [&](auto kern) {
+            kern<<<152u * (1024u / (unsigned)bd_threads), bd_threads, 0, ctx->stream>>>(
+                g, ap, bd, &cnt->dens_blocks, &cnt->dens_next, list, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
+                ctx->rho.as<float>(), ctx->aniso.as<float4>());
+        };
+        if (bd_threads == 64) tiles(k_density_tiles<64>);
+        else if (bd_threads == 256) tiles(k_density_tiles<256>);
+        else tiles(k_density_tiles<128>);
+    } else {
+        auto dens = [&](auto kern) {
+            kern<<<grid_for(n, (unsigned)bd_threads), bd_threads, 0, ctx->stream>>>(
+                g, ap, ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->rho.as<float>(),
+                ctx->aniso.as<float4>(), n);
+        };
+        if (bd_threads == 64) dens(k_density<64>);
+        else if (bd_threads == 256) dens(k_density<256>);
+        else dens(k_density<128>);
+    }
     PMS_LAUNCHED(ctx);
     // ns is on the device; grids are sized by the particle count (an upper bound)
+    // (a thread per surface particle, or a warp where there are few: enough warps for both)
+    const unsigned mom_blocks = std::max(grid_for(n, (unsigned)bm), grid_for((uint64_t)n * 32, (unsigned)bm, 152u * (2048u / (unsigned)bm)));
     auto mom = [&](auto kern) {
-        kern<<<grid_for(ctx->n, (unsigned)bm), bm, 0, ctx->stream>>>(g, ap, ctx->slist.as<uint32_t>(), cnt,
+        kern<<<mom_blocks, bm, 0, ctx->stream>>>(g, ap, ctx->slist.as<uint32_t>(), cnt,
                                                                     ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(),
                                                                     ctx->spos.as<float4>(), ctx->moments.as<float4>());
     };

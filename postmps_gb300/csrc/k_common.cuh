@@ -171,6 +171,73 @@ __device__ __forceinline__ void row_walk(const KGrid& g, float3 p, uint3 lo, uin
     }
 }
 
+// A warp's list of up to 32 index ranges, one per lane, as one sequence: `off` + position is
+// the index in the range that holds the position.
+struct WarpRows {
+    uint32_t incl, off, total;
+};
+__device__ __forceinline__ WarpRows warp_rows(uint32_t first, uint32_t n) {
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((threadIdx.x & 31u) >= (uint32_t)o) incl += v;
+    }
+    return {incl, first - (incl - n), __shfl_sync(0xffffffffu, incl, 31)};
+}
+// the range (lane) holding position p: the first whose inclusive count exceeds it
+__device__ __forceinline__ int warp_row_of(const WarpRows& w, uint32_t p) {
+    int row = 0;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+        if (__shfl_sync(0xffffffffu, w.incl, row + s - 1) <= p) row += s;
+    return row;
+}
+
+// The particles of row `row` (z, y) of the slabs [za, ..) x [ya, ya + ny) whose cells come
+// within sqrt(r2) of the box [b0, b1] (a point when they are equal), x cells clipped to
+// [xlo, xhi): first index and count.  `pad` as in row_walk.
+__device__ __forceinline__ uint32_t box_row(const KGrid& g, float3 b0, float3 b1, float r2, float pad, int z, int y, int xlo,
+                                            int xhi, const uint32_t* __restrict__ cell_start, uint32_t& first) {
+    const float cs = g.sp_cs, inv = 1.f / g.sp_cs;
+    const float z0 = g.min_pos[2] + (float)z * cs, y0 = g.min_pos[1] + (float)y * cs;
+    const float gz = fmaxf(fmaxf(z0 - pad - b1.z, b0.z - (z0 + cs + pad)), 0.f);
+    const float gy = fmaxf(fmaxf(y0 - pad - b1.y, b0.y - (y0 + cs + pad)), 0.f);
+    const float gap = gz * gz + gy * gy;
+    if (gap >= r2) return 0u;
+    const float rc = sqrtf(r2 - gap) * inv + kRangeMargin;
+    const int xa = max((int)floorf((b0.x - g.min_pos[0]) * inv - rc), xlo);
+    const int xb = min((int)floorf((b1.x - g.min_pos[0]) * inv + rc) + 1, xhi);
+    if (xa >= xb) return 0u;
+    const uint32_t row = ((uint32_t)z * g.spres[1] + (uint32_t)y) * g.spres[0];
+    first = __ldg(&cell_start[row + (uint32_t)xa]);
+    return __ldg(&cell_start[row + (uint32_t)xb]) - first;
+}
+
+// Every particle in the window [lo, hi) (hi exclusive) whose cell comes within sqrt(r2) of p,
+// 32 at a time, one per lane: body(valid, j) for all lanes together, in ascending order.
+template <class Body>
+__device__ __forceinline__ void warp_walk(const KGrid& g, float3 p, uint3 lo, uint3 hi, float r2, float pad,
+                                          const uint32_t* __restrict__ cell_start, Body&& body) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const float inv = 1.f / g.sp_cs, rc = sqrtf(r2) * inv + kRangeMargin;
+    int za, zb, ya, yb;
+    cell_range((p.z - g.min_pos[2]) * inv, rc, lo.z, hi.z, za, zb);
+    cell_range((p.y - g.min_pos[1]) * inv, rc, lo.y, hi.y, ya, yb);
+    const int ny = yb - ya, nrow = ny > 0 && zb > za ? ny * (zb - za) : 0;
+    for (int r0 = 0; r0 < nrow; r0 += 32) {
+        const int r = r0 + (int)lane;
+        uint32_t first = 0u, n = 0u;
+        if (r < nrow) n = box_row(g, p, p, r2, pad, za + r / ny, ya + r % ny, (int)lo.x, (int)hi.x, cell_start, first);
+        const WarpRows rows = warp_rows(first, n);
+        for (uint32_t q0 = 0u; q0 < rows.total; q0 += 32u) {
+            const uint32_t q = q0 + lane;
+            const int row = warp_row_of(rows, q);
+            body(q < rows.total, __shfl_sync(0xffffffffu, rows.off, row) + q);
+        }
+    }
+}
+
 // rank of bit `id` among set bits of a bitmap with exclusive word prefix sums
 __device__ __forceinline__ uint32_t bit_rank(const uint32_t* bm, const uint32_t* wprefix, uint32_t id) {
     uint32_t w = id >> 5, b = id & 31u;

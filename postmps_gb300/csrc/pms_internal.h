@@ -79,6 +79,8 @@ struct Counters {
     uint32_t l_recheck;     // certified corners of valid cubes, evaluated exactly afterwards
     uint32_t n_items;       // work items (runs or tiles) of the last field launch
     uint32_t field_next;    // the next listed tile a warp of the field takes (both 0 before a launch)
+    uint32_t dens_blocks;   // blocks of cells the density pass visits, and its ticket (0 between passes)
+    uint32_t dens_next;
     uint32_t band_next;     // the next tile a warp of the band marking takes (0 between launches)
     uint32_t n_weld;        // vertices of the welded mesh (crossed grid edges)
     uint32_t n_df_total;    // generated + carried diffuse particles of a batched frame
