@@ -18,8 +18,7 @@
 namespace pms {
 
 static constexpr int kThreads = 256;
-static constexpr uint32_t kSmallCell = 64;     // per-thread insertion sort limit
-static constexpr uint32_t kBigCell = 4096;     // per-block bitonic sort limit
+static constexpr uint32_t kBigCell = 4096;     // most particles a cell may hold
 
 // ---------------------------------------------------------------------------
 // bounding box (FileData.cpp:240-257); non-finite positions are flagged
@@ -128,80 +127,32 @@ __global__ void __launch_bounds__(kThreads) k_zero(ZeroList z) {
     }
 }
 
-// One sorted particle.
-__device__ __forceinline__ void place(uint32_t dest, uint32_t i, uint32_t key, const float* __restrict__ pos,
-                                      const float* __restrict__ vel, uint32_t* __restrict__ skeys, float4* __restrict__ spos,
-                                      float4* __restrict__ svel) {
-    skeys[dest] = key;
-    spos[dest] = make_float4(pos[3 * (size_t)i], pos[3 * (size_t)i + 1], pos[3 * (size_t)i + 2], 0.f);
-    svel[dest] = make_float4(vel[3 * (size_t)i], vel[3 * (size_t)i + 1], vel[3 * (size_t)i + 2], 0.f);
-}
-
 // Ascending input order inside every cell, what a stable sort by key yields, and the payload
-// in that order.  In a cell of up to kSmallCell particles each finds its place by counting
-// the smaller indices among the cell's entries (neighbouring threads read the same few);
-// larger cells are queued for k_cell_sort_big.  (A thread per cell sorting its entries in
-// place, then a gather, took 35 + 35 us on 2M particles and 13 + 4 us on 4k, where the
-// serial sort of a cell is the latency; this takes 39 and 5.)
+// in that order: each particle finds its place by counting the smaller indices among its
+// cell's entries (neighbouring threads read the same few).  Of a cell past kBigCell the order
+// is left as scattered: the frame fails.  (A thread per cell sorting its entries in place, a
+// block-wide sort of large cells and a gather took 35 + 2 + 35 us on 2M particles and
+// 13 + 2 + 4 us on 4k, where the serial sort of a cell is the latency; this takes 39 and 5.)
 __global__ void __launch_bounds__(kThreads) k_place(const uint32_t* __restrict__ scattered, const uint32_t* __restrict__ keys,
                                                     const uint32_t* __restrict__ cell_start, const float* __restrict__ pos,
                                                     const float* __restrict__ vel, uint32_t n, uint32_t* __restrict__ order,
                                                     uint32_t* __restrict__ skeys, float4* __restrict__ spos,
-                                                    float4* __restrict__ svel, uint32_t* __restrict__ big,
-                                                    Counters* __restrict__ cnt) {
+                                                    float4* __restrict__ svel, Counters* __restrict__ cnt) {
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const uint32_t i = __ldg(&scattered[s]), key = __ldg(&keys[i]);
         const uint32_t st = __ldg(&cell_start[key]), m = __ldg(&cell_start[key + 1u]) - st;
         uint32_t dest = s;
-        if (m <= kSmallCell) {
+        if (m <= kBigCell) {
             dest = st;
+#pragma unroll 4
             for (uint32_t t = 0; t < m; ++t) dest += __ldg(&scattered[st + t]) < i ? 1u : 0u;
         } else if (s == st) {
-            big[atomicAdd(&cnt->n_big_cells, 1u)] = key;
-            if (m > kBigCell) atomicOr(&cnt->err, kErrBigCell);
+            atomicOr(&cnt->err, kErrBigCell);
         }
         order[dest] = i;
-        place(dest, i, key, pos, vel, skeys, spos, svel);
-    }
-}
-
-// One block per queued cell: bitonic sort in shared memory (<= kBigCell entries), and the
-// payload in the sorted order.
-__global__ void __launch_bounds__(1024) k_cell_sort_big(const uint32_t* __restrict__ cell_count,
-                                                        const uint32_t* __restrict__ cell_start,
-                                                        const uint32_t* __restrict__ big, const Counters* __restrict__ cnt,
-                                                        const float* __restrict__ pos, const float* __restrict__ vel,
-                                                        uint32_t* __restrict__ order, uint32_t* __restrict__ skeys,
-                                                        float4* __restrict__ spos, float4* __restrict__ svel) {
-    __shared__ uint32_t s[kBigCell];
-    uint32_t nb = cnt->n_big_cells;
-    for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
-        uint32_t c = big[b];
-        uint32_t m = cell_count[c];
-        if (m > kBigCell) continue;
-        uint32_t* a = order + cell_start[c];
-        uint32_t p2 = 1;
-        while (p2 < m) p2 <<= 1;
-        for (uint32_t i = threadIdx.x; i < p2; i += blockDim.x) s[i] = i < m ? a[i] : 0xffffffffu;
-        __syncthreads();
-        for (uint32_t k = 2; k <= p2; k <<= 1) {
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t i = threadIdx.x; i < p2; i += blockDim.x) {
-                    uint32_t l = i ^ j;
-                    if (l > i) {
-                        bool up = (i & k) == 0;
-                        uint32_t x = s[i], y = s[l];
-                        if ((x > y) == up) { s[i] = y; s[l] = x; }
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-            a[i] = s[i];
-            place(cell_start[c] + i, s[i], c, pos, vel, skeys, spos, svel);
-        }
-        __syncthreads();
+        skeys[dest] = key;
+        spos[dest] = make_float4(pos[3 * (size_t)i], pos[3 * (size_t)i + 1], pos[3 * (size_t)i + 2], 0.f);
+        svel[dest] = make_float4(vel[3 * (size_t)i], vel[3 * (size_t)i + 1], vel[3 * (size_t)i + 2], 0.f);
     }
 }
 
@@ -235,12 +186,7 @@ pms_status launch_hash_sort(pms_ctx* ctx) {
     k_place<<<gb, kThreads, 0, ctx->stream>>>(ctx->slist.as<uint32_t>(), ctx->keys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(),
                                               ctx->in_pos.as<float>(), ctx->in_vel.as<float>(), n, ctx->order.as<uint32_t>(),
                                               ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->svel.as<float4>(),
-                                              ctx->big_cells.as<uint32_t>(), cnt);
-    PMS_LAUNCHED(ctx);
-    k_cell_sort_big<<<32, 1024, 0, ctx->stream>>>(ctx->cell_count.as<uint32_t>(), ctx->cell_start.as<uint32_t>(),
-                                                   ctx->big_cells.as<uint32_t>(), cnt, ctx->in_pos.as<float>(),
-                                                   ctx->in_vel.as<float>(), ctx->order.as<uint32_t>(), ctx->skeys.as<uint32_t>(),
-                                                   ctx->spos.as<float4>(), ctx->svel.as<float4>());
+                                              cnt);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }

@@ -55,7 +55,7 @@ template <class F>
 static void for_each_dbuf(pms_ctx* c, F f) {
     DBuf* bufs[] = {&c->in_pos, &c->in_vel, &c->in_rho, &c->keys, &c->slot, &c->order, &c->skeys, &c->spos,
                     &c->svel, &c->rho, &c->cell_count, &c->cell_start, &c->cell_info, &c->surf_count,
-                    &c->surf_start, &c->big_cells, &c->slist, &c->moments, &c->cell_rad, &c->cell_rec, &c->aniso, &c->nrm4, &c->mean4, &c->gdebug,
+                    &c->surf_start, &c->slist, &c->moments, &c->cell_rad, &c->cell_rec, &c->aniso, &c->nrm4, &c->mean4, &c->gdebug,
                     &c->nnb, &c->bm0, &c->bm, &c->wcount, &c->wprefix, &c->vlist, &c->field, &c->mc_le,
                     &c->mc_valid, &c->mc_key, &c->mc_off, &c->fdense, &c->cube, &c->fitems, &c->fitem_cnt, &c->fitem_off, &c->ftiles, &c->vert, &c->vnorm, &c->sval, &c->d_isfree, &c->d_freescan,
                     &c->d_freelist, &c->d_pot, &c->d_num, &c->d_numscan, &c->d_isdiff, &c->d_isdiffscan,
@@ -209,7 +209,6 @@ pms_status pms::ensure_particle_buffers(pms_ctx* c, uint32_t n) {
     PMS_CUDA(c, c->mean4.ensure(16 * N));
     PMS_CUDA(c, c->gdebug.ensure(40 * N));
     PMS_CUDA(c, c->nnb.ensure(4 * N));
-    PMS_CUDA(c, c->big_cells.ensure(4 * (N / 64 + 2)));
     return PMS_OK;
 }
 
@@ -678,14 +677,12 @@ extern "C" pms_status pms_download_scalar_values(pms_ctx* c, float* vel_xyz, flo
     *n_out = m;
     if (!vel_xyz && !vel_len && !rhop) return PMS_OK;
     if (cap < m) return PMS_ERR_CAPACITY;
-    std::vector<float> sv(5 * (size_t)m);
-    if (m) PMS_CUDA(c, cudaMemcpyAsync(sv.data(), c->sval.p, 20 * (size_t)m, cudaMemcpyDeviceToHost, c->stream));
+    // device layout: velocities, lengths, densities (k_scalar_values)
+    const float* sv = c->sval.as<float>();
+    if (m && vel_xyz) PMS_CUDA(c, cudaMemcpyAsync(vel_xyz, sv, 12 * m, cudaMemcpyDeviceToHost, c->stream));
+    if (m && vel_len) PMS_CUDA(c, cudaMemcpyAsync(vel_len, sv + 3 * m, 4 * m, cudaMemcpyDeviceToHost, c->stream));
+    if (m && rhop) PMS_CUDA(c, cudaMemcpyAsync(rhop, sv + 4 * m, 4 * m, cudaMemcpyDeviceToHost, c->stream));
     PMS_CUDA(c, cudaStreamSynchronize(c->stream));
-    for (uint64_t i = 0; i < m; ++i) {
-        if (vel_xyz) { vel_xyz[3 * i] = sv[5 * i]; vel_xyz[3 * i + 1] = sv[5 * i + 1]; vel_xyz[3 * i + 2] = sv[5 * i + 2]; }
-        if (vel_len) vel_len[i] = sv[5 * i + 3];
-        if (rhop) rhop[i] = sv[5 * i + 4];
-    }
     return PMS_OK;
 }
 

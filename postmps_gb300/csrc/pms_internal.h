@@ -58,7 +58,6 @@ struct Counters {
     unsigned long long df_total;  // the spawn counts' scan total, spawning << 32 | generated
     unsigned long long n_pairs;  // (vertex, particle) pairs the field launches evaluated
     uint32_t n_fp64;        // covariances solved in FP64
-    uint32_t n_big_cells;   // cells with more particles than the per-thread sort handles
     uint32_t err;           // error bits (kErr*)
     uint32_t bbox_min[3];   // order-preserving integer encodings of the bbox
     uint32_t bbox_max[3];
@@ -201,7 +200,7 @@ struct pms_ctx {
     pms::DBuf in_pos, in_vel, in_rho;
     // hashing and sorted particle data
     pms::DBuf keys, slot, order, skeys, spos, svel, rho;
-    pms::DBuf cell_count, cell_start, cell_info, surf_count, surf_start, big_cells;
+    pms::DBuf cell_count, cell_start, cell_info, surf_count, surf_start;
     // anisotropy
     pms::DBuf slist, moments, aniso, nrm4, mean4, gdebug, nnb, cell_rad, cell_rec;
     // band
