@@ -33,7 +33,7 @@ struct AnisoParams {
     float nn_d2;     // |u| <= h      <=>  |u|^2 <= nn_d2  (|u| = sqrt of |u|^2, rounded)
     float w_d2;      // |u| < 2h      <=>  |u|^2 <= w_d2
     int min_nn;
-    uint32_t sp_size, spres_x;   // where the per-row radii start; cells per row
+    uint32_t sp_size, sp_rows, spres_x;   // cells, rows of cells, cells per row
     double cond_limit;
 };
 
@@ -575,10 +575,13 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
             for (int b = 0; b < 3; ++b) gd[3 * a + b] = G[a][b];
         gd[9] = maxv;
         nnb[s] = nn;
-        // per-cell, per-row and global support radius (positive floats order like their bits)
+        // per-cell, per-row, per-stretch and global support radius (positive floats order like their bits)
         const uint32_t key = skeys[i];
         atomicMax(reinterpret_cast<unsigned int*>(&cell_rad[key]), __float_as_uint(hs));
-        atomicMax(reinterpret_cast<unsigned int*>(&cell_rad[ap.sp_size + key / ap.spres_x]), __float_as_uint(hs));
+        const uint32_t row = key / ap.spres_x, x = key - row * ap.spres_x;
+        atomicMax(reinterpret_cast<unsigned int*>(&cell_rad[ap.sp_size + row]), __float_as_uint(hs));
+        atomicMax(reinterpret_cast<unsigned int*>(&cell_rad[ap.sp_size + ap.sp_rows + row * rad_segments(ap.spres_x) + x / kRadSeg]),
+                  __float_as_uint(hs));
         atomicMax(&cnt_w->rad_max_bits, __float_as_uint(hs));
     }
 }
@@ -606,6 +609,7 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
     ap.nn_d2 = sqrt_bound(P.h, true);
     ap.w_d2 = sqrt_bound(P.aniso_radius, false);
     ap.sp_size = g.sp_size;
+    ap.sp_rows = g.spres[1] * g.spres[2];
     ap.spres_x = g.spres[0];
     Counters* cnt = ctx->counters.as<Counters>();
     // block sizes of the neighbour walks are autotuned (64, 128 or 256 threads)

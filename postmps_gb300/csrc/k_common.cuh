@@ -103,6 +103,11 @@ __device__ __forceinline__ float cell_gap2(const KGrid& g, float3 p, uint32_t x,
 // cut changes no sum.
 constexpr float kRangeMargin = 0.01f;
 
+// Cells per stretch of a row that keeps its particles' largest support (the row's own largest
+// is often a lone particle's far along it).
+constexpr int kRadSeg = 8;
+__host__ __device__ __forceinline__ uint32_t rad_segments(uint32_t res_x) { return (res_x + kRadSeg - 1u) / kRadSeg; }
+
 // Relative margin on support radii used for culling: a particle's kernel is
 // non-zero only within its support (|G r| < 1 implies |r| < maxvalue * h), and
 // float rounding of |G r|^2 moves that edge by ~1e-6 relative at most.

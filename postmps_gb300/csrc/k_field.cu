@@ -351,28 +351,32 @@ k_field_cert(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const ui
 // Bound by instruction issue.  A walk per run of vertices (18 of 32 lanes active, its
 // rows, records and cell bounds costing more than the pairs) took 2.89 / 2.56 / 7.24 ms
 // for the field stage of the crown 2M / dam 8M / spray 151k (ratio 3) frames; tiles take
-// 1.03 / 1.23 / 0.96 ms (30 of 32 lanes active).  Of that:
+// 0.91 / 1.01 / 0.77 ms (28 of 32 lanes active, 3.0 instructions a cycle on the dam).  Of that:
 // - support boxes and the separating plane leave 41, 66 and 28 staged particles per tile of
 //   about 52 band vertices; the boxes alone left 60, 99 and 42 (1.29 / 1.64 / 1.22 ms);
+// - rows are cut by the largest support of their stretch of 8 cells, tiles listed with their
+//   coordinates, and the general path taken per cell (with rows cut by their own largest
+//   support and whole chunks taken generally: 1.03 / 1.23 / 0.96 ms with the clearing of
+//   the dense field, 0.05 ms);
 // - a lane's x-neighbours go through the packed two-float operations, rounded as the
-//   scalar ones, and the early exit is a limit on |G r|^2 rather than a flag.
-// K = 2 is the default: K = 1 stages fewer particles per tile but shares less of each
-// (1.50 / 1.78 / 1.41 ms), K = 4 the reverse (1.31 / 1.53 / 1.03 ms).
+//   scalar ones, and the early exit is a limit on |G r|^2 rather than a flag.  Staging the
+//   packed operands twice, as pairs, cost more than the moves it saves (1.07 / 1.09 / 0.81).
+// K = 2 is the default: K = 1 stages fewer particles per tile but shares less of each, K = 4
+// the reverse (before the row cuts 1.50 / 1.78 / 1.41 and 1.31 / 1.53 / 1.03 ms).
 // ---------------------------------------------------------------------------
 template <int K> struct FieldTile {
     static constexpr int X = K == 4 ? 8 : 4, Y = 4, Z = K == 1 ? 2 : 4;
 };
 static constexpr uint32_t kTileTicket = 4;      // consecutive listed tiles a warp takes at once
-// Resident warps per SM the registers are capped for.  Crown 2M / dam 8M field stage: 20 warps
-// (96 registers, no spills) 1.03 / 1.23 ms, 24 (80, spilling) 1.04 / 1.25, 16 1.15 / 1.36.
+// Resident warps per SM the registers are capped for.  Crown 2M / dam 8M field stage, before the
+// row cuts: 20 warps (96 registers, no spills) 1.03 / 1.23 ms, 24 1.04 / 1.25, 16 1.15 / 1.36.
 static constexpr int kFieldWarps = 20;
 
-// The tiles holding a set bit of a bitmap over the scalar grid: list[t] its tile
-// index, mask[K t + k] the lanes whose vertex k is set.
+// The tiles holding a set bit of a bitmap over the scalar grid, 3 + K words each: the
+// first vertex's x, y, z, then for k < K the lanes whose vertex k is set.
 template <int K>
 __global__ void __launch_bounds__(256) k_field_tile_list(KGrid g, uint3 td, const uint32_t* __restrict__ bm,
-                                                         uint32_t* __restrict__ n_tiles, uint32_t* __restrict__ list,
-                                                         uint32_t* __restrict__ mask) {
+                                                         uint32_t* __restrict__ n_tiles, uint32_t* __restrict__ list) {
     using T = FieldTile<K>;
     const uint32_t ntiles = td.x * td.y * td.z;
     const uint32_t rx = g.scres[0], ry = g.scres[1], rz = g.scres[2];
@@ -382,9 +386,8 @@ __global__ void __launch_bounds__(256) k_field_tile_list(KGrid g, uint3 td, cons
         uint32_t m[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) m[k] = 0u;
+        const uint32_t tx = t % td.x, tyz = t / td.x, ty = tyz % td.y, tz = tyz / td.y, x0 = tx * T::X;
         if (t < ntiles) {
-            const uint32_t tx = t % td.x, tyz = t / td.x, ty = tyz % td.y, tz = tyz / td.y;
-            const uint32_t x0 = tx * T::X;
             const uint32_t in = rx - x0 >= (uint32_t)T::X ? (1u << T::X) - 1u : (1u << (rx - x0)) - 1u;
 #pragma unroll
             for (int z = 0; z < T::Z; ++z)
@@ -413,32 +416,32 @@ __global__ void __launch_bounds__(256) k_field_tile_list(KGrid g, uint3 td, cons
         if (lane == 0u) base = atomicAdd(n_tiles, (uint32_t)__popc(vote));
         base = __shfl_sync(0xffffffffu, base, 0);
         if (any) {
-            const uint32_t e = base + (uint32_t)__popc(vote & ((1u << lane) - 1u));
-            list[e] = t;
+            uint32_t* e = list + (size_t)(3 + K) * (base + (uint32_t)__popc(vote & ((1u << lane) - 1u)));
+            e[0] = x0; e[1] = ty * T::Y; e[2] = tz * T::Z;
 #pragma unroll
-            for (int k = 0; k < K; ++k) mask[(size_t)K * e + k] = m[k];
+            for (int k = 0; k < K; ++k) e[3 + k] = m[k];
         }
     }
 }
 
-// A staged particle: position and packed kernel, its cell key, and whether its cell
-// differs from the one before.
+// A staged particle: position and packed kernel, its cell's x, and its row of cells with
+// two flags: the first particle of a cell, a cell that needs the general path.
 struct FieldStage {
     float4 a;     // x, y, z, m00
     float4 b;     // 2 m01, 2 m02, m11, 2 m12
-    float4 c;     // m22, w, key bits, new-cell flag
+    float4 c;     // m22, w, x bits, row bits | flags
 };
 static constexpr int kFieldStage = 64;
+static constexpr uint32_t kFresh = 1u << 31, kOdd = 1u << 30;   // (a row of cells is below 2^30: a grid is 4 cells wide at least)
 static constexpr float kNever = -1.0e30f;       // below any |G r|^2
 
 template <int BT, int K>
 __global__ void __launch_bounds__(BT, kFieldWarps * 32 / BT)
-k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cnt, const uint32_t* __restrict__ n_tiles_dev,
-              uint32_t* __restrict__ next, const uint32_t* __restrict__ list, const uint32_t* __restrict__ mask,
+k_field_tiles(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_t* __restrict__ n_tiles_dev,
+              uint32_t* __restrict__ next, const uint32_t* __restrict__ list,
               const uint32_t* __restrict__ cell_start, const float* __restrict__ cell_rad,
               const uint32_t* __restrict__ skeys, const float4* __restrict__ spos, const float4* __restrict__ aniso,
               float* __restrict__ fdense, Counters* __restrict__ cnt_w) {
-    using T = FieldTile<K>;
     constexpr unsigned kAll = 0xffffffffu;
     __shared__ FieldStage stage_all[BT / 32][kFieldStage];
     const uint32_t lane = threadIdx.x & 31u;
@@ -448,7 +451,9 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
     const int srx = (int)g.spres[0], sry = (int)g.spres[1], srz = (int)g.spres[2];
     const int e2 = 2 * g.spexpand;
     const float pad = 1e-4f * g.sp_cs, cs = g.sp_cs, inv_cs = 1.f / g.sp_cs;
-    const float* __restrict__ row_rad = cell_rad + g.sp_size;
+    // largest support per stretch of kRadSeg cells of a row
+    const float* __restrict__ seg_rad = cell_rad + g.sp_size + g.spres[1] * g.spres[2];
+    const uint32_t nseg = rad_segments(g.spres[0]);
     const float rmax = fmaxf(__uint_as_float(cnt->rad_max_bits), fp.h) * fp.grow;
     const float rmax2 = rmax * rmax;
     // the lane's place in a tile
@@ -465,12 +470,11 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
         if (first >= n_tiles) break;
         const uint32_t last = min(first + ticket, n_tiles);
         for (uint32_t e = first; e < last; ++e) {
-            const uint32_t t = __ldg(&list[e]);
+            const uint32_t* tile = list + (size_t)(3 + K) * e;
             uint32_t m[K];
 #pragma unroll
-            for (int k = 0; k < K; ++k) m[k] = __ldg(&mask[(size_t)K * e + k]);
-            const uint32_t tx = t % td.x, tyz = t / td.x, ty = tyz % td.y, tz = tyz / td.y;
-            const uint32_t ix = tx * T::X + lx, iy = ty * T::Y + ly, iz = tz * T::Z + lz;
+            for (int k = 0; k < K; ++k) m[k] = __ldg(&tile[3 + k]);
+            const uint32_t ix = __ldg(&tile[0]) + lx, iy = __ldg(&tile[1]) + ly, iz = __ldg(&tile[2]) + lz;
             const float vy = sc_coord(g, iy, 1), vz = sc_coord(g, iz, 2);
             float vx[K], sum[K];
             float lim[K];                            // |G r|^2 below which a particle adds: 1, or never
@@ -486,7 +490,7 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
                 nvert += (uint32_t)__popc(m[k]);
                 if (have[k]) { x_lo = min(x_lo, ix + (uint32_t)k); x_hi = max(x_hi, ix + (uint32_t)k); some = true; }
             }
-            // the box of the tile's band vertices, and the spatial cells of its corners
+            // the box of the tile's band vertices
             x_lo = __reduce_min_sync(kAll, x_lo);
             x_hi = __reduce_max_sync(kAll, x_hi);
             const uint32_t y_lo = __reduce_min_sync(kAll, some ? iy : 0xffffffffu), y_hi = __reduce_max_sync(kAll, some ? iy : 0u);
@@ -494,25 +498,29 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
             const float bx0 = sc_coord(g, x_lo, 0), bx1 = sc_coord(g, x_hi, 0);
             const float by0 = sc_coord(g, y_lo, 1), by1 = sc_coord(g, y_hi, 1);
             const float bz0 = sc_coord(g, z_lo, 2), bz1 = sc_coord(g, z_hi, 2);
-            const uint3 c0 = sp_cell(g, bx0, by0, bz0), c1 = sp_cell(g, bx1, by1, bz1);
-            // cells some vertex's window holds [ulo, uhi), and cells that every window holds
-            // past its first column [ilo, ihi); near the grid's low side, where the reference's
-            // unsigned window wraps, every cell takes the general path
-            const bool regular = min(c0.x, min(c0.y, c0.z)) >= (uint32_t)e2;
-            const int ulx = regular ? (int)c0.x - e2 : 0, uhx = regular ? min((int)c1.x + e2, srx - 1) : srx;
-            const int uly = regular ? (int)c0.y - e2 : 0, uhy = regular ? min((int)c1.y + e2, sry - 1) : sry;
-            const int ulz = regular ? (int)c0.z - e2 : 0, uhz = regular ? min((int)c1.z + e2, srz - 1) : srz;
-            const int ilx = (int)c1.x - e2 + 1, ihx = regular ? min((int)c0.x + e2, srx - 1) : 0;
-            const int ily = (int)c1.y - e2, ihy = min((int)c0.y + e2, sry - 1);
-            const int ilz = (int)c1.z - e2, ihz = min((int)c0.z + e2, srz - 1);
             const float ux0 = (bx0 - g.min_pos[0]) * inv_cs, ux1 = (bx1 - g.min_pos[0]) * inv_cs;
             const float uy0 = (by0 - g.min_pos[1]) * inv_cs, uy1 = (by1 - g.min_pos[1]) * inv_cs;
             const float uz0 = (bz0 - g.min_pos[2]) * inv_cs, uz1 = (bz1 - g.min_pos[2]) * inv_cs;
+            // cells some vertex's window holds [u.., u..), and cells that every window holds past
+            // its first column [i.., i..), from the corners' cells taken kRangeMargin apart (the
+            // vertices' own cells lie between); near the grid's low side, where the reference's
+            // unsigned window wraps, every cell takes the general path
+            const int cx0 = (int)floorf(ux0 - kRangeMargin), cx1 = (int)floorf(ux1 + kRangeMargin);
+            const int cy0 = (int)floorf(uy0 - kRangeMargin), cy1 = (int)floorf(uy1 + kRangeMargin);
+            const int cz0 = (int)floorf(uz0 - kRangeMargin), cz1 = (int)floorf(uz1 + kRangeMargin);
+            const bool regular = min(cx0, min(cy0, cz0)) >= e2;
+            const int ulx = regular ? cx0 - e2 : 0, uhx = regular ? min(cx1 + e2, srx - 1) : srx;
+            const int uly = regular ? cy0 - e2 : 0, uhy = regular ? min(cy1 + e2, sry - 1) : sry;
+            const int ulz = regular ? cz0 - e2 : 0, uhz = regular ? min(cz1 + e2, srz - 1) : srz;
+            const int ilx = cx1 - e2 + 1, ihx = regular ? min(cx0 + e2, srx - 1) : 0;
+            const int ily = cy1 - e2, ihy = min(cy0 + e2, sry - 1);
+            const int ilz = cz1 - e2, ihz = min(cz0 + e2, srz - 1);
             // rows (z, y) within the frame's largest support of the box
             const float rc = rmax * inv_cs + kRangeMargin;
             const int za = max((int)floorf(uz0 - rc), ulz), zb = min((int)floorf(uz1 + rc) + 1, uhz);
             const int ya = max((int)floorf(uy0 - rc), uly), yb = min((int)floorf(uy1 + rc) + 1, uhy);
             const int ny = yb - ya, nrow = ny > 0 && zb > za ? ny * (zb - za) : 0;
+            const int xa0 = max((int)floorf(ux0 - rc), ulx), xb0 = min((int)floorf(ux1 + rc) + 1, uhx);
 
             int staged = 0;
             bool odd = false;                        // a staged particle needs the general path
@@ -536,11 +544,14 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
 #pragma unroll 2
                 for (int i = 0; i < staged; ++i) {
                     const float4 a = stage[i].a, b = stage[i].b, c = stage[i].c;
-                    const bool fresh = c.w != 0.f;   // the first particle of a cell
+                    const uint32_t cw = __float_as_uint(c.w);
+                    const bool fresh = (cw & kFresh) != 0u;
                     if constexpr (G) {
-                        if (fresh) {
-                            const uint32_t key = __float_as_uint(c.z);
-                            const int row = (int)(key / (uint32_t)srx), x = (int)(key - (uint32_t)row * (uint32_t)srx);
+                        if (fresh && !(cw & kOdd)) {
+#pragma unroll
+                            for (int k = 0; k < K; ++k) lim[k] = sum[k] > fp.thr ? kNever : 1.f;
+                        } else if (fresh) {
+                            const int row = (int)(cw & (kOdd - 1u)), x = __float_as_int(c.z);
                             const int z = row / sry, y = row - z * sry;
                             const bool in = y >= wy0 && y < wy1 && z >= wz0 && z < wz1;
 #pragma unroll
@@ -591,15 +602,19 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
             for (int r0 = 0; r0 < nrow; r0 += 32) {
                 // a row per lane: its cells within the row's largest support of the box
                 const int r = r0 + (int)lane;
-                uint32_t ja = 0u, n = 0u, zy = 0u;
+                uint32_t ja = 0u, n = 0u, rowi = 0u;
+                bool inner = false;
                 if (r < nrow) {
                     const int z = za + r / ny, y = ya + r % ny;
-                    const uint32_t rowi = (uint32_t)z * (uint32_t)sry + (uint32_t)y;
+                    rowi = (uint32_t)z * (uint32_t)sry + (uint32_t)y;
                     const float z0 = g.min_pos[2] + (float)z * cs, y0 = g.min_pos[1] + (float)y * cs;
                     const float gz = fmaxf(fmaxf(z0 - pad - bz1, bz0 - (z0 + cs + pad)), 0.f);
                     const float gy = fmaxf(fmaxf(y0 - pad - by1, by0 - (y0 + cs + pad)), 0.f);
                     const float gyz = gz * gz + gy * gy;
-                    const float rr = fmaxf(__ldg(&row_rad[rowi]), fp.h) * fp.grow;
+                    float rr = fp.h;                 // the row's largest support where the tile can reach it
+                    if (gyz < rmax2)
+                        for (int s = xa0 / kRadSeg; s * kRadSeg < xb0; ++s) rr = fmaxf(rr, __ldg(&seg_rad[rowi * nseg + (uint32_t)s]));
+                    rr *= fp.grow;
                     const float rr2 = rr * rr;
                     if (gyz < rr2) {
                         const float rxc = sqrtf(rr2 - gyz) * inv_cs + kRangeMargin;
@@ -610,29 +625,20 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
                             n = __ldg(&cell_start[row + (uint32_t)xb]) - ja;
                         }
                     }
-                    zy = (z >= ilz && z < ihz && y >= ily && y < ihy) ? 1u : 0u;
+                    inner = z >= ilz && z < ihz && y >= ily && y < ihy;
                 }
-                uint32_t incl = n;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t v = __shfl_up_sync(kAll, incl, o);
-                    if (lane >= (uint32_t)o) incl += v;
-                }
-                const uint32_t total = __shfl_sync(kAll, incl, 31);
-                const uint32_t off = ja - (incl - n);          // particle index = off + position in the rows' list
-                for (uint32_t p0 = 0u; p0 < total; p0 += 32u) {
+                // (the row's index, with the flag of a row outside some vertex's window)
+                const uint32_t row_tag = rowi | (inner ? 0u : kOdd);
+                const WarpRows rows = warp_rows(ja, n);
+                for (uint32_t p0 = 0u; p0 < rows.total; p0 += 32u) {
                     const uint32_t p = p0 + lane;
-                    // the row holding position p: the first whose inclusive count exceeds p
-                    int row = 0;
-#pragma unroll
-                    for (int s = 16; s > 0; s >>= 1)
-                        if (__shfl_sync(kAll, incl, row + s - 1) <= p) row += s;
-                    const uint32_t j = __shfl_sync(kAll, off, row) + p;
-                    const uint32_t inner_row = __shfl_sync(kAll, zy, row);
+                    const int row = warp_row_of(rows, p);
+                    const uint32_t j = __shfl_sync(kAll, rows.off, row) + p;
+                    const uint32_t tag = __shfl_sync(kAll, row_tag, row);
                     bool keep = false;
                     float4 q, a0, a1;
                     uint32_t key = 0u;
-                    if (p < total) {
+                    if (p < rows.total) {
                         q = __ldg(&spos[j]);
                         a0 = __ldg(&aniso[2 * (size_t)j]);
                         key = __ldg(&skeys[j]);
@@ -660,15 +666,18 @@ k_field_tiles(KGrid g, FieldParams fp, uint3 td, const Counters* __restrict__ cn
                     const uint32_t below = kept & ((1u << lane) - 1u);
                     const uint32_t prev = __shfl_sync(kAll, key, below ? 31 - __clz(below) : 0);
                     const uint32_t key_last = __shfl_sync(kAll, key, 31 - __clz(kept));
+                    bool my_odd = false;
                     if (keep) {
                         const bool fresh = key != (below ? prev : key_before);
+                        const int x = (int)(key - (tag & (kOdd - 1u)) * (uint32_t)srx);
+                        my_odd = (tag & kOdd) || x < ilx || x >= ihx;
                         FieldStage& s = stage[staged + __popc(below)];
                         s.a = make_float4(q.x, q.y, q.z, a0.x);
                         s.b = make_float4(a0.y, a0.z, a1.x, a1.y);
-                        s.c = make_float4(a1.z, a1.w, __uint_as_float(key), fresh ? 1.f : 0.f);
+                        s.c = make_float4(a1.z, a1.w, __int_as_float(x),
+                                          __uint_as_float((tag & (kOdd - 1u)) | (my_odd ? kOdd : 0u) | (fresh ? kFresh : 0u)));
                     }
-                    const int x = (int)(key % (uint32_t)srx);
-                    odd |= __any_sync(kAll, keep && !(inner_row && x >= ilx && x < ihx));
+                    odd |= __any_sync(kAll, my_odd);
                     key_before = key_last;
                     staged += __popc(kept);
                     if (staged > kFieldStage - 32) flush();
@@ -690,7 +699,7 @@ static uint3 field_tile_dims(const pms_grid& g) {
     return make_uint3((g.scres[0] + T::X - 1) / T::X, (g.scres[1] + T::Y - 1) / T::Y, (g.scres[2] + T::Z - 1) / T::Z);
 }
 
-// the listed tiles of a bitmap of at most nv set bits: an index and K lane masks each
+// the listed tiles of a bitmap of at most nv set bits
 template <int K>
 static uint64_t field_tile_most(const pms_grid& g, uint64_t nv) {
     const uint3 td = field_tile_dims<K>(g);
@@ -698,7 +707,7 @@ static uint64_t field_tile_most(const pms_grid& g, uint64_t nv) {
 }
 template <int K>
 static size_t field_tile_bytes_of(const pms_grid& g, uint64_t nv) {
-    return 4 * (size_t)(1 + K) * (field_tile_most<K>(g, nv) + 1);
+    return 4 * (size_t)(3 + K) * (field_tile_most<K>(g, nv) + 1);
 }
 size_t field_tile_bytes(const pms_grid& g, int vpt, uint64_t nv) {
     return vpt == 1 ? field_tile_bytes_of<1>(g, nv) : vpt == 4 ? field_tile_bytes_of<4>(g, nv) : field_tile_bytes_of<2>(g, nv);
@@ -719,17 +728,16 @@ static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, uint64_t n_ho
     const uint64_t ntiles = (uint64_t)td.x * td.y * td.z, most = field_tile_most<K>(ctx->grid, n_host);
     PMS_CUDA(ctx, ctx->ftiles.ensure_grow(field_tile_bytes_of<K>(ctx->grid, n_host)));
     uint32_t* list = ctx->ftiles.as<uint32_t>();
-    uint32_t* mask = list + most + 1;
     // the list's length and the next ticket start at 0: the band left them so, for one launch
     if (!ctx->field_tickets_zero) PMS_CUDA(ctx, cudaMemsetAsync(&cnt->n_items, 0, 2 * sizeof(uint32_t), ctx->stream));
     ctx->field_tickets_zero = false;
-    k_field_tile_list<K><<<grid_for(ntiles, 256), 256, 0, ctx->stream>>>(g, td, bm, &cnt->n_items, list, mask);
+    k_field_tile_list<K><<<grid_for(ntiles, 256), 256, 0, ctx->stream>>>(g, td, bm, &cnt->n_items, list);
     PMS_LAUNCHED(ctx);
     const int bt = ctx->tune.field_threads;
     const unsigned per_sm = kFieldWarps * 32u / (unsigned)bt;
     const unsigned blocks = grid_for(most, (unsigned)bt / 32u, 152u * per_sm);
     auto go = [&](auto kern) {
-        kern<<<blocks, bt, 0, ctx->stream>>>(g, fp, td, cnt, &cnt->n_items, &cnt->field_next, list, mask,
+        kern<<<blocks, bt, 0, ctx->stream>>>(g, fp, cnt, &cnt->n_items, &cnt->field_next, list,
                                              ctx->cell_start.as<uint32_t>(), ctx->cell_rad.as<float>(),
                                              ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(),
                                              ctx->fdense.as<float>(), cnt);

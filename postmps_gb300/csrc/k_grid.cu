@@ -163,7 +163,8 @@ pms_status launch_hash_sort(pms_ctx* ctx) {
     // the cell counts, the support radii the anisotropy pass raises, the band's marks: all start
     // at 0, and a stage run again on the same frame sets the same values
     const ZeroList z = {{ctx->cell_count.as<uint32_t>(), ctx->cell_rad.as<uint32_t>(), ctx->bm0.as<uint32_t>()},
-                        {g.sp_size, (uint64_t)g.sp_size + (uint64_t)g.spres[1] * g.spres[2], ((uint64_t)g.sc_size + 31) / 32}};
+                        {g.sp_size, g.sp_size + (uint64_t)g.spres[1] * g.spres[2] * (1 + rad_segments(g.spres[0])),
+                         ((uint64_t)g.sc_size + 31) / 32}};
     k_zero<<<grid_for((z.n[0] + z.n[1] + z.n[2]) / 16 + 1, kThreads, 152 * 8), kThreads, 0, ctx->stream>>>(z);
     PMS_LAUNCHED(ctx);
     const unsigned gb = grid_for(n, kThreads);

@@ -219,7 +219,8 @@ pms_status pms::ensure_grid_buffers(pms_ctx* c, const pms_grid& g) {
     PMS_CUDA(c, c->cell_info.ensure(8 * S));
     PMS_CUDA(c, c->surf_count.ensure(4 * S));
     PMS_CUDA(c, c->surf_start.ensure(4 * S));
-    PMS_CUDA(c, c->cell_rad.ensure(4 * (S + (size_t)g.spres[1] * g.spres[2])));   // per cell, then per row
+    // largest supports per cell, then per row, then per stretch of 8 cells of a row
+    PMS_CUDA(c, c->cell_rad.ensure(4 * (S + S / 8 + 2 * (size_t)g.spres[1] * g.spres[2])));
     PMS_CUDA(c, c->cell_rec.ensure(32 * S));   // two float4 per cell
     PMS_CUDA(c, c->fdense.ensure(4 * ((size_t)g.sc_size + 1)));
     const size_t W = ((uint64_t)g.sc_size + 31) / 32 + 1;
