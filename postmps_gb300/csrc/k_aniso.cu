@@ -67,8 +67,19 @@ __device__ __forceinline__ float mass_over(float mass, float r) { return r == 0.
 // beyond h adds exactly 0).  Bound by L1 (93 %: each lane loading its own neighbours)
 // before, by instruction issue now: dam 8M 1.47 -> 1.17 ms, crown 2M 0.36 -> 0.28, block 4k 23 -> 7 us.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void put_density(const AnisoParams& ap, uint32_t i, float w, uint32_t ext, float* __restrict__ rho,
-                                            float4* __restrict__ aniso) {
+//
+// The pass also writes the surface list (compactationOfParticles, Anisotropic_kernel.cuh:127-155):
+// a particle of a surface cell takes the cell's place in the scan of the surface counts plus
+// its own in the cell (a launch of its own took 30 us on 8M particles).
+struct SurfaceList {
+    const uint2* __restrict__ cell_info;      // {first particle, count | surface << 31}
+    const uint32_t* __restrict__ surf_start;
+    uint32_t* __restrict__ list;
+};
+__device__ __forceinline__ void put_density(const AnisoParams& ap, const SurfaceList& sl, uint32_t i, uint32_t key, float w,
+                                            uint32_t ext, float* __restrict__ rho, float4* __restrict__ aniso) {
+    const uint2 ci = __ldg(&sl.cell_info[key]);
+    if (ci.y & 0x80000000u) sl.list[__ldg(&sl.surf_start[key]) + (i - ci.x)] = i;
     const float r = ap.kdens * w, inv_h2 = ap.h_inv * ap.h_inv;
     rho[i] = r;
     aniso[2 * (size_t)i + 0] = make_float4(inv_h2, 0.f, 0.f, __uint_as_float(ext));
@@ -76,7 +87,8 @@ __device__ __forceinline__ void put_density(const AnisoParams& ap, uint32_t i, f
 }
 
 template <int BT>
-__global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams ap, const uint32_t* __restrict__ skeys,
+__global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams ap, SurfaceList sl,
+                                                      const uint32_t* __restrict__ skeys,
                                                       const uint32_t* __restrict__ cell_start, const float4* __restrict__ spos,
                                                       float* __restrict__ rho, float4* __restrict__ aniso, uint32_t n) {
     const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1];
@@ -97,13 +109,14 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams 
             const float s = density_term(p.x - q.x, p.y - q.y, p.z - q.z, ap.inv_h2);
             w = fmaf(s * s, s, w);
         });
-        put_density(ap, i, w, ext, rho, aniso);
+        put_density(ap, sl, i, key, w, ext, rho, aniso);
     }
 }
 
 // a warp per particle: the lanes work out 32 neighbours' terms, then add the non-zero ones in
 // their order
-__global__ void __launch_bounds__(kThreads) k_density_warp(KGrid g, AnisoParams ap, const uint32_t* __restrict__ skeys,
+__global__ void __launch_bounds__(kThreads) k_density_warp(KGrid g, AnisoParams ap, SurfaceList sl,
+                                                           const uint32_t* __restrict__ skeys,
                                                            const uint32_t* __restrict__ cell_start,
                                                            const float4* __restrict__ spos, float* __restrict__ rho,
                                                            float4* __restrict__ aniso, uint32_t n) {
@@ -131,7 +144,7 @@ __global__ void __launch_bounds__(kThreads) k_density_warp(KGrid g, AnisoParams 
                 w = fmaf(__shfl_sync(0xffffffffu, ss, l), __shfl_sync(0xffffffffu, s, l), w);
             }
         });
-        if (lane == 0u) put_density(ap, i, w, ext, rho, aniso);
+        if (lane == 0u) put_density(ap, sl, i, key, w, ext, rho, aniso);
     }
 }
 
@@ -170,7 +183,8 @@ __device__ __forceinline__ float warp_min(float v) { return from_ordered_bits(__
 __device__ __forceinline__ float warp_max(float v) { return from_ordered_bits(__reduce_max_sync(0xffffffffu, ordered_bits(v))); }
 
 template <int BT>
-__global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoParams ap, uint3 bd,
+__global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoParams ap, SurfaceList sl, uint3 bd,
+                                                                 const uint32_t* __restrict__ skeys,
                                                                  const uint32_t* __restrict__ n_blocks_dev,
                                                                  uint32_t* __restrict__ next, const uint32_t* __restrict__ list,
                                                                  const uint32_t* __restrict__ cell_start,
@@ -251,7 +265,7 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoP
                 }
             }
             if (staged) flush();
-            if (t0 + lane < mine.total) put_density(ap, id, w, ext, rho, aniso);
+            if (t0 + lane < mine.total) put_density(ap, sl, id, __ldg(&skeys[id]), w, ext, rho, aniso);
         }
     }
 }
@@ -615,9 +629,10 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
     // block sizes of the neighbour walks are autotuned (64, 128 or 256 threads)
     const int bd_threads = ctx->tune.density_threads, bm = ctx->tune.moments_threads;
     const uint32_t n = ctx->n;
+    const SurfaceList sl = {ctx->cell_info.as<uint2>(), ctx->surf_start.as<uint32_t>(), ctx->slist.as<uint32_t>()};
     if (n <= kDensityWarp) {
         k_density_warp<<<grid_for((uint64_t)n * 32, kThreads, 152u * 16u), kThreads, 0, ctx->stream>>>(
-            g, ap, ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->rho.as<float>(),
+            g, ap, sl, ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->rho.as<float>(),
             ctx->aniso.as<float4>(), n);
     } else if ((float)g.spexpand * g.sp_cs - P.h >= kRangeMargin * g.sp_cs) {
         const uint3 bd = make_uint3((g.spres[0] + kDensX - 1) / kDensX, (g.spres[1] + kDensY - 1) / kDensY,
@@ -629,7 +644,7 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
         PMS_LAUNCHED(ctx);
         auto tiles = [&](auto kern) {
             kern<<<152u * (1024u / (unsigned)bd_threads), bd_threads, 0, ctx->stream>>>(
-                g, ap, bd, &cnt->dens_blocks, &cnt->dens_next, list, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
+                g, ap, sl, bd, ctx->skeys.as<uint32_t>(), &cnt->dens_blocks, &cnt->dens_next, list, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
                 ctx->rho.as<float>(), ctx->aniso.as<float4>());
         };
         if (bd_threads == 64) tiles(k_density_tiles<64>);
@@ -638,8 +653,8 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
     } else {
         auto dens = [&](auto kern) {
             kern<<<grid_for(n, (unsigned)bd_threads), bd_threads, 0, ctx->stream>>>(
-                g, ap, ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->rho.as<float>(),
-                ctx->aniso.as<float4>(), n);
+                g, ap, sl, ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
+                ctx->rho.as<float>(), ctx->aniso.as<float4>(), n);
         };
         if (bd_threads == 64) dens(k_density<64>);
         else if (bd_threads == 256) dens(k_density<256>);

@@ -17,9 +17,10 @@
 // row needs of them; each tile row then lands in the global bitmap with at most two
 // atomics.  The dilation is a pass over the bitmap:
 // B = B0 | B0<<1 | B0<<rx | B0<<(rx*ry) in linear bit order (the reference's
-// index arithmetic, including its row wrap).  The compaction is a popcount per
-// 32-bit word, one scan over words and a per-word bit extraction.  The bitmap
-// (S_sc / 8 bytes) replaces three dense S_sc-sized uint arrays.
+// index arithmetic, including its row wrap), which also counts the band.  The bitmap
+// (S_sc / 8 bytes) replaces three dense S_sc-sized uint arrays; a list of the band (a
+// popcount per 32-bit word, one scan over words and a per-word bit extraction) is made
+// only for downloads.
 #include <algorithm>
 
 #include "pms_internal.h"
@@ -100,13 +101,14 @@ __device__ __forceinline__ uint32_t row_surface(const uint32_t* __restrict__ sur
 static constexpr int kBandThreads = 128, kBandStage = 64;
 
 __global__ void __launch_bounds__(kBandThreads, 8) k_band_tiles(KGrid g, float h, int ext, TileDims td,
-                                                                uint32_t n_tiles, uint32_t shares, uint32_t* __restrict__ next,
+                                                                uint32_t n_tiles, uint32_t shares, Counters* __restrict__ cnt,
                                                                 const uint32_t* __restrict__ surf_start,
                                                                 const uint32_t* __restrict__ surf_count,
                                                                 const uint32_t* __restrict__ slist,
                                                                 const float4* __restrict__ spos, const float4* __restrict__ nrm4,
                                                                 uint32_t* __restrict__ bm0) {
     constexpr unsigned kAll = 0xffffffffu;
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt->nv = 0u;     // the dilation counts the band
     __shared__ float4 s_p[kBandThreads / 32][kBandStage];      // p, n.x
     __shared__ float4 s_n[kBandThreads / 32][kBandStage];      // n.y, n.z, flag
     __shared__ uint2 s_m[kBandThreads / 32][kBandStage];       // x positions, tile rows inside box and AABB
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(kBandThreads, 8) k_band_tiles(KGrid g, float h
     uint32_t ti = 0u, ti_end = 0u;
     for (;;) {
         if (ti == ti_end) {
-            if (lane == 0u) ti = atomicAdd(next, ticket);
+            if (lane == 0u) ti = atomicAdd(&cnt->band_next, ticket);
             ti = __shfl_sync(kAll, ti, 0);
             if (ti >= n_work) break;
             ti_end = min(ti + ticket, n_work);
@@ -258,18 +260,29 @@ __device__ __forceinline__ uint32_t shifted_word(const uint32_t* __restrict__ b,
     return (hi << r) | (lo >> (32u - r));
 }
 
-// LOWRES dilation (Anisotropic_kernel.cuh:610-629) and popcount per word
+// LOWRES dilation (Anisotropic_kernel.cuh:610-629) and the band's size (Counters::nv, which the
+// marking set to 0)
 __global__ void __launch_bounds__(256) k_band_dilate(const uint32_t* __restrict__ bm0, uint32_t* __restrict__ bm,
-                                                     uint32_t* __restrict__ wcount, uint64_t nwords, uint64_t nbits,
+                                                     uint64_t nwords, uint64_t nbits,
                                                      uint64_t sy, uint64_t sz, Counters* __restrict__ cnt) {
     // the tickets of the next launches that take any start at 0
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt->band_next = cnt->n_items = cnt->field_next = 0u;
+    uint32_t mine = 0u;
     for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t v = bm0[w] | shifted_word(bm0, w, 1) | shifted_word(bm0, w, sy) | shifted_word(bm0, w, sz);
         if (w == nwords - 1 && (nbits & 31u)) v &= (1u << (nbits & 31u)) - 1u;
         bm[w] = v;
-        wcount[w] = __popc(v);
+        mine += (uint32_t)__popc(v);
     }
+    const uint32_t tot = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31u) == 0u && tot) atomicAdd(&cnt->nv, tot);
+}
+
+// popcount per word
+__global__ void __launch_bounds__(256) k_word_popc(const uint32_t* __restrict__ b, uint32_t* __restrict__ wcount,
+                                                   uint64_t nwords) {
+    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < nwords; w += (uint64_t)gridDim.x * blockDim.x)
+        wcount[w] = __popc(b[w]);
 }
 
 // ascending vertex list from the bitmap
@@ -307,16 +320,16 @@ pms_status launch_band(pms_ctx* ctx) {
     const uint64_t warps = 152u * 8u * (kBandThreads / 32);
     const uint32_t shares = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(warps / ntiles, 1u), 8u);
     k_band_tiles<<<grid_for(ntiles * shares * 32, kBandThreads, 152u * 8u), kBandThreads, 0, ctx->stream>>>(
-        g, ctx->prm.h, ext_dev, td, (uint32_t)ntiles, shares, &cnt->band_next, ctx->surf_start.as<uint32_t>(),
+        g, ctx->prm.h, ext_dev, td, (uint32_t)ntiles, shares, cnt, ctx->surf_start.as<uint32_t>(),
         ctx->surf_count.as<uint32_t>(), ctx->slist.as<uint32_t>(), ctx->spos.as<float4>(), ctx->nrm4.as<float4>(),
         ctx->bm0.as<uint32_t>());
     PMS_LAUNCHED(ctx);
     const uint64_t sy = g.scres[0], sz = (uint64_t)g.scres[0] * g.scres[1];
-    k_band_dilate<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(ctx->bm0.as<uint32_t>(), ctx->bm.as<uint32_t>(),
-                                                                  ctx->wcount.as<uint32_t>(), nwords, nbits, sy, sz, cnt);
+    k_band_dilate<<<grid_for(nwords, 256, 152u * 8u), 256, 0, ctx->stream>>>(ctx->bm0.as<uint32_t>(), ctx->bm.as<uint32_t>(), nwords,
+                                                                            nbits, sy, sz, cnt);
     PMS_LAUNCHED(ctx);
     ctx->field_tickets_zero = true;
-    return scan_u32(ctx, ctx->wcount.as<uint32_t>(), ctx->wprefix.as<uint32_t>(), nwords, &cnt->nv);
+    return PMS_OK;
 }
 
 pms_status launch_bits_list(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t* vlist) {
@@ -328,10 +341,13 @@ pms_status launch_bits_list(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wp
 
 pms_status launch_band_list(pms_ctx* ctx) {
     const uint64_t nwords = ((uint64_t)ctx->grid.sc_size + 31) / 32;
-    k_band_list<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(ctx->bm.as<uint32_t>(), ctx->wprefix.as<uint32_t>(),
-                                                                nwords, ctx->vlist.as<uint32_t>());
+    PMS_CUDA(ctx, ctx->wcount.ensure(4 * (nwords + 1)));
+    PMS_CUDA(ctx, ctx->wprefix.ensure(4 * (nwords + 1)));
+    k_word_popc<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(ctx->bm.as<uint32_t>(), ctx->wcount.as<uint32_t>(), nwords);
     PMS_LAUNCHED(ctx);
-    return PMS_OK;
+    pms_status st = scan_u32(ctx, ctx->wcount.as<uint32_t>(), ctx->wprefix.as<uint32_t>(), nwords, nullptr);
+    if (st != PMS_OK) return st;
+    return launch_bits_list(ctx, ctx->bm.as<uint32_t>(), ctx->wprefix.as<uint32_t>(), ctx->vlist.as<uint32_t>());
 }
 
 }  // namespace pms

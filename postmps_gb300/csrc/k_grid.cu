@@ -220,18 +220,6 @@ __global__ void __launch_bounds__(kThreads) k_surface_cells(KGrid g, const uint3
     }
 }
 
-// compactationOfParticles (Anisotropic_kernel.cuh:127-155), particle-parallel
-__global__ void __launch_bounds__(kThreads) k_surface_list(const uint32_t* __restrict__ skeys, uint32_t n,
-                                                           const uint2* __restrict__ cell_info,
-                                                           const uint32_t* __restrict__ surf_start,
-                                                           uint32_t* __restrict__ slist) {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        uint32_t c = skeys[j];
-        uint2 ci = cell_info[c];
-        if (ci.y & 0x80000000u) slist[surf_start[c] + (j - ci.x)] = j;
-    }
-}
-
 pms_status launch_surface_cells(pms_ctx* ctx) {
     const KGrid g = kgrid_of(ctx->grid);
     Counters* cnt = ctx->counters.as<Counters>();
@@ -239,13 +227,7 @@ pms_status launch_surface_cells(pms_ctx* ctx) {
         g, ctx->cell_count.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->surf_count.as<uint32_t>(),
         ctx->cell_info.as<uint2>());
     PMS_LAUNCHED(ctx);
-    pms_status st = scan_u32(ctx, ctx->surf_count.as<uint32_t>(), ctx->surf_start.as<uint32_t>(), g.sp_size, &cnt->ns);
-    if (st != PMS_OK) return st;
-    k_surface_list<<<grid_for(ctx->n, kThreads), kThreads, 0, ctx->stream>>>(
-        ctx->skeys.as<uint32_t>(), ctx->n, ctx->cell_info.as<uint2>(), ctx->surf_start.as<uint32_t>(),
-        ctx->slist.as<uint32_t>());
-    PMS_LAUNCHED(ctx);
-    return PMS_OK;
+    return scan_u32(ctx, ctx->surf_count.as<uint32_t>(), ctx->surf_start.as<uint32_t>(), g.sp_size, &cnt->ns);
 }
 
 }  // namespace pms

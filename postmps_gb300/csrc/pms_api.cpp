@@ -226,8 +226,6 @@ pms_status pms::ensure_grid_buffers(pms_ctx* c, const pms_grid& g) {
     const size_t W = ((uint64_t)g.sc_size + 31) / 32 + 1;
     PMS_CUDA(c, c->bm0.ensure(4 * W));
     PMS_CUDA(c, c->bm.ensure(4 * W));
-    PMS_CUDA(c, c->wcount.ensure(4 * W));
-    PMS_CUDA(c, c->wprefix.ensure(4 * W));
     PMS_CUDA(c, c->mc_le.ensure(4 * W));
     PMS_CUDA(c, c->mc_valid.ensure(4 * W));
     PMS_CUDA(c, c->mc_key.ensure(8 * W));
