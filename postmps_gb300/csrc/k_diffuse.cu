@@ -291,27 +291,54 @@ __global__ void __launch_bounds__(256) k_df_spawnlist(const unsigned long long* 
 
 // Particles with |s|^2 <= hd^2 (the generator's test; calculateofDiffuseType) over the
 // diffuse box, walking only the rows and cells of the box that come within hd: a cell
-// left out holds no particle the count would take, so the count is the reference's.
+// left out holds no particle the count would take, so the count is the reference's.  A
+// warp counts for one point, from the middle row on, and stops past kBubble: no type
+// depends on how many more there are.
 __device__ __forceinline__ int count_within_gen(const KGrid& g, const DiffuseParams& dp,
                                                 const uint32_t* __restrict__ cell_start, const float4* __restrict__ spos,
                                                 float px, float py, float pz) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
     uint3 lo, hi;
     diffuse_box(g, px, py, pz, lo, hi);
-    hi = make_uint3(hi.x + 1, hi.y + 1, hi.z + 1);          // row_walk takes [lo, hi)
-    const float r = dp.hd * kSupportGrow;
+    const float3 p = make_float3(px, py, pz);
+    const float r = dp.hd * kSupportGrow, pad = 1e-4f * g.sp_cs, inv = 1.f / g.sp_cs, rc = r * inv + kRangeMargin;
+    int za, zb, ya, yb;
+    cell_range((pz - g.min_pos[2]) * inv, rc, lo.z, hi.z + 1u, za, zb);
+    cell_range((py - g.min_pos[1]) * inv, rc, lo.y, hi.y + 1u, ya, yb);
+    const int ny = yb - ya, nrow = ny > 0 && zb > za ? ny * (zb - za) : 0;
     int count = 0;
-    row_walk(g, make_float3(px, py, pz), lo, hi, r * r, 1e-4f * g.sp_cs, cell_start, [&](uint32_t j) {
-        const float4 q = __ldg(&spos[j]);
-        const float sx = __fsub_rn(px, q.x), sy = __fsub_rn(py, q.y), sz = __fsub_rn(pz, q.z);
-        if (dot_rn(sx, sy, sz, sx, sy, sz) <= dp.hd_sq) ++count;
-    });
+    for (int r0 = 0; r0 < nrow; r0 += 32) {
+        int k = r0 + (int)lane;
+        uint32_t first = 0u, n = 0u;
+        if (k < nrow) {
+            k = (k + nrow / 2) % nrow;
+            n = box_row(g, p, p, r * r, pad, za + k / ny, ya + k % ny, (int)lo.x, (int)hi.x + 1, cell_start, first);
+        }
+        const WarpRows rows = warp_rows(first, n);
+        for (uint32_t q0 = 0u; q0 < rows.total; q0 += 32u) {
+            const uint32_t q = q0 + lane;
+            const int row = warp_row_of(rows, q);
+            const uint32_t j = __shfl_sync(kAll, rows.off, row) + q;
+            bool hit = false;
+            if (q < rows.total) {
+                const float4 c = __ldg(&spos[j]);
+                const float sx = __fsub_rn(px, c.x), sy = __fsub_rn(py, c.y), sz = __fsub_rn(pz, c.z);
+                hit = dot_rn(sx, sy, sz, sx, sy, sz) <= dp.hd_sq;
+            }
+            count += __popc(__ballot_sync(kAll, hit));
+            if (count > kBubble) return count;
+        }
+    }
     return count;
 }
 
 __device__ __forceinline__ int type_of(int density) { return density > kBubble ? 2 : (density < kSpray ? 0 : 1); }
 
-// calculateofDiffusePosition + calculateofDiffuseType, one spawning parent per thread
-__global__ void __launch_bounds__(kThreads, 8) k_df_spawn(KGrid g, DiffuseParams dp, const Counters* __restrict__ cnt,
+// calculateofDiffusePosition + calculateofDiffuseType, a warp per spawning parent: its lanes
+// count the parent's neighbours together and then make a child each.  (A thread per parent
+// walked alone: 2000 to 20,000 parents took 30 to 43 us whatever their number, now 6 to 28.)
+__global__ void __launch_bounds__(kThreads) k_df_spawn(KGrid g, DiffuseParams dp, const Counters* __restrict__ cnt,
                                                        const uint32_t* __restrict__ spawnlist,
                                                        const unsigned long long* __restrict__ off,
                                                        const int32_t* __restrict__ num, const uint32_t* __restrict__ cell_start,
@@ -319,10 +346,10 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_spawn(KGrid g, DiffuseParams
                                                        DiffuseParticle* __restrict__ gen, uint32_t gen_cap,
                                                        const uint32_t* __restrict__ frame_dev, uint32_t frame_off,
                                                        uint32_t* __restrict__ err) {
-    const uint32_t ns = cnt->n_spawning;
+    const uint32_t ns = cnt->n_spawning, lane = threadIdx.x & 31u;
     // a batched frame reads its number (the batch's first frame plus its place) from the device
     const uint32_t frame = frame_dev ? *frame_dev + frame_off : dp.frame;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ns; t += gridDim.x * blockDim.x) {
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ns; t += (gridDim.x * blockDim.x) >> 5) {
         const uint32_t i = spawnlist[t];
         const float4 p = spos[i], v = svel[i];
         // a vector normal to v (solveEq, myCuda.cuh:385-389), then the second axis
@@ -342,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_spawn(KGrid g, DiffuseParams
         const int k = num[i];
         const uint32_t start = (uint32_t)(off[i] & 0xffffffffull);
         const int type = type_of(count_within_gen(g, dp, cell_start, spos, p.x, p.y, p.z));
-        for (int c = 0; c < k; ++c) {
+        for (int c = (int)lane; c < k; c += 32) {
             const uint64_t idif = (uint64_t)start + (uint64_t)c;
             const float u1 = spawn_uniform(dp.seed, frame, 3 * idif + 1);
             const float u2 = spawn_uniform(dp.seed, frame, 3 * idif + 2);
@@ -716,7 +743,7 @@ static pms_status diffuse_tail(pms_ctx* ctx, const KGrid& g, const DiffuseParams
     pms_status st;
     const uint32_t total = dn.gen + dn.old;
     if (spawn_bound)
-        k_df_spawn<<<grid_for(spawn_bound, kThreads), kThreads, 0, ctx->stream>>>(
+        k_df_spawn<<<grid_for((uint64_t)spawn_bound * 32, kThreads, 152u * 16u), kThreads, 0, ctx->stream>>>(
             g, dp, cnt, ctx->d_difflist.as<uint32_t>(), ctx->d_isdiffscan.as<unsigned long long>(), ctx->d_num.as<int32_t>(),
             ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->svel.as<float4>(), ctx->d_gen.as<DiffuseParticle>(),
             dn.gen, frame_dev, frame_off, &cnt->err);

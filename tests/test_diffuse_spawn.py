@@ -1,0 +1,28 @@
+"""Spawning where the count around a parent decides its children's type: lattices of several
+spacings put 0 to more than 20 particles within the diffuse radius, and large multipliers give a
+parent more children than a warp has lanes.  Everything the spawning writes is exact against the
+oracle but the velocities (1e-5), as in the diffuse frames' own tests.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from test_diffuse import check_gpu_frames, run_gpu_frames
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("spread,multiplier", [(0.55, 40), (0.8, 4000), (1.0, 800), (1.3, 30000), (1.9, 800)])
+def test_spawned_types(pms_lib, oracle, tmp_config, spread, multiplier):
+    from postmps_gb300 import synth
+    pos = synth.lattice(12, 9, 7, 0.005 * spread, 0.0008, seed=3)
+    vel = np.random.default_rng(4).normal(0, 1.5, pos.shape).astype(np.float32)
+    rho = np.full(len(pos), 1000, np.float32)
+    text = synth.config_text(**synth.CROWN_KEYS, **{"config.isdiffusegeneration": "true",
+                                                    "diffuse.diffusetrappedairmultiplier": multiplier})
+    d = {"config": text, "seed": 11, "f0_pos": pos, "f0_vel": vel, "f0_rho": rho}
+    gpu = run_gpu_frames(pms_lib, tmp_config, d, frames=(0,))
+    if multiplier >= 4000:
+        assert gpu[0]["num"].max() > 32
+    check_gpu_frames(oracle, d, gpu, reference=False)
