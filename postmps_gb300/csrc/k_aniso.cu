@@ -26,6 +26,10 @@ namespace pms {
 static constexpr int kThreads = 128;
 // frames of up to this many particles take a warp per particle for the density
 static constexpr uint32_t kDensityWarp = 16384;
+// frames from this many particles on leave out the densities that no band vertex reads (the two
+// launches that find the blocks cost 3 to 8 us; frames: block 110k 478 -> 464 us, block 262k
+// 418 -> 411, crown 2M 3.79 -> 3.75 ms, dam 8M 3.65 -> 2.92; a batch of 110k to 300k tanks 5.90 -> 5.93)
+static constexpr uint32_t kDensityNear = 65536;
 static constexpr float kSigma = 1.56668147f;      // Define.h:11, 315/(64 pi)
 
 struct AnisoParams {
@@ -55,7 +59,7 @@ __device__ __forceinline__ float mass_over(float mass, float r) { return r == 0.
 // particles' entries.
 //
 // Three forms, chosen by the launcher:
-// - k_density_tiles: a warp per block of 4 x 2 x 2 cells.  Its particles (54 at rest, two per
+// - k_density_tiles: a warp per block of 2 x 2 x 2 cells.  Its particles (27 at rest, one per
 //   lane) share their neighbours: the warp reads each once, keeps those within h of the
 //   particles' box in shared memory, and all lanes add them.  Used where every particle's
 //   window [c - e, c + e] surely holds its support (e cells exceed h by kRangeMargin: the
@@ -65,7 +69,8 @@ __device__ __forceinline__ float mass_over(float mass, float r) { return r == 0.
 //   either, where one particle's serial walk is the pass's time.
 // All add the same contributions in the same order (ascending sorted index; what lies
 // beyond h adds exactly 0).  Bound by L1 (93 %: each lane loading its own neighbours)
-// before, by instruction issue now: dam 8M 1.47 -> 1.17 ms, crown 2M 0.36 -> 0.28, block 4k 23 -> 7 us.
+// before, by instruction issue now: dam 8M 1.47 -> 1.17 ms, crown 2M 0.36 -> 0.28, block 4k 23 -> 7 us;
+// without the blocks far from the surface dam 8M 0.45, crown 2M 0.20.
 // ---------------------------------------------------------------------------
 //
 // The pass also writes the surface list (compactationOfParticles, Anisotropic_kernel.cuh:127-155):
@@ -151,16 +156,45 @@ __global__ void __launch_bounds__(kThreads) k_density_warp(KGrid g, AnisoParams 
 static constexpr int kDensX = 2, kDensY = 2, kDensZ = 2;      // cells of a block
 static constexpr int kDensStage = 64;
 
-// the blocks that hold particles
-__global__ void __launch_bounds__(256) k_density_list(KGrid g, uint3 bd, const uint32_t* __restrict__ cell_start,
+// Which blocks of cells a density pass works on.  A frame whose fields are asked for only at
+// its band needs the densities near the surface: a band vertex lies within h per axis of a
+// surface particle, or one scalar cell further (the dilation), and a particle counts at a
+// vertex, or at a mesh vertex's scalar values, within h of it.  Blocks further than
+// 2 h + one scalar cell from every surface cell are "far": kNear writes density 0, whose
+// contribution nothing reads, for their particles; kFar makes theirs alone (launch_density_rest).
+enum class DensBlocks { kAll, kNear, kFar };
+static constexpr uint32_t kFarBlock = 1u << 31;               // (a grid holds less than 2^32 / 8 blocks)
+
+// a bit per block with a surface cell, the blocks of a row along x in whole words: a warp a word
+__global__ void __launch_bounds__(256) k_density_surface(KGrid g, uint3 bd, uint32_t wx, const uint2* __restrict__ cell_info,
+                                                         uint32_t* __restrict__ bits) {
+    const uint32_t nw = wx * bd.y * bd.z, lane = threadIdx.x & 31u;
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nw; w += (gridDim.x * blockDim.x) >> 5) {
+        const uint32_t bx = (w % wx) * 32u + lane, y0 = w / wx % bd.y * kDensY, z0 = w / wx / bd.y * kDensZ;
+        uint32_t any = 0u;
+        if (bx < bd.x) {
+            const uint32_t x0 = bx * kDensX, x1 = min(x0 + kDensX, g.spres[0]);
+            for (uint32_t z = z0; z < min(z0 + kDensZ, g.spres[2]); ++z)
+                for (uint32_t y = y0; y < min(y0 + kDensY, g.spres[1]); ++y)
+                    for (uint32_t x = x0; x < x1; ++x) any |= __ldg(&cell_info[(z * g.spres[1] + y) * g.spres[0] + x].y);
+        }
+        const uint32_t vote = __ballot_sync(0xffffffffu, (any >> 31) != 0u);
+        if (lane == 0u) bits[w] = vote;
+    }
+}
+
+// the blocks that hold particles (and, for kNear, whether they are far), a warp per 32 blocks along x
+__global__ void __launch_bounds__(256) k_density_list(KGrid g, uint3 bd, uint32_t wx, DensBlocks which, int reach,
+                                                      const uint32_t* __restrict__ bits, const uint32_t* __restrict__ cell_start,
                                                       uint32_t* __restrict__ n_blocks, uint32_t* __restrict__ list) {
-    const uint32_t nb = bd.x * bd.y * bd.z;
-    for (uint32_t t0 = blockIdx.x * blockDim.x; t0 < nb; t0 += gridDim.x * blockDim.x) {    // whole warps together
-        const uint32_t t = t0 + threadIdx.x;
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t nw = wx * bd.y * bd.z, lane = threadIdx.x & 31u;
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nw; w += (gridDim.x * blockDim.x) >> 5) {
+        const uint32_t wi = w % wx, bx = wi * 32u + lane, by = w / wx % bd.y, bz = w / wx / bd.y;
+        const uint32_t t = (bz * bd.y + by) * bd.x + bx;
         bool any = false;
-        if (t < nb) {
-            const uint32_t x0 = t % bd.x * kDensX, y0 = t / bd.x % bd.y * kDensY, z0 = t / bd.x / bd.y * kDensZ;
-            const uint32_t x1 = min(x0 + kDensX, g.spres[0]);
+        if (bx < bd.x) {
+            const uint32_t x0 = bx * kDensX, y0 = by * kDensY, z0 = bz * kDensZ, x1 = min(x0 + kDensX, g.spres[0]);
 #pragma unroll
             for (int k = 0; k < kDensY * kDensZ; ++k) {
                 const uint32_t y = y0 + k % kDensY, z = z0 + k / kDensY;
@@ -169,13 +203,30 @@ __global__ void __launch_bounds__(256) k_density_list(KGrid g, uint3 bd, const u
                 any |= __ldg(&cell_start[row + x0]) != __ldg(&cell_start[row + x1]);
             }
         }
-        const uint32_t vote = __ballot_sync(0xffffffffu, any);
+        uint32_t vote = __ballot_sync(kAll, any), near = kAll;
+        if (which != DensBlocks::kAll && vote) {
+            // the surface bits of the (2 reach + 1)^2 rows of blocks around, spread by reach along x
+            const int side = 2 * reach + 1;
+            near = 0u;
+            for (int r = (int)lane; r < side * side; r += 32) {
+                const int y = (int)by + r % side - reach, z = (int)bz + r / side - reach;
+                if (y < 0 || z < 0 || y >= (int)bd.y || z >= (int)bd.z) continue;
+                const uint32_t* row = bits + ((uint32_t)z * bd.y + (uint32_t)y) * wx;
+                const uint32_t c = __ldg(&row[wi]), lo = wi ? __ldg(&row[wi - 1u]) : 0u, hi = wi + 1u < wx ? __ldg(&row[wi + 1u]) : 0u;
+                near |= c;
+                for (int s = 1; s <= reach; ++s)
+                    near |= __funnelshift_l(lo, c, s) | __funnelshift_r(c, hi, s);
+            }
+            near = __reduce_or_sync(kAll, near);
+            if (which == DensBlocks::kFar) vote &= ~near;
+        }
         if (!vote) continue;
-        const uint32_t lane = threadIdx.x & 31u;
         uint32_t base = 0u;
         if (lane == 0u) base = atomicAdd(n_blocks, (uint32_t)__popc(vote));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (any) list[base + (uint32_t)__popc(vote & ((1u << lane) - 1u))] = t;
+        base = __shfl_sync(kAll, base, 0);
+        if ((vote >> lane) & 1u)
+            list[base + (uint32_t)__popc(vote & ((1u << lane) - 1u))] =
+                t | (which == DensBlocks::kNear && !((near >> lane) & 1u) ? kFarBlock : 0u);
     }
 }
 
@@ -202,7 +253,7 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoP
         if (lane == 0u) bi = atomicAdd(next, 1u);
         bi = __shfl_sync(kAll, bi, 0);
         if (bi >= n_blocks) break;
-        const uint32_t t = __ldg(&list[bi]);
+        const uint32_t entry = __ldg(&list[bi]), t = entry & ~kFarBlock;
         // the block's particles: a contiguous range per row of cells
         const uint32_t x0 = t % bd.x * kDensX, y0 = t / bd.x % bd.y * kDensY, z0 = t / bd.x / bd.y * kDensZ;
         uint32_t first = 0u, n = 0u;
@@ -220,6 +271,10 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoP
             const uint32_t own = min(t0 + lane, mine.total - 1u);
             const int own_row = warp_row_of(mine, own);
             const uint32_t id = __shfl_sync(kAll, mine.off, own_row) + own;
+            if (entry != t) {                                  // a far block
+                if (t0 + lane < mine.total) put_density(ap, sl, id, __ldg(&skeys[id]), 0.f, ext, rho, aniso);
+                continue;
+            }
             const float4 pi4 = __ldg(&spos[id]);
             const float3 b0 = make_float3(warp_min(pi4.x), warp_min(pi4.y), warp_min(pi4.z));
             const float3 b1 = make_float3(warp_max(pi4.x), warp_max(pi4.y), warp_max(pi4.z));
@@ -611,8 +666,7 @@ static float sqrt_bound(float r, bool inclusive) {
     return x;
 }
 
-pms_status launch_density_aniso(pms_ctx* ctx) {
-    const KGrid g = kgrid_of(ctx->grid);
+static AnisoParams aniso_params(const pms_ctx* ctx, const KGrid& g) {
     const pms_params& P = ctx->prm;
     AnisoParams ap;
     ap.h = P.h; ap.h_sq = P.h_sq; ap.h_inv = P.h_inv; ap.r2h = P.aniso_radius; ap.mass = P.mass;
@@ -625,31 +679,81 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
     ap.sp_size = g.sp_size;
     ap.sp_rows = g.spres[1] * g.spres[2];
     ap.spres_x = g.spres[0];
+    return ap;
+}
+
+// Blocks of cells between a surface cell and the first far block: cells whose indices
+// differ by k are (k - 1) cells apart at least.
+static int density_reach(const KGrid& g, float h) {
+    const float cells = 1.001f * (2.f * h + g.sc_cs) / g.sp_cs + 2.f * kRangeMargin;
+    return ((int)floorf(cells) + 2) / 2;
+}
+
+// the block form of the density over the blocks `which` names
+static pms_status density_blocks(pms_ctx* ctx, const KGrid& g, const AnisoParams& ap, const SurfaceList& sl, DensBlocks which) {
+    Counters* cnt = ctx->counters.as<Counters>();
+    const int bd_threads = ctx->tune.density_threads;
+    const uint3 bd = make_uint3((g.spres[0] + kDensX - 1) / kDensX, (g.spres[1] + kDensY - 1) / kDensY,
+                                (g.spres[2] + kDensZ - 1) / kDensZ);
+    const uint32_t wx = (bd.x + 31u) / 32u;
+    const uint64_t words = (uint64_t)wx * bd.y * bd.z;
+    // (the moments' buffer holds the list until the moments are made: at most a block per particle;
+    // the certification's cell records, made after the band, hold the bits: a word per cell is plenty)
+    uint32_t *list = ctx->moments.as<uint32_t>(), *bits = ctx->cell_rec.as<uint32_t>();
+    if (which != DensBlocks::kAll) {
+        k_density_surface<<<grid_for(words * 32, 256), 256, 0, ctx->stream>>>(g, bd, wx, ctx->cell_info.as<uint2>(), bits);
+        PMS_LAUNCHED(ctx);
+    }
+    k_density_list<<<grid_for(words * 32, 256), 256, 0, ctx->stream>>>(
+        g, bd, wx, which, density_reach(g, ap.h), bits, ctx->cell_start.as<uint32_t>(), &cnt->dens_blocks, list);
+    PMS_LAUNCHED(ctx);
+    auto tiles = [&](auto kern) {
+        kern<<<152u * (1024u / (unsigned)bd_threads), bd_threads, 0, ctx->stream>>>(
+            g, ap, sl, bd, ctx->skeys.as<uint32_t>(), &cnt->dens_blocks, &cnt->dens_next, list, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
+            ctx->rho.as<float>(), ctx->aniso.as<float4>());
+    };
+    if (bd_threads == 64) tiles(k_density_tiles<64>);
+    else if (bd_threads == 256) tiles(k_density_tiles<256>);
+    else tiles(k_density_tiles<128>);
+    PMS_LAUNCHED(ctx);
+    return PMS_OK;
+}
+
+// The densities of the far blocks that a frame left out (downloads of all densities).
+pms_status launch_density_rest(pms_ctx* ctx) {
+    if (!ctx->dens_far) return PMS_OK;
+    const KGrid g = kgrid_of(ctx->grid);
+    Counters* cnt = ctx->counters.as<Counters>();
+    const SurfaceList sl = {ctx->cell_info.as<uint2>(), ctx->surf_start.as<uint32_t>(), ctx->slist.as<uint32_t>()};
+    pms_status st = density_blocks(ctx, g, aniso_params(ctx, g), sl, DensBlocks::kFar);
+    if (st) return st;
+    // (between frames the tickets are zero: the anisotropy pass resets them)
+    PMS_CUDA(ctx, cudaMemsetAsync(&cnt->dens_blocks, 0, sizeof(uint32_t), ctx->stream));
+    PMS_CUDA(ctx, cudaMemsetAsync(&cnt->dens_next, 0, sizeof(uint32_t), ctx->stream));
+    ctx->dens_far = false;
+    return PMS_OK;
+}
+
+pms_status launch_density_aniso(pms_ctx* ctx) {
+    const KGrid g = kgrid_of(ctx->grid);
+    const pms_params& P = ctx->prm;
+    const AnisoParams ap = aniso_params(ctx, g);
     Counters* cnt = ctx->counters.as<Counters>();
     // block sizes of the neighbour walks are autotuned (64, 128 or 256 threads)
     const int bd_threads = ctx->tune.density_threads, bm = ctx->tune.moments_threads;
     const uint32_t n = ctx->n;
     const SurfaceList sl = {ctx->cell_info.as<uint2>(), ctx->surf_start.as<uint32_t>(), ctx->slist.as<uint32_t>()};
+    pms_status st;
+    ctx->dens_far = false;
     if (n <= kDensityWarp) {
         k_density_warp<<<grid_for((uint64_t)n * 32, kThreads, 152u * 16u), kThreads, 0, ctx->stream>>>(
             g, ap, sl, ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->rho.as<float>(),
             ctx->aniso.as<float4>(), n);
-    } else if ((float)g.spexpand * g.sp_cs - P.h >= kRangeMargin * g.sp_cs) {
-        const uint3 bd = make_uint3((g.spres[0] + kDensX - 1) / kDensX, (g.spres[1] + kDensY - 1) / kDensY,
-                                    (g.spres[2] + kDensZ - 1) / kDensZ);
-        // (the moments' buffer holds the list until the moments are made: at most a block per particle)
-        uint32_t* list = ctx->moments.as<uint32_t>();
-        k_density_list<<<grid_for((uint64_t)bd.x * bd.y * bd.z, 256), 256, 0, ctx->stream>>>(
-            g, bd, ctx->cell_start.as<uint32_t>(), &cnt->dens_blocks, list);
         PMS_LAUNCHED(ctx);
-        auto tiles = [&](auto kern) {
-            kern<<<152u * (1024u / (unsigned)bd_threads), bd_threads, 0, ctx->stream>>>(
-                g, ap, sl, bd, ctx->skeys.as<uint32_t>(), &cnt->dens_blocks, &cnt->dens_next, list, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
-                ctx->rho.as<float>(), ctx->aniso.as<float4>());
-        };
-        if (bd_threads == 64) tiles(k_density_tiles<64>);
-        else if (bd_threads == 256) tiles(k_density_tiles<256>);
-        else tiles(k_density_tiles<128>);
+    } else if ((float)g.spexpand * g.sp_cs - P.h >= kRangeMargin * g.sp_cs) {
+        // (a scalar cell above h would let the dilation wrap past the grid's margin of 2 h)
+        ctx->dens_far = ctx->dens_near && n >= kDensityNear && 2.f * g.sc_cs <= P.h && density_reach(g, P.h) < 32;
+        if ((st = density_blocks(ctx, g, ap, sl, ctx->dens_far ? DensBlocks::kNear : DensBlocks::kAll))) return st;
     } else {
         auto dens = [&](auto kern) {
             kern<<<grid_for(n, (unsigned)bd_threads), bd_threads, 0, ctx->stream>>>(
@@ -659,8 +763,8 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
         if (bd_threads == 64) dens(k_density<64>);
         else if (bd_threads == 256) dens(k_density<256>);
         else dens(k_density<128>);
+        PMS_LAUNCHED(ctx);
     }
-    PMS_LAUNCHED(ctx);
     // ns is on the device; grids are sized by the particle count (an upper bound)
     // (a thread per surface particle, or a warp where there are few: enough warps for both)
     const unsigned mom_blocks = std::max(grid_for(n, (unsigned)bm), grid_for((uint64_t)n * 32, (unsigned)bm, 152u * (2048u / (unsigned)bm)));

@@ -237,6 +237,7 @@ namespace pms {
 pms_status ensure_band_buffers(pms_ctx* c, uint32_t nv);
 void mark_stage(pms_ctx* c, int boundary);
 pms_status plain_band(pms_ctx* c);
+pms_status anisotropy_stage(pms_ctx* c, bool near);
 }  // namespace pms
 
 // a record per valid cube (at most nv): their number changes from frame to frame, so with headroom
@@ -527,10 +528,14 @@ extern "C" pms_status pms_build_grid(pms_ctx* c) {
     return PMS_OK;
 }
 
-extern "C" pms_status pms_anisotropy(pms_ctx* c) {
+// The anisotropy stage.  Inside a surface reconstruction the stages after it read densities
+// near the surface only (near); a caller of the stage alone gets every particle's.
+pms_status pms::anisotropy_stage(pms_ctx* c, bool near) {
     if (!c) return PMS_ERR_INVALID_ARGUMENT;
     if (!c->have_grid) return pms_fail(c, PMS_ERR_STATE, "pms_anisotropy before pms_build_grid");
     cudaSetDevice(c->device);
+    c->dens_far = false;
+    c->dens_near = near;
     if (c->n == 0) { c->have_aniso = true; return PMS_OK; }
     pms_status st;
     if ((st = launch_surface_cells(c))) return st;
@@ -539,6 +544,8 @@ extern "C" pms_status pms_anisotropy(pms_ctx* c) {
     mark(c, kStageAniso + 1);
     return PMS_OK;
 }
+
+extern "C" pms_status pms_anisotropy(pms_ctx* c) { return pms::anisotropy_stage(c, false); }
 
 // The band's size on the host, from counters just synchronised.
 static pms_status take_band_size(pms_ctx* c) {
@@ -687,7 +694,7 @@ extern "C" pms_status pms_download_scalar_values(pms_ctx* c, float* vel_xyz, flo
 
 extern "C" pms_status pms_surface(pms_ctx* c) {
     pms_status st;
-    if ((st = pms_anisotropy(c))) return st;
+    if ((st = pms::anisotropy_stage(c, true))) return st;
     if ((st = band_stage(c, true))) return st;
     if ((st = pms_field(c))) return st;
     return pms_marching_cubes(c);
@@ -747,7 +754,7 @@ static pms_status run_frame_overlapped(pms_ctx* c) {
         PMS_CUDA(c, cudaEventCreateWithFlags(&c->df_join, cudaEventDisableTiming));
         PMS_CUDA(c, c->df_tmp.ensure(64));
     }
-    if ((st = pms_anisotropy(c))) return st;
+    if ((st = pms::anisotropy_stage(c, true))) return st;
     PMS_CUDA(c, cudaEventRecord(c->df_fork, c->stream));
     PMS_CUDA(c, cudaStreamWaitEvent(c->df_stream, c->df_fork, 0));
     DiffuseJoin join{c};
@@ -969,6 +976,7 @@ extern "C" pms_status pms_debug_download(pms_ctx* c, int id, void* dst, uint64_t
         case PMS_ARRAY_KEYS_SORTED: case PMS_ARRAY_PERM: case PMS_ARRAY_DENSITY: {
             if (!c->have_grid) return PMS_ERR_STATE;
             if (id == PMS_ARRAY_DENSITY && !c->have_aniso) return PMS_ERR_STATE;
+            if (id == PMS_ARRAY_DENSITY && n && (st = launch_density_rest(c))) return st;
             const DBuf& b = id == PMS_ARRAY_KEYS_SORTED ? c->skeys : id == PMS_ARRAY_PERM ? c->order : c->rho;
             std::vector<uint32_t> v;
             if ((st = d2h(c, v, b.p, n))) return st;

@@ -183,7 +183,10 @@ static pms_status capture_frame(pms_ctx* c, BatchState* b, uint32_t f, int band,
     }
     if ((st = launch_hash_sort(c))) return st;
     if ((st = launch_surface_cells(c))) return st;
-    if ((st = launch_density_aniso(c))) return st;
+    c->dens_near = true;
+    st = launch_density_aniso(c);
+    c->dens_near = c->dens_far = false;      // (a lane's context hands out no densities)
+    if (st) return st;
     if (fork) PMS_CUDA(c, cudaEventRecord(fork, c->stream));
     if (band) {
         if ((st = launch_band(c))) return st;

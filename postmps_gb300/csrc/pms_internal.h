@@ -194,6 +194,8 @@ struct pms_ctx {
     // host mirrors of device counters, valid after the stage that syncs
     uint32_t ns = 0, nv = 0, nvalid = 0;
     uint64_t nmesh = 0;
+    bool dens_near = false;      // asked: the stages after the anisotropy read densities near the surface only
+    bool dens_far = false;       // the last density pass left out the blocks far from the surface
     bool nv_pending = false;     // nv is on the device: the marching cubes' synchronisation reads it
 
     // particle inputs
@@ -323,6 +325,7 @@ pms_status launch_publish_counters(pms_ctx* ctx);
 pms_status launch_hash_sort(pms_ctx* ctx);
 pms_status launch_surface_cells(pms_ctx* ctx);
 pms_status launch_density_aniso(pms_ctx* ctx);
+pms_status launch_density_rest(pms_ctx* ctx);
 pms_status launch_band(pms_ctx* ctx);
 pms_status launch_band_list(pms_ctx* ctx);
 pms_status launch_field(pms_ctx* ctx);

@@ -17,6 +17,7 @@ namespace pms {
 pms_status ensure_band_buffers(pms_ctx* c, uint32_t nv);
 void mark_stage(pms_ctx* c, int boundary);
 pms_status plain_band(pms_ctx* c);
+pms_status anisotropy_stage(pms_ctx* c, bool near);
 }  // namespace pms
 
 static pms_status zero_learn_counters(pms_ctx* c) {
@@ -159,7 +160,7 @@ extern "C" pms_status pms_band_learned(pms_ctx* c) {
 
 extern "C" pms_status pms_surface_learned(pms_ctx* c) {
     pms_status st;
-    if ((st = pms_anisotropy(c))) return st;
+    if ((st = anisotropy_stage(c, true))) return st;
     if ((st = pms_band_learned(c))) return st;
     return pms_marching_cubes(c);
 }
