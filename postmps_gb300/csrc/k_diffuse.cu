@@ -100,25 +100,56 @@ __device__ __forceinline__ void diffuse_box(const KGrid& g, float x, float y, fl
     box_clamp(g, c, (uint32_t)g.spexpand_diffuse, lo, hi);
 }
 
-// ---------------------------------------------------------------------------
-// free-surface list and the starting normals
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_df_free(const uint32_t* __restrict__ skeys, const uint2* __restrict__ cell_info,
-                                                 const float4* __restrict__ nrm4, int have_surface_normals, uint32_t n,
-                                                 uint32_t* __restrict__ isfree, float4* __restrict__ nrm) {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const bool surf = (cell_info[skeys[j]].y & 0x80000000u) != 0;
-        isfree[j] = surf ? 1u : 0u;
-        // the surface pass leaves normals on surface particles; other particles start at zero
-        const float4 q = (surf && have_surface_normals) ? nrm4[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        nrm[j] = make_float4(q.x, q.y, q.z, 0.f);
-    }
+__device__ __forceinline__ float phi_clamp(float I, float tmin, float tmax) {
+    return __fdiv_rn(__fsub_rn(fminf(I, tmax), fminf(I, tmin)), __fsub_rn(tmax, tmin));
 }
 
-__global__ void __launch_bounds__(256) k_df_freelist(const uint32_t* __restrict__ isfree, const uint32_t* __restrict__ scan,
-                                                     uint32_t n, uint32_t* __restrict__ list) {
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-        if (isfree[j]) list[scan[j]] = j;
+// Appends i to a list for the lanes that `take`, all lanes of the warp together (one atomic; the
+// lists' order does not matter: each entry's work is its own).
+__device__ __forceinline__ void list_append(bool take, uint32_t i, uint32_t* __restrict__ n, uint32_t* __restrict__ list) {
+    const uint32_t vote = __ballot_sync(0xffffffffu, take), lane = threadIdx.x & 31u;
+    if (!vote) return;
+    uint32_t base = 0u;
+    if (lane == 0u) base = atomicAdd(n, (uint32_t)__popc(vote));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (take) list[base + (uint32_t)__popc(vote & ((1u << lane) - 1u))] = i;
+}
+
+// ---------------------------------------------------------------------------
+// the starting normals, the kinetic energies, and the particles that can spawn.  The free
+// surface is the particles of surface cells, counted by the scan of the surface counts.
+//
+// A particle spawns floor(ke (ta_mult TA + wc_mult WC) dt) diffuse particles with ke its clamped
+// kinetic energy: where ke clamps to 0 (a particle at rest) the count is 0 whatever its trapped
+// air and wave crest, so its potentials stay 0; every count, and so every output, is the
+// reference's.  The others are listed, and the walks below run over lists: lanes that had
+// nothing to walk for waited for those that had (9 of 32 walked in the trapped-air pass, 5 in the
+// crests', on a 2M-particle crown).
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_df_begin(DiffuseParams dp, const uint32_t* __restrict__ skeys,
+                                                  const uint2* __restrict__ cell_info, const float4* __restrict__ nrm4,
+                                                  int have_surface_normals, const float4* __restrict__ svel, uint32_t n,
+                                                  float4* __restrict__ nrm, float4* __restrict__ pot,
+                                                  Counters* __restrict__ cnt, uint32_t* __restrict__ active) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt->n_free = cnt->ns;
+    for (uint32_t j0 = blockIdx.x * blockDim.x; j0 < n; j0 += gridDim.x * blockDim.x) {       // whole warps together
+        const uint32_t j = j0 + threadIdx.x;
+        bool spawns = false;
+        if (j < n) {
+            const bool surf = (cell_info[skeys[j]].y & 0x80000000u) != 0;
+            // the surface pass leaves normals on surface particles; other particles start at zero
+            const float4 q = (surf && have_surface_normals) ? nrm4[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            nrm[j] = make_float4(q.x, q.y, q.z, 0.f);
+            const float4 v = svel[j];
+            // 0.5 * (double)m * (double)|v|^2 rounded to float: the double product of two floats
+            // is exact and the halving too, so it is the float product rounded once, halved (the
+            // two could differ only for energies below the normal float range, ~1e-38)
+            const float ke = 0.5f * __fmul_rn(dp.mass, v.x * v.x + v.y * v.y + v.z * v.z);
+            pot[j] = make_float4(0.f, 0.f, ke, 0.f);
+            spawns = phi_clamp(ke, dp.min_ke, dp.max_ke) != 0.f;
+        }
+        list_append(spawns, j, &cnt->df_active, active);
+    }
 }
 
 // calculationofNormal: thread t < NumFree computes the normal of particle t
@@ -158,31 +189,27 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_normal(KGrid g, DiffuseParam
 // ---------------------------------------------------------------------------
 // potentials
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float phi_clamp(float I, float tmin, float tmax) {
-    return __fdiv_rn(__fsub_rn(fminf(I, tmax), fminf(I, tmin)), __fsub_rn(tmax, tmin));
-}
-
-// calculationofTrappedairpotential: every particle.  A particle spawns
-// floor(ke (ta_mult TA + wc_mult WC) dt) diffuse particles with ke its clamped kinetic
-// energy: where ke clamps to 0 (a particle at rest) the count is 0 whatever its
-// trapped air and wave crest, so those walks are skipped and the potentials left 0;
-// every count, and so every output, is the reference's.
+// calculationofTrappedairpotential: the particles that can spawn; those of the free surface that
+// move outwards are listed for the wave crests
 __global__ void __launch_bounds__(kThreads, 8) k_df_trapped(KGrid g, DiffuseParams dp, const uint32_t* __restrict__ cell_start,
                                                          const float4* __restrict__ spos, const float4* __restrict__ svel,
-                                                         uint32_t n, float4* __restrict__ pot) {
+                                                         const uint32_t* __restrict__ active, const float4* __restrict__ nrm,
+                                                         const uint32_t* __restrict__ skeys, const uint2* __restrict__ cell_info,
+                                                         float4* __restrict__ pot, Counters* __restrict__ cnt,
+                                                         uint32_t* __restrict__ crests) {
+    const uint32_t na = cnt->df_active;
     const float pad = 1e-4f * g.sp_cs, r2 = dp.hd_sq;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 p4 = spos[i], v = svel[i];
+    for (uint32_t t0 = blockIdx.x * blockDim.x; t0 < na; t0 += gridDim.x * blockDim.x) {      // whole warps together
+        const bool in = t0 + threadIdx.x < na;
+        const uint32_t i = active[in ? t0 + threadIdx.x : t0];
+        const float4 p4 = spos[i], v = svel[i], ni = nrm[i];
         const float3 p = make_float3(p4.x, p4.y, p4.z);
-        // 0.5 * (double)m * (double)|v|^2 rounded to float: the double product of two floats
-        // is exact and the halving too, so it is the float product rounded once, halved (the
-        // two could differ only for energies below the normal float range, ~1e-38)
-        const float ke = 0.5f * __fmul_rn(dp.mass, v.x * v.x + v.y * v.y + v.z * v.z);
-        pot[i].z = ke;
-        if (phi_clamp(ke, dp.min_ke, dp.max_ke) == 0.f) {
-            pot[i].y = 0.f;
-            continue;
-        }
+        // the reference's zero cases of the wave crests
+        const bool crest = in && (cell_info[skeys[i]].y & 0x80000000u) != 0 && !(dot_rn(ni.x, ni.y, ni.z, ni.x, ni.y, ni.z) <= kEpsDown) &&
+                           !(dot_rn(v.x, v.y, v.z, v.x, v.y, v.z) <= kEpsDown) &&
+                           !(dot_rn(v.x, v.y, v.z, ni.x, ni.y, ni.z) < k06Up);
+        list_append(crest, i, &cnt->df_crests, crests);
+        if (!in) continue;
         uint3 lo, hi;
         diffuse_box(g, p.x, p.y, p.z, lo, hi);
         hi = make_uint3(hi.x + 1, hi.y + 1, hi.z + 1);
@@ -211,27 +238,18 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_trapped(KGrid g, DiffusePara
     }
 }
 
-// calculationofWavecrests: free-surface particles
+// calculationofWavecrests: the listed free-surface particles
 __global__ void __launch_bounds__(kThreads, 8) k_df_crests(KGrid g, DiffuseParams dp, const Counters* __restrict__ cnt,
-                                                        const uint32_t* __restrict__ freelist,
+                                                        const uint32_t* __restrict__ crests,
                                                         const uint32_t* __restrict__ cell_start,
-                                                        const float4* __restrict__ spos, const float4* __restrict__ svel,
+                                                        const float4* __restrict__ spos,
                                                         const float4* __restrict__ nrm, float4* __restrict__ pot) {
-    const uint32_t nf = cnt->n_free;
+    const uint32_t nc = cnt->df_crests;
     const float pad = 1e-4f * g.sp_cs, r2 = dp.hd_sq;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nf; t += gridDim.x * blockDim.x) {
-        const uint32_t i = freelist[t];
-        const float4 p4 = spos[i], v = svel[i], ni = nrm[i];
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nc; t += gridDim.x * blockDim.x) {
+        const uint32_t i = crests[t];
+        const float4 p4 = spos[i], ni = nrm[i];
         const float3 p = make_float3(p4.x, p4.y, p4.z);
-        const float nn = dot_rn(ni.x, ni.y, ni.z, ni.x, ni.y, ni.z);
-        const float vv = dot_rn(v.x, v.y, v.z, v.x, v.y, v.z);
-        // the reference's zero cases, and a particle that spawns nothing (its clamped kinetic
-        // energy, from the trapped-air pass, is 0)
-        if (nn <= kEpsDown || vv <= kEpsDown || dot_rn(v.x, v.y, v.z, ni.x, ni.y, ni.z) < k06Up ||
-            phi_clamp(pot[i].z, dp.min_ke, dp.max_ke) == 0.f) {
-            pot[i].x = 0.f;
-            continue;
-        }
         uint3 lo, hi;
         diffuse_box(g, p.x, p.y, p.z, lo, hi);
         hi = make_uint3(hi.x + 1, hi.y + 1, hi.z + 1);
@@ -262,7 +280,9 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_crests(KGrid g, DiffuseParam
 
 // calculateofNumberofdiffuseparticles; key = spawning << 32 | count for one 64-bit scan
 __global__ void __launch_bounds__(256) k_df_count(DiffuseParams dp, float4* __restrict__ pot, uint32_t n,
-                                                  int32_t* __restrict__ num, unsigned long long* __restrict__ key) {
+                                                  int32_t* __restrict__ num, unsigned long long* __restrict__ key,
+                                                  Counters* __restrict__ cnt) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt->df_active = cnt->df_crests = 0u;     // the lists are done with
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 q = pot[i];
         q.x = phi_clamp(q.x, dp.min_wc, dp.max_wc);
@@ -694,9 +714,8 @@ static pms_status diffuse_front(pms_ctx* ctx, const KGrid& g, const DiffuseParam
     const uint32_t n = ctx->n;
     const size_t N = n;
     pms_status st;
-    PMS_CUDA(ctx, ctx->d_isfree.ensure(4 * N));
-    PMS_CUDA(ctx, ctx->d_freescan.ensure(4 * N));
-    PMS_CUDA(ctx, ctx->d_freelist.ensure(4 * N));
+    PMS_CUDA(ctx, ctx->d_active.ensure(4 * N));
+    PMS_CUDA(ctx, ctx->d_crests.ensure(4 * N));
     PMS_CUDA(ctx, ctx->d_nrm_free.ensure(16 * N));
     PMS_CUDA(ctx, ctx->d_pot.ensure(16 * N));
     PMS_CUDA(ctx, ctx->d_num.ensure(4 * N));
@@ -704,26 +723,23 @@ static pms_status diffuse_front(pms_ctx* ctx, const KGrid& g, const DiffuseParam
     PMS_CUDA(ctx, ctx->d_isdiffscan.ensure(8 * N));
     PMS_CUDA(ctx, ctx->d_difflist.ensure(4 * N));
     const unsigned gb = grid_for(n, 256), gk = grid_for(n, kThreads);
-    k_df_free<<<gb, 256, 0, ctx->stream>>>(ctx->skeys.as<uint32_t>(), ctx->cell_info.as<uint2>(), ctx->nrm4.as<float4>(),
-                                           ctx->have_aniso ? 1 : 0, n, ctx->d_isfree.as<uint32_t>(), ctx->d_nrm_free.as<float4>());
-    PMS_LAUNCHED(ctx);
-    if ((st = scan_u32(ctx, ctx->d_isfree.as<uint32_t>(), ctx->d_freescan.as<uint32_t>(), n, &cnt->n_free))) return st;
-    k_df_freelist<<<gb, 256, 0, ctx->stream>>>(ctx->d_isfree.as<uint32_t>(), ctx->d_freescan.as<uint32_t>(), n,
-                                               ctx->d_freelist.as<uint32_t>());
+    k_df_begin<<<gb, 256, 0, ctx->stream>>>(dp, ctx->skeys.as<uint32_t>(), ctx->cell_info.as<uint2>(), ctx->nrm4.as<float4>(),
+                                            ctx->have_aniso ? 1 : 0, ctx->svel.as<float4>(), n, ctx->d_nrm_free.as<float4>(),
+                                            ctx->d_pot.as<float4>(), cnt, ctx->d_active.as<uint32_t>());
     PMS_LAUNCHED(ctx);
     k_df_normal<<<gk, kThreads, 0, ctx->stream>>>(g, dp, cnt, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), n,
                                                   ctx->d_nrm_free.as<float4>());
     PMS_LAUNCHED(ctx);
-    PMS_CUDA(ctx, cudaMemsetAsync(ctx->d_pot.p, 0, 16 * N, ctx->stream));
     k_df_trapped<<<gk, kThreads, 0, ctx->stream>>>(g, dp, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
-                                                   ctx->svel.as<float4>(), n, ctx->d_pot.as<float4>());
+                                                   ctx->svel.as<float4>(), ctx->d_active.as<uint32_t>(), ctx->d_nrm_free.as<float4>(),
+                                                   ctx->skeys.as<uint32_t>(), ctx->cell_info.as<uint2>(), ctx->d_pot.as<float4>(),
+                                                   cnt, ctx->d_crests.as<uint32_t>());
     PMS_LAUNCHED(ctx);
-    k_df_crests<<<gk, kThreads, 0, ctx->stream>>>(g, dp, cnt, ctx->d_freelist.as<uint32_t>(), ctx->cell_start.as<uint32_t>(),
-                                                  ctx->spos.as<float4>(), ctx->svel.as<float4>(),
-                                                  ctx->d_nrm_free.as<float4>(), ctx->d_pot.as<float4>());
+    k_df_crests<<<gk, kThreads, 0, ctx->stream>>>(g, dp, cnt, ctx->d_crests.as<uint32_t>(), ctx->cell_start.as<uint32_t>(),
+                                                  ctx->spos.as<float4>(), ctx->d_nrm_free.as<float4>(), ctx->d_pot.as<float4>());
     PMS_LAUNCHED(ctx);
     k_df_count<<<gb, 256, 0, ctx->stream>>>(dp, ctx->d_pot.as<float4>(), n, ctx->d_num.as<int32_t>(),
-                                            ctx->d_isdiff.as<unsigned long long>());
+                                            ctx->d_isdiff.as<unsigned long long>(), cnt);
     PMS_LAUNCHED(ctx);
     if ((st = scan_u64(ctx, ctx->d_isdiff.as<unsigned long long>(), ctx->d_isdiffscan.as<unsigned long long>(), n,
                        &cnt->df_total)))
@@ -853,7 +869,7 @@ pms_status launch_diffuse(pms_ctx* ctx) {
 // every buffer of a batched frame's diffuse stage, for frames of up to nmax particles
 pms_status ensure_diffuse_batch_buffers(pms_ctx* ctx, uint32_t nmax, uint32_t gen_cap, uint32_t old_cap) {
     const size_t N = nmax ? nmax : 1, G = gen_cap ? gen_cap : 1, O = old_cap ? old_cap : 1;
-    for (DBuf* b : {&ctx->d_isfree, &ctx->d_freescan, &ctx->d_freelist, &ctx->d_num, &ctx->d_difflist})
+    for (DBuf* b : {&ctx->d_active, &ctx->d_crests, &ctx->d_num, &ctx->d_difflist})
         PMS_CUDA(ctx, b->ensure(4 * N));
     for (DBuf* b : {&ctx->d_nrm_free, &ctx->d_pot}) PMS_CUDA(ctx, b->ensure(16 * N));
     for (DBuf* b : {&ctx->d_isdiff, &ctx->d_isdiffscan}) PMS_CUDA(ctx, b->ensure(8 * N));

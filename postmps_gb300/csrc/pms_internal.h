@@ -80,6 +80,8 @@ struct Counters {
     uint32_t field_next;    // the next listed tile a warp of the field takes (both 0 before a launch)
     uint32_t dens_blocks;   // blocks of cells the density pass visits, and its ticket (0 between passes)
     uint32_t dens_next;
+    uint32_t df_active;     // particles that can spawn, and those of them with a wave crest: the lists'
+    uint32_t df_crests;     // lengths (0 between frames)
     uint32_t band_next;     // the next tile a warp of the band marking takes (0 between launches)
     uint32_t n_weld;        // vertices of the welded mesh (crossed grid edges)
     uint32_t n_df_total;    // generated + carried diffuse particles of a batched frame
@@ -227,7 +229,7 @@ struct pms_ctx {
     // mesh asks for them, else on the first download that does
     bool mesh_normals = false;
     // diffuse
-    pms::DBuf d_isfree, d_freescan, d_freelist, d_pot, d_num, d_numscan, d_isdiff, d_isdiffscan,
+    pms::DBuf d_active, d_crests, d_pot, d_num, d_numscan, d_isdiff, d_isdiffscan,
               d_difflist, d_gen, d_old, d_all, d_rand, d_typescan, d_nrm_free, d_tkey, d_tscan, d_perm;
     // learned band: coarse counts, model, cube bitmaps, merge buffers, training data
     pms::DBuf l_dens, l_clist;   // bf16 coarse density pairs (padded grid), candidate cube records

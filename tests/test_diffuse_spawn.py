@@ -26,3 +26,20 @@ def test_spawned_types(pms_lib, oracle, tmp_config, spread, multiplier):
     if multiplier >= 4000:
         assert gpu[0]["num"].max() > 32
     check_gpu_frames(oracle, d, gpu, reference=False)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 257, 1000])
+@pytest.mark.parametrize("moving", [0.0, 0.4, 1.0])
+def test_listed_particles(pms_lib, oracle, tmp_config, n, moving):
+    """Frames in which none, some and all of the particles move fast enough to spawn: the walks'
+    lists end at every place in a warp, and are empty."""
+    from postmps_gb300 import synth
+    rng = np.random.default_rng(n)
+    pos = synth.lattice(10, 10, 10, 0.005, 0.0005, seed=8)[rng.permutation(1000)[:n]]
+    vel = rng.normal(0, 2.0, pos.shape).astype(np.float32)
+    vel[rng.random(n) >= moving] = 0.0
+    text = synth.config_text(**synth.CROWN_KEYS, **{"config.isdiffusegeneration": "true"})
+    d = {"config": text, "seed": 5}
+    for f in (0, 1):
+        d.update({f"f{f}_pos": pos, f"f{f}_vel": vel, f"f{f}_rho": np.full(n, 1000, np.float32)})
+    check_gpu_frames(oracle, d, run_gpu_frames(pms_lib, tmp_config, d), reference=False)
