@@ -659,6 +659,11 @@ __global__ void __launch_bounds__(256) k_features(KGrid g, LearnDims ld, const u
 //             sum_s dh[s][j] (db1) and D2[64 + j][65] = sum_s h[s][j] dz[s] (dw2):
 //             all three gradients from one accumulator (dh, h, dz rounded to bf16,
 //             fp32 accumulation).  db2 and the loss are warp reductions.
+// Bound by latency: 64 blocks of a batch of 8192 take what one block takes.  Each thread holds
+// its sample in registers (eight 16-byte loads), from where it becomes the forward's row and the
+// backward's column; through shared memory, rows 128 bytes apart, every one of those accesses met
+// 32-way bank conflicts, and W1 came in strided 2-byte loads: 33 us for 8192 samples then, 8 now;
+// a step over 65,536 sampled candidates took 242 us, now 78.
 // One thread issues the MMAs; their completion arrives on an mbarrier whose waits
 // are bounded (a wait that runs out sets an error bit, waits once more for the
 // MMA in flight and frees the tensor memory).
@@ -668,8 +673,7 @@ static constexpr uint32_t kTrCols = 256;                 // tensor-memory column
 static constexpr uint32_t kTrColA = 64, kTrColD2 = 128;  // X (32 columns), D2 (80 columns)
 static constexpr uint32_t kTrN2 = 80;                     // D2 columns: 64 features, ones, dz, zero padding
 static constexpr uint32_t kTrBytesA2 = 128u * 128u * 2u, kTrBytesB2 = kTrN2 * 128u * 2u;
-static constexpr uint32_t kTrSmem = 1024u + kTcBytesB + kTrBytesA2 + kTrBytesB2 + kBlockSamples * kIn * 2 +
-                                    kBlockSamples * 4 + 2 * kHid * 4 + 64;
+static constexpr uint32_t kTrSmem = 1024u + kTcBytesB + kTrBytesA2 + kTrBytesB2 + 2 * kHid * 4 + 64;
 constexpr uint32_t kTrIdesc2 = (1u << 4) | (1u << 7) | (1u << 10) | ((kTrN2 >> 3) << 17) | ((128u >> 4) << 24);
 static_assert(kTrN2 % 16 == 0 && kTrColD2 + kTrN2 <= kTrCols && kTrColA + 32 <= kTrColD2, "tensor-memory plan");
 
@@ -731,49 +735,54 @@ __global__ void __launch_bounds__(kTrainThreads) k_learn_train(KGrid g, LearnDim
     uint8_t* sW1 = sm;
     uint8_t* sA2 = sW1 + kTcBytesB;
     uint8_t* sB2 = sA2 + kTrBytesA2;
-    uint16_t* s_x = reinterpret_cast<uint16_t*>(sB2 + kTrBytesB2);        // [sample][feature]
-    float* s_y = reinterpret_cast<float*>(s_x + kBlockSamples * kIn);
-    float* s_b1 = s_y + kBlockSamples;
+    float* s_b1 = reinterpret_cast<float*>(sB2 + kTrBytesB2);
     float* s_w2 = s_b1 + kHid;
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_w2 + kHid);
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + 1);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t s_base = blockIdx.x * kBlockSamples;
+    const uint32_t s = blockIdx.x * kBlockSamples + tid;
     const float inv_batch = 1.f / (float)in.batch;
-    // features and labels of the block's samples (rows past the batch: zero, label -1)
-    for (uint32_t e = tid; e < (uint32_t)(kBlockSamples * kIn); e += kTrainThreads) {
-        const uint32_t r = e / kIn, f = e % kIn;
-        const uint32_t s = s_base + r;
-        uint16_t v = 0;
-        float y = -1.f;
-        if (s < in.batch) {
-            if (in.x) {
-                v = in.x[(size_t)s * kIn + f];
-                y = in.y[s] ? 1.f : 0.f;
-            } else {
-                const uint32_t slot = (uint32_t)(mix64(in.seed ^ (0x9E3779B97F4A7C15ull * (s + 1))) % in.n_cand);
-                const uint32_t id = in.cand[slot];
-                const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
-                const int c[3] = {(int)(id % rx), (int)((id / rx) % g.scres[1]), (int)(id / rxy)};
-                const int d[3] = {(int)(f & 3u), (int)((f >> 2) & 3u), (int)(f >> 4)};
-                int cc[3];
-                bool inside = true;
+    // this thread's sample: its 64 features, two to a register, and its label (past the batch: zero
+    // and -1).  A sample's features are needed as a row by the forward and as a column by the
+    // backward: both are written from these registers.
+    uint32_t xr[kIn / 2];
+    float y = -1.f;
+    if (s < in.batch && in.x) {
+        const uint4* row = reinterpret_cast<const uint4*>(in.x + (size_t)s * kIn);
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    cc[a] = patch_cell(c[a] >> 1, c[a] & 1, d[a]);
-                    inside = inside && cc[a] >= 0 && cc[a] < (int)ld.cres[a];
-                }
-                const uint32_t cnt = inside ? in.counts[((size_t)cc[2] * ld.cres[1] + cc[1]) * ld.cres[0] + cc[0]] : 0u;
-                v = __bfloat16_as_ushort(__float2bfloat16_rn(feature_of(cnt, ld.inv_expected)));
-                y = ((in.labels[id >> 5] >> (id & 31u)) & 1u) ? 1.f : 0.f;
-            }
+        for (int k = 0; k < kIn / 8; ++k) {
+            const uint4 v = __ldg(&row[k]);
+            xr[4 * k] = v.x; xr[4 * k + 1] = v.y; xr[4 * k + 2] = v.z; xr[4 * k + 3] = v.w;
         }
-        s_x[r * kIn + f] = v;
-        if (f == 0) s_y[r] = y;
+        y = in.y[s] ? 1.f : 0.f;
+    } else if (s < in.batch) {
+        const uint32_t slot = (uint32_t)(mix64(in.seed ^ (0x9E3779B97F4A7C15ull * (s + 1))) % in.n_cand);
+        const uint32_t id = in.cand[slot];
+        const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
+        const int c[3] = {(int)(id % rx), (int)((id / rx) % g.scres[1]), (int)(id / rxy)};
+        auto feature = [&](int f) {
+            const int d[3] = {f & 3, (f >> 2) & 3, f >> 4};
+            int cc[3];
+            bool inside = true;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                cc[a] = patch_cell(c[a] >> 1, c[a] & 1, d[a]);
+                inside = inside && cc[a] >= 0 && cc[a] < (int)ld.cres[a];
+            }
+            const uint32_t cnt = inside ? in.counts[((size_t)cc[2] * ld.cres[1] + cc[1]) * ld.cres[0] + cc[0]] : 0u;
+            return __bfloat16_as_ushort(__float2bfloat16_rn(feature_of(cnt, ld.inv_expected)));
+        };
+#pragma unroll
+        for (int k = 0; k < kIn / 2; ++k) xr[k] = pack_raw(feature(2 * k), feature(2 * k + 1));
+        y = ((in.labels[id >> 5] >> (id & 31u)) & 1u) ? 1.f : 0.f;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kIn / 2; ++k) xr[k] = 0u;
     }
     // W1 as the forward's B operand (row j = hidden unit, K = input feature i)
-    for (uint32_t e = tid; e < (uint32_t)(kHid * kIn / 2); e += kTrainThreads) {
-        const uint32_t j = e / (kIn / 2), i = (e % (kIn / 2)) * 2;
+#pragma unroll
+    for (uint32_t k = 0; k < (uint32_t)(kHid * kIn / 2) / kTrainThreads; ++k) {
+        const uint32_t e = k * kTrainThreads + tid, j = e % kHid, i = e / kHid * 2;
         *reinterpret_cast<uint32_t*>(sW1 + umma_off(j, i)) = pack_raw(model->w1[i * kHid + j], model->w1[(i + 1) * kHid + j]);
     }
     if (tid < (uint32_t)kHid) {
@@ -796,12 +805,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_learn_train(KGrid g, LearnDim
     const uint32_t tmem = *s_tmem;
     const uint32_t t_row = tmem + ((warp * 32u) << 16);
     // forward: this sample's features into its lane, then D1 = X W1
-    {
-        uint32_t xr[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) xr[i] = pack_raw(s_x[tid * kIn + 2 * i], s_x[tid * kIn + 2 * i + 1]);
-        tc_st32(t_row + kTrColA, xr);
-    }
+    tc_st32(t_row + kTrColA, xr);
     tc_before_sync();
     __syncthreads();
     if (tid == 0) {
@@ -826,7 +830,6 @@ __global__ void __launch_bounds__(kTrainThreads) k_learn_train(KGrid g, LearnDim
         float z = model->b2;
 #pragma unroll
         for (int j = 0; j < kHid; ++j) z += fmaxf(acc[j], 0.f) * s_w2[j];
-        const float y = s_y[tid];
         if (y >= 0.f) {
             const float p = 1.f / (1.f + expf(-z));
             const float wy = in.pos_weight * y;
@@ -845,12 +848,11 @@ __global__ void __launch_bounds__(kTrainThreads) k_learn_train(KGrid g, LearnDim
                 __bfloat16_as_ushort(__float2bfloat16_rn(fmaxf(acc[j], 0.f)));
         }
     }
-#pragma unroll 8
+    const uint16_t dz16 = __bfloat16_as_ushort(__float2bfloat16_rn(dz));
+#pragma unroll
     for (uint32_t n = 0; n < kTrN2; ++n) {
-        const uint16_t v = n < (uint32_t)kIn ? s_x[tid * kIn + n]
-                                             : (n == (uint32_t)kIn ? (uint16_t)0x3F80u
-                                                                   : (n == (uint32_t)kIn + 1u ? __bfloat16_as_ushort(__float2bfloat16_rn(dz))
-                                                                                              : (uint16_t)0u));
+        const uint16_t v = n < (uint32_t)kIn ? (uint16_t)(xr[n < (uint32_t)kIn ? n / 2 : 0] >> (16u * (n & 1u)))
+                                             : (n == (uint32_t)kIn ? (uint16_t)0x3F80u : (n == (uint32_t)kIn + 1u ? dz16 : (uint16_t)0u));
         *reinterpret_cast<uint16_t*>(sB2 + umma_off128(n, tid)) = v;
     }
     // db2 and the loss, one atomic per warp
