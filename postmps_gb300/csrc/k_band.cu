@@ -98,6 +98,8 @@ __device__ __forceinline__ uint32_t row_surface(const uint32_t* __restrict__ sur
 // and tile another 0.06 / 0.05 / 0.06; this takes 0.23 / 0.25 / 0.23, list included (an empty
 // tile costs its rows' bounds).  Cells cut to the AABB's reach instead of a cell more on each
 // side: 0.37 -> 0.24 ms on the crown.  A 4k-particle frame: 16 + 22 -> 10 us with shares.
+// Particles whose plane leaves their whole part of the tile on one side, settled before the rows
+// look at them: spray 0.23 -> 0.20, dam 0.25 -> 0.23, crown and blocks unchanged.
 static constexpr int kBandThreads = 128, kBandStage = 64;
 
 __global__ void __launch_bounds__(kBandThreads, 8) k_band_tiles(KGrid g, float h, int ext, TileDims td,
@@ -205,6 +207,8 @@ __global__ void __launch_bounds__(kBandThreads, 8) k_band_tiles(KGrid g, float h
                     int blo[3], bhi[3];
                     particle_box(g, ext, p, blo, bhi);
                     uint32_t in[3];
+                    const float n[3] = {n4.x, n4.y, n4.z};
+                    float near = 0.f, far = 0.f, size = 0.f;   // bounds of n . (v - p) over those vertices
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         // vertices i of [box and tile] with a <= v(i) <= b: v rises with i, so they are
@@ -219,6 +223,19 @@ __global__ void __launch_bounds__(kBandThreads, 8) k_band_tiles(KGrid g, float h
                         while (i1 >= b0 && sc_coord_i(g, i1, k) > b) --i1;
                         // at most 32 positions of the tile
                         in[k] = i0 <= i1 ? (kAll >> (31 - (i1 - i0))) << (i0 - t0[k]) : 0u;
+                        const float d0 = __fmul_rn(n[k], __fsub_rn(sc_coord_i(g, i0, k), p[k]));
+                        const float d1 = __fmul_rn(n[k], __fsub_rn(sc_coord_i(g, i1, k), p[k]));
+                        near += fminf(d0, d1);
+                        far += fmaxf(d0, d1);
+                        size += fmaxf(fabsf(d0), fabsf(d1));
+                    }
+                    // a plane that leaves the whole part of the tile on one side needs no test per
+                    // row: all of it is marked, or none.  (Each rounded product of a vertex between the
+                    // ends lies between theirs; sums of three in any order differ by less than 1e-6 of
+                    // their sizes.)
+                    if (n4.w == 0.f) {
+                        if (near > 1e-6f * size) n4.w = 1.f;
+                        else if (far < -1e-6f * size) in[0] = 0u;
                     }
                     xin = in[0];
                     // row (y, z) of the tile is lane 4 z + y
