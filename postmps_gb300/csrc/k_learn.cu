@@ -148,82 +148,86 @@ __global__ void __launch_bounds__(256) k_coarse_dens(const uint32_t* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// candidates over tiles of 4 x 4 x 4 coarse cells (8 x 8 x 8 fine cubes):
-// each tile lists its candidate cubes and appends them to one list
+// Candidates.  A warp takes 16 coarse cells along x (its lanes are the 32 cubes along x of each of
+// a cell row's four (y, z) parities) and walks kCandCells of them along z: the patches' vertices
+// as bits (some density, below one half) of a row, four rows of y to a plane, four planes to
+// a cell.  The candidates go to the list row by row of cubes, so the network's 32 consecutive
+// ones mostly share their coarse rows and read each as one or two lines (the network on 13 M
+// candidates: 373 us with a list from tiles of 4 x 4 x 4 cells, in no order, 341 so).  A block per
+// such tile, testing 64 densities per cell, took 162 us, mostly for its barriers and tests; a block
+// per 16 x 2 x 2 cells on these bits 234, waiting for its own loads; this takes 96.
 // ---------------------------------------------------------------------------
-static constexpr int kTile = 4;                 // coarse cells per tile axis
-static constexpr int kHalo = 1;                 // patch vertices k - 1 .. k + 2 of the tile's cells k
-static constexpr int kSm = 8;                   // tile + halo = 7 coarse vertices per axis, padded
+static constexpr int kCandX = 16, kCandCells = 8;     // coarse cells along x and z
 static constexpr int kCandThreads = 128;
 
 // clist[i] = {cube id, padded coarse vertex of the cube's coarse cell | parity
 // x << 29 | parity y << 30 | parity z << 31}
 __global__ void __launch_bounds__(kCandThreads) k_learn_cand(KGrid g, LearnDims ld, const uint32_t* __restrict__ counts,
                                                              uint2* __restrict__ clist, uint32_t* __restrict__ n_cand) {
-    __shared__ float s_cnt[kSm][kSm][kSm];        // densities of the coarse vertices the tile's cubes read
-    __shared__ uint8_t s_mixed[kTile * kTile * kTile];
-    __shared__ uint16_t s_list[512];
-    __shared__ uint32_t s_n, s_base;
-    const int tid = threadIdx.x;
-    const uint32_t tx = ld.tiles[0], ty = ld.tiles[1];
-    const uint32_t tile = blockIdx.x;
-    const int T0[3] = {(int)(tile % tx) * kTile, (int)((tile / tx) % ty) * kTile, (int)(tile / (tx * ty)) * kTile};
-    if (T0[2] >= (int)ld.cres[2]) return;
-    // the coarse densities of the tile plus halo (outside the grid: empty)
-    int any = 0, all = 1;
-    for (int e = tid; e < kSm * kSm * kSm; e += kCandThreads) {
-        const int lx = e % kSm, ly = (e / kSm) % kSm, lz = e / (kSm * kSm);
-        const int cx = T0[0] - kHalo + lx, cy = T0[1] - kHalo + ly, cz = T0[2] - kHalo + lz;
-        uint32_t c = 0;
-        // the padding plane (index 7) lies beyond every patch: load it as empty without a read
-        if (lx < 7 && ly < 7 && lz < 7 && cx >= 0 && cy >= 0 && cz >= 0 && cx < (int)ld.cres[0] && cy < (int)ld.cres[1] &&
-            cz < (int)ld.cres[2])
-            c = __ldg(&counts[((size_t)cz * ld.cres[1] + cy) * ld.cres[0] + cx]);
-        const float d = density_of(c, ld.inv_expected);
-        s_cnt[lz][ly][lx] = d;
-        if (lx < 7 && ly < 7 && lz < 7) {
-            any |= d > 0.f;
-            all &= d >= 0.5f;
+    constexpr unsigned kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, n_tiles = ld.tiles[0] * ld.tiles[1] * ld.tiles[2];
+    const uint32_t tile = (blockIdx.x * kCandThreads + threadIdx.x) >> 5;
+    if (tile >= n_tiles) return;                       // whole warps
+    const int x0 = (int)(tile % ld.tiles[0]) * kCandX, y0 = (int)(tile / ld.tiles[0] % ld.tiles[1]),
+              z0 = (int)(tile / ld.tiles[0] / ld.tiles[1]) * kCandCells;
+    // planes z0 - 1 .. z0 + kCandCells + 1 of the vertices the patches read (outside the grid: empty)
+    const int cx = x0 - 1 + (int)lane;
+    const bool col = lane < (uint32_t)(kCandX + 3) && cx >= 0 && cx < (int)ld.cres[0];
+    uint32_t c[kCandCells + 3][4], some[kCandCells + 3], low[kCandCells + 3];
+#pragma unroll
+    for (int p = 0; p < kCandCells + 3; ++p)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {                  // all in flight together
+            const int cy = y0 - 1 + r, cz = z0 - 1 + p;
+            c[p][r] = col && cy >= 0 && cz >= 0 && cy < (int)ld.cres[1] && cz < (int)ld.cres[2]
+                          ? __ldg(&counts[((size_t)cz * ld.cres[1] + cy) * ld.cres[0] + cx]) : 0u;
         }
+#pragma unroll
+    for (int p = 0; p < kCandCells + 3; ++p) {
+        bool any = false, under = false;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const float d = density_of(c[p][r], ld.inv_expected);
+            any |= d > 0.f;
+            under |= d < 0.5f;
+        }
+        some[p] = __ballot_sync(kAll, any);
+        low[p] = __ballot_sync(kAll, under);
     }
-    if (tid == 0) s_n = 0;
-    const int any_b = __syncthreads_or(any), all_b = __syncthreads_and(all);
-    if (!any_b || all_b) return;                 // uniformly empty or full: no candidates
-    // mixed flag of each coarse cell of the tile over its 4^3 patch vertices
-    if (tid < kTile * kTile * kTile) {
-        const int cx = tid % kTile, cy = (tid / kTile) % kTile, cz = tid / (kTile * kTile);
-        bool nz = false, lo = false;
-        for (int dz = 0; dz < 4; ++dz)
-            for (int dy = 0; dy < 4; ++dy)
-                for (int dx = 0; dx < 4; ++dx) {
-                    const float v = s_cnt[cz + dz][cy + dy][cx + dx];
-                    nz |= v > 0.f;
-                    lo |= v < 0.5f;
-                }
-        s_mixed[tid] = (nz && lo) ? 1 : 0;
+    const uint32_t fx = 2u * (uint32_t)x0 + lane;
+    const uint32_t row = __ballot_sync(kAll, fx + 1u < g.scres[0]);        // cubes of the grid along x
+    // the cubes of each cell row: pairs of lanes of the mixed cells
+    uint32_t cubes[kCandCells], n = 0u;
+#pragma unroll
+    for (int k = 0; k < kCandCells; ++k) {
+        uint32_t s = some[k] | some[k + 1] | some[k + 2] | some[k + 3], l = low[k] | low[k + 1] | low[k + 2] | low[k + 3];
+        s |= s >> 1; s |= s >> 2;                      // any of the four vertices from bit x on
+        l |= l >> 1; l |= l >> 2;
+        cubes[k] = __ballot_sync(kAll, ((s & l) >> (lane >> 1)) & 1u) & row;
+        const uint32_t fy = 2u * (uint32_t)y0, fz = 2u * (uint32_t)(z0 + k);
+        const uint32_t ny = (fy + 1u < g.scres[1] ? 1u : 0u) + (fy + 2u < g.scres[1] ? 1u : 0u);
+        const uint32_t nz = (fz + 1u < g.scres[2] ? 1u : 0u) + (fz + 2u < g.scres[2] ? 1u : 0u);
+        n += (uint32_t)__popc(cubes[k]) * ny * nz;
     }
-    __syncthreads();
-    // candidate cubes of the tile (local index q = (lz * 8 + ly) * 8 + lx)
-    const uint32_t rxy = g.scres[0] * g.scres[1];
-    for (int q = tid; q < 512; q += kCandThreads) {
-        const int lx = q & 7, ly = (q >> 3) & 7, lz = q >> 6;
-        const int fx = 2 * T0[0] + lx, fy = 2 * T0[1] + ly, fz = 2 * T0[2] + lz;
-        const bool in = fx < (int)g.scres[0] - 1 && fy < (int)g.scres[1] - 1 && fz < (int)g.scres[2] - 1;
-        if (in && s_mixed[((lz >> 1) * kTile + (ly >> 1)) * kTile + (lx >> 1)]) s_list[atomicAdd(&s_n, 1u)] = (uint16_t)q;
-    }
-    __syncthreads();
-    const uint32_t ncand = s_n;
-    if (ncand == 0) return;
-    if (tid == 0) s_base = atomicAdd(n_cand, ncand);
-    __syncthreads();
+    if (!n) return;
+    uint32_t at = 0u;
+    if (lane == 0u) at = atomicAdd(n_cand, n);
+    at = __shfl_sync(kAll, at, 0);
     const PadDims pd = pad_dims(ld);
-    for (uint32_t e = tid; e < ncand; e += kCandThreads) {
-        const int q = s_list[e];
-        const int lx = q & 7, ly = (q >> 3) & 7, lz = q >> 6;
-        const uint32_t fx = 2 * T0[0] + lx, fy = 2 * T0[1] + ly, fz = 2 * T0[2] + lz;
-        const uint32_t pv = (((fz >> 1) + 1) * pd.p1 + (fy >> 1) + 1) * pd.p0 + (fx >> 1) + 1;
-        clist[s_base + e] = make_uint2(fz * rxy + fy * g.scres[0] + fx,
-                                       pv | ((fx & 1u) << 29) | ((fy & 1u) << 30) | ((fz & 1u) << 31));
+#pragma unroll
+    for (int k = 0; k < kCandCells; ++k) {
+        const uint32_t v = cubes[k];
+        if (!v) continue;
+        const uint32_t pv = (((uint32_t)(z0 + k) + 1u) * pd.p1 + (uint32_t)y0 + 1u) * pd.p0 + (fx >> 1) + 1u;
+        const uint32_t rank = (uint32_t)__popc(v & ((1u << lane) - 1u));
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+            const uint32_t fy = 2u * (uint32_t)y0 + (q & 1u), fz = 2u * (uint32_t)(z0 + k) + (q >> 1);
+            if (fy + 1u >= g.scres[1] || fz + 1u >= g.scres[2]) continue;
+            if ((v >> lane) & 1u)
+                clist[at + rank] = make_uint2((fz * g.scres[1] + fy) * g.scres[0] + fx, pv | ((lane & 1u) << 29) | (q << 30));
+            at += (uint32_t)__popc(v);
+        }
     }
 }
 
@@ -238,21 +242,6 @@ struct PredictOut {
     uint32_t cand_cap;
     uint32_t* n_pred;         // device counter
 };
-
-// W1 as B fragments: b[kk][nt][0..1] for k-step kk (features 16kk..16kk+15) and
-// n-tile nt (hidden 8nt..8nt+7)
-__device__ __forceinline__ void load_w1_frags(const DevModel* __restrict__ m, uint32_t (&b)[4][8][2], int lane) {
-    const uint16_t* w1 = m->w1;
-    const int kq = (lane & 3) * 2, n = lane >> 2;
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            const int i0 = kk * 16 + kq, j = nt * 8 + n;
-            b[kk][nt][0] = pack_raw(w1[(i0 + 0) * kHid + j], w1[(i0 + 1) * kHid + j]);
-            b[kk][nt][1] = pack_raw(w1[(i0 + 8) * kHid + j], w1[(i0 + 9) * kHid + j]);
-        }
-}
 
 // The A-fragment registers of one cube for a lane: features (dz, dy, dx) with
 // dx in {dx0, dx0 + 1} (one dens2 pair) and dy in {dy0, dy0 + 2}, for dz = kk.
@@ -305,7 +294,13 @@ static constexpr uint32_t kTcBytesB = kHid * kIn * 2;
 static constexpr uint32_t kTcSmem = 50u * 1024u;
 static constexpr uint32_t kTcSpin = 1u << 22;                   // bound on the polls of one mbarrier phase
 static constexpr int kTcBlocksPerSm = 4;
-static_assert(kTcBytesB + 2 * kHid * 4 + 64 + 1024 <= kTcSmem, "shared memory plan");
+static_assert(kTcBytesB + 64 + 1024 <= kTcSmem, "shared memory plan");
+// What follows the first layer, as a kernel parameter: every thread reads all of it for its
+// row, and from shared memory those broadcasts took more of L1's bandwidth (84 % busy) than the
+// gathers: 341 us for 13 M candidates, 261 from the constant bank.
+struct MlpTail {
+    float b1[kHid], w2[kHid], b2, threshold;
+};
 static_assert(kIn == 64 && kHid == 64, "the tile plan assumes 64 features and 64 hidden units");
 
 // byte offset of element (row r, k) of a K-major operand with 64 K elements (bf16)
@@ -381,8 +376,8 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
 
 __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm) k_learn_mlp(LearnDims ld, const uint32_t* __restrict__ dens2,
                                                           const uint2* __restrict__ clist, const uint32_t* __restrict__ n_dev,
-                                                          const DevModel* __restrict__ model, int use_model, PredictOut out,
-                                                          uint32_t* __restrict__ err, uint32_t wait_polls) {
+                                                          const DevModel* __restrict__ model, MlpTail tail, int use_model,
+                                                          PredictOut out, uint32_t* __restrict__ err, uint32_t wait_polls) {
     const uint32_t n = *n_dev;
     if (!use_model) {
         // collect only
@@ -394,24 +389,17 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm) k_learn_mlp(LearnD
     extern __shared__ uint8_t tc_smem[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem) + 1023u) & ~(uintptr_t)1023u);
     uint8_t* sB = sm;
-    float* s_b1 = reinterpret_cast<float*>(sB + kTcBytesB);
-    float* s_w2 = s_b1 + kHid;
-    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_w2 + kHid);
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(sB + kTcBytesB);
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + 1);
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     const uint32_t b_saddr = (uint32_t)__cvta_generic_to_shared(sB);
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
     // W1 as the B operand (row j = hidden unit, K = input feature i)
-    for (uint32_t e = tid; e < (uint32_t)(kHid * kIn / 2); e += kTcThreads) {
-        const uint32_t j = e / (kIn / 2), i = (e % (kIn / 2)) * 2;
+#pragma unroll
+    for (uint32_t k = 0; k < (uint32_t)(kHid * kIn / 2) / kTcThreads; ++k) {
+        const uint32_t q = k * kTcThreads + tid, j = q % kHid, i = q / kHid * 2;
         *reinterpret_cast<uint32_t*>(sB + umma_off(j, i)) =
             pack_raw(model->w1[i * kHid + j], model->w1[(i + 1) * kHid + j]);
-    }
-    // {b1[j], b1[j + 1], w2[j], w2[j + 1]} for even j, one 16-byte load per two columns
-    if (tid < (uint32_t)kHid / 2) {
-        const uint32_t j = 2 * tid;
-        reinterpret_cast<float4*>(s_b1)[tid] =
-            make_float4(model->b1[j], model->b1[j + 1], bf16_to_f(model->w2[j]), bf16_to_f(model->w2[j + 1]));
     }
     if (tid == 0) mbar_init(bar, 1);
     if (warp == 0) {
@@ -427,7 +415,6 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm) k_learn_mlp(LearnD
     tc_after_sync();
     const uint32_t tmem = *s_tmem;
     const uint32_t t_row = tmem + ((warp * 32u) << 16);      // this warp's 32 lanes
-    const float b2 = model->b2, thr = model->threshold;
     const PadDims pd = pad_dims(ld);
     const uint32_t p01 = pd.p0 * pd.p1;
     const uint32_t ntiles = (n + kTcRows - 1) / kTcRows;
@@ -516,23 +503,19 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm) k_learn_mlp(LearnD
         }
         phase ^= 1u;
         tc_after_sync();
-        float z = b2;
+        float z = tail.b2;
 #pragma unroll
         for (uint32_t q = 0; q < 4; ++q) {
             float v[16];
             tc_ld16(t_row + q * 16u, v);
 #pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-                const float4 bw = reinterpret_cast<const float4*>(s_b1)[(q * 16 + i) / 2];
-                z += fmaxf(v[i] + bw.x, 0.f) * bw.z;
-                z += fmaxf(v[i + 1] + bw.y, 0.f) * bw.w;
-            }
+            for (int i = 0; i < 16; ++i) z += fmaxf(v[i] + tail.b1[q * 16 + i], 0.f) * tail.w2[q * 16 + i];
         }
         if (live) {
             if (out.logit) {
                 if (e < out.cand_cap) { out.cand[e] = id; out.logit[e] = z; }
                 ++npred;
-            } else if (z > thr) {
+            } else if (z > tail.threshold) {
                 atomicOr(&out.q[id >> 5], 1u << (id & 31u));
                 ++npred;
             }
@@ -934,9 +917,10 @@ __global__ void __launch_bounds__(256) k_adam(float* __restrict__ w, const float
 LearnDims learn_dims(const pms_ctx* ctx) {
     const pms_grid& g = ctx->grid;
     LearnDims ld;
+    const uint32_t cells[3] = {kCandX, 1u, kCandCells};
     for (int a = 0; a < 3; ++a) {
         ld.cres[a] = g.scres[a] / 2u + 2u;                        // coarse vertices per axis
-        ld.tiles[a] = ((g.scres[a] + 1u) / 2u + kTile - 1) / kTile;  // tiles over the coarse cells holding cubes
+        ld.tiles[a] = ((g.scres[a] + 1u) / 2u + cells[a] - 1u) / cells[a];    // over the coarse cells holding cubes
     }
     const double side = 2.0 * (double)g.sc_grid_size, sp = (double)ctx->prm.particle_spacing;
     const double expected = (side / sp) * (side / sp) * (side / sp);
@@ -971,7 +955,7 @@ pms_status launch_predict(pms_ctx* ctx, int use_model, uint32_t* q, uint32_t* ca
     Counters* cnt = ctx->counters.as<Counters>();
     // candidates are distinct cubes: at most one per scalar-grid vertex
     PMS_CUDA(ctx, ctx->l_clist.ensure(8 * ((size_t)g.sc_size + 1)));
-    k_learn_cand<<<(unsigned)ntiles, kCandThreads, 0, ctx->stream>>>(g, ld, ctx->l_counts.as<uint32_t>(),
+    k_learn_cand<<<(unsigned)((ntiles + kCandThreads / 32 - 1) / (kCandThreads / 32)), kCandThreads, 0, ctx->stream>>>(g, ld, ctx->l_counts.as<uint32_t>(),
                                                                     ctx->l_clist.as<uint2>(), &cnt->l_cand);
     PMS_LAUNCHED(ctx);
     PredictOut out;
@@ -980,9 +964,20 @@ pms_status launch_predict(pms_ctx* ctx, int use_model, uint32_t* q, uint32_t* ca
     PMS_CUDA(ctx, cudaFuncSetAttribute(k_learn_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
     PMS_CUDA(ctx, cudaFuncSetAttribute(k_learn_mlp, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared));
+    MlpTail tail = {};
+    if (use_model) {
+        const pms_band_model& m = ctx->h_model;
+        for (int j = 0; j < kHid; ++j) {
+            const uint32_t w = (uint32_t)m.w2[j] << 16;            // bf16 bits
+            memcpy(&tail.w2[j], &w, 4);
+            tail.b1[j] = m.b1[j];
+        }
+        tail.b2 = m.b2;
+        tail.threshold = m.threshold;
+    }
     k_learn_mlp<<<152u * kTcBlocksPerSm, kTcThreads, kTcSmem, ctx->stream>>>(
         ld, ctx->l_dens.as<uint32_t>(), ctx->l_clist.as<uint2>(), &cnt->l_cand,
-        ctx->l_model.as<DevModel>(), use_model, out, &cnt->err, ctx->tc_wait_polls ? ctx->tc_wait_polls - 1u : kTcSpin);
+        ctx->l_model.as<DevModel>(), tail, use_model, out, &cnt->err, ctx->tc_wait_polls ? ctx->tc_wait_polls - 1u : kTcSpin);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }

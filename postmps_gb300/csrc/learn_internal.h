@@ -18,7 +18,7 @@ using DevModel = pms_band_model;
 // coarse density grid: a vertex on every second scalar-grid vertex
 struct LearnDims {
     uint32_t cres[3];        // coarse vertices per axis
-    uint32_t tiles[3];       // prediction tiles per axis (4 coarse cells each)
+    uint32_t tiles[3];       // candidate tiles per axis (k_learn_cand)
     float inv_expected;      // 1 / particles per coarse cell at the lattice spacing
 };
 

@@ -71,6 +71,7 @@ struct BatchState {
     uint32_t captures = 0;
     uint64_t sig = 0;                 // signature of the buffers the graph was captured against
     uint32_t nlanes_captured = 0;
+    uint32_t model_captured = 0;      // the model's last layer in the captured launches
     uint32_t wait_captured = 0;       // the debug wait limit baked into the captured launches
     // diffuse generation
     pms_ctx* dlane = nullptr;                    // the diffuse lane
@@ -343,6 +344,7 @@ static pms_status ensure_lane(pms_ctx* lc, pms_ctx* c, uint32_t nmax, const pms_
         PMS_CUDA(lc, lc->l_model.ensure(sizeof(pms_band_model)));
         PMS_CUDA(lc, cudaMemcpyAsync(lc->l_model.p, c->l_model.p, sizeof(pms_band_model), cudaMemcpyDeviceToDevice, c->stream));
         PMS_CUDA(lc, cudaStreamSynchronize(c->stream));
+        lc->h_model = c->h_model;
         lc->have_model = true;
     }
     return PMS_OK;
@@ -488,6 +490,7 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
         b->darena_cap = std::max<uint64_t>(b->darena_cap, (uint64_t)k * (b->old_cap / 2));
     }
     if (nlanes != b->nlanes_captured || c->tc_wait_polls != b->wait_captured) grids_same = false;
+    if (band == 1 && c->model_serial != b->model_captured) grids_same = false;
     uint64_t want_cap = 0;
     for (uint32_t f = 0; f < k; ++f) {
         const uint64_t sx = grid[f].scres[0], sy = grid[f].scres[1], sz = grid[f].scres[2];
@@ -519,6 +522,7 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
             b->sig = batch_signature(c, b, nlanes, diffuse);
             b->nlanes_captured = nlanes;
             b->wait_captured = c->tc_wait_polls;
+            b->model_captured = c->model_serial;
             grids_same = true;
         }
         if (diffuse) {

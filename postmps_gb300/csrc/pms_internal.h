@@ -238,6 +238,8 @@ struct pms_ctx {
     // (l_e_list: scratch of the candidate downloads)
     pms::DBuf l_counts, l_model, l_q, l_cert, l_e_bm, l_e_list, l_n_bm, l_n_wc, l_n_wp, l_n_list,
               l_field_new, l_cand, l_logit, l_label;
+    pms_band_model h_model;            // the model's host copy, and how often it changed (batch graphs hold its last
+    uint32_t model_serial = 0;         // layer in their launches)
     bool have_model = false, band_learned = false, mc_classified = false, mc_compacted = false;
     // polls + 1 of the first bounded wait on the tensor cores (0: the default bound)
     uint32_t tc_wait_polls = 0;

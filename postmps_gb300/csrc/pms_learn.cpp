@@ -35,6 +35,8 @@ extern "C" pms_status pms_set_band_model(pms_ctx* c, const pms_band_model* m) {
     PMS_CUDA(c, c->l_model.ensure(sizeof(pms_band_model)));
     PMS_CUDA(c, cudaMemcpyAsync(c->l_model.p, m, sizeof(pms_band_model), cudaMemcpyHostToDevice, c->stream));
     PMS_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (!c->have_model || memcmp(&c->h_model, m, sizeof(*m)) != 0) c->model_serial++;
+    c->h_model = *m;
     c->have_model = true;
     return PMS_OK;
 }
