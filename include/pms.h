@@ -139,7 +139,8 @@ typedef struct pms_counts {
     uint32_t n_band_exact;             /* band vertices evaluated exactly first (corners of predicted cubes) */
     uint32_t n_band_certified;         /* band vertices certified above iso without an exact value */
     uint32_t n_band_rechecked;         /* ... of those, corners of valid cubes, then evaluated exactly */
-    uint64_t n_field_pairs;            /* (band vertex, particle) pairs the field evaluated this frame */
+    uint64_t n_field_pairs;            /* (band vertex, particle) pairs the field evaluated this frame (a tile's vertices all
+                                          evaluate the particles that reach the tile) */
 } pms_counts;
 
 typedef struct pms_ctx pms_ctx;
@@ -311,7 +312,8 @@ typedef enum pms_array {
     PMS_ARRAY_CELL_END = 4,      /* uint32[sp_size] */
     PMS_ARRAY_SURF_COUNT = 5,    /* uint32[sp_size]  numSurParticleGrid */
     PMS_ARRAY_SURF_LIST = 6,     /* uint32[ns]  sorted index of each surface particle */
-    PMS_ARRAY_DENSITY = 7,       /* float[n]   density of each sorted particle */
+    PMS_ARRAY_DENSITY = 7,       /* float[n]   density of each sorted particle (pms_run_frame and the surface calls make
+                                          those near the surface; this makes the rest) */
     PMS_ARRAY_MEAN = 8,          /* float[3 ns] weighted mean of each surface particle */
     PMS_ARRAY_G = 9,             /* float[10 ns] G row-major + maxvalue (MatrixValue layout) */
     PMS_ARRAY_NORMAL = 10,       /* float[3 ns] oriented normal of each surface particle */
@@ -493,7 +495,8 @@ pms_status pms_batch_info(pms_ctx* ctx, uint32_t* graph_kernels, uint32_t* captu
  * ------------------------------------------------------------------------- */
 typedef struct pms_tune {
     int field_threads, field_waves, density_threads, moments_threads;
-    int field_vpt;                     /* x-neighbouring band vertices a thread of the field owns: 1, 2 or 4 */
+    int field_vpt;                     /* band vertices a lane of the field owns: 1, 2 or 4 (field_waves caps the resident
+                                          blocks of the certification alone) */
     float anisotropy_ms, field_ms;     /* the chosen shapes' times on the tuning frame */
 } pms_tune;
 pms_status pms_autotune(pms_ctx* ctx, pms_tune* out);

@@ -7,10 +7,11 @@
 // myCuda.cuh:84-119, 193-203, 403-415 (wij, matrixMul, determinant,
 // wij_density), SVD3.cuh (a float32 3x3 SVD).
 //
-// GB300 design: one thread per particle walks the sorted cells around it;
-// cells whose box lies beyond the kernel support are skipped (their
-// contributions are exactly zero), so the (4e+1)^3 box shrinks to the cells
-// that can matter.  The covariance is symmetric positive definite (it is seeded
+// GB300 design: a thread, a warp or a warp per block of cells (by frame size; the sums
+// are the same) walks the sorted cells around a particle; cells whose box lies beyond
+// the kernel support are skipped (their contributions are exactly zero), so the
+// (4e+1)^3 box shrinks to the cells that can matter, and a surface reconstruction
+// leaves out the densities that nothing after it reads.  The covariance is symmetric positive definite (it is seeded
 // with h^2 I), so its SVD is its eigen decomposition: a cyclic Jacobi solver
 // with exact rotations runs in float32, and covariances whose condition
 // number exceeds cfg.fp64_svd_cond are re-solved in float64.  Sums are

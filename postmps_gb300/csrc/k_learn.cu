@@ -27,9 +27,8 @@
 // empty neighbourhood is deep inside or far outside the fluid).
 //
 // Network.  h = relu(x W1 + b1), z = h . w2 + b2; the cube is predicted when
-// z > threshold.  The first layer runs on the tensor cores, 16 cubes per warp
-// per mma.sync.m16n8k16 (bf16 inputs, fp32 accumulate), weights held in
-// registers as B fragments; the second layer is a quad shuffle reduction.
+// z > threshold.  The first layer runs on the fifth-generation tensor cores, 128
+// cubes per block (bf16 inputs, fp32 accumulate); each thread then finishes one cube.
 //
 // Training.  Weighted binary cross-entropy on cubes the plain method labels
 // (valid marching cube = 1).  Forward as above; backward dz = sigmoid(z) (pw y
