@@ -95,6 +95,13 @@ __device__ __forceinline__ float cell_gap2(const KGrid& g, float3 p, uint32_t x,
     return dx * dx + dy * dy + dz * dz;
 }
 
+// The frame's counters into the context's mapped pinned mirror, by one block: the last work of a
+// kernel whose results the host waits for (a launch of its own costs 2.6 us).
+__device__ __forceinline__ void publish_counters(const Counters* cnt, uint32_t* mirror) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(cnt);
+    for (uint32_t i = threadIdx.x; i < sizeof(Counters) / 4; i += blockDim.x) mirror[i] = __ldcg(&src[i]);
+}
+
 // Margin, in cells, added to every range that the neighbour walks cut from a
 // support radius.  The ranges are computed from the point's position in cell
 // units, u = (p - min) / cell, whose rounding error (like that of a particle's

@@ -742,7 +742,7 @@ static pms_status diffuse_front(pms_ctx* ctx, const KGrid& g, const DiffuseParam
                                             ctx->d_isdiff.as<unsigned long long>(), cnt);
     PMS_LAUNCHED(ctx);
     if ((st = scan_u64(ctx, ctx->d_isdiff.as<unsigned long long>(), ctx->d_isdiffscan.as<unsigned long long>(), n,
-                       &cnt->df_total)))
+                       &cnt->df_total, nullptr, ctx->df_publish)))
         return st;
     k_df_spawnlist<<<gb, 256, 0, ctx->stream>>>(ctx->d_isdiff.as<unsigned long long>(),
                                                 ctx->d_isdiffscan.as<unsigned long long>(), n, cnt,
@@ -821,8 +821,13 @@ pms_status diffuse_part_tail(pms_ctx* ctx) {
     const DiffuseParams dp = diffuse_params(ctx);
     Counters* cnt = ctx->counters.as<Counters>();
     pms_status st;
-    if ((st = sync_counters(ctx))) return st;
-    const uint32_t n_gen = ctx->h_counters->n_generated, n_spawn = ctx->h_counters->n_spawning;
+    if (!ctx->df_publish) {
+        if ((st = sync_counters(ctx))) return st;
+    } else {
+        PMS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
+    const unsigned long long counts = ctx->h_counters->df_total;      // spawning << 32 | generated
+    const uint32_t n_gen = (uint32_t)counts, n_spawn = (uint32_t)(counts >> 32);
     const uint32_t n_old = ctx->diffuse_old;
     const size_t total = (size_t)n_gen + n_old;
     ctx->df_total = total;
@@ -861,8 +866,13 @@ pms_status diffuse_part_finish(pms_ctx* ctx) {
 }
 
 pms_status launch_diffuse(pms_ctx* ctx) {
-    PMS_CHECK(diffuse_part_front(ctx));
-    PMS_CHECK(diffuse_part_tail(ctx));
+    // alone on the context's stream, the front's last scan publishes the counters itself (beside
+    // the surface stages another stream's publication could overtake it)
+    ctx->df_publish = true;
+    pms_status st = diffuse_part_front(ctx);
+    if (!st) st = diffuse_part_tail(ctx);
+    ctx->df_publish = false;
+    PMS_CHECK(st);
     return diffuse_part_finish(ctx);
 }
 

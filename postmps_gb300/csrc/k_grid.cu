@@ -23,7 +23,8 @@ static constexpr uint32_t kBigCell = 4096;     // most particles a cell may hold
 // ---------------------------------------------------------------------------
 // bounding box (FileData.cpp:240-257); non-finite positions are flagged
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) k_bbox(const float* __restrict__ pos, uint32_t n, Counters* __restrict__ cnt) {
+__global__ void __launch_bounds__(kThreads) k_bbox(const float* __restrict__ pos, uint32_t n, Counters* __restrict__ cnt,
+                                                   uint32_t* __restrict__ mirror) {
     uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
     bool bad = false;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -55,6 +56,16 @@ __global__ void __launch_bounds__(kThreads) k_bbox(const float* __restrict__ pos
         atomicMax(&cnt->bbox_max[k], hi);
     }
     if (any_bad && threadIdx.x == 0) atomicOr(&cnt->err, kErrNonFinite);
+    if (!mirror) return;
+    // the last block publishes: every block's atomics come before its own count
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&cnt->bbox_blocks, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    publish_counters(cnt, mirror);
 }
 
 __global__ void k_counters_init(Counters* cnt, uint32_t n) {
@@ -79,11 +90,12 @@ pms_status launch_publish_counters(pms_ctx* ctx) {
     return PMS_OK;
 }
 
-pms_status launch_bbox(pms_ctx* ctx) {
+pms_status launch_bbox(pms_ctx* ctx, bool publish) {
     Counters* cnt = ctx->counters.as<Counters>();
     k_counters_init<<<1, 1, 0, ctx->stream>>>(cnt, ctx->n);
     PMS_LAUNCHED(ctx);
-    k_bbox<<<grid_for(ctx->n, kThreads, 152 * 4), kThreads, 0, ctx->stream>>>(ctx->in_pos.as<float>(), ctx->n, cnt);
+    k_bbox<<<grid_for(ctx->n, kThreads, 152 * 4), kThreads, 0, ctx->stream>>>(ctx->in_pos.as<float>(), ctx->n, cnt,
+                                                                           publish ? ctx->h_counters_dev : nullptr);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }

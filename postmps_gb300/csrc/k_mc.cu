@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kThreads) k_mc_emit(KGrid g, float iso, Counte
     }
 }
 
-pms_status launch_mc_count(pms_ctx* ctx) {
+pms_status launch_mc_count(pms_ctx* ctx, bool publish) {
     const KGrid g = kgrid_of(ctx->grid);
     Counters* cnt = ctx->counters.as<Counters>();
     const uint64_t nwords = ((uint64_t)g.sc_size + 31) / 32, rx = g.scres[0], rxy = rx * g.scres[1];
@@ -360,7 +360,8 @@ pms_status launch_mc_count(pms_ctx* ctx) {
     k_mc_count<<<grid_for(nwords, 256), 256, 0, ctx->stream>>>(nwords, rx, rxy, ctx->bm.as<uint32_t>(), ctx->mc_le.as<uint32_t>(),
                                                                ctx->mc_valid.as<uint32_t>(), ctx->mc_key.as<unsigned long long>());
     PMS_LAUNCHED(ctx);
-    return scan_u64(ctx, ctx->mc_key.as<unsigned long long>(), ctx->mc_off.as<unsigned long long>(), nwords, &cnt->mc_total);
+    return scan_u64(ctx, ctx->mc_key.as<unsigned long long>(), ctx->mc_off.as<unsigned long long>(), nwords, &cnt->mc_total,
+                    nullptr, publish);
 }
 
 pms_status launch_mc_compact(pms_ctx* ctx) {

@@ -508,9 +508,9 @@ extern "C" pms_status pms_build_grid(pms_ctx* c) {
     if (!c->have_particles) return pms_fail(c, PMS_ERR_STATE, "pms_build_grid before pms_upload_particles");
     cudaSetDevice(c->device);
     mark(c, kStageGrid);
-    pms_status st = launch_bbox(c);
+    pms_status st = launch_bbox(c, true);
     if (st) return st;
-    if ((st = sync_counters(c))) return st;
+    PMS_CUDA(c, cudaStreamSynchronize(c->stream));
     if ((st = check_device_errors(c))) return st;
     if (c->n == 0) {
         memset(&c->grid, 0, sizeof(c->grid));
@@ -609,9 +609,13 @@ extern "C" pms_status pms_marching_cubes(pms_ctx* c) {
     if (c->nv || c->nv_pending) {
         pms_status st;
         // the learned band has classified already
-        if (!c->mc_classified && (st = launch_mc_count(c))) return st;
+        if (!c->mc_classified && (st = launch_mc_count(c, true))) return st;
         if (!(c->mc_classified && c->mc_compacted)) {
-            if ((st = sync_counters(c))) return st;
+            if (c->mc_classified) {
+                if ((st = sync_counters(c))) return st;
+            } else {
+                PMS_CUDA(c, cudaStreamSynchronize(c->stream));
+            }
             if (c->nv_pending && (st = take_band_size(c))) return st;
             const uint64_t total = c->h_counters->mc_total;
             if ((st = ensure_band(c, (uint32_t)(total >> 32)))) return st;

@@ -84,6 +84,7 @@ struct Counters {
     uint32_t df_crests;     // lengths (0 between frames)
     uint32_t band_next;     // the next tile a warp of the band marking takes (0 between launches)
     uint32_t n_weld;        // vertices of the welded mesh (crossed grid edges)
+    uint32_t bbox_blocks;   // blocks of the bounding box that are done
     uint32_t n_df_total;    // generated + carried diffuse particles of a batched frame
     uint32_t mc_piece[kMaxMcPieces + 1];  // first cube of each streamed emission range, then nvalid
 };
@@ -184,6 +185,7 @@ struct pms_ctx {
     cudaEvent_t df_fork = nullptr, df_join = nullptr;
     pms::ScanTemp df_scan;
     pms::DBuf df_tmp;
+    bool df_publish = false;           // the diffuse front's scan published its counters
     bool df_run = false;               // the frame's diffuse parts have work (particles)
     size_t df_total = 0;               // generated + carried particles of the frame
     bool own_stream = false;
@@ -305,12 +307,13 @@ inline unsigned grid_for(uint64_t n, unsigned block, unsigned max_blocks = 152u 
 pms_status scan_u32(pms_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total_dev,
                     const uint32_t* n_dev = nullptr);
 pms_status scan_u64(pms_ctx* ctx, const unsigned long long* in, unsigned long long* out, uint64_t n,
-                    unsigned long long* total_dev, const uint32_t* n_dev = nullptr);
+                    unsigned long long* total_dev, const uint32_t* n_dev = nullptr, bool publish = false);
 
 size_t scan_scratch_bytes();   // what a scan keeps in ScanTemp (captured launches: allocated before)
 
 // stage launchers (one .cu each)
-pms_status launch_bbox(pms_ctx* ctx);
+// (publish: the pass also copies the counters to the host's mirror, as launch_publish_counters)
+pms_status launch_bbox(pms_ctx* ctx, bool publish = false);
 // Streamed-output queues (pms_api.cpp).  copy_stream_ready creates the copy stream and
 // both queues' events.  out_begin picks the record slot of a frame about to stream into
 // `host`: records still pending on that buffer (and every older one) are waited for and
@@ -346,7 +349,7 @@ pms_status launch_field_gather(pms_ctx* ctx, const uint32_t* vlist, const uint32
 // ascending list of the set bits of a bitmap over the scalar grid
 pms_status launch_bits_list(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t* vlist);
 // the valid cubes per word and their scan (Counters::mc_total); then the compaction; classify = both
-pms_status launch_mc_count(pms_ctx* ctx);
+pms_status launch_mc_count(pms_ctx* ctx, bool publish = false);
 pms_status launch_mc_compact(pms_ctx* ctx);
 pms_status launch_mc_classify(pms_ctx* ctx);
 // case and / or vertex count of every band vertex's cube (vlist made before)

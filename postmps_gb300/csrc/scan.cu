@@ -52,7 +52,8 @@ __device__ __forceinline__ T warp_sum(T v) {
 
 template <class T>
 __global__ void __launch_bounds__(kClusterThreads) k_scan_cluster(const T* __restrict__ in, T* __restrict__ out, uint32_t n,
-                                                                  T* __restrict__ total_out, const uint32_t* __restrict__ n_dev) {
+                                                                  T* total_out, const uint32_t* __restrict__ n_dev,
+                                                                  const Counters* cnt, uint32_t* mirror) {
     __shared__ T warp_tot[kClusterThreads / 32];
     __shared__ T block_tot;
     const cg::cluster_group cluster = cg::this_cluster();
@@ -88,6 +89,10 @@ __global__ void __launch_bounds__(kClusterThreads) k_scan_cluster(const T* __res
         __syncthreads();
     }
     if (total_out && blockIdx.x == gridDim.x - 1u && threadIdx.x == 0u) *total_out = before + block_tot;
+    if (mirror && blockIdx.x == gridDim.x - 1u) {
+        __syncthreads();
+        publish_counters(cnt, mirror);
+    }
     before += warp_tot[wid];
 #pragma unroll
     for (int r = 0; r < kRows; ++r)
@@ -149,7 +154,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restric
 template <class T, int V>
 __global__ void __launch_bounds__(kScanThreads) k_scan_down(const T* __restrict__ in, T* __restrict__ out, uint64_t n,
                                                             const T* __restrict__ block_sum, const T* __restrict__ warp_sums,
-                                                            T* __restrict__ total_out, const uint32_t* __restrict__ n_dev) {
+                                                            T* total_out, const uint32_t* __restrict__ n_dev,
+                                                            const Counters* cnt, uint32_t* mirror) {
     __shared__ T ws[kScanWarps];
     const uint64_t nn = n_dev && (uint64_t)*n_dev < n ? (uint64_t)*n_dev : n;
     const Stretch s = scan_stretch<V>(nn);
@@ -164,6 +170,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const T* __restrict_
 #pragma unroll
     for (int w = 0; w < kScanWarps; ++w) run += ws[w];
     if (total_out && blockIdx.x == gridDim.x - 1u && threadIdx.x == 0u) *total_out = run + block_sum[blockIdx.x];
+    if (mirror && blockIdx.x == gridDim.x - 1u) {
+        __syncthreads();
+        publish_counters(cnt, mirror);
+    }
     for (uint32_t w = 0; w < wid; ++w) run += warp_sums[(size_t)blockIdx.x * kScanWarps + w];
 #pragma unroll 2
     for (uint64_t r = s.begin; r < s.end; r += 32u * V) {
@@ -190,19 +200,22 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const T* __restrict_
 }
 
 template <class T, int V>
-static pms_status scan_two(pms_ctx* ctx, const T* in, T* out, uint64_t n, T* total_dev, const uint32_t* n_dev) {
+static pms_status scan_two(pms_ctx* ctx, const T* in, T* out, uint64_t n, T* total_dev, const uint32_t* n_dev,
+                            uint32_t* mirror) {
     const uint64_t per = 4u * 32u * V * kScanWarps;          // at least four rows for each warp
     const unsigned nb = (unsigned)std::min<uint64_t>((n + per - 1) / per, kMaxBlocks);
     T *block_sum = ctx->scan.partial.as<T>(), *warp_sums = block_sum + kMaxBlocks;
     k_scan_reduce<T, V><<<nb, kScanThreads, 0, ctx->stream>>>(in, n, block_sum, warp_sums, n_dev);
     PMS_LAUNCHED(ctx);
-    k_scan_down<T, V><<<nb, kScanThreads, 0, ctx->stream>>>(in, out, n, block_sum, warp_sums, total_dev, n_dev);
+    k_scan_down<T, V><<<nb, kScanThreads, 0, ctx->stream>>>(in, out, n, block_sum, warp_sums, total_dev, n_dev,
+                                                       ctx->counters.as<Counters>(), mirror);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }
 
 template <class T>
-static pms_status scan_impl(pms_ctx* ctx, const T* in, T* out, uint64_t n, T* total_dev, const uint32_t* n_dev) {
+static pms_status scan_impl(pms_ctx* ctx, const T* in, T* out, uint64_t n, T* total_dev, const uint32_t* n_dev,
+                            uint32_t* mirror) {
     if (n == 0) {
         if (total_dev) PMS_CUDA(ctx, cudaMemsetAsync(total_dev, 0, sizeof(T), ctx->stream));
         return PMS_OK;
@@ -220,24 +233,25 @@ static pms_status scan_impl(pms_ctx* ctx, const T* in, T* out, uint64_t n, T* to
         cfg.stream = ctx->stream;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        PMS_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_scan_cluster<T>, in, out, (uint32_t)n, total_dev, n_dev));
+        PMS_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_scan_cluster<T>, in, out, (uint32_t)n, total_dev, n_dev,
+                                         (const Counters*)ctx->counters.as<Counters>(), mirror));
         PMS_LAUNCHED(ctx);
         return PMS_OK;
     }
     PMS_CUDA(ctx, ctx->scan.partial.ensure(scan_scratch_bytes()));
     constexpr int V = 16 / (int)sizeof(T);
     // 16-byte accesses where both arrays start on a 16-byte boundary
-    if (((uintptr_t)in | (uintptr_t)out) & 15u) return scan_two<T, 1>(ctx, in, out, n, total_dev, n_dev);
-    return scan_two<T, V>(ctx, in, out, n, total_dev, n_dev);
+    if (((uintptr_t)in | (uintptr_t)out) & 15u) return scan_two<T, 1>(ctx, in, out, n, total_dev, n_dev, mirror);
+    return scan_two<T, V>(ctx, in, out, n, total_dev, n_dev, mirror);
 }
 
 pms_status scan_u32(pms_ctx* ctx, const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* total_dev,
                     const uint32_t* n_dev) {
-    return scan_impl<uint32_t>(ctx, in, out, n, total_dev, n_dev);
+    return scan_impl<uint32_t>(ctx, in, out, n, total_dev, n_dev, nullptr);
 }
 pms_status scan_u64(pms_ctx* ctx, const unsigned long long* in, unsigned long long* out, uint64_t n,
-                    unsigned long long* total_dev, const uint32_t* n_dev) {
-    return scan_impl<unsigned long long>(ctx, in, out, n, total_dev, n_dev);
+                    unsigned long long* total_dev, const uint32_t* n_dev, bool publish) {
+    return scan_impl<unsigned long long>(ctx, in, out, n, total_dev, n_dev, publish ? ctx->h_counters_dev : nullptr);
 }
 
 }  // namespace pms
