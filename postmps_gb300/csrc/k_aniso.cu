@@ -422,10 +422,11 @@ __device__ __forceinline__ void moments_warp(const KGrid& g, const AnisoParams& 
                                              const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ cell_start,
                                              const float4* __restrict__ spos, float4* __restrict__ mom) {
     constexpr unsigned kAll = 0xffffffffu;
-    // five columns of staged neighbours {w, ux, uy, uz, 1}, padded so that the ten lanes' 16-byte
-    // reads fall on different banks
+    // eight columns of staged neighbours {w, w ux, w uy, w uz, 1, ux, uy, uz}, padded so that the
+    // ten lanes' 16-byte reads fall on different banks (the products made by all lanes as they
+    // stage, not by the ten as they add: block 262k 64 -> 60 us)
     constexpr int kCol = 68;
-    __shared__ __align__(16) float hits_all[BT / 32][5 * kCol];
+    __shared__ __align__(16) float hits_all[BT / 32][8 * kCol];
     float* hits = hits_all[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t k = lane; k < 64u; k += 32u) hits[4 * kCol + k] = 1.f;
@@ -433,8 +434,8 @@ __device__ __forceinline__ void moments_warp(const KGrid& g, const AnisoParams& 
     const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1];
     const float pad = 1e-4f * g.sp_cs, r2h_sq = ap.r2h * ap.r2h, inv_r2h = 1.f / ap.r2h;
     // lane q's sum adds (w f1) f2: s0 | sx sy sz | sxx sxy sxz syy syz szz
-    const int f1 = lane == 0u ? 4 : (lane < 4u ? (int)lane : (lane < 7u ? 1 : (lane < 9u ? 2 : 3)));
-    const int f2 = lane < 4u ? 4 : (lane < 7u ? (int)lane - 3 : (lane < 9u ? (int)lane - 5 : 3));
+    const int f1 = lane < 4u ? (int)lane : (lane < 7u ? 1 : (lane < 9u ? 2 : 3));
+    const int f2 = lane < 4u ? 4 : (lane < 7u ? (int)lane + 1 : (lane < 9u ? (int)lane - 1 : 7));
     for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < ns; s += (gridDim.x * blockDim.x) >> 5) {
         const uint32_t i = slist[s];
         const float4 pi4 = spos[i];
@@ -450,17 +451,16 @@ __device__ __forceinline__ void moments_warp(const KGrid& g, const AnisoParams& 
         auto flush = [&]() {
             __syncwarp();
             if (lane < 10u) {
-                const float *W = hits, *A = hits + kCol * f1, *B = hits + kCol * f2;
+                const float *A = hits + kCol * f1, *B = hits + kCol * f2;
                 int k = 0;
                 for (; k + 4 <= staged; k += 4) {
-                    const float4 w = *reinterpret_cast<const float4*>(W + k), a = *reinterpret_cast<const float4*>(A + k),
-                                 b = *reinterpret_cast<const float4*>(B + k);
-                    acc = __fmaf_rn(__fmul_rn(w.x, a.x), b.x, acc);
-                    acc = __fmaf_rn(__fmul_rn(w.y, a.y), b.y, acc);
-                    acc = __fmaf_rn(__fmul_rn(w.z, a.z), b.z, acc);
-                    acc = __fmaf_rn(__fmul_rn(w.w, a.w), b.w, acc);
+                    const float4 a = *reinterpret_cast<const float4*>(A + k), b = *reinterpret_cast<const float4*>(B + k);
+                    acc = __fmaf_rn(a.x, b.x, acc);
+                    acc = __fmaf_rn(a.y, b.y, acc);
+                    acc = __fmaf_rn(a.z, b.z, acc);
+                    acc = __fmaf_rn(a.w, b.w, acc);
                 }
-                for (; k < staged; ++k) acc = __fmaf_rn(__fmul_rn(W[k], A[k]), B[k], acc);
+                for (; k < staged; ++k) acc = __fmaf_rn(A[k], B[k], acc);
             }
             __syncwarp();
             staged = 0;
@@ -479,7 +479,8 @@ __device__ __forceinline__ void moments_warp(const KGrid& g, const AnisoParams& 
             const uint32_t kept = __ballot_sync(kAll, keep);
             if (keep) {
                 float* h = hits + staged + __popc(kept & ((1u << lane) - 1u));
-                h[0] = w; h[kCol] = ux; h[2 * kCol] = uy; h[3 * kCol] = uz;
+                h[0] = w; h[kCol] = __fmul_rn(w, ux); h[2 * kCol] = __fmul_rn(w, uy); h[3 * kCol] = __fmul_rn(w, uz);
+                h[5 * kCol] = ux; h[6 * kCol] = uy; h[7 * kCol] = uz;
             }
             staged += __popc(kept);
             if (staged > 32) flush();
