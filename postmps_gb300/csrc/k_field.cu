@@ -361,8 +361,7 @@ k_field_cert(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const ui
 // - a lane's x-neighbours go through the packed two-float operations, rounded as the
 //   scalar ones, and the early exit is a limit on |G r|^2 rather than a flag.  Staging the
 //   packed operands twice, as pairs, cost more than the moves it saves (1.07 / 1.09 / 0.81).
-// K = 2 is the default: K = 1 stages fewer particles per tile but shares less of each, K = 4
-// the reverse (before the row cuts 1.50 / 1.78 / 1.41 and 1.31 / 1.53 / 1.03 ms).
+// K trades what a tile shares for what its vertices add in vain (pick_k has the rule).
 // ---------------------------------------------------------------------------
 template <int K> struct FieldTile {
     static constexpr int X = K == 4 ? 8 : 4, Y = 4, Z = K == 1 ? 2 : 4;
@@ -372,12 +371,34 @@ static constexpr uint32_t kTileTicket = 4;      // consecutive listed tiles a wa
 // row cuts: 20 warps (96 registers, no spills) 1.03 / 1.23 ms, 24 1.04 / 1.25, 16 1.15 / 1.36.
 static constexpr int kFieldWarps = 20;
 
+// How many vertices a lane takes, from the number of vertices to evaluate (a device count: the
+// host does not know the band's size yet).  Both launches decide alike.
+// - Below 160,000 vertices tiles of 64 do not fill the GPU: tiles of 32.  Field stage with 1 / 2:
+//   block 4k 22 / 25 us, 10k 29 / 33, one scalar cell per spacing (3k to 60k) 33 to 39 / 45 to
+//   51; the sides meet near 180,000 (crown 10k 31 / 33, 30k 49 / 47; block 30k 45 / 43).
+// - Tiles of 128 where many vertices share the same particles.  With 2 / 4: from three scalar
+//   cells per spacing on and 500,000 vertices, block 200k 213 / 178 us, crown 400k 723 / 590, dam
+//   1M 913 / 768, spray 100k 537 / 393 (338,000 vertices: 39 / 41); at two cells, from h = 4
+//   spacings on, dam 1M 2.18 / 2.02 ms, crown 400k 1.60 / 1.48, block 200k 0.54 / 0.46, and for
+//   sparse frames (droplets: particles fill less than a tenth of their box, a tile meets few of
+//   them), spray 151k (h = 3) 0.76 / 0.65 ms, 30k 0.23 / 0.17.  Elsewhere they lose: h = 2 and two
+//   cells, dam 1M 424 / 449 us, block 200k 104 / 119; one cell 1.3 to 2 times.
+struct FieldPick {
+    uint32_t few, many;                    // below: 1, from here on: 4
+    const uint32_t* __restrict__ count;
+};
+__device__ __forceinline__ uint32_t pick_k(const FieldPick& p) {
+    const uint32_t v = *p.count;
+    return v < p.few ? 1u : (v >= p.many ? 4u : 2u);
+}
+
 // The tiles holding a set bit of a bitmap over the scalar grid, 3 + K words each: the
 // first vertex's x, y, z, then for k < K the lanes whose vertex k is set.
 template <int K>
-__global__ void __launch_bounds__(256) k_field_tile_list(KGrid g, uint3 td, const uint32_t* __restrict__ bm,
-                                                         uint32_t* __restrict__ n_tiles, uint32_t* __restrict__ list) {
+__device__ __forceinline__ void field_tile_list(const KGrid& g, const uint32_t* __restrict__ bm,
+                                                uint32_t* __restrict__ n_tiles, uint32_t* __restrict__ list) {
     using T = FieldTile<K>;
+    const uint3 td = make_uint3((g.scres[0] + T::X - 1) / T::X, (g.scres[1] + T::Y - 1) / T::Y, (g.scres[2] + T::Z - 1) / T::Z);
     const uint32_t ntiles = td.x * td.y * td.z;
     const uint32_t rx = g.scres[0], ry = g.scres[1], rz = g.scres[2];
     // whole warps stay in the loop together (the append is a warp vote)
@@ -424,6 +445,17 @@ __global__ void __launch_bounds__(256) k_field_tile_list(KGrid g, uint3 td, cons
     }
 }
 
+// K = 0: by the rule (a launch whose K the host knows saves the look at the count: 6 us of the
+// dam's 980)
+template <int K>
+__global__ void __launch_bounds__(256) k_field_tile_list(KGrid g, FieldPick pick, const uint32_t* __restrict__ bm,
+                                                         uint32_t* __restrict__ n_tiles, uint32_t* __restrict__ list) {
+    const uint32_t k = K ? (uint32_t)K : pick_k(pick);
+    if (k == 1u) field_tile_list<1>(g, bm, n_tiles, list);
+    else if (k == 4u) field_tile_list<4>(g, bm, n_tiles, list);
+    else field_tile_list<2>(g, bm, n_tiles, list);
+}
+
 // A staged particle: position and packed kernel, its cell's x, and its row of cells with
 // two flags: the first particle of a cell, a cell that needs the general path.
 struct FieldStage {
@@ -436,16 +468,14 @@ static constexpr uint32_t kFresh = 1u << 31, kOdd = 1u << 30;   // (a row of cel
 static constexpr float kNever = -1.0e30f;       // below any |G r|^2
 
 template <int BT, int K>
-__global__ void __launch_bounds__(BT, kFieldWarps * 32 / BT)
-k_field_tiles(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const uint32_t* __restrict__ n_tiles_dev,
-              uint32_t* __restrict__ next, const uint32_t* __restrict__ list,
-              const uint32_t* __restrict__ cell_start, const float* __restrict__ cell_rad,
-              const uint32_t* __restrict__ skeys, const float4* __restrict__ spos, const float4* __restrict__ aniso,
-              float* __restrict__ fdense, Counters* __restrict__ cnt_w) {
+__device__ __forceinline__ void
+field_tiles(const KGrid& g, const FieldParams& fp, FieldStage* stage, const Counters* __restrict__ cnt,
+            const uint32_t* __restrict__ n_tiles_dev, uint32_t* __restrict__ next, const uint32_t* __restrict__ list,
+            const uint32_t* __restrict__ cell_start, const float* __restrict__ cell_rad,
+            const uint32_t* __restrict__ skeys, const float4* __restrict__ spos, const float4* __restrict__ aniso,
+            float* __restrict__ fdense, Counters* __restrict__ cnt_w) {
     constexpr unsigned kAll = 0xffffffffu;
-    __shared__ FieldStage stage_all[BT / 32][kFieldStage];
     const uint32_t lane = threadIdx.x & 31u;
-    FieldStage* stage = stage_all[threadIdx.x >> 5];
     const uint32_t n_tiles = *n_tiles_dev;
     const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
     const int srx = (int)g.spres[0], sry = (int)g.spres[1], srz = (int)g.spres[2];
@@ -693,28 +723,62 @@ k_field_tiles(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const u
     if (lane == 0u && my_pairs) atomicAdd(&cnt_w->n_pairs, my_pairs);
 }
 
-template <int K>
-static uint3 field_tile_dims(const pms_grid& g) {
-    using T = FieldTile<K>;
-    return make_uint3((g.scres[0] + T::X - 1) / T::X, (g.scres[1] + T::Y - 1) / T::Y, (g.scres[2] + T::Z - 1) / T::Z);
+template <int BT, int K>
+__global__ void __launch_bounds__(BT, kFieldWarps * 32 / BT)
+k_field_tiles(KGrid g, FieldParams fp, FieldPick pick, const Counters* __restrict__ cnt, const uint32_t* __restrict__ n_tiles_dev,
+              uint32_t* __restrict__ next, const uint32_t* __restrict__ list,
+              const uint32_t* __restrict__ cell_start, const float* __restrict__ cell_rad,
+              const uint32_t* __restrict__ skeys, const float4* __restrict__ spos, const float4* __restrict__ aniso,
+              float* __restrict__ fdense, Counters* __restrict__ cnt_w) {
+    __shared__ FieldStage stage_all[BT / 32][kFieldStage];
+    FieldStage* stage = stage_all[threadIdx.x >> 5];
+    const uint32_t k = K ? (uint32_t)K : pick_k(pick);
+    if (k == 1u)
+        field_tiles<BT, 1>(g, fp, stage, cnt, n_tiles_dev, next, list, cell_start, cell_rad, skeys, spos, aniso, fdense, cnt_w);
+    else if (k == 4u)
+        field_tiles<BT, 4>(g, fp, stage, cnt, n_tiles_dev, next, list, cell_start, cell_rad, skeys, spos, aniso, fdense, cnt_w);
+    else
+        field_tiles<BT, 2>(g, fp, stage, cnt, n_tiles_dev, next, list, cell_start, cell_rad, skeys, spos, aniso, fdense, cnt_w);
 }
 
 // the listed tiles of a bitmap of at most nv set bits
 template <int K>
 static uint64_t field_tile_most(const pms_grid& g, uint64_t nv) {
-    const uint3 td = field_tile_dims<K>(g);
-    return std::min<uint64_t>((uint64_t)td.x * td.y * td.z, nv);
+    using T = FieldTile<K>;
+    const uint64_t n = (uint64_t)((g.scres[0] + T::X - 1) / T::X) * ((g.scres[1] + T::Y - 1) / T::Y) * ((g.scres[2] + T::Z - 1) / T::Z);
+    return std::min<uint64_t>(n, nv);
 }
 template <int K>
 static size_t field_tile_bytes_of(const pms_grid& g, uint64_t nv) {
     return 4 * (size_t)(3 + K) * (field_tile_most<K>(g, nv) + 1);
 }
-size_t field_tile_bytes(const pms_grid& g, int vpt, uint64_t nv) {
-    return vpt == 1 ? field_tile_bytes_of<1>(g, nv) : vpt == 4 ? field_tile_bytes_of<4>(g, nv) : field_tile_bytes_of<2>(g, nv);
+// (room for any choice: the number of vertices is the device's)
+size_t field_tile_bytes(const pms_grid& g, uint64_t nv) {
+    return std::max(field_tile_bytes_of<1>(g, nv), std::max(field_tile_bytes_of<2>(g, nv), field_tile_bytes_of<4>(g, nv)));
+}
+
+// pick_k's lines for this frame, and the choice itself where the host knows it (else 0): a shape
+// that was set, or the middle one where nothing asks for 4 and a body of so many particles
+// has a band above `few` (30,000 in a block: 239,000 vertices at h = 2 and two cells).
+static int field_pick(const pms_ctx* ctx, FieldPick& p) {
+    p.few = 160000u;
+    p.many = 0xffffffffu;
+    if (!ctx->tune.field_auto) return ctx->tune.field_vpt;
+    const pms_params& P = ctx->prm;
+    const pms_grid& g = ctx->grid;
+    // the particles' share of their bounding box (the scalar grid has 2 h around it)
+    double box = 1.0;
+    for (int k = 0; k < 3; ++k)
+        box *= std::max((double)g.scmax_pos[k] - (double)g.scmin_pos[k] - 4.0 * P.h, (double)P.particle_spacing);
+    const double sp = P.particle_spacing;
+    const bool sparse = (double)ctx->n * sp * sp * sp < 0.1 * box;
+    if (P.sc_scale >= 3) p.many = 500000u;
+    else if (P.sc_scale == 2 && (P.smoothing_radius_ratio >= 4 || sparse)) p.many = 1000000u;
+    return p.many == 0xffffffffu && P.sc_scale == 2 && ctx->n >= 24576u ? 2 : 0;
 }
 
 template <int K>
-static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, uint64_t n_host) {
+static pms_status field_tiles_of(pms_ctx* ctx, const FieldPick& pick, const uint32_t* bm, uint64_t n_host) {
     const KGrid g = kgrid_of(ctx->grid);
     const pms_params& P = ctx->prm;
     FieldParams fp;
@@ -724,20 +788,19 @@ static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, uint64_t n_ho
     fp.quick = 0.f;
     fp.ext_unit = extent_unit(P.h);
     Counters* cnt = ctx->counters.as<Counters>();
-    const uint3 td = field_tile_dims<K>(ctx->grid);
-    const uint64_t ntiles = (uint64_t)td.x * td.y * td.z, most = field_tile_most<K>(ctx->grid, n_host);
-    PMS_CUDA(ctx, ctx->ftiles.ensure_grow(field_tile_bytes_of<K>(ctx->grid, n_host)));
+    constexpr int kGrid = K ? K : 2;            // what sizes the launches (both loop over what there is)
+    PMS_CUDA(ctx, ctx->ftiles.ensure_grow(field_tile_bytes(ctx->grid, n_host)));
     uint32_t* list = ctx->ftiles.as<uint32_t>();
     // the list's length and the next ticket start at 0: the band left them so, for one launch
     if (!ctx->field_tickets_zero) PMS_CUDA(ctx, cudaMemsetAsync(&cnt->n_items, 0, 2 * sizeof(uint32_t), ctx->stream));
     ctx->field_tickets_zero = false;
-    k_field_tile_list<K><<<grid_for(ntiles, 256), 256, 0, ctx->stream>>>(g, td, bm, &cnt->n_items, list);
+    k_field_tile_list<K><<<grid_for(field_tile_most<kGrid>(ctx->grid, ~0ull), 256), 256, 0, ctx->stream>>>(g, pick, bm, &cnt->n_items, list);
     PMS_LAUNCHED(ctx);
     const int bt = ctx->tune.field_threads;
     const unsigned per_sm = kFieldWarps * 32u / (unsigned)bt;
-    const unsigned blocks = grid_for(most, (unsigned)bt / 32u, 152u * per_sm);
+    const unsigned blocks = grid_for(field_tile_most<kGrid>(ctx->grid, n_host), (unsigned)bt / 32u, 152u * per_sm);
     auto go = [&](auto kern) {
-        kern<<<blocks, bt, 0, ctx->stream>>>(g, fp, cnt, &cnt->n_items, &cnt->field_next, list,
+        kern<<<blocks, bt, 0, ctx->stream>>>(g, fp, pick, cnt, &cnt->n_items, &cnt->field_next, list,
                                              ctx->cell_start.as<uint32_t>(), ctx->cell_rad.as<float>(),
                                              ctx->skeys.as<uint32_t>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(),
                                              ctx->fdense.as<float>(), cnt);
@@ -749,10 +812,14 @@ static pms_status field_tiles_of(pms_ctx* ctx, const uint32_t* bm, uint64_t n_ho
     return PMS_OK;
 }
 
-pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, uint64_t n_host) {
-    if (ctx->tune.field_vpt == 1) return field_tiles_of<1>(ctx, bm, n_host);
-    if (ctx->tune.field_vpt == 4) return field_tiles_of<4>(ctx, bm, n_host);
-    return field_tiles_of<2>(ctx, bm, n_host);
+pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, uint64_t n_host, const uint32_t* n_dev) {
+    FieldPick pick = {0u, 0u, n_dev};
+    switch (field_pick(ctx, pick)) {
+        case 1: return field_tiles_of<1>(ctx, pick, bm, n_host);
+        case 2: return field_tiles_of<2>(ctx, pick, bm, n_host);
+        case 4: return field_tiles_of<4>(ctx, pick, bm, n_host);
+        default: return field_tiles_of<0>(ctx, pick, bm, n_host);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -864,7 +931,8 @@ pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t
 }
 
 pms_status launch_field(pms_ctx* ctx) {
-    return launch_field_bits(ctx, ctx->bm.as<uint32_t>(), ctx->nv_pending ? ctx->grid.sc_size : ctx->nv);
+    return launch_field_bits(ctx, ctx->bm.as<uint32_t>(), ctx->nv_pending ? ctx->grid.sc_size : ctx->nv,
+                             &ctx->counters.as<Counters>()->nv);
 }
 
 // field[t] = fdense[vlist[t]]: the band-order field of a vertex list whose values are all computed

@@ -325,7 +325,7 @@ static pms_status ensure_lane(pms_ctx* lc, pms_ctx* c, uint32_t nmax, const pms_
     PMS_CUDA(lc, lc->scan.partial.ensure(scan_scratch_bytes()));
     lc->tune = c->tune;
     lc->tc_wait_polls = c->tc_wait_polls;     // the debug wait limit holds on every lane
-    for (const pms_grid& g : grid) PMS_CUDA(lc, lc->ftiles.ensure(field_tile_bytes(g, c->tune.field_vpt, g.sc_size)));
+    for (const pms_grid& g : grid) PMS_CUDA(lc, lc->ftiles.ensure(field_tile_bytes(g, g.sc_size)));
     if (!learned) return PMS_OK;
     const size_t S = (size_t)gmax.sc_size + 1;
     if ((st = ensure_learned_buffers(lc, gmax.sc_size, gmax.sc_size))) return st;

@@ -134,6 +134,7 @@ struct ScanTemp {
 // the neighbour walks and the field's resident-block cap (blocks per SM).
 struct Tune {
     int field_threads = 128, field_waves = 8, density_threads = 128, moments_threads = 128, field_vpt = 2;
+    bool field_auto = true;    // the field picks its vertices per lane itself (until a shape is set)
 };
 
 // Stage timing events.
@@ -342,9 +343,9 @@ pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t
                              uint32_t* n_cert);
 // exact field at the vertices of a bitmap over the scalar grid (n_host: a bound of their
 // number), into fdense
-pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, uint64_t n_host);
-// bytes of the tile list such a launch needs (field_vpt vertices per lane)
-size_t field_tile_bytes(const pms_grid& g, int vpt, uint64_t nv);
+pms_status launch_field_bits(pms_ctx* ctx, const uint32_t* bm, uint64_t n_host, const uint32_t* n_dev);
+// bytes of the tile list such a launch needs, whatever number of vertices a lane takes
+size_t field_tile_bytes(const pms_grid& g, uint64_t nv);
 pms_status launch_field_gather(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, float* out);
 // ascending list of the set bits of a bitmap over the scalar grid
 pms_status launch_bits_list(pms_ctx* ctx, const uint32_t* bm, const uint32_t* wprefix, uint32_t* vlist);

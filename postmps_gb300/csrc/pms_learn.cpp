@@ -116,13 +116,13 @@ pms_status pms::learned_field(pms_ctx* c) {
     const uint32_t nvb = c->nv;
     pms_status st;
     PMS_CUDA(c, cudaMemsetAsync(c->l_cert.p, 0, 4 * W, c->stream));
-    if ((st = launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nvb))) return st;
+    if ((st = launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nvb, &cnt->l_exact))) return st;
     if ((st = launch_field_cert(c, c->l_n_list.as<uint32_t>(), &cnt->l_nlist, nvb, c->l_cert.as<uint32_t>(), &cnt->l_cert)))
         return st;
     if ((st = launch_mc_classify(c))) return st;
     // the certified corners of valid cubes: E's bitmap holds them from here on
     if ((st = launch_recheck_bits(c, c->l_cert.as<uint32_t>(), c->l_e_bm.as<uint32_t>()))) return st;
-    return launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nvb);
+    return launch_field_bits(c, c->l_e_bm.as<uint32_t>(), nvb, &cnt->l_recheck);
 }
 
 extern "C" pms_status pms_band_learned(pms_ctx* c) {

@@ -62,12 +62,14 @@ extern "C" pms_status pms_autotune(pms_ctx* c, pms_tune* out) {
             for (int bt : sizes)
                 for (int w : waves) {
                     c->tune.field_vpt = k;
+                    c->tune.field_auto = false;
                     c->tune.field_threads = bt;
                     c->tune.field_waves = w;
                     float ms;
                     if ((st = time_ms(c, 3, &ms, launch_field))) return st;
                     if (ms < best_field) {
                         best_field = ms; best.field_threads = bt; best.field_waves = w; best.field_vpt = k;
+                        best.field_auto = false;
                     }
                 }
     }
@@ -99,6 +101,7 @@ extern "C" pms_status pms_set_tune(pms_ctx* c, const pms_tune* t) {
     c->tune.field_threads = t->field_threads;
     c->tune.field_waves = t->field_waves;
     c->tune.field_vpt = t->field_vpt;
+    c->tune.field_auto = false;
     c->tune.density_threads = t->density_threads;
     c->tune.moments_threads = t->moments_threads;
     return PMS_OK;
