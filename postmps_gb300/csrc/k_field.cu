@@ -37,7 +37,6 @@
 // `cert`; a vertex whose walk ran to the end has exactly the reference's value
 // (no early exit fired, the sum never exceeded iso).
 #include <algorithm>
-#include <type_traits>
 
 #include "pms_internal.h"
 #include "k_common.cuh"
@@ -879,6 +878,12 @@ __global__ void __launch_bounds__(256) k_field_items(const uint32_t* __restrict_
     }
 }
 
+// The certification's launch shape, which the field's tuned shape says nothing about: runs of two,
+// 128 threads, 8 waves of blocks.  Crown 2M: 0.81 ms; 64 or 256 threads 0.80 / 0.83, 2, 4 or 16 waves
+// 0.89 / 0.84 / 0.81.
+static constexpr uint32_t kCertRun = 2u;
+static constexpr unsigned kCertThreads = 128u, kCertWaves = 8u;
+
 pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t* n_dev, uint32_t n_host, uint32_t* cert,
                              uint32_t* n_cert) {
     const KGrid g = kgrid_of(ctx->grid);
@@ -891,7 +896,7 @@ pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t
     fp.ext_unit = 0.f;
     Counters* cnt = ctx->counters.as<Counters>();
     if ((uint64_t)n_host >= (1ull << kItemShift)) return pms_fail(ctx, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices");
-    const uint32_t K = (uint32_t)ctx->tune.field_vpt;
+    constexpr uint32_t K = kCertRun;
     const uint32_t ngroups = (n_host + K - 1u) / K;
     PMS_CUDA(ctx, ctx->fitem_cnt.ensure(4 * ((size_t)ngroups + 1)));
     PMS_CUDA(ctx, ctx->fitem_off.ensure(4 * ((size_t)ngroups + 1)));
@@ -908,24 +913,10 @@ pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t
     k_field_items<<<gb, 256, 0, ctx->stream>>>(vlist, n_dev, ngroups, K, g.scres[0], ctx->fitem_off.as<uint32_t>(),
                                                ctx->fitems.as<uint32_t>());
     PMS_LAUNCHED(ctx);
-    const int bt = ctx->tune.field_threads;
-    const unsigned per_sm = (K == 1 ? 1280u : 1024u) / (unsigned)bt;
-    const unsigned blocks = grid_for(n_host, (unsigned)bt, 152u * (unsigned)ctx->tune.field_waves * per_sm);
-    auto go = [&](auto kern) {
-        kern<<<blocks, bt, 0, ctx->stream>>>(g, fp, cnt, &cnt->n_items, ctx->fitems.as<uint32_t>(), vlist,
-                                             ctx->cell_start.as<uint32_t>(), ctx->cell_rad.as<float>(),
-                                             ctx->cell_rec.as<float4>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(),
-                                             ctx->fdense.as<float>(), cert, n_cert, cnt);
-    };
-    auto by_vpt = [&](auto bt_tag) {
-        constexpr int B = decltype(bt_tag)::value;
-        if (K == 1) go(k_field_cert<B, 1>);
-        else if (K == 4) go(k_field_cert<B, 4>);
-        else go(k_field_cert<B, 2>);
-    };
-    if (bt == 64) by_vpt(std::integral_constant<int, 64>());
-    else if (bt == 256) by_vpt(std::integral_constant<int, 256>());
-    else by_vpt(std::integral_constant<int, 128>());
+    const unsigned blocks = grid_for(n_host, kCertThreads, 152u * kCertWaves * (1024u / kCertThreads));
+    k_field_cert<kCertThreads, (int)kCertRun><<<blocks, kCertThreads, 0, ctx->stream>>>(
+        g, fp, cnt, &cnt->n_items, ctx->fitems.as<uint32_t>(), vlist, ctx->cell_start.as<uint32_t>(), ctx->cell_rad.as<float>(),
+        ctx->cell_rec.as<float4>(), ctx->spos.as<float4>(), ctx->aniso.as<float4>(), ctx->fdense.as<float>(), cert, n_cert, cnt);
     PMS_LAUNCHED(ctx);
     return PMS_OK;
 }

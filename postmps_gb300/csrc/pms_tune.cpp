@@ -42,7 +42,6 @@ extern "C" pms_status pms_autotune(pms_ctx* c, pms_tune* out) {
     PMS_CUDA(c, cudaMemcpyAsync(&saved, c->counters.p, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream));
     PMS_CUDA(c, cudaStreamSynchronize(c->stream));
     const int sizes[3] = {64, 128, 256};
-    const int waves[4] = {1, 2, 4, 8};
     const int vpts[3] = {1, 2, 4};
     pms_status st;
     Tune best = c->tune;
@@ -59,19 +58,17 @@ extern "C" pms_status pms_autotune(pms_ctx* c, pms_tune* out) {
     c->tune.moments_threads = best.moments_threads;
     if (c->nv) {
         for (int k : vpts)
-            for (int bt : sizes)
-                for (int w : waves) {
-                    c->tune.field_vpt = k;
-                    c->tune.field_auto = false;
-                    c->tune.field_threads = bt;
-                    c->tune.field_waves = w;
-                    float ms;
-                    if ((st = time_ms(c, 3, &ms, launch_field))) return st;
-                    if (ms < best_field) {
-                        best_field = ms; best.field_threads = bt; best.field_waves = w; best.field_vpt = k;
-                        best.field_auto = false;
-                    }
+            for (int bt : sizes) {
+                c->tune.field_vpt = k;
+                c->tune.field_auto = false;
+                c->tune.field_threads = bt;
+                float ms;
+                if ((st = time_ms(c, 3, &ms, launch_field))) return st;
+                if (ms < best_field) {
+                    best_field = ms; best.field_threads = bt; best.field_vpt = k;
+                    best.field_auto = false;
                 }
+            }
     }
     c->tune = best;
     // leave the frame's results as they were (the last re-runs used other shapes; values are identical)
