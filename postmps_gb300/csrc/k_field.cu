@@ -350,7 +350,8 @@ k_field_cert(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const ui
 // Bound by instruction issue.  A walk per run of vertices (18 of 32 lanes active, its
 // rows, records and cell bounds costing more than the pairs) took 2.89 / 2.56 / 7.24 ms
 // for the field stage of the crown 2M / dam 8M / spray 151k (ratio 3) frames; tiles take
-// 0.91 / 1.01 / 0.77 ms (28 of 32 lanes active, 3.0 instructions a cycle on the dam).  Of that:
+// 0.91 / 1.01 / 0.65 ms (28 of 32 lanes active, 3.0 instructions a cycle on the dam; the spray
+// 0.77 with K = 2, as in the figures here).  Of that:
 // - support boxes and the separating plane leave 41, 66 and 28 staged particles per tile of
 //   about 52 band vertices; the boxes alone left 60, 99 and 42 (1.29 / 1.64 / 1.22 ms);
 // - rows are cut by the largest support of their stretch of 8 cells, tiles listed with their

@@ -397,6 +397,9 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
     }
     BatchState* b = batch_of(c);
     if (k == 0) { b->n.clear(); b->hcnt.clear(); return PMS_OK; }
+    // the context is a lane, and its arrays are about to be the frames': downloads make nothing from them any more
+    c->dens_far = false;
+    c->arrays_lent = true;
     // ---- pass 1: arena, uploads, bounding boxes
     uint64_t total = 0;
     std::vector<uint64_t> off(k);

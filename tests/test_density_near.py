@@ -48,3 +48,28 @@ def test_frame_matches_stages(pms_lib, tmp_config, kind, ratio, sc):
             for a, b in zip(results(ctx), want, strict=True):
                 np.testing.assert_array_equal(a, b)
             np.testing.assert_array_equal(ctx.debug("density"), want[-2])
+
+
+def test_download_after_a_batch(pms_lib, tmp_config):
+    """A batch runs its frames in the context's own arrays, also when its graph is only launched again:
+    a frame before it leaves nothing that a download could still make.  The frame run after it gives
+    its own."""
+    from postmps_gb300 import synth
+    pos = scene("block")
+    frames = [(synth.lattice(30, 20, 25, 0.01, 0.001, seed=k), None, None) for k in range(2)]
+    with pms_lib.Context(pms_lib.load_config(tmp_config(synth.config_text())), 0) as ctx:
+        ctx.run_batch(frames)
+        ctx.upload(pos)
+        ctx.run_frame()
+        want = ctx.debug("density")
+        ctx.upload(pos)
+        ctx.run_frame()
+        names = ("density", "band_list", "field", "cube_case", "cube_nvert")
+        before = [ctx.debug(k) for k in names]
+        ctx.run_batch(frames)
+        assert [len(ctx.debug(k)) for k in names] == [len(b) for b in before]
+        ctx.upload(pos)
+        ctx.run_frame()
+        for k, b in zip(names, before):
+            np.testing.assert_array_equal(ctx.debug(k), b)
+        np.testing.assert_array_equal(ctx.debug("density"), want)
