@@ -57,7 +57,7 @@ static void for_each_dbuf(pms_ctx* c, F f) {
                     &c->svel, &c->rho, &c->cell_count, &c->cell_start, &c->cell_info, &c->surf_count,
                     &c->surf_start, &c->slist, &c->moments, &c->cell_rad, &c->cell_rec, &c->aniso, &c->nrm4, &c->mean4, &c->gdebug,
                     &c->nnb, &c->bm0, &c->bm, &c->wcount, &c->wprefix, &c->vlist, &c->field, &c->mc_le,
-                    &c->mc_valid, &c->mc_key, &c->mc_off, &c->fdense, &c->cube, &c->fitems, &c->fitem_cnt, &c->fitem_off, &c->ftiles, &c->vert, &c->vnorm, &c->sval, &c->d_active, &c->d_crests,
+                    &c->mc_valid, &c->mc_key, &c->mc_off, &c->fdense, &c->cube, &c->fitems, &c->fitem_cnt, &c->fitem_off, &c->ftiles, &c->vert, &c->vnorm, &c->sval, &c->d_active, &c->d_crests, &c->d_marks,
                     &c->d_pot, &c->d_num, &c->d_numscan, &c->d_isdiff, &c->d_isdiffscan,
                     &c->d_difflist, &c->d_gen, &c->d_old, &c->d_all, &c->d_rand, &c->d_typescan,
                     &c->d_nrm_free, &c->d_tkey, &c->d_tscan, &c->d_perm, &c->counters, &c->scan.partial, &c->tmp,
@@ -75,7 +75,7 @@ static void release_all(pms_ctx* c) {
 
 uint64_t pms::dbuf_signature(pms_ctx* c, bool diffuse) {
     // the diffuse stage's buffers (d_*): used by a graph only on its diffuse lane
-    const DBuf* dfirst[] = {&c->d_active, &c->d_crests, &c->d_pot, &c->d_num, &c->d_numscan,
+    const DBuf* dfirst[] = {&c->d_active, &c->d_crests, &c->d_marks, &c->d_pot, &c->d_num, &c->d_numscan,
                             &c->d_isdiff, &c->d_isdiffscan, &c->d_difflist, &c->d_gen, &c->d_old, &c->d_all,
                             &c->d_rand, &c->d_typescan, &c->d_nrm_free, &c->d_tkey, &c->d_tscan, &c->d_perm};
     uint64_t h = 1469598103934665603ull;
@@ -509,6 +509,7 @@ extern "C" pms_status pms_build_grid(pms_ctx* c) {
     cudaSetDevice(c->device);
     mark(c, kStageGrid);
     c->arrays_lent = false;
+    c->df_normals_near = false;
     pms_status st = launch_bbox(c, true);
     if (st) return st;
     PMS_CUDA(c, cudaStreamSynchronize(c->stream));

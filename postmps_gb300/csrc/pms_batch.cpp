@@ -513,7 +513,7 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
     for (int attempt = 0; attempt < attempts; ++attempt) {
         if (diffuse) {
             pms_ctx* dl = b->dlane;
-            if ((st = ensure_diffuse_batch_buffers(dl, nmax, b->gen_cap, b->old_cap))) return st;
+            if ((st = ensure_diffuse_batch_buffers(dl, nmax, b->gen_cap, b->old_cap, grid.data(), k))) return st;
             PMS_CUDA(c, dl->scan.partial.ensure(scan_scratch_bytes()));
             PMS_CUDA(c, b->dcnt.ensure(2 * sizeof(uint32_t)));
             PMS_CUDA(c, b->drun.ensure(sizeof(unsigned long long)));

@@ -186,6 +186,7 @@ struct pms_ctx {
     cudaEvent_t df_fork = nullptr, df_join = nullptr;
     pms::ScanTemp df_scan;
     pms::DBuf df_tmp;
+    bool df_normals_near = false;      // the last frame's diffuse normals were made where crests read them only
     bool df_publish = false;           // the diffuse front's scan published its counters
     bool df_run = false;               // the frame's diffuse parts have work (particles)
     size_t df_total = 0;               // generated + carried particles of the frame
@@ -233,7 +234,7 @@ struct pms_ctx {
     // mesh asks for them, else on the first download that does
     bool mesh_normals = false;
     // diffuse
-    pms::DBuf d_active, d_crests, d_pot, d_num, d_numscan, d_isdiff, d_isdiffscan,
+    pms::DBuf d_active, d_crests, d_marks, d_pot, d_num, d_numscan, d_isdiff, d_isdiffscan,
               d_difflist, d_gen, d_old, d_all, d_rand, d_typescan, d_nrm_free, d_tkey, d_tscan, d_perm;
     // learned band: coarse counts, model, cube bitmaps, merge buffers, training data
     pms::DBuf l_dens, l_clist;   // bf16 coarse density pairs (padded grid), candidate cube records
@@ -389,7 +390,8 @@ struct DiffuseBatch {
     void* arena = nullptr;                   // 32-byte diffuse records
     uint64_t arena_cap = 0;                  // records the arena holds
 };
-pms_status ensure_diffuse_batch_buffers(pms_ctx* ctx, uint32_t nmax, uint32_t gen_cap, uint32_t old_cap);
+pms_status ensure_diffuse_batch_buffers(pms_ctx* ctx, uint32_t nmax, uint32_t gen_cap, uint32_t old_cap, const pms_grid* grid,
+                                        uint32_t n_grids);
 pms_status launch_diffuse_bounded(pms_ctx* ctx, const DiffuseBatch& db);
 pms_status upload_mc_tables(pms_ctx* ctx);
 

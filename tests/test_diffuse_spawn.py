@@ -43,3 +43,26 @@ def test_listed_particles(pms_lib, oracle, tmp_config, n, moving):
     for f in (0, 1):
         d.update({f"f{f}_pos": pos, f"f{f}_vel": vel, f"f{f}_rho": np.full(n, 1000, np.float32)})
     check_gpu_frames(oracle, d, run_gpu_frames(pms_lib, tmp_config, d), reference=False)
+
+
+@pytest.mark.parametrize("moving", [0.0, 0.02, 1.0])
+@pytest.mark.parametrize("surface", ["true", "false"])
+def test_normals_do_not_depend_on_who_moves(pms_lib, tmp_config, moving, surface):
+    """Normals are made only where a particle that can spawn may read them; a download makes the rest,
+    bit for bit those of a frame in which every particle moves."""
+    from postmps_gb300 import synth
+    pos = synth.lattice(31, 27, 14, 0.005, 0.0008, seed=9)
+    rho = np.full(len(pos), 1000, np.float32)
+    text = synth.config_text(**synth.CROWN_KEYS, **{"config.isdiffusegeneration": "true", "config.issurfacereconstruct": surface})
+    normals = []
+    for share in (1.0, moving):
+        rng = np.random.default_rng(3)
+        vel = rng.normal(0, 3.0, pos.shape).astype(np.float32)
+        vel[rng.random(len(pos)) >= share] = 0.0
+        with pms_lib.Context(pms_lib.load_config(tmp_config(text)), 0) as ctx:
+            ctx.upload(pos, vel, rho)
+            ctx.run_frame()
+            normals.append((ctx.debug("free_normal"), ctx.debug("free_normal")))
+    assert np.any(normals[0][0] != 0)
+    for n in normals[1]:
+        np.testing.assert_array_equal(n, normals[0][0])
