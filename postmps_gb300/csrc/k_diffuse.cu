@@ -848,7 +848,8 @@ pms_status diffuse_part_front(pms_ctx* ctx) {
     const DiffuseParams dp = diffuse_params(ctx);
     Counters* cnt = ctx->counters.as<Counters>();
     pms_status st;
-    if (!ctx->have_aniso && (st = launch_surface_cells(ctx))) return st;
+    // (counted by the anisotropy pass, unless the grid was built again since)
+    if (!ctx->surf_current && (st = launch_surface_cells(ctx))) return st;
     // earlier frames' live particles (moved in place below) may still be on their way to the host
     PMS_CHECK(out_device_wait(ctx, ctx->diffuse_q));
     return diffuse_front(ctx, g, dp, cnt);

@@ -239,7 +239,9 @@ pms_status launch_surface_cells(pms_ctx* ctx) {
         g, ctx->cell_count.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->surf_count.as<uint32_t>(),
         ctx->cell_info.as<uint2>());
     PMS_LAUNCHED(ctx);
-    return scan_u32(ctx, ctx->surf_count.as<uint32_t>(), ctx->surf_start.as<uint32_t>(), g.sp_size, &cnt->ns);
+    pms_status st = scan_u32(ctx, ctx->surf_count.as<uint32_t>(), ctx->surf_start.as<uint32_t>(), g.sp_size, &cnt->ns);
+    ctx->surf_current = st == PMS_OK;
+    return st;
 }
 
 }  // namespace pms

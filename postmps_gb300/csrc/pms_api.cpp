@@ -510,6 +510,7 @@ extern "C" pms_status pms_build_grid(pms_ctx* c) {
     mark(c, kStageGrid);
     c->arrays_lent = false;
     c->df_normals_near = false;
+    c->surf_current = false;           // (its counters start again, also on the same upload)
     pms_status st = launch_bbox(c, true);
     if (st) return st;
     PMS_CUDA(c, cudaStreamSynchronize(c->stream));
