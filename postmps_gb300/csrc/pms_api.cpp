@@ -238,6 +238,7 @@ pms_status ensure_band_buffers(pms_ctx* c, uint32_t nv);
 void mark_stage(pms_ctx* c, int boundary);
 pms_status plain_band(pms_ctx* c);
 pms_status anisotropy_stage(pms_ctx* c, bool near);
+pms_status anisotropy_ready(pms_ctx* c);
 }  // namespace pms
 
 // a record per valid cube (at most nv): their number changes from frame to frame, so with headroom
@@ -510,7 +511,8 @@ extern "C" pms_status pms_build_grid(pms_ctx* c) {
     mark(c, kStageGrid);
     c->arrays_lent = false;
     c->df_normals_near = false;
-    c->surf_current = false;           // (its counters start again, also on the same upload)
+    // (the counters start again, also on the same upload)
+    c->surf_current = c->aniso_current = c->mc_classified = c->mc_compacted = false;
     pms_status st = launch_bbox(c, true);
     if (st) return st;
     PMS_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -539,16 +541,20 @@ pms_status pms::anisotropy_stage(pms_ctx* c, bool near) {
     cudaSetDevice(c->device);
     c->dens_far = false;
     c->dens_near = near;
-    if (c->n == 0) { c->have_aniso = true; return PMS_OK; }
+    if (c->n == 0) { c->have_aniso = c->aniso_current = true; return PMS_OK; }
     pms_status st;
     if ((st = launch_surface_cells(c))) return st;
     if ((st = launch_density_aniso(c))) return st;
-    c->have_aniso = true;
+    c->have_aniso = c->aniso_current = true;
     mark(c, kStageAniso + 1);
     return PMS_OK;
 }
 
 extern "C" pms_status pms_anisotropy(pms_ctx* c) { return pms::anisotropy_stage(c, false); }
+
+// Before a stage that reads what the anisotropy pass leaves (counters, surface list, support
+// radii): made again where the grid was built again since.
+pms_status pms::anisotropy_ready(pms_ctx* c) { return c->aniso_current ? PMS_OK : anisotropy_stage(c, c->dens_near); }
 
 // The band's size on the host, from counters just synchronised.
 static pms_status take_band_size(pms_ctx* c) {
@@ -576,8 +582,9 @@ static pms_status band_stage(pms_ctx* c, bool defer) {
     c->band_learned = c->mc_classified = c->mc_compacted = false;
     c->l_ncand = c->l_npred = c->l_nexact = c->l_ncert = c->l_nrecheck = 0;
     if (c->n == 0) { c->nv = 0; c->have_band = true; return PMS_OK; }
-    pms_status st = defer ? launch_band(c) : plain_band(c);
-    if (st) return st;
+    pms_status st;
+    if ((st = anisotropy_ready(c))) return st;
+    if ((st = defer ? launch_band(c) : plain_band(c))) return st;
     c->nv_pending = defer;
     c->have_band = true;
     mark(c, kStageBand + 1);
@@ -595,7 +602,10 @@ extern "C" pms_status pms_field(pms_ctx* c) {
     if (!c) return PMS_ERR_INVALID_ARGUMENT;
     if (!c->have_band) return pms_fail(c, PMS_ERR_STATE, "pms_field before pms_band");
     cudaSetDevice(c->device);
-    if (c->nv || c->nv_pending) { pms_status st = launch_field(c); if (st) return st; }
+    pms_status st;
+    // (a grid built again since the band took the band's count with it too)
+    if (!c->aniso_current && (st = band_stage(c, false))) return st;
+    if ((c->nv || c->nv_pending) && (st = launch_field(c))) return st;
     c->have_field = true;
     mark(c, kStageField + 1);
     return PMS_OK;

@@ -19,6 +19,7 @@ pms_status ensure_band_buffers(pms_ctx* c, uint32_t nv);
 void mark_stage(pms_ctx* c, int boundary);
 pms_status plain_band(pms_ctx* c);
 pms_status anisotropy_stage(pms_ctx* c, bool near);
+pms_status anisotropy_ready(pms_ctx* c);
 }  // namespace pms
 
 static pms_status zero_learn_counters(pms_ctx* c) {
@@ -138,6 +139,7 @@ extern "C" pms_status pms_band_learned(pms_ctx* c) {
     if (c->n == 0) { c->nv = 0; c->have_band = c->have_field = true; return PMS_OK; }
     pms_status st;
     // the plain band: where the field exists (a cube with a corner off it is never valid)
+    if ((st = anisotropy_ready(c))) return st;
     if ((st = plain_band(c))) return st;
     if ((st = ensure_learned_buffers(c, c->grid.sc_size, c->nv))) return st;
     if (c->nv && (st = learned_split(c, predict))) return st;

@@ -37,13 +37,15 @@ extern "C" pms_status pms_autotune(pms_ctx* c, pms_tune* out) {
     if (!c) return PMS_ERR_INVALID_ARGUMENT;
     if (!c->have_field || c->n == 0) return pms_fail(c, PMS_ERR_STATE, "pms_autotune needs a reconstructed frame");
     cudaSetDevice(c->device);
+    pms_status st;
+    // (a grid built again since took the anisotropy's and the band's counters with it)
+    if (!c->aniso_current && (st = pms_band(c))) return st;
     // the re-runs below bump device counters (FP64 solves); keep the frame's
     Counters saved;
     PMS_CUDA(c, cudaMemcpyAsync(&saved, c->counters.p, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream));
     PMS_CUDA(c, cudaStreamSynchronize(c->stream));
     const int sizes[3] = {64, 128, 256};
     const int vpts[3] = {1, 2, 4};
-    pms_status st;
     Tune best = c->tune;
     float best_aniso = 1e30f, best_field = 1e30f;
     for (int bd : sizes)

@@ -40,3 +40,42 @@ def test_diffuse_after_a_second_grid(pms_lib, tmp_config, before):
     for one, two in zip(*results):
         for a, b in zip(one, two, strict=True):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("band", ["band", "band_learned"])
+@pytest.mark.parametrize("first", ["band", "field", "marching_cubes"])
+def test_surface_after_a_second_grid(pms_lib, tmp_config, band, first):
+    """The surface stages from `first` on run after a second grid, on what the stages before left."""
+    pos, vel, text = scene()
+    once = ["anisotropy", "band", "field", "marching_cubes"] if band == "band" else ["anisotropy", band, "marching_cubes"]
+    then = once[1:] if first == "band" else ["field", "marching_cubes"] if first == "field" else ["marching_cubes"]
+    results = []
+    for again in (False, True):
+        with pms_lib.Context(pms_lib.load_config(tmp_config(text)), 0) as ctx:
+            ctx.set_band_mode("certified")                      # (read by band_learned alone)
+            ctx.upload(pos, vel)
+            for stage in ["build_grid"] + once + (["build_grid"] + then if again else []):
+                getattr(ctx, stage)()
+            results.append([ctx.mesh(False)[0], ctx.weld(False)])
+            if first != "marching_cubes":
+                results[-1] += [ctx.debug("band_list"), ctx.debug("surf_list")]
+                if band == "band":
+                    results[-1].append(ctx.debug("field"))
+    assert len(results[0][0]) > 0
+    for a, b in zip(*results, strict=True):
+        for x, y in zip(a, b, strict=True) if isinstance(a, tuple) else [(a, b)]:
+            np.testing.assert_array_equal(x, y)
+
+
+def test_autotune_after_a_second_grid(pms_lib, tmp_config):
+    pos, vel, text = scene()
+    with pms_lib.Context(pms_lib.load_config(tmp_config(text)), 0) as ctx:
+        ctx.upload(pos, vel)
+        ctx.build_grid()
+        ctx.surface()
+        mesh, field = ctx.mesh(False)[0], ctx.debug("field")
+        ctx.build_grid()
+        assert ctx.autotune()["field_ms"] > 0
+        ctx.marching_cubes()
+        np.testing.assert_array_equal(ctx.mesh(False)[0], mesh)
+        np.testing.assert_array_equal(ctx.debug("field"), field)
