@@ -170,16 +170,17 @@ __global__ void __launch_bounds__(256) k_df_begin(KGrid g, DiffuseParams dp, con
     }
 }
 
-// calculationofNormal: thread t < NumFree computes the normal of particle t.  With marks, only
-// where a wave crest may read it (NumFree counts the surface, but the particles are the first in
-// cell order, mostly the bottom of a pool at rest: three frames of a 1M-particle crown spent
-// 0.24 of 1.70 ms on normals that nothing read, 0.02 now); a download of the normals makes the rest.
+// calculationofNormal: thread t < NumFree (the particles of surface cells, Counters::ns) computes
+// the normal of particle t.  With marks, only where a wave crest may read it (NumFree counts the
+// surface, but the particles are the first in cell order, mostly the bottom of a pool at rest:
+// three frames of a 1M-particle crown spent 0.24 of 1.70 ms on normals that nothing read, 0.02
+// now); a download of the normals makes the rest.
 __global__ void __launch_bounds__(kThreads, 8) k_df_normal(KGrid g, DiffuseParams dp, const Counters* __restrict__ cnt,
                                                         const uint32_t* __restrict__ cell_start,
                                                         const float4* __restrict__ spos, uint32_t n,
                                                         const uint32_t* __restrict__ skeys, const uint8_t* __restrict__ marks,
                                                         float4* __restrict__ nrm) {
-    const uint32_t nf = min(cnt->n_free, n);
+    const uint32_t nf = min(cnt->ns, n);
     const float pad = 1e-4f * g.sp_cs, r2 = dp.hd_sq;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nf; t += gridDim.x * blockDim.x) {
         if (marks) {
@@ -919,6 +920,8 @@ pms_status launch_diffuse(pms_ctx* ctx) {
 // The normals that the last frame left out.
 static pms_status launch_normals_rest(pms_ctx* ctx) {
     if (!ctx->df_normals_near || ctx->arrays_lent || !ctx->n) return PMS_OK;
+    pms_status st;
+    if (!ctx->surf_current && (st = launch_surface_cells(ctx))) return st;     // the grid was built again since
     k_df_normal<<<grid_for(ctx->n, kThreads), kThreads, 0, ctx->stream>>>(
         kgrid_of(ctx->grid), diffuse_params(ctx), ctx->counters.as<Counters>(), ctx->cell_start.as<uint32_t>(),
         ctx->spos.as<float4>(), ctx->n, ctx->skeys.as<uint32_t>(), nullptr, ctx->d_nrm_free.as<float4>());

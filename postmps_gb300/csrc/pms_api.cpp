@@ -365,6 +365,7 @@ static void begin_frame(pms_ctx* c, uint32_t n) {
     c->ns = c->nv = c->nvalid = 0;
     c->nmesh = 0;
     c->nv_pending = false;
+    c->df_normals_near = false;
     for (int i = 0; i < kNumStages; ++i) c->ev_recorded[i] = false;
 }
 
@@ -510,7 +511,6 @@ extern "C" pms_status pms_build_grid(pms_ctx* c) {
     cudaSetDevice(c->device);
     mark(c, kStageGrid);
     c->arrays_lent = false;
-    c->df_normals_near = false;
     // (the counters start again, also on the same upload)
     c->surf_current = c->aniso_current = c->mc_classified = c->mc_compacted = false;
     pms_status st = launch_bbox(c, true);

@@ -79,3 +79,19 @@ def test_autotune_after_a_second_grid(pms_lib, tmp_config):
         ctx.marching_cubes()
         np.testing.assert_array_equal(ctx.mesh(False)[0], mesh)
         np.testing.assert_array_equal(ctx.debug("field"), field)
+
+
+def test_normals_after_a_second_grid(pms_lib, tmp_config):
+    """The colour-gradient normals that a frame left out are still made after a second grid."""
+    pos, vel, text = scene()
+    vel[len(vel) // 20:] = 0.0                                  # few particles that can spawn
+    normals = []
+    for again in (False, True):
+        with pms_lib.Context(pms_lib.load_config(tmp_config(text)), 0) as ctx:
+            ctx.upload(pos, vel)
+            ctx.run_frame()
+            if again:
+                ctx.build_grid()
+            normals.append(ctx.debug("free_normal"))
+    assert np.any(normals[0] != 0)
+    np.testing.assert_array_equal(normals[1], normals[0])
