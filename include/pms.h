@@ -450,7 +450,8 @@ pms_status pms_trainer_get_model(pms_trainer* t, pms_band_model* out);
  * continue one sequence); pms_batch_diffuse reads a frame's live particles.
  * With PMS_BATCH_LEARNED the learned band is used (PMS_BATCH_CERTIFIED: its
  * sign certification without the network); every frame's result equals its
- * single-frame run, and the plain band's.
+ * single-frame run, and the plain band's.  A frame that the context holds stays
+ * as it is: its results can be downloaded and worked on after a batch, too.
  * ------------------------------------------------------------------------- */
 typedef struct pms_frame {
     const float* pos_xyz;

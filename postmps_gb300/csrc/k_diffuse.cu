@@ -919,7 +919,7 @@ pms_status launch_diffuse(pms_ctx* ctx) {
 
 // The normals that the last frame left out.
 static pms_status launch_normals_rest(pms_ctx* ctx) {
-    if (!ctx->df_normals_near || ctx->arrays_lent || !ctx->n) return PMS_OK;
+    if (!ctx->df_normals_near || !ctx->n) return PMS_OK;
     pms_status st;
     if (!ctx->surf_current && (st = launch_surface_cells(ctx))) return st;     // the grid was built again since
     k_df_normal<<<grid_for(ctx->n, kThreads), kThreads, 0, ctx->stream>>>(

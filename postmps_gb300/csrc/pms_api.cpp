@@ -510,7 +510,6 @@ extern "C" pms_status pms_build_grid(pms_ctx* c) {
     if (!c->have_particles) return pms_fail(c, PMS_ERR_STATE, "pms_build_grid before pms_upload_particles");
     cudaSetDevice(c->device);
     mark(c, kStageGrid);
-    c->arrays_lent = false;
     // (the counters start again, also on the same upload)
     c->surf_current = c->aniso_current = c->mc_classified = c->mc_compacted = false;
     pms_status st = launch_bbox(c, true);
@@ -1084,11 +1083,6 @@ extern "C" pms_status pms_debug_download(pms_ctx* c, int id, void* dst, uint64_t
             const bool ok = id == PMS_ARRAY_BAND_LIST ? c->have_band : id == PMS_ARRAY_FIELD ? c->have_field : c->have_mc;
             if (!ok) return PMS_ERR_STATE;
             // the stages keep the band as bits and the field over the grid: the band-order arrays are made here
-            // (zeros once a batch has run in the frame's arrays)
-            if (c->arrays_lent) {
-                out.assign(4 * (size_t)nv, 0);
-                break;
-            }
             if (nv) {
                 PMS_CUDA(c, c->vlist.ensure(4 * (size_t)nv));
                 PMS_CUDA(c, c->field.ensure(4 * (size_t)nv));

@@ -9,13 +9,14 @@
 // into one CUDA graph whose kernels size their work from counts kept on the
 // device -- one Counters record per frame -- with host-side launch grids and
 // buffers sized by per-frame bounds, so nothing in the graph waits for the
-// host.  Frames run one after another on the context's buffers; meshes land
-// behind each other in one arena (the running offset lives on the device).
-// The graph is kept and relaunched while the frames' grids stay the same.
-// Frames are spread over lanes -- the context and up to three sub-contexts,
-// each with its own buffers and stream -- that fork from and join the
-// capture stream, so independent frames overlap on the GPU; a frame's mesh
-// claims its stretch of the arena with an atomic add.
+// host.  Meshes land behind each other in one arena (the running offset lives
+// on the device).  The graph is kept and relaunched while the frames' grids stay
+// the same.  Frames are spread over up to four lanes, each with its own buffers
+// and stream, that fork from and join the capture stream, so independent frames
+// overlap on the GPU; a frame's mesh claims its stretch of the arena with an
+// atomic add.  The lanes are sub-contexts, but a context that never held a frame
+// is the first lane itself; one that did keeps its arrays, so that what its frame
+// left can be downloaded and worked on after a batch as before it.
 //
 // With the learned band, the graph holds each frame's plain band, prediction,
 // split, exact field at the predicted corners, sign certification of the rest,
@@ -62,8 +63,8 @@ struct BatchState {
     std::vector<Counters> hcnt;
     std::vector<unsigned long long> hbase;
     std::vector<cudaEvent_t> ev, ev_end;         // per-frame start / end, recorded inside the graph
-    std::vector<pms_ctx*> lanes;                 // sub-contexts (lane 0 is the context itself)
-    std::vector<cudaEvent_t> join;
+    std::vector<pms_ctx*> lanes;                 // sub-contexts (lane 0 null: the context itself)
+    std::vector<cudaEvent_t> join;               // one per lane
     cudaEvent_t fork = nullptr;
     cudaGraphExec_t exec = nullptr;
     int flags = -1;
@@ -93,7 +94,8 @@ struct BatchState {
         for (cudaEvent_t e : ev_end) cudaEventDestroy(e);
         for (cudaEvent_t e : join) cudaEventDestroy(e);
         if (fork) cudaEventDestroy(fork);
-        for (pms_ctx* l : lanes) pms_destroy(l);
+        for (pms_ctx* l : lanes)
+            if (l) pms_destroy(l);
         for (cudaEvent_t e : ev_surf) cudaEventDestroy(e);
         for (cudaEvent_t e : ev_diff) cudaEventDestroy(e);
         if (djoin) cudaEventDestroy(djoin);
@@ -209,8 +211,8 @@ static pms_status capture_frame(pms_ctx* c, BatchState* b, uint32_t f, int band,
 
 static constexpr uint32_t kBatchLanes = 4;
 
-// lane l of the batch: the context itself for l = 0, else a sub-context
-static pms_ctx* lane_ctx(pms_ctx* c, BatchState* b, uint32_t l) { return l == 0 ? c : b->lanes[l - 1]; }
+// lane l of the batch
+static pms_ctx* lane_ctx(pms_ctx* c, BatchState* b, uint32_t l) { return b->lanes[l] ? b->lanes[l] : c; }
 
 static pms_status capture(pms_ctx* c, BatchState* b, int band, uint32_t nlanes, bool diffuse) {
     if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
@@ -235,7 +237,8 @@ static pms_status capture(pms_ctx* c, BatchState* b, int band, uint32_t nlanes, 
     cudaError_t e = cudaMemsetAsync(b->base.as<unsigned long long>() + k, 0, sizeof(unsigned long long), c->stream);
     if (e == cudaSuccess && dl) e = cudaMemsetAsync(b->drun.p, 0, sizeof(unsigned long long), c->stream);
     if (e == cudaSuccess) e = cudaEventRecord(b->fork, c->stream);
-    for (uint32_t l = 1; l < nlanes && e == cudaSuccess; ++l) e = cudaStreamWaitEvent(lane_ctx(c, b, l)->stream, b->fork, 0);
+    for (uint32_t l = 0; l < nlanes && e == cudaSuccess; ++l)
+        if (b->lanes[l]) e = cudaStreamWaitEvent(b->lanes[l]->stream, b->fork, 0);
     if (e == cudaSuccess && dl) e = cudaStreamWaitEvent(dl->stream, b->fork, 0);
     if (e != cudaSuccess) st = PMS_ERR_CUDA;
     {
@@ -280,9 +283,9 @@ static pms_status capture(pms_ctx* c, BatchState* b, int band, uint32_t nlanes, 
         }
         if (dl) b->d_out = dl->d_old.p;
     }
-    for (uint32_t l = 1; l < nlanes && !st; ++l) {
-        if (cudaEventRecord(b->join[l - 1], lane_ctx(c, b, l)->stream) != cudaSuccess ||
-            cudaStreamWaitEvent(c->stream, b->join[l - 1], 0) != cudaSuccess)
+    for (uint32_t l = 0; l < nlanes && !st; ++l) {
+        if (b->lanes[l] && (cudaEventRecord(b->join[l], b->lanes[l]->stream) != cudaSuccess ||
+                            cudaStreamWaitEvent(c->stream, b->join[l], 0) != cudaSuccess))
             st = PMS_ERR_CUDA;
     }
     if (dl && !st &&
@@ -302,8 +305,8 @@ static pms_status capture(pms_ctx* c, BatchState* b, int band, uint32_t nlanes, 
     if (st) {
         if (graph) cudaGraphDestroy(graph);
         // a lane's failure message lives on the lane
-        for (uint32_t l = 1; l < nlanes; ++l)
-            if (!lane_ctx(c, b, l)->last_error.empty()) c->last_error = lane_ctx(c, b, l)->last_error;
+        for (uint32_t l = 0; l < nlanes; ++l)
+            if (b->lanes[l] && !b->lanes[l]->last_error.empty()) c->last_error = b->lanes[l]->last_error;
         if (dl && !dl->last_error.empty()) c->last_error = dl->last_error;
         return st;
     }
@@ -397,9 +400,6 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
     }
     BatchState* b = batch_of(c);
     if (k == 0) { b->n.clear(); b->hcnt.clear(); return PMS_OK; }
-    // the context is a lane, and its arrays are about to be the frames': downloads make nothing from them any more
-    c->dens_far = false;
-    c->arrays_lent = true;
     // ---- pass 1: arena, uploads, bounding boxes
     uint64_t total = 0;
     std::vector<uint64_t> off(k);
@@ -459,15 +459,20 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
     b->grid = grid;
     // ---- lanes and their capacities (nothing may allocate inside the graph)
     const uint32_t nlanes = std::min<uint32_t>(kBatchLanes, k);
-    while (b->lanes.size() + 1 < nlanes) {
+    for (uint32_t l = 0; l < nlanes; ++l) {
+        if (b->lanes.size() == l) {
+            cudaEvent_t e;
+            PMS_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            b->join.push_back(e);
+            b->lanes.push_back(nullptr);
+        }
+        if (b->lanes[l] || (l == 0 && !c->have_particles)) continue;
         pms_ctx* lc = nullptr;
         pms_config lcfg = c->cfg;
         lcfg.band_model[0] = 0;
         if ((st = pms_create(&lcfg, c->device, &lc))) return pms_fail(c, st, "batch lane context");
-        b->lanes.push_back(lc);
-        cudaEvent_t e;
-        PMS_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        b->join.push_back(e);
+        b->lanes[l] = lc;
+        grids_same = false;
     }
     if (!b->fork) PMS_CUDA(c, cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
     for (uint32_t l = 0; l < nlanes; ++l)

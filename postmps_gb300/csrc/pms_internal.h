@@ -203,7 +203,6 @@ struct pms_ctx {
     bool surf_current = false;   // the present grid's surface cells are counted (Counters::ns, surf_start, cell_info)
     bool aniso_current = false;  // the anisotropy pass ran on the present grid (its counters, surface list and radii)
     bool dens_near = false;      // asked: the stages after the anisotropy read densities near the surface only
-    bool arrays_lent = false;    // a batch has run in the context's arrays since its last grid
     bool dens_far = false;       // the last density pass left out the blocks far from the surface
     bool nv_pending = false;     // nv is on the device: the marching cubes' synchronisation reads it
 
