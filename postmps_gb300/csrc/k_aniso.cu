@@ -63,7 +63,7 @@ __device__ __forceinline__ float mass_over(float mass, float r) { return r == 0.
 // - k_density_tiles: a warp per block of 2 x 2 x 2 cells.  Its particles (27 at rest, one per
 //   lane) share their neighbours: the warp reads each once, keeps those within h of the
 //   particles' box in shared memory, and all lanes add them.  Used where every particle's
-//   window [c - e, c + e] surely holds its support (e cells exceed h by kRangeMargin: the
+//   window [c - e, c + e] surely holds its support (e cells exceed h by the margin: the
 //   sum then does not depend on the window).
 // - k_density: a thread per particle over its own window, else.
 // - k_density_warp: a warp per particle for frames too small to fill the GPU with
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density(KGrid g, AnisoParams 
                                                       const uint32_t* __restrict__ cell_start, const float4* __restrict__ spos,
                                                       float* __restrict__ rho, float4* __restrict__ aniso, uint32_t n) {
     const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1];
-    const float pad = 1e-4f * g.sp_cs;
+    const float pad = g.pad;
     const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 pi4 = spos[i];
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kThreads) k_density_warp(KGrid g, AnisoParams 
                                                            const float4* __restrict__ spos, float* __restrict__ rho,
                                                            float4* __restrict__ aniso, uint32_t n) {
     const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1], lane = threadIdx.x & 31u;
-    const float pad = 1e-4f * g.sp_cs;
+    const float pad = g.pad;
     const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
         const float4 pi4 = spos[i];
@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoP
     __shared__ float4 stage_all[BT / 32][kDensStage];
     float4* stage = stage_all[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u, n_blocks = *n_blocks_dev;
-    const float pad = 1e-4f * g.sp_cs, inv_cs = 1.f / g.sp_cs;
-    const float rc = ap.h * inv_cs + kRangeMargin, reach2 = ap.h_sq * 1.001f;
+    const float pad = g.pad, inv_cs = 1.f / g.sp_cs;
+    const float rc = ap.h * inv_cs + g.margin, reach2 = ap.h_sq * 1.001f;
     const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
     for (;;) {
         uint32_t bi = 0u;
@@ -432,7 +432,7 @@ __device__ __forceinline__ void moments_warp(const KGrid& g, const AnisoParams& 
     for (uint32_t k = lane; k < 64u; k += 32u) hits[4 * kCol + k] = 1.f;
     __syncwarp();
     const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1];
-    const float pad = 1e-4f * g.sp_cs, r2h_sq = ap.r2h * ap.r2h, inv_r2h = 1.f / ap.r2h;
+    const float pad = g.pad, r2h_sq = ap.r2h * ap.r2h, inv_r2h = 1.f / ap.r2h;
     // lane q's sum adds (w f1) f2: s0 | sx sy sz | sxx sxy sxz syy syz szz
     const int f1 = lane < 4u ? (int)lane : (lane < 7u ? 1 : (lane < 9u ? 2 : 3));
     const int f2 = lane < 4u ? 4 : (lane < 7u ? (int)lane + 1 : (lane < 9u ? (int)lane - 1 : 7));
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_moments(KGrid g, AnisoParams 
                                                       float4* __restrict__ mom) {
     const uint32_t ns = cnt->ns;
     const uint32_t rx = g.spres[0], rxy = g.spres[0] * g.spres[1];
-    const float pad = 1e-4f * g.sp_cs;
+    const float pad = g.pad;
     const float r2h_sq = ap.r2h * ap.r2h;
     const float inv_r2h = 1.f / ap.r2h;
     if (ns <= kMomentsWarp) {
@@ -687,7 +687,7 @@ static AnisoParams aniso_params(const pms_ctx* ctx, const KGrid& g) {
 // Blocks of cells between a surface cell and the first far block: cells whose indices
 // differ by k are (k - 1) cells apart at least.
 static int density_reach(const KGrid& g, float h) {
-    const float cells = 1.001f * (2.f * h + g.sc_cs) / g.sp_cs + 2.f * kRangeMargin;
+    const float cells = 1.001f * (2.f * h + g.sc_cs) / g.sp_cs + 2.f * g.margin;
     return ((int)floorf(cells) + 2) / 2;
 }
 
@@ -752,7 +752,7 @@ pms_status launch_density_aniso(pms_ctx* ctx) {
             g, ap, sl, ctx->skeys.as<uint32_t>(), ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(), ctx->rho.as<float>(),
             ctx->aniso.as<float4>(), n);
         PMS_LAUNCHED(ctx);
-    } else if ((float)g.spexpand * g.sp_cs - P.h >= kRangeMargin * g.sp_cs) {
+    } else if ((float)g.spexpand * g.sp_cs - P.h >= g.margin * g.sp_cs) {
         // (a scalar cell above h would let the dilation wrap past the grid's margin of 2 h)
         ctx->dens_far = ctx->dens_near && n >= kDensityNear && 2.f * g.sc_cs <= P.h && density_reach(g, P.h) < 32;
         if ((st = density_blocks(ctx, g, ap, sl, ctx->dens_far ? DensBlocks::kNear : DensBlocks::kAll))) return st;

@@ -48,7 +48,7 @@ __device__ __forceinline__ void particle_box(const KGrid& g, int ext, const floa
 }
 
 // Spatial cells of the particles whose AABB p +- h can hold a vertex of the tile [t0, t1]:
-// kRangeMargin cells, and four units in the last place of the largest coordinate, cover the
+// range_margin cells, and four units in the last place of the largest coordinate, cover the
 // rounding of cell keys, vertex coordinates and p +- h.
 struct TileCells {
     int lo[3], hi[3];
@@ -57,7 +57,7 @@ __device__ __forceinline__ TileCells tile_cells(const KGrid& g, float h, float i
     TileCells c;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const float slack = (fabsf(g.min_pos[k]) + (float)g.spres[k] * g.sp_cs) * 0x1p-21f + kRangeMargin * g.sp_cs;
+        const float slack = (fabsf(g.min_pos[k]) + (float)g.spres[k] * g.sp_cs) * 0x1p-21f + g.margin * g.sp_cs;
         const float a = sc_coord_i(g, t0[k], k) - h - slack - g.min_pos[k], b = sc_coord_i(g, t1[k], k) + h + slack - g.min_pos[k];
         c.lo[k] = max((int)floorf(a * inv_sp), 0);
         c.hi[k] = min((int)floorf(b * inv_sp), (int)g.spres[k] - 1);

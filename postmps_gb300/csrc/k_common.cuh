@@ -1,6 +1,7 @@
 // k_common.cuh -- device helpers shared by the libpms kernels.
 #pragma once
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include "pms_internal.h"
 
@@ -13,7 +14,22 @@ struct KGrid {
     uint32_t spres[3], scres[3];
     int32_t spexpand, scexpand, spexpand_diffuse;
     uint32_t sp_size, sc_size;
+    float margin, pad;        // range_margin in cells; what a cell's box is widened by, a length
 };
+
+// Margin, in cells, added to every range that the neighbour walks cut from a
+// support radius, and to the cells that a tile's windows are taken from.  The
+// ranges are computed from the point's position in cell units, u = (p - min) / cell:
+// the difference, the reciprocal, the product and the sum with the radius are each
+// rounded by up to 2^-24 of u, as are the difference and the quotient of a
+// particle's key, so a cell is up to 6 x 2^-24 of the longest axis off.  0.01 cells
+// cover that up to 20,971 cells per axis, 2^-21 of the axis beyond.  A cell left out
+// by a cut therefore holds no particle within the support, and the cut changes no sum.
+// (0.01 on every grid gave a sheet 262,144 cells from a stray particle field values
+// that were up to 2 % off.)
+inline float range_margin(const uint32_t res[3]) {
+    return std::max(0.01f, 0x1p-21f * (float)std::max(res[0], std::max(res[1], res[2])));
+}
 
 inline KGrid kgrid_of(const pms_grid& g) {
     KGrid k;
@@ -30,6 +46,8 @@ inline KGrid kgrid_of(const pms_grid& g) {
     k.spexpand_diffuse = g.spexpand_diffuse;
     k.sp_size = g.sp_size;
     k.sc_size = g.sc_size;
+    k.margin = range_margin(g.spres);
+    k.pad = (k.margin > 0.01f ? k.margin : 1e-4f) * g.sp_grid_size;
     return k;
 }
 
@@ -102,14 +120,6 @@ __device__ __forceinline__ void publish_counters(const Counters* cnt, uint32_t* 
     for (uint32_t i = threadIdx.x; i < sizeof(Counters) / 4; i += blockDim.x) mirror[i] = __ldcg(&src[i]);
 }
 
-// Margin, in cells, added to every range that the neighbour walks cut from a
-// support radius.  The ranges are computed from the point's position in cell
-// units, u = (p - min) / cell, whose rounding error (like that of a particle's
-// own key) stays below 1e-3 cells on grids of up to 8000 cells per axis; a cell
-// left out by the cut therefore holds no particle within the support, and the
-// cut changes no sum.
-constexpr float kRangeMargin = 0.01f;
-
 // Cells per stretch of a row that keeps its particles' largest support (the row's own largest
 // is often a lone particle's far along it).
 constexpr int kRadSeg = 8;
@@ -159,21 +169,21 @@ __device__ __forceinline__ void row_walk(const KGrid& g, float3 p, uint3 lo, uin
     const float cs = g.sp_cs, inv = 1.f / g.sp_cs;
     const float ux = (p.x - g.min_pos[0]) * inv, uy = (p.y - g.min_pos[1]) * inv, uz = (p.z - g.min_pos[2]) * inv;
     int za, zb;
-    cell_range(uz, sqrtf(r2) * inv + kRangeMargin, lo.z, hi.z, za, zb);
+    cell_range(uz, sqrtf(r2) * inv + g.margin, lo.z, hi.z, za, zb);
     for (int z = za; z < zb; ++z) {
         const float z0 = g.min_pos[2] + (float)z * cs;
         const float gz0 = axis_gap(p.z, z0 - pad, z0 + cs + pad);
         const float gz = gz0 * gz0;
         if (gz >= r2) continue;
         int ya, yb;
-        cell_range(uy, sqrtf(r2 - gz) * inv + kRangeMargin, lo.y, hi.y, ya, yb);
+        cell_range(uy, sqrtf(r2 - gz) * inv + g.margin, lo.y, hi.y, ya, yb);
         for (int y = ya; y < yb; ++y) {
             const float y0 = g.min_pos[1] + (float)y * cs;
             const float gy0 = axis_gap(p.y, y0 - pad, y0 + cs + pad);
             const float gyz = gz + gy0 * gy0;
             if (gyz >= r2) continue;
             int xa, xb;
-            cell_range(ux, sqrtf(r2 - gyz) * inv + kRangeMargin, lo.x, hi.x, xa, xb);
+            cell_range(ux, sqrtf(r2 - gyz) * inv + g.margin, lo.x, hi.x, xa, xb);
             if (xa >= xb) continue;
             const uint32_t row = (uint32_t)z * srxy + (uint32_t)y * srx;
             const uint32_t ja = __ldg(&cell_start[row + (uint32_t)xa]), jb = __ldg(&cell_start[row + (uint32_t)xb]);
@@ -217,7 +227,7 @@ __device__ __forceinline__ uint32_t box_row(const KGrid& g, float3 b0, float3 b1
     const float gy = fmaxf(fmaxf(y0 - pad - b1.y, b0.y - (y0 + cs + pad)), 0.f);
     const float gap = gz * gz + gy * gy;
     if (gap >= r2) return 0u;
-    const float rc = sqrtf(r2 - gap) * inv + kRangeMargin;
+    const float rc = sqrtf(r2 - gap) * inv + g.margin;
     const int xa = max((int)floorf((b0.x - g.min_pos[0]) * inv - rc), xlo);
     const int xb = min((int)floorf((b1.x - g.min_pos[0]) * inv + rc) + 1, xhi);
     if (xa >= xb) return 0u;
@@ -232,7 +242,7 @@ template <class Body>
 __device__ __forceinline__ void warp_walk(const KGrid& g, float3 p, uint3 lo, uint3 hi, float r2, float pad,
                                           const uint32_t* __restrict__ cell_start, Body&& body) {
     const uint32_t lane = threadIdx.x & 31u;
-    const float inv = 1.f / g.sp_cs, rc = sqrtf(r2) * inv + kRangeMargin;
+    const float inv = 1.f / g.sp_cs, rc = sqrtf(r2) * inv + g.margin;
     int za, zb, ya, yb;
     cell_range((p.z - g.min_pos[2]) * inv, rc, lo.z, hi.z, za, zb);
     cell_range((p.y - g.min_pos[1]) * inv, rc, lo.y, hi.y, ya, yb);

@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_normal(KGrid g, DiffuseParam
                                                         const uint32_t* __restrict__ skeys, const uint8_t* __restrict__ marks,
                                                         float4* __restrict__ nrm) {
     const uint32_t nf = min(cnt->ns, n);
-    const float pad = 1e-4f * g.sp_cs, r2 = dp.hd_sq;
+    const float pad = g.pad, r2 = dp.hd_sq;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nf; t += gridDim.x * blockDim.x) {
         if (marks) {
             const uint32_t key = skeys[t], rx = g.spres[0], row = key / rx;
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_trapped(KGrid g, DiffusePara
                                                          float4* __restrict__ pot, Counters* __restrict__ cnt,
                                                          uint32_t* __restrict__ crests) {
     const uint32_t na = cnt->df_active;
-    const float pad = 1e-4f * g.sp_cs, r2 = dp.hd_sq;
+    const float pad = g.pad, r2 = dp.hd_sq;
     for (uint32_t t0 = blockIdx.x * blockDim.x; t0 < na; t0 += gridDim.x * blockDim.x) {      // whole warps together
         const bool in = t0 + threadIdx.x < na;
         const uint32_t i = active[in ? t0 + threadIdx.x : t0];
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_crests(KGrid g, DiffuseParam
                                                         const float4* __restrict__ spos,
                                                         const float4* __restrict__ nrm, float4* __restrict__ pot) {
     const uint32_t nc = cnt->df_crests;
-    const float pad = 1e-4f * g.sp_cs, r2 = dp.hd_sq;
+    const float pad = g.pad, r2 = dp.hd_sq;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nc; t += gridDim.x * blockDim.x) {
         const uint32_t i = crests[t];
         const float4 p4 = spos[i], ni = nrm[i];
@@ -356,7 +356,7 @@ __device__ __forceinline__ int count_within_gen(const KGrid& g, const DiffusePar
     uint3 lo, hi;
     diffuse_box(g, px, py, pz, lo, hi);
     const float3 p = make_float3(px, py, pz);
-    const float r = dp.hd * kSupportGrow, pad = 1e-4f * g.sp_cs, inv = 1.f / g.sp_cs, rc = r * inv + kRangeMargin;
+    const float r = dp.hd * kSupportGrow, pad = g.pad, inv = 1.f / g.sp_cs, rc = r * inv + g.margin;
     int za, zb, ya, yb;
     cell_range((pz - g.min_pos[2]) * inv, rc, lo.z, hi.z + 1u, za, zb);
     cell_range((py - g.min_pos[1]) * inv, rc, lo.y, hi.y + 1u, ya, yb);
@@ -557,7 +557,7 @@ __device__ __forceinline__ int count_within_near(const KGrid& g, const DiffusePa
     hi = make_uint3(hi.x + 1, hi.y + 1, hi.z + 1);          // row_walk takes [lo, hi)
     const float r = dp.hd * kSupportGrow;
     int count = 0;
-    row_walk(g, make_float3(px, py, pz), lo, hi, r * r, 1e-4f * g.sp_cs, cell_start, [&](uint32_t j) {
+    row_walk(g, make_float3(px, py, pz), lo, hi, r * r, g.pad, cell_start, [&](uint32_t j) {
         const float4 q = __ldg(&spos[j]);
         const float sx = __fsub_rn(px, q.x), sy = __fsub_rn(py, q.y), sz = __fsub_rn(pz, q.z);
         if (dot_rn(sx, sy, sz, sx, sy, sz) <= dp.d2_hd) ++count;   // |s| <= hd
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_update(KGrid g, DiffuseParam
             diffuse_box(g, px, py, pz, lo, hi);
             hi = make_uint3(hi.x + 1, hi.y + 1, hi.z + 1);
             const float r = 2.f * dp.hd * kSupportGrow;
-            row_walk(g, make_float3(px, py, pz), lo, hi, r * r, 1e-4f * g.sp_cs, cell_start, [&](uint32_t j) {
+            row_walk(g, make_float3(px, py, pz), lo, hi, r * r, g.pad, cell_start, [&](uint32_t j) {
                 const float4 q = __ldg(&spos[j]);
                 const float sx = __fsub_rn(px, q.x), sy = __fsub_rn(py, q.y), sz = __fsub_rn(pz, q.z);
                 if (dot_rn(sx, sy, sz, sx, sy, sz) <= dp.d2_hd) ++density;   // |s| <= hd

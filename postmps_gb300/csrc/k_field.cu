@@ -96,7 +96,7 @@ k_field_cert(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const ui
     const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
     const uint32_t srx = g.spres[0], sry = g.spres[1];
     const uint32_t e2 = 2u * (uint32_t)g.spexpand;
-    const float pad = 1e-4f * g.sp_cs, inv_cs = 1.f / g.sp_cs;
+    const float pad = g.pad, inv_cs = 1.f / g.sp_cs;
     const float* __restrict__ row_rad = cell_rad + g.sp_size;
     // largest support of any particle this frame
     const float rmax = fmaxf(__uint_as_float(cnt->rad_max_bits), fp.h) * fp.grow;
@@ -198,12 +198,12 @@ k_field_cert(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const ui
             }
         }
         int za, zb;
-        cell_range(uz, rmax * inv_cs + kRangeMargin, lo.z, hi.z, za, zb);
+        cell_range(uz, rmax * inv_cs + g.margin, lo.z, hi.z, za, zb);
         for (int z = za; z < zb; ++z) {
             const float gz = gap2_axis(vz, g.min_pos[2] + (float)z * g.sp_cs, g.sp_cs, pad);
             if (gz >= rmax2) continue;
             int ya, yb;
-            cell_range(uy, sqrtf(rmax2 - gz) * inv_cs + kRangeMargin, lo.y, hi.y, ya, yb);
+            cell_range(uy, sqrtf(rmax2 - gz) * inv_cs + g.margin, lo.y, hi.y, ya, yb);
             for (int y = ya; y < yb; ++y) {
                 const float gyz = gz + gap2_axis(vy, g.min_pos[1] + (float)y * g.sp_cs, g.sp_cs, pad);
                 const uint32_t rowi = (uint32_t)z * sry + (uint32_t)y;
@@ -212,7 +212,7 @@ k_field_cert(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const ui
                 if (gyz >= rr2) continue;           // every cell of the row adds 0
                 const uint32_t row = rowi * srx;
                 // each vertex's cells of this row: those the row's largest support reaches
-                const float rxc = sqrtf(rr2 - gyz) * inv_cs + kRangeMargin;
+                const float rxc = sqrtf(rr2 - gyz) * inv_cs + g.margin;
                 int xs[K], xe[K];
                 bool live[K];
                 int X0 = 0x7fffffff, X1 = -1;
@@ -480,7 +480,7 @@ field_tiles(const KGrid& g, const FieldParams& fp, FieldStage* stage, const Coun
     const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
     const int srx = (int)g.spres[0], sry = (int)g.spres[1], srz = (int)g.spres[2];
     const int e2 = 2 * g.spexpand;
-    const float pad = 1e-4f * g.sp_cs, cs = g.sp_cs, inv_cs = 1.f / g.sp_cs;
+    const float pad = g.pad, cs = g.sp_cs, inv_cs = 1.f / g.sp_cs;
     // largest support per stretch of kRadSeg cells of a row
     const float* __restrict__ seg_rad = cell_rad + g.sp_size + g.spres[1] * g.spres[2];
     const uint32_t nseg = rad_segments(g.spres[0]);
@@ -532,12 +532,12 @@ field_tiles(const KGrid& g, const FieldParams& fp, FieldStage* stage, const Coun
             const float uy0 = (by0 - g.min_pos[1]) * inv_cs, uy1 = (by1 - g.min_pos[1]) * inv_cs;
             const float uz0 = (bz0 - g.min_pos[2]) * inv_cs, uz1 = (bz1 - g.min_pos[2]) * inv_cs;
             // cells some vertex's window holds [u.., u..), and cells that every window holds past
-            // its first column [i.., i..), from the corners' cells taken kRangeMargin apart (the
+            // its first column [i.., i..), from the corners' cells taken a margin apart (the
             // vertices' own cells lie between); near the grid's low side, where the reference's
             // unsigned window wraps, every cell takes the general path
-            const int cx0 = (int)floorf(ux0 - kRangeMargin), cx1 = (int)floorf(ux1 + kRangeMargin);
-            const int cy0 = (int)floorf(uy0 - kRangeMargin), cy1 = (int)floorf(uy1 + kRangeMargin);
-            const int cz0 = (int)floorf(uz0 - kRangeMargin), cz1 = (int)floorf(uz1 + kRangeMargin);
+            const int cx0 = (int)floorf(ux0 - g.margin), cx1 = (int)floorf(ux1 + g.margin);
+            const int cy0 = (int)floorf(uy0 - g.margin), cy1 = (int)floorf(uy1 + g.margin);
+            const int cz0 = (int)floorf(uz0 - g.margin), cz1 = (int)floorf(uz1 + g.margin);
             const bool regular = min(cx0, min(cy0, cz0)) >= e2;
             const int ulx = regular ? cx0 - e2 : 0, uhx = regular ? min(cx1 + e2, srx - 1) : srx;
             const int uly = regular ? cy0 - e2 : 0, uhy = regular ? min(cy1 + e2, sry - 1) : sry;
@@ -546,7 +546,7 @@ field_tiles(const KGrid& g, const FieldParams& fp, FieldStage* stage, const Coun
             const int ily = cy1 - e2, ihy = min(cy0 + e2, sry - 1);
             const int ilz = cz1 - e2, ihz = min(cz0 + e2, srz - 1);
             // rows (z, y) within the frame's largest support of the box
-            const float rc = rmax * inv_cs + kRangeMargin;
+            const float rc = rmax * inv_cs + g.margin;
             const int za = max((int)floorf(uz0 - rc), ulz), zb = min((int)floorf(uz1 + rc) + 1, uhz);
             const int ya = max((int)floorf(uy0 - rc), uly), yb = min((int)floorf(uy1 + rc) + 1, uhy);
             const int ny = yb - ya, nrow = ny > 0 && zb > za ? ny * (zb - za) : 0;
@@ -647,7 +647,7 @@ field_tiles(const KGrid& g, const FieldParams& fp, FieldStage* stage, const Coun
                     rr *= fp.grow;
                     const float rr2 = rr * rr;
                     if (gyz < rr2) {
-                        const float rxc = sqrtf(rr2 - gyz) * inv_cs + kRangeMargin;
+                        const float rxc = sqrtf(rr2 - gyz) * inv_cs + g.margin;
                         const int xa = max((int)floorf(ux0 - rxc), ulx), xb = min((int)floorf(ux1 + rxc) + 1, uhx);
                         if (xa < xb) {
                             const uint32_t row = rowi * (uint32_t)srx;

@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kThreads) k_scalar_values(KGrid g, float h, co
                                                             const float4* __restrict__ spos, const float4* __restrict__ svel,
                                                             const float* __restrict__ rho, float* __restrict__ out) {
     const unsigned long long m = cnt->nmesh;
-    const float pad = 1e-4f * g.sp_cs;
+    const float pad = g.pad;
     for (unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; t < m;
          t += (unsigned long long)gridDim.x * blockDim.x) {
         const float3 v = make_float3(vert[3 * t], vert[3 * t + 1], vert[3 * t + 2]);
