@@ -492,13 +492,14 @@ pms_status pms_batch_info(pms_ctx* ctx, uint32_t* graph_kernels, uint32_t* captu
  * moments and field, and the field's 1/2/4 vertices per lane --
  * keeps the fastest in the context (results do not depend on the shape) and
  * reports it.  pms_set_tune applies a shape chosen earlier (e.g. cached by
- * the caller per workload); batches use the context's shape.
+ * the caller per workload; what pms_get_tune reported before a tuning undoes
+ * it); batches use the context's shape.
  * ------------------------------------------------------------------------- */
 typedef struct pms_tune {
     int field_threads, field_waves, density_threads, moments_threads;
-    int field_vpt;                     /* band vertices a lane of the field owns: 1, 2 or 4 (until a shape is tuned or set
-                                          the field chooses per frame; field_waves is kept for callers, no launch
-                                          depends on it) */
+    int field_vpt;                     /* band vertices a lane of the field owns: 1, 2 or 4, or 0 (as a context starts): the
+                                          field chooses per frame.  field_waves (1 to 64) is kept for callers, no
+                                          launch depends on it */
     float anisotropy_ms, field_ms;     /* the chosen shapes' times on the tuning frame */
 } pms_tune;
 pms_status pms_autotune(pms_ctx* ctx, pms_tune* out);

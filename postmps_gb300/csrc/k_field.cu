@@ -763,7 +763,7 @@ size_t field_tile_bytes(const pms_grid& g, uint64_t nv) {
 static int field_pick(const pms_ctx* ctx, FieldPick& p) {
     p.few = 160000u;
     p.many = 0xffffffffu;
-    if (!ctx->tune.field_auto) return ctx->tune.field_vpt;
+    if (ctx->tune.field_vpt) return ctx->tune.field_vpt;
     const pms_params& P = ctx->prm;
     const pms_grid& g = ctx->grid;
     // the particles' share of their bounding box (the scalar grid has 2 h around it)

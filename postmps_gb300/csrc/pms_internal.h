@@ -131,10 +131,10 @@ struct ScanTemp {
 };
 
 // Launch shapes chosen by the autotuner (pms_autotune): threads per block of
-// the neighbour walks and the field's resident-block cap (blocks per SM).
+// the neighbour walks and the field's vertices per lane (0: it picks them itself, per frame).
+// field_waves is only handed back: no launch depends on it.
 struct Tune {
-    int field_threads = 128, field_waves = 8, density_threads = 128, moments_threads = 128, field_vpt = 2;
-    bool field_auto = true;    // the field picks its vertices per lane itself (until a shape is set)
+    int field_threads = 128, field_waves = 8, density_threads = 128, moments_threads = 128, field_vpt = 0;
 };
 
 // Stage timing events.

@@ -1,8 +1,7 @@
 // pms_tune.cpp -- the project's autotuner: picks launch shapes of the
-// neighbour-walk kernels (threads per block, the field's resident-block cap and
-// vertices per work item)
-// by timing every candidate on the frame the context holds.  No counterpart
-// in the reference, whose launches use fixed block sizes.
+// neighbour-walk kernels (threads per block, the field's vertices per lane) by timing
+// every candidate on the frame the context holds.  No counterpart in the reference,
+// whose launches use fixed block sizes.
 #include <algorithm>
 #include <vector>
 
@@ -62,14 +61,10 @@ extern "C" pms_status pms_autotune(pms_ctx* c, pms_tune* out) {
         for (int k : vpts)
             for (int bt : sizes) {
                 c->tune.field_vpt = k;
-                c->tune.field_auto = false;
                 c->tune.field_threads = bt;
                 float ms;
                 if ((st = time_ms(c, 3, &ms, launch_field))) return st;
-                if (ms < best_field) {
-                    best_field = ms; best.field_threads = bt; best.field_vpt = k;
-                    best.field_auto = false;
-                }
+                if (ms < best_field) { best_field = ms; best.field_threads = bt; best.field_vpt = k; }
             }
     }
     c->tune = best;
@@ -95,12 +90,12 @@ static bool valid_threads(int t) { return t == 64 || t == 128 || t == 256; }
 extern "C" pms_status pms_set_tune(pms_ctx* c, const pms_tune* t) {
     if (!c || !t) return PMS_ERR_INVALID_ARGUMENT;
     if (!valid_threads(t->field_threads) || !valid_threads(t->density_threads) || !valid_threads(t->moments_threads) ||
-        t->field_waves < 1 || t->field_waves > 64 || (t->field_vpt != 1 && t->field_vpt != 2 && t->field_vpt != 4))
+        t->field_waves < 1 || t->field_waves > 64 ||
+        (t->field_vpt != 0 && t->field_vpt != 1 && t->field_vpt != 2 && t->field_vpt != 4))
         return pms_fail(c, PMS_ERR_INVALID_ARGUMENT, "launch shape outside the tuned set");
     c->tune.field_threads = t->field_threads;
     c->tune.field_waves = t->field_waves;
     c->tune.field_vpt = t->field_vpt;
-    c->tune.field_auto = false;
     c->tune.density_threads = t->density_threads;
     c->tune.moments_threads = t->moments_threads;
     return PMS_OK;

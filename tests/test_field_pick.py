@@ -40,3 +40,20 @@ def test_choice_keeps_the_field(pms_lib, tmp_config, kind, ratio, sc, low, high)
     assert low <= n < high, n
     for f in fields[1:]:
         np.testing.assert_array_equal(fields[0], f)
+
+
+def test_saved_shape_restores_the_choice(pms_lib, tmp_config):
+    """What get_tune reports before a tuning brings the frame's own choice back, and keeps it."""
+    from postmps_gb300 import synth
+    with pms_lib.Context(pms_lib.load_config(tmp_config(synth.config_text())), 0) as ctx:
+        saved = ctx.get_tune()
+        ctx.upload(synth.lattice(12, 12, 12, 0.01, 0.001, seed=2))
+        ctx.run_frame()
+        field = ctx.debug("field")
+        assert ctx.autotune()["field_vpt"] in (1, 2, 4)
+        ctx.set_tune(saved)
+        assert ctx.get_tune()["field_vpt"] == saved["field_vpt"] == 0
+        ctx.run_frame()
+        np.testing.assert_array_equal(ctx.debug("field"), field)
+        with pytest.raises(pms_lib.PmsError):
+            ctx.set_tune({**saved, "field_vpt": 3})
