@@ -758,8 +758,10 @@ size_t field_tile_bytes(const pms_grid& g, uint64_t nv) {
 }
 
 // pick_k's lines for this frame, and the choice itself where the host knows it (else 0): a shape
-// that was set, or the middle one where nothing asks for 4 and a body of so many particles
-// has a band above `few` (30,000 in a block: 239,000 vertices at h = 2 and two cells).
+// that was set, or the middle one where nothing asks for 4 and even a block of so many particles
+// has a band above `few`: at two cells 24,389 have 171,000 vertices at h = 2, 200,000 at h = 3; at
+// h = 1 24,389 have 94,000 and 64,000 have 214,000.  (Field stage there, the middle one / by the
+// device's count: 27,000 particles 26.6 / 24.6 us, 39,304 and 64,000 equal.)
 static int field_pick(const pms_ctx* ctx, FieldPick& p) {
     p.few = 160000u;
     p.many = 0xffffffffu;
@@ -774,7 +776,7 @@ static int field_pick(const pms_ctx* ctx, FieldPick& p) {
     const bool sparse = (double)ctx->n * sp * sp * sp < 0.1 * box;
     if (P.sc_scale >= 3) p.many = 500000u;
     else if (P.sc_scale == 2 && (P.smoothing_radius_ratio >= 4 || sparse)) p.many = 1000000u;
-    return p.many == 0xffffffffu && P.sc_scale == 2 && ctx->n >= 24576u ? 2 : 0;
+    return p.many == 0xffffffffu && P.sc_scale == 2 && ctx->n >= (P.smoothing_radius_ratio >= 2 ? 24576u : 65536u) ? 2 : 0;
 }
 
 template <int K>
