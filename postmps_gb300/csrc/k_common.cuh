@@ -102,17 +102,6 @@ __device__ __forceinline__ float from_ordered_bits(uint32_t u) {
     return __uint_as_float(b);
 }
 
-// Squared distance from p to the box of spatial cell (x, y, z), the box widened
-// by `pad` so particles whose key rounded into the cell from just outside are
-// still covered.
-__device__ __forceinline__ float cell_gap2(const KGrid& g, float3 p, uint32_t x, uint32_t y, uint32_t z, float pad) {
-    const float x0 = g.min_pos[0] + (float)x * g.sp_cs - pad, x1 = x0 + g.sp_cs + 2.f * pad;
-    const float y0 = g.min_pos[1] + (float)y * g.sp_cs - pad, y1 = y0 + g.sp_cs + 2.f * pad;
-    const float z0 = g.min_pos[2] + (float)z * g.sp_cs - pad, z1 = z0 + g.sp_cs + 2.f * pad;
-    const float dx = axis_gap(p.x, x0, x1), dy = axis_gap(p.y, y0, y1), dz = axis_gap(p.z, z0, z1);
-    return dx * dx + dy * dy + dz * dz;
-}
-
 // The frame's counters into the context's mapped pinned mirror, by one block: the last work of a
 // kernel whose results the host waits for (a launch of its own costs 2.6 us).
 __device__ __forceinline__ void publish_counters(const Counters* cnt, uint32_t* mirror) {
@@ -260,11 +249,6 @@ __device__ __forceinline__ void warp_walk(const KGrid& g, float3 p, uint3 lo, ui
     }
 }
 
-// rank of bit `id` among set bits of a bitmap with exclusive word prefix sums
-__device__ __forceinline__ uint32_t bit_rank(const uint32_t* bm, const uint32_t* wprefix, uint32_t id) {
-    uint32_t w = id >> 5, b = id & 31u;
-    return wprefix[w] + __popc(bm[w] & ((1u << b) - 1u));
-}
 __device__ __forceinline__ bool bit_get(const uint32_t* bm, uint64_t nbits, uint64_t id) {
     return id < nbits && ((bm[id >> 5] >> (id & 31u)) & 1u);
 }

@@ -74,8 +74,7 @@ __device__ __forceinline__ float gap2_axis(float p, float lo, float cs, float pa
 // that vertex alone gives.
 static constexpr uint32_t kItemShift = 29;
 
-// BT threads per block (autotuned: 64, 128 or 256), K vertices per item (1, 2
-// or 4, autotuned).  cell_rad holds sp_size per-cell support radii followed by
+// BT threads per block, K vertices per item.  cell_rad holds sp_size per-cell support radii followed by
 // one radius per row (z, y): the largest maxvalue * h of the row's particles
 // (0 where none is anisotropic).  The z and y ranges are cut from the largest
 // support of the frame, each row's x range from the row's own radius, and each
@@ -272,7 +271,7 @@ k_field_cert(KGrid g, FieldParams fp, const Counters* __restrict__ cnt, const ui
 #pragma unroll 1
                         for (uint32_t j = j0; j < j1; ++j) {
                             const float4 q = __ldg(&spos[j]);
-                            const float4 a0 = __ldg(&aniso[2 * (size_t)j]);      // {m00, 2 m01, 2 m02, h_s^2}
+                            const float4 a0 = __ldg(&aniso[2 * (size_t)j]);      // {m00, 2 m01, 2 m02, extents}
                             const float4 a1 = __ldg(&aniso[2 * (size_t)j + 1]);  // {m11, 2 m12, m22, w}
                             // r^T M r with every rounding spelled out, so that the value does
                             // not depend on how many vertices share the loads
