@@ -255,3 +255,25 @@ pms_status scan_u64(pms_ctx* ctx, const unsigned long long* in, unsigned long lo
 }
 
 }  // namespace pms
+
+// The scans on device arrays of 4- or 8-byte elements, for tests (exported, not part of
+// pms.h's stable surface): n elements or the first *d_n of them; the sum comes back by way
+// of the context's counters, for 8-byte elements as the scan itself publishes them.
+extern "C" pms_status pms_debug_scan(pms_ctx* ctx, int elem_bytes, const void* d_in, void* d_out, uint64_t n,
+                                     const uint32_t* d_n, uint64_t* total) {
+    using namespace pms;
+    if (!ctx || !total || (elem_bytes != 4 && elem_bytes != 8)) return PMS_ERR_INVALID_ARGUMENT;
+    cudaSetDevice(ctx->device);
+    Counters* cnt = ctx->counters.as<Counters>();
+    if (elem_bytes == 8) {
+        PMS_CHECK(scan_u64(ctx, static_cast<const unsigned long long*>(d_in), static_cast<unsigned long long*>(d_out), n,
+                           &cnt->mc_total, d_n, true));
+        PMS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        *total = ctx->h_counters->mc_total;
+    } else {
+        PMS_CHECK(scan_u32(ctx, static_cast<const uint32_t*>(d_in), static_cast<uint32_t*>(d_out), n, &cnt->n_weld, d_n));
+        PMS_CHECK(sync_counters(ctx));
+        *total = ctx->h_counters->n_weld;
+    }
+    return PMS_OK;
+}
