@@ -283,3 +283,26 @@ def test_batch_meshes_streamed_inside_the_graph(pms_lib):
         ctx.batch_stream_meshes(0, 0)
         ctx.run_batch(frames)
         assert np.array_equal(ctx.batch_mesh(3), ref[3])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("band", ["plain", "certified"])
+def test_large_frames_in_a_batch(pms_lib, band):
+    """Frames large enough that the densities far from the surface are left out inside the graph:
+    each frame's mesh and counts are those of its stages one by one, which make every density."""
+    pms = pms_lib
+    frames = _frames(3, spacing=0.008)
+    assert min(len(f[0]) for f in frames) >= 65536
+    with _ctx(pms, 0.008) as ctx:
+        for _ in range(2):                                   # captured, then launched again
+            ctx.run_batch(frames, learned=band)
+        got = [(ctx.batch_frame(f)[0], ctx.batch_mesh(f)) for f in range(len(frames))]
+    with _ctx(pms, 0.008) as ctx:
+        for (c, mesh), fr in zip(got, frames, strict=True):
+            ctx.upload(*fr)
+            for stage in ("build_grid", "anisotropy", "band", "field", "marching_cubes"):
+                getattr(ctx, stage)()
+            want = ctx.counts()
+            np.testing.assert_array_equal(mesh, ctx.mesh(normals=False)[0])
+            assert (c.n_surface_particles, c.n_band_vertices, c.n_valid_cubes, c.n_mesh_vertices) == \
+                   (want.n_surface_particles, want.n_band_vertices, want.n_valid_cubes, want.n_mesh_vertices)
