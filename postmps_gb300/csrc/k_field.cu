@@ -73,6 +73,7 @@ __device__ __forceinline__ float gap2_axis(float p, float lo, float cs, float pa
 // contributions in the reference's order, so each value is the one a walk of
 // that vertex alone gives.
 static constexpr uint32_t kItemShift = 29;
+static_assert(kMaxBand == 1u << kItemShift, "an item holds a band index and a count");
 
 // BT threads per block, K vertices per item.  cell_rad holds sp_size per-cell support radii followed by
 // one radius per row (z, y): the largest maxvalue * h of the row's particles
@@ -897,7 +898,7 @@ pms_status launch_field_cert(pms_ctx* ctx, const uint32_t* vlist, const uint32_t
     fp.quick = P.iso_value * (1.f + 1.f / 512.f);
     fp.ext_unit = 0.f;
     Counters* cnt = ctx->counters.as<Counters>();
-    if ((uint64_t)n_host >= (1ull << kItemShift)) return pms_fail(ctx, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices");
+    if (n_host >= kMaxBand) return pms_fail(ctx, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices");
     constexpr uint32_t K = kCertRun;
     const uint32_t ngroups = (n_host + K - 1u) / K;
     PMS_CUDA(ctx, ctx->fitem_cnt.ensure(4 * ((size_t)ngroups + 1)));

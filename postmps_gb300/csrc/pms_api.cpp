@@ -562,8 +562,13 @@ static pms_status take_band_size(pms_ctx* c) {
     c->ns = c->h_counters->ns;
     c->nv = c->h_counters->nv;
     c->nv_pending = false;
-    if (c->nv >= (1u << 29)) return pms_fail(c, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices");
     return PMS_OK;
+}
+
+// The most band vertices that have a field: its stages count mesh vertices in 32 bits, and the
+// certification's items hold 29 bits.
+static pms_status check_band_size(pms_ctx* c) {
+    return c->nv >= kMaxBand ? pms_fail(c, PMS_ERR_UNSUPPORTED, "band above 2^29 vertices") : PMS_OK;
 }
 
 // The plain band's bitmap and count (one synchronisation).
@@ -604,6 +609,7 @@ extern "C" pms_status pms_field(pms_ctx* c) {
     pms_status st;
     // (a grid built again since the band took the band's count with it too)
     if (!c->aniso_current && (st = band_stage(c, false))) return st;
+    if (!c->nv_pending && (st = check_band_size(c))) return st;
     if ((c->nv || c->nv_pending) && (st = launch_field(c))) return st;
     c->have_field = true;
     mark(c, kStageField + 1);
@@ -628,7 +634,7 @@ extern "C" pms_status pms_marching_cubes(pms_ctx* c) {
             } else {
                 PMS_CUDA(c, cudaStreamSynchronize(c->stream));
             }
-            if (c->nv_pending && (st = take_band_size(c))) return st;
+            if (c->nv_pending && ((st = take_band_size(c)) || (st = check_band_size(c)))) return st;
             const uint64_t total = c->h_counters->mc_total;
             if ((st = ensure_band(c, (uint32_t)(total >> 32)))) return st;
             if ((st = launch_mc_compact(c))) return st;

@@ -448,6 +448,8 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
         float bmin[3], bmax[3];
         for (int a = 0; a < 3; ++a) { bmin[a] = decode_ordered(b->hcnt[f].bbox_min[a]); bmax[a] = decode_ordered(b->hcnt[f].bbox_max[a]); }
         if ((st = pms_grid_from_bbox(&c->prm, bmin, bmax, &grid[f]))) return pms_fail(c, st, "frame %u: grid too large", f);
+        // (nothing in the graph looks at the band's size: its bound has to fit)
+        if (grid[f].sc_size >= kMaxBand) return pms_fail(c, PMS_ERR_UNSUPPORTED, "frame %u: band above 2^29 vertices", f);
         gmax.sp_size = std::max(gmax.sp_size, grid[f].sp_size);
         gmax.sc_size = std::max(gmax.sc_size, grid[f].sc_size);
         // rows of the largest frame (the per-row radii follow the per-cell ones)

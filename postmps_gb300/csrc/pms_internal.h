@@ -46,6 +46,7 @@ struct DBuf {
 };
 
 // Counters kept on the device between stages (read back only on demand).
+static constexpr uint32_t kMaxBand = 1u << 29;   // band vertices a field is made for
 static constexpr int kMaxMcPieces = 4;  // vertex ranges a streamed mesh is emitted in
 
 struct Counters {
