@@ -429,6 +429,7 @@ extern "C" pms_status pms_run_batch(pms_ctx* c, const pms_frame* frames, uint32_
     b->n = n;
     b->off = off;
     b->flags = shape_flags;
+    if (!shape_same) b->grid.clear();        // (of other frames: this batch may be refused before it has its own)
     pms_status st;
     {
         FrameView view(c);

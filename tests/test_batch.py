@@ -306,3 +306,28 @@ def test_large_frames_in_a_batch(pms_lib, band):
             np.testing.assert_array_equal(mesh, ctx.mesh(normals=False)[0])
             assert (c.n_surface_particles, c.n_band_vertices, c.n_valid_cubes, c.n_mesh_vertices) == \
                    (want.n_surface_particles, want.n_band_vertices, want.n_valid_cubes, want.n_mesh_vertices)
+
+
+@pytest.mark.gpu
+def test_batch_after_a_refused_one(pms_lib):
+    """Frames of other sizes in the same boxes, refused once for a NaN and then run: their own meshes,
+    not a relaunch of what was captured before them."""
+    pms = pms_lib
+    rng = np.random.default_rng(1)
+    corners = np.array([[x, y, z] for x in (0, 0.3) for y in (0, 0.2) for z in (0, 0.2)], np.float32)
+
+    def frames(*n):
+        return [(np.concatenate([corners, rng.random((m, 3)).astype(np.float32) * 0.2]), None, None) for m in n]
+    first, second = frames(900, 900), frames(900, 400)
+    bad = [(p.copy(), None, None) for p, _, _ in second]
+    bad[1][0][20, 0] = np.nan
+    with _ctx(pms, 0.02) as ctx:
+        ctx.run_batch(second)
+        want = [ctx.batch_mesh(f) for f in range(2)]
+    with _ctx(pms, 0.02) as ctx:
+        ctx.run_batch(first)
+        with pytest.raises(pms.PmsError):
+            ctx.run_batch(bad)
+        ctx.run_batch(second)
+        for f in range(2):
+            np.testing.assert_array_equal(ctx.batch_mesh(f), want[f])
