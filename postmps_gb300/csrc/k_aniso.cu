@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(kThreads) k_density_warp(KGrid g, AnisoParams 
 
 static constexpr int kDensX = 2, kDensY = 2, kDensZ = 2;      // cells of a block
 static constexpr int kDensStage = 64;
+static constexpr uint32_t kDensEntry = 64;                     // most particles of an entry of the pass's list
 
 // Which blocks of cells a density pass works on.  A frame whose fields are asked for only at
 // its band needs the densities near the surface: a band vertex lies within h per axis of a
@@ -184,16 +185,21 @@ __global__ void __launch_bounds__(256) k_density_surface(KGrid g, uint3 bd, uint
     }
 }
 
-// the blocks that hold particles (and, for kNear, whether they are far), a warp per 32 blocks along x
+// the work of the pass, an entry {block, which kDensEntry of its particles} each: the blocks that hold
+// particles (and, for kNear, whether they are far), a warp per 32 blocks along x.  A block at rest is
+// one entry; a frame of crowded cells has few blocks, and a warp per block then leaves the GPU idle
+// (anisotropy stage of 300,000 particles, 200 or 1000 to a cell: 25 / 268 ms with a warp per block,
+// 6.7 / 26 with a thread per particle, 5.7 / 22 so; entries of 32: 5.5 / 21, but crown and dam frames
+// 0.2 to 0.5 % slower).
 __global__ void __launch_bounds__(256) k_density_list(KGrid g, uint3 bd, uint32_t wx, DensBlocks which, int reach,
                                                       const uint32_t* __restrict__ bits, const uint32_t* __restrict__ cell_start,
-                                                      uint32_t* __restrict__ n_blocks, uint32_t* __restrict__ list) {
+                                                      uint32_t* __restrict__ n_entries, uint2* __restrict__ list) {
     constexpr unsigned kAll = 0xffffffffu;
     const uint32_t nw = wx * bd.y * bd.z, lane = threadIdx.x & 31u;
     for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nw; w += (gridDim.x * blockDim.x) >> 5) {
         const uint32_t wi = w % wx, bx = wi * 32u + lane, by = w / wx % bd.y, bz = w / wx / bd.y;
         const uint32_t t = (bz * bd.y + by) * bd.x + bx;
-        bool any = false;
+        uint32_t m = 0u;
         if (bx < bd.x) {
             const uint32_t x0 = bx * kDensX, y0 = by * kDensY, z0 = bz * kDensZ, x1 = min(x0 + kDensX, g.spres[0]);
 #pragma unroll
@@ -201,10 +207,10 @@ __global__ void __launch_bounds__(256) k_density_list(KGrid g, uint3 bd, uint32_
                 const uint32_t y = y0 + k % kDensY, z = z0 + k / kDensY;
                 if (y >= g.spres[1] || z >= g.spres[2]) continue;
                 const uint32_t row = (z * g.spres[1] + y) * g.spres[0];
-                any |= __ldg(&cell_start[row + x0]) != __ldg(&cell_start[row + x1]);
+                m += __ldg(&cell_start[row + x1]) - __ldg(&cell_start[row + x0]);
             }
         }
-        uint32_t vote = __ballot_sync(kAll, any), near = kAll;
+        uint32_t vote = __ballot_sync(kAll, m != 0u), near = kAll;
         if (which != DensBlocks::kAll && vote) {
             // the surface bits of the (2 reach + 1)^2 rows of blocks around, spread by reach along x
             const int side = 2 * reach + 1;
@@ -222,12 +228,13 @@ __global__ void __launch_bounds__(256) k_density_list(KGrid g, uint3 bd, uint32_
             if (which == DensBlocks::kFar) vote &= ~near;
         }
         if (!vote) continue;
+        const uint32_t parts = (vote >> lane) & 1u ? (m + kDensEntry - 1u) / kDensEntry : 0u;
+        const WarpRows at = warp_rows(0u, parts);
         uint32_t base = 0u;
-        if (lane == 0u) base = atomicAdd(n_blocks, (uint32_t)__popc(vote));
-        base = __shfl_sync(kAll, base, 0);
-        if ((vote >> lane) & 1u)
-            list[base + (uint32_t)__popc(vote & ((1u << lane) - 1u))] =
-                t | (which == DensBlocks::kNear && !((near >> lane) & 1u) ? kFarBlock : 0u);
+        if (lane == 0u) base = atomicAdd(n_entries, at.total);
+        base = __shfl_sync(kAll, base, 0) + at.incl - parts;
+        const uint32_t tag = t | (which == DensBlocks::kNear && !((near >> lane) & 1u) ? kFarBlock : 0u);
+        for (uint32_t k = 0u; k < parts; ++k) list[base + k] = make_uint2(tag, k);
     }
 }
 
@@ -237,15 +244,15 @@ __device__ __forceinline__ float warp_max(float v) { return from_ordered_bits(__
 template <int BT>
 __global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoParams ap, SurfaceList sl, uint3 bd,
                                                                  const uint32_t* __restrict__ skeys,
-                                                                 const uint32_t* __restrict__ n_blocks_dev,
-                                                                 uint32_t* __restrict__ next, const uint32_t* __restrict__ list,
+                                                                 const uint32_t* __restrict__ n_entries_dev,
+                                                                 uint32_t* __restrict__ next, const uint2* __restrict__ list,
                                                                  const uint32_t* __restrict__ cell_start,
                                                                  const float4* __restrict__ spos, float* __restrict__ rho,
                                                                  float4* __restrict__ aniso) {
     constexpr unsigned kAll = 0xffffffffu;
     __shared__ float4 stage_all[BT / 32][kDensStage];
     float4* stage = stage_all[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31u, n_blocks = *n_blocks_dev;
+    const uint32_t lane = threadIdx.x & 31u, n_entries = *n_entries_dev;
     const float pad = g.pad, inv_cs = 1.f / g.sp_cs;
     const float rc = ap.h * inv_cs + g.margin, reach2 = ap.h_sq * 1.001f;
     const uint32_t ext = pack_extents(ap.h, ap.h, ap.h, ap.h);
@@ -253,8 +260,9 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoP
         uint32_t bi = 0u;
         if (lane == 0u) bi = atomicAdd(next, 1u);
         bi = __shfl_sync(kAll, bi, 0);
-        if (bi >= n_blocks) break;
-        const uint32_t entry = __ldg(&list[bi]), t = entry & ~kFarBlock;
+        if (bi >= n_entries) break;
+        const uint2 entry = __ldg(&list[bi]);
+        const uint32_t t = entry.x & ~kFarBlock;
         // the block's particles: a contiguous range per row of cells
         const uint32_t x0 = t % bd.x * kDensX, y0 = t / bd.x % bd.y * kDensY, z0 = t / bd.x / bd.y * kDensZ;
         uint32_t first = 0u, n = 0u;
@@ -267,12 +275,13 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_density_tiles(KGrid g, AnisoP
             }
         }
         const WarpRows mine = warp_rows(first, n);
-        for (uint32_t t0 = 0u; t0 < mine.total; t0 += 32u) {
+        const uint32_t end = min((entry.y + 1u) * kDensEntry, mine.total);
+        for (uint32_t t0 = entry.y * kDensEntry; t0 < end; t0 += 32u) {
             // lanes past the block's particles repeat its last one
             const uint32_t own = min(t0 + lane, mine.total - 1u);
             const int own_row = warp_row_of(mine, own);
             const uint32_t id = __shfl_sync(kAll, mine.off, own_row) + own;
-            if (entry != t) {                                  // a far block
+            if (entry.x != t) {                                // a far block
                 if (t0 + lane < mine.total) put_density(ap, sl, id, __ldg(&skeys[id]), 0.f, ext, rho, aniso);
                 continue;
             }
@@ -556,7 +565,7 @@ __global__ void __launch_bounds__(kThreads) k_eigen(AnisoParams ap, const uint32
                                                     uint32_t* __restrict__ nnb, float* __restrict__ cell_rad,
                                                     Counters* __restrict__ cnt_w) {
     const uint32_t ns = cnt->ns;
-    if (blockIdx.x == 0 && threadIdx.x == 0) cnt_w->dens_blocks = cnt_w->dens_next = 0u;   // the next density pass's tickets
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnt_w->dens_entries = cnt_w->dens_next = 0u;   // the next density pass's tickets
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
         const uint32_t i = slist[s];
         const float4 pi4 = spos[i];
@@ -699,19 +708,20 @@ static pms_status density_blocks(pms_ctx* ctx, const KGrid& g, const AnisoParams
                                 (g.spres[2] + kDensZ - 1) / kDensZ);
     const uint32_t wx = (bd.x + 31u) / 32u;
     const uint64_t words = (uint64_t)wx * bd.y * bd.z;
-    // (the moments' buffer holds the list until the moments are made: at most a block per particle;
+    // (the moments' buffer holds the list until the moments are made: at most an entry per particle;
     // the certification's cell records, made after the band, hold the bits: a word per cell is plenty)
-    uint32_t *list = ctx->moments.as<uint32_t>(), *bits = ctx->cell_rec.as<uint32_t>();
+    uint2* list = ctx->moments.as<uint2>();
+    uint32_t* bits = ctx->cell_rec.as<uint32_t>();
     if (which != DensBlocks::kAll) {
         k_density_surface<<<grid_for(words * 32, 256), 256, 0, ctx->stream>>>(g, bd, wx, ctx->cell_info.as<uint2>(), bits);
         PMS_LAUNCHED(ctx);
     }
     k_density_list<<<grid_for(words * 32, 256), 256, 0, ctx->stream>>>(
-        g, bd, wx, which, density_reach(g, ap.h), bits, ctx->cell_start.as<uint32_t>(), &cnt->dens_blocks, list);
+        g, bd, wx, which, density_reach(g, ap.h), bits, ctx->cell_start.as<uint32_t>(), &cnt->dens_entries, list);
     PMS_LAUNCHED(ctx);
     auto tiles = [&](auto kern) {
         kern<<<152u * (1024u / (unsigned)bd_threads), bd_threads, 0, ctx->stream>>>(
-            g, ap, sl, bd, ctx->skeys.as<uint32_t>(), &cnt->dens_blocks, &cnt->dens_next, list, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
+            g, ap, sl, bd, ctx->skeys.as<uint32_t>(), &cnt->dens_entries, &cnt->dens_next, list, ctx->cell_start.as<uint32_t>(), ctx->spos.as<float4>(),
             ctx->rho.as<float>(), ctx->aniso.as<float4>());
     };
     if (bd_threads == 64) tiles(k_density_tiles<64>);
@@ -730,7 +740,7 @@ pms_status launch_density_rest(pms_ctx* ctx) {
     pms_status st = density_blocks(ctx, g, aniso_params(ctx, g), sl, DensBlocks::kFar);
     if (st) return st;
     // (between frames the tickets are zero: the anisotropy pass resets them)
-    PMS_CUDA(ctx, cudaMemsetAsync(&cnt->dens_blocks, 0, sizeof(uint32_t), ctx->stream));
+    PMS_CUDA(ctx, cudaMemsetAsync(&cnt->dens_entries, 0, sizeof(uint32_t), ctx->stream));
     PMS_CUDA(ctx, cudaMemsetAsync(&cnt->dens_next, 0, sizeof(uint32_t), ctx->stream));
     ctx->dens_far = false;
     return PMS_OK;

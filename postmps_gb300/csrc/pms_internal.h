@@ -79,7 +79,7 @@ struct Counters {
     uint32_t l_recheck;     // certified corners of valid cubes, evaluated exactly afterwards
     uint32_t n_items;       // work items (runs or tiles) of the last field launch
     uint32_t field_next;    // the next listed tile a warp of the field takes (both 0 before a launch)
-    uint32_t dens_blocks;   // blocks of cells the density pass visits, and its ticket (0 between passes)
+    uint32_t dens_entries;  // the density pass's list, and its ticket (0 between passes)
     uint32_t dens_next;
     uint32_t df_active;     // particles that can spawn, and those of them with a wave crest: the lists'
     uint32_t df_crests;     // lengths (0 between frames)
