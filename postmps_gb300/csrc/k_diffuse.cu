@@ -115,6 +115,19 @@ __device__ __forceinline__ void list_append(bool take, uint32_t i, uint32_t* __r
     if (take) list[base + (uint32_t)__popc(vote & ((1u << lane) - 1u))] = i;
 }
 
+// A list of n walks over the launch's threads: one walk to every 2^spread-th thread, as sparse as
+// fills the GPU (at most a walk per warp).  Lanes of a warp walk at different places, so each of
+// their loads takes up to 32 lines, and a short list in full warps waits for them on a few SMs.
+// (Trapped air / crests of 100,000 particles, 20 to a cell, few of them moving: 467 / 563 us in full
+// warps, 166 / 137 with a thread per particle of the frame, 130 / 143 so; appending to the lists by
+// blocks instead of by warps changed nothing.)
+__device__ __forceinline__ uint32_t walk_spread(uint32_t n) {
+    const uint64_t threads = min((uint64_t)gridDim.x * blockDim.x, (uint64_t)152u * 1024u);
+    uint32_t s = 0u;
+    while (s < 5u && ((uint64_t)n << (s + 1u)) <= threads) ++s;
+    return s;
+}
+
 // Blocks of kMarkSide^3 cells with a particle that can spawn, a byte each.  Only the wave crests of
 // such particles read normals: their own, and those within the diffuse window around them.
 static constexpr uint32_t kMarkSide = 4;
@@ -233,9 +246,12 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_trapped(KGrid g, DiffusePara
                                                          uint32_t* __restrict__ crests) {
     const uint32_t na = cnt->df_active;
     const float pad = g.pad, r2 = dp.hd_sq;
-    for (uint32_t t0 = blockIdx.x * blockDim.x; t0 < na; t0 += gridDim.x * blockDim.x) {      // whole warps together
-        const bool in = t0 + threadIdx.x < na;
-        const uint32_t i = active[in ? t0 + threadIdx.x : t0];
+    const uint32_t spread = walk_spread(na);
+    const uint64_t end = (uint64_t)na << spread;
+    for (uint64_t t0 = blockIdx.x * blockDim.x; t0 < end; t0 += gridDim.x * blockDim.x) {     // whole warps together
+        const uint64_t t = t0 + threadIdx.x;
+        const bool in = t < end && (t & ((1u << spread) - 1u)) == 0u;
+        const uint32_t i = active[in ? t >> spread : 0u];
         const float4 p4 = spos[i], v = svel[i], ni = nrm[i];
         const float3 p = make_float3(p4.x, p4.y, p4.z);
         // the reference's zero cases of the wave crests
@@ -280,8 +296,11 @@ __global__ void __launch_bounds__(kThreads, 8) k_df_crests(KGrid g, DiffuseParam
                                                         const float4* __restrict__ nrm, float4* __restrict__ pot) {
     const uint32_t nc = cnt->df_crests;
     const float pad = g.pad, r2 = dp.hd_sq;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nc; t += gridDim.x * blockDim.x) {
-        const uint32_t i = crests[t];
+    const uint32_t spread = walk_spread(nc);
+    const uint64_t end = (uint64_t)nc << spread;
+    for (uint64_t t = blockIdx.x * blockDim.x + threadIdx.x; t < end; t += gridDim.x * blockDim.x) {
+        if (t & ((1u << spread) - 1u)) continue;
+        const uint32_t i = crests[t >> spread];
         const float4 p4 = spos[i], ni = nrm[i];
         const float3 p = make_float3(p4.x, p4.y, p4.z);
         uint3 lo, hi;

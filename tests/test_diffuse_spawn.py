@@ -66,3 +66,16 @@ def test_normals_do_not_depend_on_who_moves(pms_lib, tmp_config, moving, surface
     assert np.any(normals[0][0] != 0)
     for n in normals[1]:
         np.testing.assert_array_equal(n, normals[0][0])
+
+
+@pytest.mark.parametrize("moving", [0.3, 0.15, 0.08, 0.04, 0.02, 0.01])
+def test_short_lists(pms_lib, oracle, tmp_config, moving):
+    """Few particles that can spawn, in crowded cells: the walks' lists are spread over 2 to 32 lanes each."""
+    from postmps_gb300 import synth
+    pos = synth.lattice(13, 13, 13, 0.003, 0.0003, seed=8)
+    rng = np.random.default_rng(5)
+    vel = rng.normal(0, 3.0, pos.shape).astype(np.float32)
+    vel[rng.random(len(pos)) >= moving] = 0.0
+    text = synth.config_text(**synth.CROWN_KEYS, **{"config.isdiffusegeneration": "true"})
+    d = {"config": text, "seed": 5, "f0_pos": pos, "f0_vel": vel, "f0_rho": np.full(len(pos), 1000, np.float32)}
+    check_gpu_frames(oracle, d, run_gpu_frames(pms_lib, tmp_config, d, frames=(0,)), reference=False)
