@@ -224,10 +224,11 @@ __global__ void __launch_bounds__(kThreads) k_mc_cases(KGrid g, float iso, const
 // holds values at band vertices only; elsewhere it is whatever an earlier frame left)
 __device__ __forceinline__ float grid_value(const KGrid& g, const uint32_t* __restrict__ bm, const float* __restrict__ fdense,
                                             int x, int y, int z) {
-    if (x < 0 || y < 0 || z < 0 || (uint32_t)x >= g.scres[0] || (uint32_t)y >= g.scres[1] || (uint32_t)z >= g.scres[2])
-        return 0.f;
-    const size_t i = ((size_t)z * g.scres[1] + (size_t)y) * g.scres[0] + (size_t)x;
-    return (__ldg(&bm[i >> 5]) >> (i & 31u)) & 1u ? __ldg(&fdense[i]) : 0.f;
+    // (no branch: the loads of several values are in flight together)
+    const bool in = (uint32_t)x < g.scres[0] && (uint32_t)y < g.scres[1] && (uint32_t)z < g.scres[2];
+    const uint32_t i = in ? ((uint32_t)z * g.scres[1] + (uint32_t)y) * g.scres[0] + (uint32_t)x : 0u;
+    const float f = __ldg(&fdense[i]);
+    return in && ((__ldg(&bm[i >> 5]) >> (i & 31u)) & 1u) ? f : 0.f;
 }
 
 __device__ __forceinline__ float3 normalized(float3 v) {
@@ -599,47 +600,69 @@ __device__ __forceinline__ uint32_t nth_bit(uint32_t b, uint32_t n) {
     return pos;
 }
 
-// One welded vertex per set edge bit, at the edge's rank.  A warp takes the edges of 32 words
-// together, a lane each (a thread per word walked its edges one after the other: 33 us for
-// the 24k edges of a 27k-particle block with normals, 19 now).
+// The welded vertex of an edge, at rank r.
+__device__ __forceinline__ void weld_vertex(const KGrid& g, float iso, uint64_t key, uint64_t r, const uint32_t* __restrict__ bm,
+                                            const float* __restrict__ fdense, float* __restrict__ vert, float* __restrict__ vnorm) {
+    const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1];
+    const uint32_t v = (uint32_t)(key / 3ull), axis = (uint32_t)(key - 3ull * v);
+    const int z = (int)(v / rxy), rem = (int)(v - (uint32_t)z * rxy), y = rem / (int)rx, x = rem - y * (int)rx;
+    const int X = x + (axis == 0), Y = y + (axis == 1), Z = z + (axis == 2);
+    // the ends are corners of a valid cube, so band vertices, but the high one may lie past the
+    // grid's side (a cube wrapped into the next row) and is 0 then
+    const bool in = (uint32_t)X < rx && (uint32_t)Y < g.scres[1] && (uint32_t)Z < g.scres[2];
+    const float fa = __ldg(&fdense[v]), fb = in ? __ldg(&fdense[(uint32_t)Z * rxy + (uint32_t)Y * rx + (uint32_t)X]) : 0.f;
+    const float d = fb - fa;
+    const float tt = fabsf(d) < 1.0e-7f ? 0.5f : (iso - fa) / d;   // getLerpFac's test, as above
+    const float ax = sc_coord_i(g, x, 0), ay = sc_coord_i(g, y, 1), az = sc_coord_i(g, z, 2);
+    const float bx = sc_coord_i(g, X, 0), by = sc_coord_i(g, Y, 1), bz = sc_coord_i(g, Z, 2);
+    vert[3 * r + 0] = ax + tt * (bx - ax);
+    vert[3 * r + 1] = ay + tt * (by - ay);
+    vert[3 * r + 2] = az + tt * (bz - az);
+    if (vnorm) {
+        const float sgn = (iso < 0.f) ? -1.f : 1.f;
+        const float3 na = vertex_normal(g, bm, fdense, x, y, z), nb = vertex_normal(g, bm, fdense, X, Y, Z);
+        const float3 nn = normalized(make_float3(na.x + tt * (nb.x - na.x), na.y + tt * (nb.y - na.y),
+                                                 na.z + tt * (nb.z - na.z)));
+        vnorm[3 * r + 0] = sgn * nn.x;
+        vnorm[3 * r + 1] = sgn * nn.y;
+        vnorm[3 * r + 2] = sgn * nn.z;
+    }
+}
+
+// One welded vertex per set edge bit, at the edge's rank.  A thread per word of edges makes its
+// edges one after the other; for a small mesh with normals, whose time is one thread's chain of loads,
+// a warp takes the edges of 32 words together, a lane each.  Bound by the latency of those loads
+// (a value's bit and field are read side by side and without branches: 104 -> 75 us for 3.3M).  Thread / warp form, us, by soup vertices, with normals: 17k 26 / 16, 42k 26 / 19, 146k
+// 28 / 25, 373k 28 / 27, 661k 33 / 36, 3.3M 75 / 97, a sheet's 1.1M 30 / 42; without: 42k 10 / 10, 146k
+// 11 / 12, 3.3M 31 / 53.
+static constexpr uint64_t kWeldWarp = 400000u;    // soup vertices
+template <bool kWarp>
 __global__ void __launch_bounds__(256) k_weld_vertices(KGrid g, float iso, const uint32_t* __restrict__ ebits,
                                                        const uint32_t* __restrict__ wprefix, uint64_t nw,
                                                        const uint32_t* __restrict__ bm, const float* __restrict__ fdense, uint64_t cap,
                                                        float* __restrict__ vert, float* __restrict__ vnorm) {
-    const uint32_t rx = g.scres[0], rxy = g.scres[0] * g.scres[1], lane = threadIdx.x & 31u;
-    const float sgn = (iso < 0.f) ? -1.f : 1.f;
-    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t w0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; w0 < nw; w0 += step) {
-        const uint32_t mine = w0 + lane < nw ? ebits[w0 + lane] : 0u;
-        if (!__any_sync(0xffffffffu, mine != 0u)) continue;
-        const WarpRows rows = warp_rows(0u, (uint32_t)__popc(mine));
-        const uint32_t rank0 = wprefix[w0];
-        for (uint32_t e0 = 0u; e0 < rows.total; e0 += 32u) {
-            const uint32_t e = e0 + lane;
-            const int i = warp_row_of(rows, e);
-            const uint32_t bits = __shfl_sync(0xffffffffu, mine, i), n = __shfl_sync(0xffffffffu, rows.off, i) + e;
-            const uint64_t r = (uint64_t)rank0 + e;
-            if (e >= rows.total || r >= cap) continue;   // (the host sizes vert for every soup vertex)
-            const uint64_t key = 32ull * (w0 + (uint32_t)i) + nth_bit(bits, n);
-            const uint32_t v = (uint32_t)(key / 3ull), axis = (uint32_t)(key - 3ull * v);
-            const int z = (int)(v / rxy), rem = (int)(v - (uint32_t)z * rxy), y = rem / (int)rx, x = rem - y * (int)rx;
-            const int X = x + (axis == 0), Y = y + (axis == 1), Z = z + (axis == 2);
-            const float fa = grid_value(g, bm, fdense, x, y, z), fb = grid_value(g, bm, fdense, X, Y, Z);
-            const float d = fb - fa;
-            const float tt = fabsf(d) < 1.0e-7f ? 0.5f : (iso - fa) / d;   // getLerpFac's test, as above
-            const float ax = sc_coord_i(g, x, 0), ay = sc_coord_i(g, y, 1), az = sc_coord_i(g, z, 2);
-            const float bx = sc_coord_i(g, X, 0), by = sc_coord_i(g, Y, 1), bz = sc_coord_i(g, Z, 2);
-            vert[3 * r + 0] = ax + tt * (bx - ax);
-            vert[3 * r + 1] = ay + tt * (by - ay);
-            vert[3 * r + 2] = az + tt * (bz - az);
-            if (vnorm) {
-                const float3 na = vertex_normal(g, bm, fdense, x, y, z), nb = vertex_normal(g, bm, fdense, X, Y, Z);
-                const float3 nn = normalized(make_float3(na.x + tt * (nb.x - na.x), na.y + tt * (nb.y - na.y),
-                                                         na.z + tt * (nb.z - na.z)));
-                vnorm[3 * r + 0] = sgn * nn.x;
-                vnorm[3 * r + 1] = sgn * nn.y;
-                vnorm[3 * r + 2] = sgn * nn.z;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x, w1 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if constexpr (kWarp) {
+        const uint32_t lane = threadIdx.x & 31u;
+        for (uint64_t w0 = w1 & ~31ull; w0 < nw; w0 += step) {
+            const uint32_t mine = w0 + lane < nw ? ebits[w0 + lane] : 0u;
+            if (!__any_sync(0xffffffffu, mine != 0u)) continue;
+            const WarpRows rows = warp_rows(0u, (uint32_t)__popc(mine));
+            const uint32_t rank0 = wprefix[w0];
+            for (uint32_t e0 = 0u; e0 < rows.total; e0 += 32u) {
+                const uint32_t e = e0 + lane;
+                const int i = warp_row_of(rows, e);
+                const uint32_t bits = __shfl_sync(0xffffffffu, mine, i), n = __shfl_sync(0xffffffffu, rows.off, i) + e;
+                const uint64_t r = (uint64_t)rank0 + e;
+                if (e >= rows.total || r >= cap) continue;   // (the host sizes vert for every soup vertex)
+                weld_vertex(g, iso, 32ull * (w0 + (uint32_t)i) + nth_bit(bits, n), r, bm, fdense, vert, vnorm);
             }
+        }
+    } else {
+        for (uint64_t w = w1; w < nw; w += step) {
+            uint64_t r = wprefix[w];
+            for (uint32_t bits = ebits[w]; bits && r < cap; bits &= bits - 1u, ++r)
+                weld_vertex(g, iso, 32ull * w + (uint32_t)(__ffs((int)bits) - 1), r, bm, fdense, vert, vnorm);
         }
     }
 }
@@ -677,9 +700,9 @@ pms_status launch_weld(pms_ctx* ctx, uint32_t* ebits, uint32_t* wc, uint32_t* wp
     pms_status st = scan_u32(ctx, wc, wprefix, nw, n_unique);
     if (st) return st;
     if (vert) {
-        k_weld_vertices<<<grid_for(nw, 256), 256, 0, ctx->stream>>>(g, ctx->prm.iso_value, ebits, wprefix, nw,
-                                                                    ctx->bm.as<uint32_t>(), ctx->fdense.as<float>(), cap, vert,
-                                                                    vnorm);
+        auto kern = vnorm && ctx->nmesh < kWeldWarp ? k_weld_vertices<true> : k_weld_vertices<false>;
+        kern<<<grid_for(nw, 256), 256, 0, ctx->stream>>>(g, ctx->prm.iso_value, ebits, wprefix, nw, ctx->bm.as<uint32_t>(),
+                                                         ctx->fdense.as<float>(), cap, vert, vnorm);
         PMS_LAUNCHED(ctx);
     }
     if (idx) {
