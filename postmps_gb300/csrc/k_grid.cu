@@ -68,10 +68,13 @@ __global__ void __launch_bounds__(kThreads) k_bbox(const float* __restrict__ pos
     publish_counters(cnt, mirror);
 }
 
-__global__ void k_counters_init(Counters* cnt, uint32_t n) {
+__global__ void k_counters_init(Counters* cnt, uint32_t n, uint32_t nv, uint32_t nvalid, unsigned long long nmesh) {
     Counters c;
     memset(&c, 0, sizeof(c));
     c.n = n;
+    c.nv = nv;
+    c.nvalid = nvalid;
+    c.nmesh = nmesh;
     for (int k = 0; k < 3; ++k) { c.bbox_min[k] = 0xffffffffu; c.bbox_max[k] = 0u; }
     *cnt = c;
 }
@@ -92,7 +95,10 @@ pms_status launch_publish_counters(pms_ctx* ctx) {
 
 pms_status launch_bbox(pms_ctx* ctx, bool publish) {
     Counters* cnt = ctx->counters.as<Counters>();
-    k_counters_init<<<1, 1, 0, ctx->stream>>>(cnt, ctx->n);
+    // (a grid built again on the same upload: the band and the mesh made before it stay, and what is
+    // made from them on demand reads their sizes here)
+    const bool kept = publish && ctx->have_mc;
+    k_counters_init<<<1, 1, 0, ctx->stream>>>(cnt, ctx->n, kept ? ctx->nv : 0u, kept ? ctx->nvalid : 0u, kept ? ctx->nmesh : 0ull);
     PMS_LAUNCHED(ctx);
     k_bbox<<<grid_for(ctx->n, kThreads, 152 * 4), kThreads, 0, ctx->stream>>>(ctx->in_pos.as<float>(), ctx->n, cnt,
                                                                            publish ? ctx->h_counters_dev : nullptr);

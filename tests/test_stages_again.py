@@ -95,3 +95,20 @@ def test_normals_after_a_second_grid(pms_lib, tmp_config):
             normals.append(ctx.debug("free_normal"))
     assert np.any(normals[0] != 0)
     np.testing.assert_array_equal(normals[1], normals[0])
+
+
+def test_results_on_demand_after_a_second_grid(pms_lib, tmp_config):
+    """A mesh made before the second grid: its normals, welded mesh and scalar values."""
+    pos, vel, text = scene()
+    results = []
+    for again in (False, True):
+        with pms_lib.Context(pms_lib.load_config(tmp_config(text)), 0) as ctx:
+            ctx.upload(pos, vel)
+            ctx.run_frame()
+            if again:
+                ctx.build_grid()
+            results.append([*ctx.mesh(True), *ctx.weld(True), *(v for _, v in sorted(ctx.scalar_values().items())),
+                            ctx.debug("band_list"), ctx.debug("field"), np.array(ctx.counts().n_mesh_vertices)])
+    assert len(results[0][0]) > 0
+    for a, b in zip(*results, strict=True):
+        np.testing.assert_array_equal(a, b)
