@@ -120,8 +120,9 @@ def dominant_stage(stage_ms: dict, alg: dict, diffuse: bool) -> str:
     """The stage whose kernel the roofline reports: the longest on the frame's stream.  With
     surface and diffuse on, the diffuse stage runs on its own stream beside the band, field
     and marching cubes, so its time is a span from the anisotropy's end, not a cost of its
-    own, and it is left out."""
-    serial = [k for k in alg if not (diffuse and k == "diffuse")]
+    own, and it is left out; so are the marching cubes, whose span is mostly the diffuse tail
+    beside them (0.9 ms on the crown frame, 0.35 of them its own)."""
+    serial = [k for k in alg if not (diffuse and k in ("diffuse", "marching_cubes"))]
     return max(serial, key=lambda k: stage_ms.get(k, 0.0))
 
 
@@ -899,6 +900,9 @@ def run_pms(args) -> None:
             line["field_compute"] = {"pair_evals": pairs, "pair_evals_per_s": rate, "flops_per_pair": 10,
                                      "achieved_tflops": rate * 10 / 1e12, "peak_tflops_fp32": peak_fp32,
                                      "frac": rate * 10 / 1e12 / peak_fp32,
+                                     "pairs_note": "every pair a tile's vertices evaluate, those out of reach too "
+                                                   "(about 1.8 times a vertex's own): no rate to compare with a "
+                                                   "walk's of each vertex alone",
                                      "peak_source": "nominal: 152 SMs x 128 FP32 lanes x 2 x the sampled SM clock"}
         line["stage_ms"] = stage_ms
         if diffuse:
