@@ -198,7 +198,9 @@ pms_status pms_upload_particles_device(pms_ctx* ctx, const float* d_pos_xyz, con
 pms_status pms_stage_particles(pms_ctx* ctx, const float* pos_xyz, const float* vel_xyz, const float* rhop, uint32_t n);
 pms_status pms_upload_staged(pms_ctx* ctx);
 
-/* Stages (asynchronous on the context stream unless stated). */
+/* Stages (asynchronous on the context stream unless stated).  Building the grid again
+ * on the same upload keeps what later stages made from the first one; a stage run
+ * after it gives what it gives on one grid. */
 pms_status pms_build_grid(pms_ctx* ctx);        /* NeighborSearch::SpatialGridBuilding, NeighborSearch.cu:37-76 */
 pms_status pms_anisotropy(pms_ctx* ctx);        /* Anisotropic::processingOfParticles, Anisotropic.cu:30-40 */
 pms_status pms_band(pms_ctx* ctx);              /* Anisotropic::processingOfVertices, Anisotropic.cu:43-50 */
