@@ -629,40 +629,41 @@ __device__ __forceinline__ void weld_vertex(const KGrid& g, float iso, uint64_t 
     }
 }
 
-// One welded vertex per set edge bit, at the edge's rank.  A thread per word of edges makes its
-// edges one after the other; for a small mesh with normals, whose time is one thread's chain of loads,
-// a warp takes the edges of 32 words together, a lane each.  Bound by the latency of those loads
-// (a value's bit and field are read side by side and without branches: 104 -> 75 us for 3.3M).  Thread / warp form, us, by soup vertices, with normals: 17k 26 / 16, 42k 26 / 19, 146k
-// 28 / 25, 373k 28 / 27, 661k 33 / 36, 3.3M 75 / 97, a sheet's 1.1M 30 / 42; without: 42k 10 / 10, 146k
-// 11 / 12, 3.3M 31 / 53.
-static constexpr uint64_t kWeldWarp = 400000u;    // soup vertices
-template <bool kWarp>
+// One welded vertex per set edge bit, at the edge's rank.  A warp takes 32 words: a lane per word, its
+// edges one after the other, or all their edges together, a lane each, where that takes at most half
+// the rounds (a round of the latter costs the ranking of its lanes too).  Bound by the latency of a
+// round's loads (a value's bit and field are read side by side and without branches).  With normals, a
+// lane per word / all together / this rule, us: block 27k 28 / 25 / 18, block 1M at three scalar cells
+// 75 / 97 / 84, a sheet of 1.1M soup vertices 30 / 42 / 29, 20,000 isolated particles 653 / 270 / 215 (lane
+// per word with branches); at most as many rounds instead of half 24 / 99 / 43 / 216.
+static constexpr uint32_t kWeldShare = 2u;
 __global__ void __launch_bounds__(256) k_weld_vertices(KGrid g, float iso, const uint32_t* __restrict__ ebits,
                                                        const uint32_t* __restrict__ wprefix, uint64_t nw,
                                                        const uint32_t* __restrict__ bm, const float* __restrict__ fdense, uint64_t cap,
                                                        float* __restrict__ vert, float* __restrict__ vnorm) {
-    const uint64_t step = (uint64_t)gridDim.x * blockDim.x, w1 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if constexpr (kWarp) {
-        const uint32_t lane = threadIdx.x & 31u;
-        for (uint64_t w0 = w1 & ~31ull; w0 < nw; w0 += step) {
-            const uint32_t mine = w0 + lane < nw ? ebits[w0 + lane] : 0u;
-            if (!__any_sync(0xffffffffu, mine != 0u)) continue;
-            const WarpRows rows = warp_rows(0u, (uint32_t)__popc(mine));
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t w0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; w0 < nw; w0 += step) {
+        const uint32_t mine = w0 + lane < nw ? ebits[w0 + lane] : 0u, n_mine = (uint32_t)__popc(mine);
+        const uint32_t most = __reduce_max_sync(0xffffffffu, n_mine);
+        if (!most) continue;
+        const uint32_t total = __reduce_add_sync(0xffffffffu, n_mine);
+        if ((total + 31u) / 32u * kWeldShare > most) {
+            uint64_t r = w0 + lane < nw ? wprefix[w0 + lane] : 0u;
+            for (uint32_t bits = mine; bits && r < cap; bits &= bits - 1u, ++r)
+                weld_vertex(g, iso, 32ull * (w0 + lane) + (uint32_t)(__ffs((int)bits) - 1), r, bm, fdense, vert, vnorm);
+            __syncwarp();
+        } else {
+            const WarpRows rows = warp_rows(0u, n_mine);
             const uint32_t rank0 = wprefix[w0];
-            for (uint32_t e0 = 0u; e0 < rows.total; e0 += 32u) {
+            for (uint32_t e0 = 0u; e0 < total; e0 += 32u) {
                 const uint32_t e = e0 + lane;
                 const int i = warp_row_of(rows, e);
                 const uint32_t bits = __shfl_sync(0xffffffffu, mine, i), n = __shfl_sync(0xffffffffu, rows.off, i) + e;
                 const uint64_t r = (uint64_t)rank0 + e;
-                if (e >= rows.total || r >= cap) continue;   // (the host sizes vert for every soup vertex)
+                if (e >= total || r >= cap) continue;        // (the host sizes vert for every soup vertex)
                 weld_vertex(g, iso, 32ull * (w0 + (uint32_t)i) + nth_bit(bits, n), r, bm, fdense, vert, vnorm);
             }
-        }
-    } else {
-        for (uint64_t w = w1; w < nw; w += step) {
-            uint64_t r = wprefix[w];
-            for (uint32_t bits = ebits[w]; bits && r < cap; bits &= bits - 1u, ++r)
-                weld_vertex(g, iso, 32ull * w + (uint32_t)(__ffs((int)bits) - 1), r, bm, fdense, vert, vnorm);
         }
     }
 }
@@ -700,9 +701,8 @@ pms_status launch_weld(pms_ctx* ctx, uint32_t* ebits, uint32_t* wc, uint32_t* wp
     pms_status st = scan_u32(ctx, wc, wprefix, nw, n_unique);
     if (st) return st;
     if (vert) {
-        auto kern = vnorm && ctx->nmesh < kWeldWarp ? k_weld_vertices<true> : k_weld_vertices<false>;
-        kern<<<grid_for(nw, 256), 256, 0, ctx->stream>>>(g, ctx->prm.iso_value, ebits, wprefix, nw, ctx->bm.as<uint32_t>(),
-                                                         ctx->fdense.as<float>(), cap, vert, vnorm);
+        k_weld_vertices<<<grid_for(nw, 256), 256, 0, ctx->stream>>>(g, ctx->prm.iso_value, ebits, wprefix, nw, ctx->bm.as<uint32_t>(),
+                                                                    ctx->fdense.as<float>(), cap, vert, vnorm);
         PMS_LAUNCHED(ctx);
     }
     if (idx) {
